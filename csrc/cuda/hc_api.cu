@@ -213,13 +213,7 @@ static int decompress_call(hc_codec* c, const uint8_t* d_in, size_t in_size, siz
   p.ring_epoch = want;
   p.eb = eb;
   p.ws = next_workspace(c, stream);
-  bool flagged = false;
-  if (!d_tile_flags) {
-    flagged = stage_offsets(c, p.ws, &d_in, &in_size, 1, n, &p.seg[0].in_ready, stream);
-    if (flagged) p.ring_epoch = p.ws.epoch;
-    else p.seg[0].in_ready = nullptr;
-  }
-  return hc::launch_decode(mode, p, stream, flagged) == cudaSuccess ? hc::kOk : hc::kErrCuda;
+  return hc::launch_decode(mode, p, stream) == cudaSuccess ? hc::kOk : hc::kErrCuda;
 }
 
 int hc_decompress(hc_codec* c, const uint8_t* d_in, size_t in_size, size_t n, float eb, int mode, float* d_x,
@@ -256,13 +250,7 @@ int hc_decompress_sum(hc_codec* c, int n_in, const uint8_t* const* d_in, const s
   }
   p.eb = eb;
   p.ws = next_workspace(c, stream);
-  const uint64_t* ready[hc::kMaxIn] = {};
-  const bool flagged = stage_offsets(c, p.ws, d_in, in_size, p.n_seg, n, ready, stream);
-  if (flagged) {
-    p.ring_epoch = p.ws.epoch;
-    for (int q = 0; q < n_in; ++q) p.seg[q].in_ready = ready[q];
-  }
-  return hc::launch_decode(hc::kModeOutlier, p, stream, flagged) == cudaSuccess ? hc::kOk : hc::kErrCuda;
+  return hc::launch_decode(hc::kModeOutlier, p, stream) == cudaSuccess ? hc::kOk : hc::kErrCuda;
 }
 
 // Several independent tensors compressed by one launch (segments); sizes land in d_sizes[g].

@@ -4,13 +4,13 @@
 #include <stdio.h>
 
 #include "hc_launch.h"
+#include "hc_host.cuh"
+#include "hc_warp.cuh"
 
 namespace hc {
 namespace dev {
 
 constexpr int kEncThreads = kComputeThreads + 64;  // + loader warp + scanner warp
-constexpr int kDecThreads = kComputeThreads + 32;  // + loader warp
-constexpr uint32_t kNoTile = 0xffffffffu;
 
 constexpr int kMaxStages = 2;
 constexpr int kRing = 8;  // tiles a CTA may have between "total known" and "payload copied out"
@@ -38,12 +38,6 @@ struct __align__(16) EncShared {
   uint16_t in_rel[2][kTileBlocks];
   uint8_t in_rate[2][kTileBlocks];
 };
-
-__device__ __forceinline__ void note_error(uint32_t* ctrl, uint32_t code) { atomicMax(ctrl + 2, code); }
-// timeouts and peer failures end the launch early; capacity / truncation errors only skip data
-__device__ __forceinline__ bool fatal_error(const uint32_t* ctrl) {
-  return *((volatile const uint32_t*)(ctrl + 2)) >= (uint32_t)kErrTimeout;
-}
 
 // Optional per-CTA timeline (compile with -DHC_TIMELINE): nanosecond stamps of the first tile's way
 // through the roles (slots 0-15) and, for the first compute warp, SM-clock cycles accumulated per
@@ -92,31 +86,7 @@ __device__ __forceinline__ unsigned long long timeline_now() {
 #define HC_PH_COUNT()
 #endif
 
-// the last CTA to leave re-arms the ticket counter for the next launch
-// (returns true in thread 0 of that CTA)
-__device__ __forceinline__ bool cta_epilogue(uint32_t* tick) {
-  __syncthreads();
-  bool last = false;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    uint32_t done = atomicAdd(tick + 1, 1u);
-    if (done == gridDim.x - 1) {
-      tick[0] = 0;
-      tick[1] = 0;
-      __threadfence();
-      last = true;
-    }
-  }
-  return last;
-}
-
-// bounded mbarrier wait that records a timeout
-// `site` says which wait it was; the first one to run out is kept in ctrl[3] (hc_codec_status_site),
-// because every later time-out of the launch is only a consequence of it
-enum WaitSite : uint32_t {
-  kSiteLoaderStageFree = 1, kSiteLoaderInFree = 2, kSiteComputeInFull = 3, kSiteComputeTile = 4, kSiteComputeRing = 5,
-  kSiteScannerTotal = 6, kSiteCopierBase = 7, kSiteCopierPacked = 8, kSiteDecodeInFree = 9, kSiteDecodeInFull = 10,
-};
+// bounded mbarrier wait that records a timeout; `site` says which wait it was
 __device__ __forceinline__ bool wait_or_flag(uint64_t* bar, uint32_t parity, const Workspace& ws, volatile uint32_t* abort,
                                              uint32_t site) {
   if (mbar_wait_bounded(bar, parity, ws.spin_limit_ns)) return true;
@@ -193,25 +163,6 @@ __device__ __forceinline__ void loader_stage_stream(const uint8_t* in, uint64_t 
       mbar_arrive(full);
     }
   }
-}
-
-// collective steps: one non-blocking look at the tile's arrival flag; 0 = not raised yet
-__device__ __forceinline__ uint64_t flag_peek(const uint64_t* flag, uint32_t call) {
-  uint64_t w = 0;
-  if ((threadIdx.x & 31) == 0) {
-    w = ld_acquire_sys_u64(flag);
-    if (!flag_matches(w, call)) w = 0;
-  }
-  return __shfl_sync(0xffffffffu, w, 0);
-}
-// collective steps: bounded wait for the tile's arrival flag; 0 = the peer never delivered
-__device__ __forceinline__ uint64_t flag_wait_warp(const uint64_t* flag, uint32_t call, const Workspace& ws) {
-  uint64_t w = 0;
-  if ((threadIdx.x & 31) == 0) {
-    w = wait_tile_flag(flag, call, ws.spin_limit_ns, ws.ctrl + 2);
-    if (w == 0) note_error(ws.ctrl, kErrPeer);
-  }
-  return __shfl_sync(0xffffffffu, w, 0);
 }
 
 // Shared-memory plan of the stream-producing kernel (offsets from a 1024-byte aligned base):
@@ -710,209 +661,6 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
   }
 }
 
-struct __align__(16) DecShared {
-  uint64_t in_full[2];
-  uint64_t in_free[2];
-  uint32_t tile[4];
-  uint32_t in_phase[2];
-  uint32_t abort;
-  uint16_t in_rel[2][kTileBlocks];
-  uint8_t in_rate[2][kTileBlocks];
-};
-
-// SUM: the n_seg streams hold contributions to ONE array (every rank's whole message in the one-step
-// form of the allreduce): a CTA stages tile lt of every stream in turn, adds the decoded quantised
-// values in registers and writes seg[0].out once per tile.  Tickets then count tiles, not (tile, stream).
-template <int MODE, bool SUM>
-__global__ void __launch_bounds__(kDecThreads, SUM ? 3 : 4)
-hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const DecParams p) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ DecShared sh;
-  // one output tile (its TMA store has a whole tile time to read it out) + two staging buffers:
-  // 51 KB per CTA, four CTAs per SM
-  uint8_t* const obuf = smem;
-  uint8_t* cbuf[2] = {smem + kTileBytes, smem + kTileBytes + kBufBytes};
-
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  const Workspace& ws = p.ws;
-  HC_TL_DECL(ws.epoch);
-  const float eb = p.eb;
-  const uint32_t groups_per_seg = p.tiles_per_seg / 32 + 1;
-
-  if (tid == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&sh.in_full[i], 1);
-      mbar_init(&sh.in_free[i], kComputeThreads);
-    }
-    fence_mbar_init();
-    sh.abort = fatal_error(ws.ctrl) ? 1u : 0u;
-    HC_TL_ZERO();
-    launch_dependents();  // a following launch with programmatic serialisation may fill the SMs as CTAs leave
-  }
-  __syncthreads();
-  volatile uint32_t* abort = &sh.abort;
-  if (tid == 0) HC_STAMP(0);
-
-  if (warp == kComputeThreads / 32) {
-    // ================================ loader warp ================================================
-    // CTA i starts with tile i, later tiles come from the shared ticket counter.  Software pipeline
-    // over this CTA's tiles: the ticket is taken two turns ahead and the rate bytes one turn ahead,
-    // so neither round trip sits between two look-backs.
-    uint32_t handed = kNoTile, handed_sg = 0;  // SUM: the (tile, stream) pair handed out last
-    auto take = [&]() -> uint32_t {  // lane 0 takes a ticket, every lane gets it
-      if (SUM && handed != kNoTile && handed_sg + 1 < p.n_seg) {
-        ++handed_sg;
-        return ++handed;  // the next stream of the same tile
-      }
-      uint32_t t = kNoTile;
-      if (lane == 0 && !*abort) t = gridDim.x + atomicAdd(ws.tick, 1u);
-      t = __shfl_sync(0xffffffffu, t, 0);
-      if (!SUM) return t < p.n_tiles ? t : kNoTile;
-      handed = t < p.tiles_per_seg ? t * p.n_seg : kNoTile;
-      handed_sg = 0;
-      return handed;
-    };
-    // non-blocking; fw receives the tile's arrival flag word when the segment has flags
-    auto try_fetch = [&](uint32_t t, uint32_t (&r)[kRatesPerLane], uint64_t& fw) -> bool {
-      if (t == kNoTile) return false;
-      const uint32_t lt = t / p.n_seg, sg = t - lt * p.n_seg;  // tickets go round the segments
-      const DecSegment& seg = p.seg[sg];
-      fw = 0;
-      // a segment shorter than the longest one of the launch has tickets past its own tiles: nothing to
-      // wait for and nothing to read there (its producer never raises those flags)
-      if ((uint64_t)lt * kTileBlocks >= rate_bytes(seg.n)) {
-#pragma unroll
-        for (int i = 0; i < kRatesPerLane; ++i) r[i] = 0u;
-        return true;
-      }
-      if (seg.in_ready && (fw = flag_peek(seg.in_ready + lt, p.ring_epoch)) == 0) return false;
-      loader_fetch_rates(seg.in, seg.in_size, lt, r);
-      return true;
-    };
-    uint32_t tile = (!*abort && blockIdx.x < (SUM ? p.tiles_per_seg : p.n_tiles)) ? blockIdx.x : kNoTile;
-    if (SUM && tile != kNoTile) tile = handed = tile * p.n_seg;
-    if (lane == 0) HC_STAMP(1);
-    uint32_t tile_n = tile != kNoTile ? take() : kNoTile;
-    uint32_t rates[kRatesPerLane] = {}, rates_n[kRatesPerLane] = {};
-    uint64_t fw = 0, fw_n = 0;
-    bool have = try_fetch(tile, rates, fw), have_n = false;
-    for (uint32_t k = 0;; ++k) {
-      const int s = k & 1;
-      if (tile == kNoTile) {
-        // end marker; the buffer's previous phase must have been consumed before it is re-armed
-        if (k >= 2) wait_or_flag(&sh.in_free[s], ((k >> 1) - 1) & 1, ws, abort, kSiteDecodeInFree);
-        if (lane == 0) sh.tile[k & 3] = kNoTile;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh.in_full[s]);
-        break;
-      }
-      const uint32_t tile_nn = tile_n != kNoTile ? take() : kNoTile;
-      have_n = try_fetch(tile_n, rates_n, fw_n);
-      const uint32_t lt = tile / p.n_seg, sg = tile - lt * p.n_seg;
-      const DecSegment& seg = p.seg[sg];
-      bool usable = true;
-      if (!have) {  // (tickets past the segment's own tiles always come back from try_fetch with `have`)
-        fw = 0;
-        if (seg.in_ready && (fw = flag_wait_warp(seg.in_ready + lt, p.ring_epoch, ws)) == 0) usable = false;
-        if (usable) loader_fetch_rates(seg.in, seg.in_size, lt, rates);
-      }
-      const bool flagged_in = seg.in_ready != nullptr;
-      if (flagged_in && (fw & kFlagOffsetMask) == kFlagOffsetMask) usable = false;  // the producer gave up
-      const Chain chain{ws.st_a + (size_t)sg * p.tiles_per_seg, ws.grp_a + (size_t)sg * groups_per_seg};
-      if (lane == 0) sh.tile[k & 3] = tile;  // ring of 4 > 2 buffers: nobody still reads this slot
-      loader_stage_stream(seg.in, seg.in_size, rate_bytes(seg.n), lt, chain, ws, cbuf[s], &sh.in_full[s], sh.in_rel[s],
-                          sh.in_rate[s], &sh.in_phase[s], usable, rates, &sh.in_free[s], ((k >> 1) - 1) & 1, k >= 2,
-                          abort, flagged_in, fw & kFlagOffsetMask);
-      if (lane == 0 && fatal_error(ws.ctrl)) *abort = 1;
-      tile = tile_n;
-      tile_n = tile_nn;
-      have = have_n;
-      fw = fw_n;
-#pragma unroll
-      for (int i = 0; i < kRatesPerLane; ++i) rates[i] = rates_n[i];
-    }
-    if (lane == 0) HC_STAMP(6);
-  } else {
-    // ================================ compute warps ==============================================
-    if (tid == 0) HC_PH_START();
-    int32_t acc[SUM ? 32 : 1];
-    for (uint32_t k = 0;; ++k) {
-      const int s = k & 1;
-      bool alive = wait_or_flag(&sh.in_full[s], (k >> 1) & 1, ws, abort, kSiteDecodeInFull);
-      if (tid == 0) HC_PH(0);
-      if (k == 0 && tid == 0) HC_STAMP(2);
-      const uint32_t tile = alive ? sh.tile[k & 3] : kNoTile;
-      if (tile == kNoTile) break;
-      const uint32_t lt = tile / p.n_seg, sg = tile - lt * p.n_seg;
-      const DecSegment& seg = p.seg[SUM ? 0u : sg];  // where the tile goes
-      const bool tma = seg.use_tma != 0;
-      const uint64_t full_rows = seg.n / kBlock;
-      const uint32_t rate = sh.in_rate[s][tid];
-      const uint32_t pos = sh.in_phase[s] + sh.in_rel[s][tid];
-      int W = plane_width(rate & 31u);
-      W = __reduce_max_sync(0xffffffffu, W);
-      int32_t d[32];
-      if (__any_sync(0xffffffffu, rate != 0)) {
-        decode_block_quant<MODE>(cbuf[s], pos, rate, W, d);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) d[i] = 0;
-      }
-      mbar_arrive(&sh.in_free[s]);
-      if (SUM) {
-        if (sg == 0) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[i] = d[i];
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[i] += d[i];
-        }
-        if (sg + 1 < p.n_seg) continue;  // more streams of this tile to come
-#pragma unroll
-        for (int i = 0; i < 32; ++i) d[i] = acc[i];
-      }
-      if (tid == 0) HC_PH(1);
-      if (k == 0 && tid == 0) HC_STAMP(3);
-      uint32_t w[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(__fmul_rn(__fmul_rn((float)d[i], eb), 2.0f));
-
-      const uint64_t row = (uint64_t)lt * kTileBlocks + tid;
-      const bool ragged = row * kBlock < seg.n && (row + 1) * kBlock > seg.n;
-      // the TMA store of the previous tile must have finished reading obuf
-      if (tid == 0) HC_PH(2);
-      if (tid == 0) tma_wait_group_read<0>();
-      compute_barrier();
-      if (tid == 0) HC_PH(3);
-      if (tma) {
-        store_row_swizzled(obuf, tid, w);
-        fence_proxy_async();
-      }
-      compute_barrier();
-      if (tid == 0) {
-        HC_PH(4);
-        HC_PH_COUNT();
-        if (tma && (uint64_t)lt * kTileBlocks < full_rows)
-          tma_store_2d(&tmaps.m[SUM ? 0u : sg], 0, (int)(lt * kTileBlocks), obuf);
-        tma_commit_group();
-        if (k == 0) HC_STAMP(5);
-      }
-      if (!tma || ragged) {
-        const uint64_t o = row * kBlock;
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (o + i < seg.n) seg.out[o + i] = __uint_as_float(w[i]);
-      }
-    }
-    if (tid == 0) tma_wait_group<0>();
-  }
-  if (lane == 0) HC_STAMP_MAX(7);
-  cta_epilogue(ws.tick);
-}
-
 // Pre-pass for the stand-alone stream consumers (decompress and the homomorphic adds on streams that
 // no collective step has flagged): reads the rate bytes of up to kMaxIn streams and writes, for every
 // tile, the byte offset of its payload in the arrival-flag format (dev::flag_pack(tag, offset)), so
@@ -1038,96 +786,8 @@ __global__ void __launch_bounds__(256) hc_sum_kernel(float* __restrict__ dst, co
 
 namespace {
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
-}
-
-// 2-D view {32, rows} of a 4-byte-element array, box {32, 256}, 128-byte swizzle
-bool make_rows_map(CUtensorMap* map, const void* base, uint64_t rows) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn || rows == 0 || (reinterpret_cast<uintptr_t>(base) & 15u)) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)kBlock, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)kBlock * 4};
-  cuuint32_t box[2] = {(cuuint32_t)kBlock, (cuuint32_t)kTileBlocks};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
-
-struct DeviceInfo {
-  int sms = 0;
-  bool ready = false;
-};
-DeviceInfo& device_info() {
-  static thread_local DeviceInfo info[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  DeviceInfo& d = info[dev & 63];
-  if (!d.ready) {
-    cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
-    d.ready = true;
-  }
-  return d;
-}
-
 constexpr int enc_smem_bytes(int op, int ns, bool inplace) {
   return dev::enc_cbuf_off(op, ns, inplace) + (op == kOpCompress ? 0 : 2 * kBufBytes) + 1024;
-}
-constexpr int kDecSmem = kTileBytes + 2 * kBufBytes + 1024;
-
-template <typename K>
-cudaError_t set_smem(K kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
-// launch with programmatic stream serialisation (see launch_encode in hc_launch.h)
-template <typename... Params, typename... Args>
-cudaError_t launch_overlapped(void (*kernel)(Params...), int grid, int block, int smem, cudaStream_t stream,
-                              const Args&... args) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  memset(&attr, 0, sizeof(attr));
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
-// CTAs of `kernel` that one GPU holds at the same time, asked of the runtime once per device.  The
-// kernels are written for a grid that is resident as a whole (CTA i owns tile i, and every look-back
-// waits for tiles held by other CTAs of the grid), so the grid is cut to this number, never assumed.
-template <typename K>
-int resident_ctas(K kernel, int threads, int smem, int* cache) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int& c = cache[dev & 63];
-  if (c == 0) {
-    if (set_smem(kernel, smem) != cudaSuccess) return 0;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, (size_t)smem) != cudaSuccess) return 0;
-    c = per_sm * device_info().sms;
-  }
-  return c;
 }
 
 template <int OP, int MODE, bool INPLACE = false>
@@ -1159,20 +819,6 @@ cudaError_t launch_encode_m(int mode, const TensorMaps& map, const EncParams& p,
     case kModeVec: return launch_encode_t<OP, kModeVec>(map, p, stream, overlap);
     default: return cudaErrorInvalidValue;
   }
-}
-
-template <int MODE, bool SUM = false>
-cudaError_t launch_decode_t(const TensorMaps& maps, const DecParams& p, cudaStream_t stream, bool overlap) {
-  static thread_local int cache[64] = {};
-  const int cap = resident_ctas(dev::hc_decode_kernel<MODE, SUM>, dev::kDecThreads, kDecSmem, cache);
-  if (cap <= 0) return cudaErrorLaunchOutOfResources;
-  const uint32_t tickets = SUM ? p.tiles_per_seg : p.n_tiles;
-  int grid = (int)(tickets < (uint32_t)cap ? tickets : (uint32_t)cap);
-  if (p.grid_limit && (int)p.grid_limit < grid) grid = (int)p.grid_limit;
-  if (overlap)
-    return launch_overlapped(dev::hc_decode_kernel<MODE, SUM>, grid, dev::kDecThreads, kDecSmem, stream, maps, p);
-  dev::hc_decode_kernel<MODE, SUM><<<grid, dev::kDecThreads, kDecSmem, stream>>>(maps, p);
-  return cudaGetLastError();
 }
 
 }  // namespace
@@ -1229,7 +875,7 @@ cudaError_t launch_encode(int op, int mode, EncParams p, cudaStream_t stream, bo
     if (op != kOpAddStream && p.n[g]) {
       // int32 deltas are stored in whole blocks; fp32 data may end in a ragged row
       uint64_t rows = op == kOpAddI32 ? num_blocks(p.n[g]) : p.n[g] / kBlock;
-      p.use_tma[g] = make_rows_map(&maps.m[g], p.local[g], rows) ? 1u : 0u;
+      p.use_tma[g] = make_rows_map(&maps.m[g], p.local[g], rows, kTileBlocks) ? 1u : 0u;
     }
   }
   if (op == kOpAddF32 && mode == kModeOutlier) {
@@ -1248,33 +894,6 @@ cudaError_t launch_encode(int op, int mode, EncParams p, cudaStream_t stream, bo
     case kOpAddF32: return launch_encode_m<kOpAddF32>(mode, maps, p, stream, overlap);
     case kOpAddI32: return launch_encode_m<kOpAddI32>(mode, maps, p, stream, overlap);
     case kOpAddStream: return launch_encode_m<kOpAddStream>(mode, maps, p, stream, overlap);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-cudaError_t launch_decode(int mode, DecParams p, cudaStream_t stream, bool overlap) {
-  if (p.n_seg == 0 || p.n_seg > (uint32_t)kMaxDst) return cudaErrorInvalidValue;
-  uint64_t n_max = 0;
-  for (uint32_t i = 0; i < p.n_seg; ++i) n_max = p.seg[i].n > n_max ? p.seg[i].n : n_max;
-  if (n_max == 0) return cudaSuccess;
-  p.tiles_per_seg = (uint32_t)(rate_bytes(n_max) / kTileBlocks);
-  p.n_tiles = p.tiles_per_seg * p.n_seg;
-  TensorMaps maps;
-  memset(&maps, 0, sizeof(maps));
-  if (p.sum) {
-    // one output: every stream must describe the same array
-    for (uint32_t i = 1; i < p.n_seg; ++i)
-      if (p.seg[i].n != p.seg[0].n) return cudaErrorInvalidValue;
-    if (mode == kModeVec) return cudaErrorInvalidValue;
-    p.seg[0].use_tma = make_rows_map(&maps.m[0], p.seg[0].out, p.seg[0].n / kBlock) ? 1u : 0u;
-    return launch_decode_t<kModeOutlier, true>(maps, p, stream, overlap);
-  }
-  for (uint32_t i = 0; i < p.n_seg; ++i)
-    p.seg[i].use_tma = make_rows_map(&maps.m[i], p.seg[i].out, p.seg[i].n / kBlock) ? 1u : 0u;
-  switch (mode) {
-    case kModeOutlier:
-    case kModePlain: return launch_decode_t<kModeOutlier>(maps, p, stream, overlap);
-    case kModeVec: return launch_decode_t<kModeVec>(maps, p, stream, overlap);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -1318,16 +937,12 @@ cudaError_t launch_sum(float* dst, const float* a, const float* b, const float* 
 }  // namespace hc
 
 // CTAs of one launch that the current device holds at once: op 0 compress, 1 fused add, 2 fused add
-// in place (the variant for launches of about one tile per CTA), 3 decode
+// in place (the variant for launches of about one tile per CTA)
 extern "C" int hc_resident_ctas(int op) {
   switch (op) {
     case 0: return hc::encode_capacity<hc::kOpCompress, hc::kModeOutlier, false>();
     case 1: return hc::encode_capacity<hc::kOpAddF32, hc::kModeOutlier, false>();
     case 2: return hc::encode_capacity<hc::kOpAddF32, hc::kModeOutlier, true>();
-    case 3: {
-      static thread_local int cache[64] = {};
-      return hc::resident_ctas(hc::dev::hc_decode_kernel<hc::kModeOutlier, false>, hc::dev::kDecThreads, hc::kDecSmem, cache);
-    }
     default: return 0;
   }
 }

@@ -33,8 +33,7 @@
 // thread, and needs a 4-byte device-to-host copy after every launch
 // (HomComp/src/GSZ.cu:33-756, HomComp/src/GSZ_entry.cu:263-301).
 #pragma once
-#include "hc_bitplane.h"
-#include "hc_device.cuh"
+#include "hc_block.cuh"
 
 namespace hc {
 
@@ -118,9 +117,16 @@ struct DecParams {
   uint32_t n_tiles;  // n_seg * tiles_per_seg
   uint32_t ring_epoch;
   float eb;
+  float scale;          // 2 eb * 2^23 where one multiplication by it gives the bits of (q * eb) * 2; else 0
   uint32_t grid_limit;  // at most this many CTAs (0: as many as the GPU holds)
   uint32_t sum;         // 1: the n_seg streams are contributions to one array of seg[0].n values; their
                         //    quantised values are added tile by tile and seg[0].out receives the sum
+  uint32_t parts;       // flagged segments: tickets per tile, 1 (a warp takes all four quarters) or 4
+  // stand-alone streams (no in_ready; set by the launcher): one word per CTA and stream for the exchange of payload
+  // totals; sub-tiles of every warp's run that are handed out one by one, and their payload offsets as flag words
+  uint64_t* chain;
+  uint64_t* flags;
+  uint32_t pool;
   Workspace ws;
 };
 struct TensorMaps {
@@ -142,37 +148,6 @@ struct OffsetParams {
 namespace dev {
 
 // ---- per-thread block arithmetic ------------------------------------------------------------
-
-__device__ __forceinline__ int32_t quantise(float x, float recip) {
-  float t = __fmul_rn(x, recip);  // two roundings: the stream is defined without FMA contraction
-  float u = __fadd_rn(t, 0.5f);
-  return __float2int_rz(u) - ((t >= -0.5f) ? 0 : 1);
-}
-
-// 32 values of row `row` from a tile stored with the 128-byte TMA swizzle
-__device__ __forceinline__ void load_row_swizzled(const uint8_t* stage, int row, uint32_t (&w)[32]) {
-  const uint8_t* r = stage + row * 128;
-  const int x = row & 7;
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint4 v = *reinterpret_cast<const uint4*>(r + ((c ^ x) << 4));
-    w[4 * c + 0] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
-  }
-}
-__device__ __forceinline__ void store_row_swizzled(uint8_t* stage, int row, const uint32_t (&w)[32]) {
-  uint8_t* r = stage + row * 128;
-  const int x = row & 7;
-#pragma unroll
-  for (int c = 0; c < 8; ++c)
-    *reinterpret_cast<uint4*>(r + ((c ^ x) << 4)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
-}
-
-// plain-load path (unaligned base, tiny inputs) and the ragged last row
-__device__ __forceinline__ void load_row_global(const uint32_t* base, uint64_t n, uint64_t row, uint32_t (&w)[32]) {
-  uint64_t o = row * kBlock;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) w[i] = (o + i < n) ? __ldg(base + o + i) : 0u;
-}
 
 template <int MODE>
 __device__ __forceinline__ void lorenzo_forward(const int32_t (&q)[32], int32_t (&d)[32]) {
@@ -229,6 +204,7 @@ __device__ __forceinline__ void transpose_forward(uint32_t (&A)[32], int W) {
   switch (W) {
     case 4: planes_from_rows<4>(A); break;
     case 8: planes_from_rows<8>(A); break;
+    case 12: planes_from_rows<12>(A); break;
     case 16: planes_from_rows<16>(A); break;
     case 32: planes_from_rows<32>(A); break;
     default: break;
@@ -288,6 +264,7 @@ __device__ __forceinline__ void write_payload(uint8_t* obuf, uint32_t pos, const
     }
     case 4: write_payload_w<4>(obuf, pos, c, T); break;
     case 8: write_payload_w<8>(obuf, pos, c, T); break;
+    case 12: write_payload_w<12>(obuf, pos, c, T); break;
     case 16: write_payload_w<16>(obuf, pos, c, T); break;
     default: write_payload_w<32>(obuf, pos, c, T); break;
   }
@@ -348,6 +325,7 @@ __device__ __forceinline__ uint32_t decode_magnitudes(const uint8_t* cbuf, uint3
       break;
     case 4: read_payload_w<4>(cbuf, pos, rate, sign_mem, a0, T); rows_from_planes<4>(T); break;
     case 8: read_payload_w<8>(cbuf, pos, rate, sign_mem, a0, T); rows_from_planes<8>(T); break;
+    case 12: read_payload_w<12>(cbuf, pos, rate, sign_mem, a0, T); rows_from_planes<12>(T); break;
     case 16: read_payload_w<16>(cbuf, pos, rate, sign_mem, a0, T); rows_from_planes<16>(T); break;
     default: read_payload_w<32>(cbuf, pos, rate, sign_mem, a0, T); rows_from_planes<32>(T); break;
   }

@@ -1,0 +1,125 @@
+// Warp- and CTA-level helpers of the codec kernels: status words, bounded waits, rate bytes -> payload offsets.
+#pragma once
+#include "hc_kernels.cuh"
+
+namespace hc {
+namespace dev {
+
+constexpr uint32_t kNoTile = 0xffffffffu;
+
+__device__ __forceinline__ void note_error(uint32_t* ctrl, uint32_t code) { atomicMax(ctrl + 2, code); }
+// timeouts and peer failures end the launch early; capacity / truncation errors only skip data
+__device__ __forceinline__ bool fatal_error(const uint32_t* ctrl) {
+  return *((volatile const uint32_t*)(ctrl + 2)) >= (uint32_t)kErrTimeout;
+}
+
+// which wait ran out; the first one is kept in ctrl[3] (hc_codec_status_site), because every later time-out of
+// the launch is only a consequence of it
+enum WaitSite : uint32_t {
+  kSiteLoaderStageFree = 1, kSiteLoaderInFree = 2, kSiteComputeInFull = 3, kSiteComputeTile = 4, kSiteComputeRing = 5,
+  kSiteScannerTotal = 6, kSiteCopierBase = 7, kSiteCopierPacked = 8, kSiteDecodeInFree = 9, kSiteDecodeInFull = 10,
+  kSiteLookBack = 11,
+};
+__device__ __forceinline__ void note_timeout(const Workspace& ws, uint32_t site) {
+  if (!fatal_error(ws.ctrl)) atomicCAS(ws.ctrl + 3, 0u, site);
+  note_error(ws.ctrl, kErrTimeout);
+}
+// bounded mbarrier wait of a whole warp; false: gave up (recorded)
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const Workspace& ws, uint32_t site) {
+  const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, ws.spin_limit_ns));
+  if (!ok && (threadIdx.x & 31) == 0) note_timeout(ws, site);
+  return ok;
+}
+
+// collective steps: one non-blocking look at the tile's arrival flag; 0 = not raised yet
+__device__ __forceinline__ uint64_t flag_peek(const uint64_t* flag, uint32_t call) {
+  uint64_t w = 0;
+  if ((threadIdx.x & 31) == 0) {
+    w = ld_acquire_sys_u64(flag);
+    if (!flag_matches(w, call)) w = 0;
+  }
+  return __shfl_sync(0xffffffffu, w, 0);
+}
+// collective steps: bounded wait for the tile's arrival flag; 0 = the peer never delivered
+__device__ __forceinline__ uint64_t flag_wait_warp(const uint64_t* flag, uint32_t call, const Workspace& ws) {
+  uint64_t w = 0;
+  if ((threadIdx.x & 31) == 0) {
+    w = wait_tile_flag(flag, call, ws.spin_limit_ns, ws.ctrl + 2);
+    if (w == 0) note_error(ws.ctrl, kErrPeer);
+  }
+  return __shfl_sync(0xffffffffu, w, 0);
+}
+
+// bounded wait for a flag that some CTA of the same launch writes; ~0: gave up
+__device__ __forceinline__ uint64_t own_flag_wait(const uint64_t* flag, uint32_t tag, const Workspace& ws) {
+  uint64_t w = 0;
+  if ((threadIdx.x & 31) == 0) {
+    const long long t0 = clock64();
+    const long long limit_clk = (long long)ws.spin_limit_ns * 2;
+    for (uint32_t it = 0; it < (1u << 24); ++it) {
+      w = ld_relaxed_gpu_u64(flag);
+      if (flag_matches(w, tag)) break;
+      w = ~0ull;
+      __nanosleep(100);
+      if ((it & 15u) == 15u && (clock64() - t0 > limit_clk || fatal_error(ws.ctrl))) break;
+    }
+    if (w == ~0ull) note_timeout(ws, kSiteLookBack);
+  }
+  return __shfl_sync(0xffffffffu, w, 0);
+}
+
+// ---- rate bytes -> offsets ------------------------------------------------------------------------------
+// rate bytes b .. b+3 of a stream as a word; bytes past the end of the stream count as 0
+__device__ __forceinline__ uint32_t load_rates4(const uint8_t* in, uint64_t in_size, uint64_t b) {
+  if (b + 4 <= in_size && ((reinterpret_cast<uintptr_t>(in) + b) & 3u) == 0)
+    return __ldcg(reinterpret_cast<const uint32_t*>(in + b));
+  uint32_t r = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (b + k < in_size) r |= ld_cg_u8(in + b + k) << (8 * k);
+  return r;
+}
+
+constexpr int kMaxCtas = 160;  // CTAs of a launch with one CTA per SM
+// Sum of the status words words[0 .. n) of this launch (n <= 32 * U), one warp; polls until all are there (bounded)
+template <int U>
+__device__ __forceinline__ uint64_t sum_status_words(const uint64_t* words, uint32_t n, const Workspace& ws) {
+  const uint32_t lane = threadIdx.x & 31;
+  const long long t0 = clock64();
+  const long long limit_clk = (long long)ws.spin_limit_ns * 2;
+  for (uint32_t it = 0; it < (1u << 24); ++it) {
+    uint64_t w[U], sum = 0;
+    bool ready = true;
+#pragma unroll
+    for (int u = 0; u < U; ++u) w[u] = lane + 32u * u < n ? ld_relaxed_gpu_u64(words + lane + 32u * u) : st_pack(kStAgg, ws.epoch, 0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      ready = ready && st_state(w[u], ws.epoch) != 0;
+      sum += st_value(w[u]);
+    }
+    if (__all_sync(0xffffffffu, ready)) return warp_sum_u64(sum);
+    if ((it & 15u) == 15u && __any_sync(0xffffffffu, clock64() - t0 > limit_clk || fatal_error(ws.ctrl))) break;
+  }
+  if (lane == 0) note_timeout(ws, kSiteLookBack);
+  return 0;
+}
+
+// the last CTA to leave re-arms the ticket counter for the next launch (true in thread 0 of that CTA)
+__device__ __forceinline__ bool cta_epilogue(uint32_t* tick) {
+  __syncthreads();
+  bool last = false;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    uint32_t done = atomicAdd(tick + 1, 1u);
+    if (done == gridDim.x - 1) {
+      tick[0] = 0;
+      tick[1] = 0;
+      __threadfence();
+      last = true;
+    }
+  }
+  return last;
+}
+
+}  // namespace dev
+}  // namespace hc

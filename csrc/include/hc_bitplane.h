@@ -7,7 +7,7 @@
 //
 // The transpose is five independent stages (one per index bit); stage `s` swaps bit s of the row
 // index with bit s of the column index.  Stages 16 and 8 are byte permutes (PRMT), stages 4, 2, 1
-// are shift-xor swaps.  When every magnitude of the block fits W bits (W = 4, 8, 16) the upper rows
+// are shift-xor swaps.  When every magnitude of the block fits W bits (W = 4, 8, 12, 16) the upper rows
 // of the result are known zero and most of the network disappears, which is what makes the
 // thread-per-block layout cheaper than one warp ballot per plane: cost is ~2.6 (W=8) to ~9.5 (W=32)
 // integer instructions per element, independent of F.
@@ -29,20 +29,22 @@ HC_HD uint32_t perm(uint32_t a, uint32_t b, uint32_t sel) {
 #endif
 }
 
-// swap the bits of A[k] selected by (m << s) with the bits of A[k + s] selected by m
+// swap the bits of A[k] selected by ~m with the bits of A[k + s] selected by m (m << s == ~m).  Written as two
+// bit selects: two shifts and two 3-input logic operations a pair, one operation less than the xor-swap form
 template <int S>
 HC_HD void swap_stage(uint32_t& lo, uint32_t& hi) {
   constexpr uint32_t m = S == 4 ? 0x0f0f0f0fu : (S == 2 ? 0x33333333u : 0x55555555u);
-  uint32_t t = ((lo >> S) ^ hi) & m;
-  hi ^= t;
-  lo ^= t << S;
+  const uint32_t l = lo, h = hi;
+  lo = (l & m) | ((h << S) & ~m);
+  hi = ((l >> S) & m) | (h & ~m);
 }
 
 // Forward: rows A[0..31] hold values below 2^W; on return A[0..W-1] hold planes 0..W-1.
-// Rows W..31 are unspecified afterwards.
+// Rows W..31 are unspecified afterwards.  For W <= 16 the bits of the rows at and above 16 are ignored
+// (stage 16 picks the low halves).
 template <int W>
 HC_HD void planes_from_rows(uint32_t (&A)[32]) {
-  static_assert(W == 4 || W == 8 || W == 16 || W == 32, "W");
+  static_assert(W == 4 || W == 8 || W == 12 || W == 16 || W == 32, "W");
   // stage 16
 #pragma unroll
   for (int k = 0; k < 16; ++k) {
@@ -60,7 +62,7 @@ HC_HD void planes_from_rows(uint32_t (&A)[32]) {
       if (W > 8) A[k + 8] = perm(lo, hi, 0x7351);
     }
   }
-  constexpr int R = W;  // live rows from here on
+  constexpr int R = W == 12 ? 8 : W;  // rows with a full stage 4
   // stage 4
   if (W == 4) {
 #pragma unroll
@@ -69,12 +71,16 @@ HC_HD void planes_from_rows(uint32_t (&A)[32]) {
 #pragma unroll
     for (int k = 0; k < R; ++k)
       if ((k & 4) == 0) swap_stage<4>(A[k], A[k + 4]);
+    if (W == 12) {
+#pragma unroll
+      for (int k = 8; k < 12; ++k) A[k] = (A[k] & 0x0f0f0f0fu) | ((A[k + 4] << 4) & 0xf0f0f0f0u);
+    }
   }
 #pragma unroll
-  for (int k = 0; k < R; ++k)
+  for (int k = 0; k < W; ++k)
     if ((k & 2) == 0) swap_stage<2>(A[k], A[k + 2]);
 #pragma unroll
-  for (int k = 0; k < R; ++k)
+  for (int k = 0; k < W; ++k)
     if ((k & 1) == 0) swap_stage<1>(A[k], A[k + 1]);
 }
 
@@ -82,32 +88,44 @@ HC_HD void planes_from_rows(uint32_t (&A)[32]) {
 // Entries A[W..31] are ignored on input.
 template <int W>
 HC_HD void rows_from_planes(uint32_t (&A)[32]) {
-  static_assert(W == 4 || W == 8 || W == 16 || W == 32, "W");
-  constexpr int R = W;
+  static_assert(W == 4 || W == 8 || W == 12 || W == 16 || W == 32, "W");
 #pragma unroll
-  for (int k = 0; k < R; ++k)
+  for (int k = 0; k < W; ++k)
     if ((k & 1) == 0) swap_stage<1>(A[k], A[k + 1]);
 #pragma unroll
-  for (int k = 0; k < R; ++k)
+  for (int k = 0; k < W; ++k)
     if ((k & 2) == 0) swap_stage<2>(A[k], A[k + 2]);
-  if (W == 4) {
+  constexpr int R = W == 12 ? 8 : W;  // rows with a full stage 4
+  if (W == 4 || W == 12) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = W - 4; k < W; ++k) {
       uint32_t v = A[k];
       A[k] = v & 0x0f0f0f0fu;
       A[k + 4] = (v >> 4) & 0x0f0f0f0fu;
     }
-  } else {
+  }
+  if (W != 4) {
 #pragma unroll
     for (int k = 0; k < R; ++k)
       if ((k & 4) == 0) swap_stage<4>(A[k], A[k + 4]);
+  }
+  if (W <= 8) {  // stages 8 and 16 at once: every byte of the eight registers is a row
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t v = A[k];
+      A[k] = perm(v, 0u, 0x4440);
+      A[k + 8] = perm(v, 0u, 0x4441);
+      A[k + 16] = perm(v, 0u, 0x4442);
+      A[k + 24] = perm(v, 0u, 0x4443);
+    }
+    return;
   }
   // stage 8
 #pragma unroll
   for (int h = 0; h < (W > 16 ? 32 : 16); h += 16) {
 #pragma unroll
     for (int k = h; k < h + 8; ++k) {
-      uint32_t lo = A[k], hi = (W > 8) ? A[k + 8] : 0u;
+      uint32_t lo = A[k], hi = A[k + 8];
       A[k] = perm(lo, hi, 0x6240);
       A[k + 8] = perm(lo, hi, 0x7351);
     }
@@ -122,6 +140,8 @@ HC_HD void rows_from_planes(uint32_t (&A)[32]) {
 }
 
 // smallest supported width that holds F planes (F in 0..31); 0 means "no planes at all"
-HC_HD int plane_width(uint32_t F) { return F == 0 ? 0 : (F <= 4 ? 4 : (F <= 8 ? 8 : (F <= 16 ? 16 : 32))); }
+HC_HD int plane_width(uint32_t F) {
+  return F == 0 ? 0 : (F <= 4 ? 4 : (F <= 8 ? 8 : (F <= 12 ? 12 : (F <= 16 ? 16 : 32))));
+}
 
 }  // namespace hc
