@@ -31,33 +31,6 @@ hc::Workspace next_workspace(hc_codec* c, cudaStream_t stream) {
   return hc::workspace_view(c->ws_mem, c->max_elems, c->epoch, c->spin_limit_ns);
 }
 
-// Streams of at least this many tiles get their tile offsets from the pre-pass (launch_offsets):
-// below it the consuming kernel has a tile or two per CTA and its own look-back costs nothing extra.
-constexpr uint32_t kPrepassMinTiles = 1024;
-
-// Enqueues the pre-pass over `n_in` streams of n values each and returns the flag rows it fills
-// (in the look-back words of the input chains, which the consumer then does not use); false when the
-// streams are small or the workspace has no room, in which case the consumer walks the chains itself.
-bool stage_offsets(hc_codec* c, const hc::Workspace& ws, const uint8_t* const* in, const size_t* in_size, uint32_t n_in,
-                   size_t n, const uint64_t** flags, cudaStream_t stream) {
-  const uint32_t tiles = (uint32_t)(hc::rate_bytes(n) / hc::kTileBlocks);
-  if (!c->prepass || tiles < kPrepassMinTiles || !hc::offsets_fit(ws, c->max_elems, n_in, tiles)) return false;
-  hc::OffsetParams o;
-  memset(&o, 0, sizeof(o));
-  o.n_in = n_in;
-  o.tiles_per_seg = tiles;
-  o.nrate = hc::rate_bytes(n);
-  o.tag = ws.epoch;  // below 2^22: can never match a look-back status word left in the same place
-  o.ws = ws;
-  for (uint32_t q = 0; q < n_in; ++q) {
-    o.in[q] = in[q];
-    o.in_size[q] = in_size[q];
-    o.flags[q] = ws.st_a + (size_t)q * tiles;
-    flags[q] = o.flags[q];
-  }
-  return hc::launch_offsets(o, stream) == cudaSuccess;
-}
-
 int check_call(hc_codec* c, size_t n, float eb, bool needs_eb) {
   if (!c) return hc::kErrArgument;
   if (n > c->max_elems) return hc::kErrArgument;
@@ -73,7 +46,7 @@ int encode_call(hc_codec* c, int op, int mode, const void* local, const uint8_t*
     if (d_size) cudaMemsetAsync(d_size, 0, sizeof(uint64_t), stream);
     return hc::kOk;
   }
-  hc::EncParams p;
+  hc::SoloParams p;
   memset(&p, 0, sizeof(p));
   p.n_seg = 1;
   p.local[0] = local;
@@ -84,21 +57,11 @@ int encode_call(hc_codec* c, int op, int mode, const void* local, const uint8_t*
   p.in_size[0] = in_size;
   p.in[1] = in2;
   p.in_size[1] = in2_size;
-  p.n_dst = 1;
   p.out[0] = out;
   p.out_cap = cap;
   p.size_out = d_size;
   p.ws = next_workspace(c, stream);
-  bool flagged = false;
-  if (p.n_in) {
-    const uint8_t* ins[2] = {in, in2};
-    const size_t sizes[2] = {in_size, in2_size};
-    flagged = stage_offsets(c, p.ws, ins, sizes, p.n_in, n, p.in_ready, stream);
-    if (flagged) p.ring_epoch = p.ws.epoch;
-    else p.in_ready[0] = p.in_ready[1] = nullptr;
-  }
-  // behind its pre-pass the kernel starts at once and consumes tiles as their flags appear
-  return hc::launch_encode(op, mode, p, stream, flagged) == cudaSuccess ? hc::kOk : hc::kErrCuda;
+  return hc::launch_encode_solo(op, mode, p, stream) == cudaSuccess ? hc::kOk : hc::kErrCuda;
 }
 
 }  // namespace
@@ -257,7 +220,7 @@ int hc_decompress_sum(hc_codec* c, int n_in, const uint8_t* const* d_in, const s
 int hc_compress_batch(hc_codec* c, int n_seg, const float* const* d_x, const size_t* n, float eb, int mode,
                       uint8_t* const* d_out, size_t cap_each, uint64_t* d_sizes, hc_stream_t stream) {
   if (!c || n_seg < 1 || n_seg > hc::kMaxDst || !(eb > 0.0f) || !d_x || !n || !d_out) return hc::kErrArgument;
-  hc::EncParams p;
+  hc::SoloParams p;
   memset(&p, 0, sizeof(p));
   size_t total = 0;
   for (int g = 0; g < n_seg; ++g) {
@@ -269,12 +232,11 @@ int hc_compress_batch(hc_codec* c, int n_seg, const float* const* d_x, const siz
   }
   if (total > hc::rate_bytes(c->max_elems) * hc::kBlock) return hc::kErrArgument;
   p.n_seg = (uint32_t)n_seg;
-  p.n_dst = 1;
   p.recip = 0.5f / eb;
   p.out_cap = cap_each;
   p.size_out = d_sizes;
   p.ws = next_workspace(c, stream);
-  return hc::launch_encode(hc::kOpCompress, mode, p, stream) == cudaSuccess ? hc::kOk : hc::kErrCuda;
+  return hc::launch_encode_solo(hc::kOpCompress, mode, p, stream) == cudaSuccess ? hc::kOk : hc::kErrCuda;
 }
 
 // n_in streams (+) fp32 -> stream: every stream is decoded to deltas and summed in the integer
@@ -285,7 +247,7 @@ int hc_hom_add_multi(hc_codec* c, int n_in, const uint8_t* const* d_in, const si
   if (n_in < 1 || n_in > hc::kMaxIn || !d_in || !in_size || !d_local || !d_out) return hc::kErrArgument;
   if ((size_t)n_in * hc::rate_bytes(n) > hc::rate_bytes(c->max_elems) + 64) return hc::kErrArgument;
   if (n == 0) return hc::kOk;
-  hc::EncParams p;
+  hc::SoloParams p;
   memset(&p, 0, sizeof(p));
   p.n_seg = 1;
   p.local[0] = d_local;
@@ -296,16 +258,11 @@ int hc_hom_add_multi(hc_codec* c, int n_in, const uint8_t* const* d_in, const si
     p.in[q] = d_in[q];
     p.in_size[q] = in_size[q];
   }
-  p.n_dst = 1;
   p.out[0] = d_out;
   p.out_cap = cap;
   p.size_out = d_size;
   p.ws = next_workspace(c, stream);
-  const bool flagged = stage_offsets(c, p.ws, d_in, in_size, p.n_in, n, p.in_ready, stream);
-  if (flagged) p.ring_epoch = p.ws.epoch;
-  else
-    for (int q = 0; q < n_in; ++q) p.in_ready[q] = nullptr;
-  return hc::launch_encode(hc::kOpAddF32, mode, p, stream, flagged) == cudaSuccess ? hc::kOk : hc::kErrCuda;
+  return hc::launch_encode_solo(hc::kOpAddF32, mode, p, stream) == cudaSuccess ? hc::kOk : hc::kErrCuda;
 }
 
 int hc_quant_pred(const float* d_x, size_t n, float eb, int mode, int32_t* d_deltas, hc_stream_t stream) {

@@ -24,6 +24,14 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+// stores v when j <= limit, as a predicated store (no branch)
+__device__ __forceinline__ void sts32_upto(uint32_t addr, uint32_t v, uint32_t j, uint32_t limit) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.le.u32 p, %2, %3;\n\t@p st.shared.u32 [%0], %1;\n\t}" ::"r"(addr), "r"(v), "r"(j), "r"(limit)
+               : "memory");
+}
 // (a & b) | c in one operation, with b and c kept from being split into two immediates
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
@@ -150,6 +158,159 @@ __device__ __forceinline__ void decode_rows(const uint8_t* buf, uint32_t pos, ui
 __device__ __forceinline__ float sign_scale(uint32_t sign, int i) { return as_f(and_or(sign << i, kMsb, 0x7e800000u)); }
 // |d_i| and sign -> d_i as a subnormal
 __device__ __forceinline__ float signed_sub(uint32_t mag, uint32_t sign, int i) { return as_f(mag ^ ((sign << i) & kMsb)); }
+
+
+// ---- block -> stream --------------------------------------------------------------------------------
+template <int MODE>
+__host__ __device__ constexpr int lorenzo_stride() { return MODE == kModeVec ? 4 : 1; }
+
+struct BlockCode {
+  uint32_t rate;  // rate byte
+  uint32_t len;   // payload bytes
+  uint32_t a0;    // |d_0|
+  uint32_t sign;  // sign map, element i at bit 31 - i
+};
+
+// values (float bits) -> deltas of the quantised values as subnormals, in place
+template <int MODE>
+__device__ __forceinline__ void deltas_sub(uint32_t (&w)[32], float recip) {
+  constexpr int S = lorenzo_stride<MODE>();
+#pragma unroll
+  for (int i = 0; i < 32; ++i) w[i] = as_u(quantise_sub(as_f(w[i]), recip));
+#pragma unroll
+  for (int i = 31; i >= S; --i) w[i] = as_u(__fsub_rn(as_f(w[i]), as_f(w[i - S])));
+}
+// the same in int32
+template <int MODE>
+__device__ __forceinline__ void deltas_int(uint32_t (&w)[32], float recip) {
+  constexpr int S = lorenzo_stride<MODE>();
+#pragma unroll
+  for (int i = 0; i < 32; ++i) w[i] = (uint32_t)quantise(as_f(w[i]), recip);
+#pragma unroll
+  for (int i = 31; i >= S; --i) w[i] -= w[i - S];
+}
+// a whole number held as a subnormal -> int32
+__device__ __forceinline__ uint32_t sub_to_int(uint32_t bits) {
+  const uint32_t m = (uint32_t)((int32_t)bits >> 31);
+  return ((bits & 0x7fffffffu) ^ m) - m;
+}
+// int32 -> sign and magnitude, 31 bits (INT_MIN folds to -0, whose sign the stream keeps)
+__device__ __forceinline__ uint32_t sign_magnitude(uint32_t d) { return ((uint32_t)abs((int32_t)d) & 0x7fffffffu) | (d & kMsb); }
+
+// OR of the magnitudes of d_1 .. d_31
+__device__ __forceinline__ uint32_t or_tail_of(const uint32_t (&d)[32]) {
+  uint32_t o = d[31];
+#pragma unroll
+  for (int i = 1; i < 31; i += 2) o |= d[i] | d[i + 1];  // one 3-input operation per pair
+  return o & 0x7fffffffu;
+}
+// the same of the rows of a decoded block (T[i ^ 7] = |d_i|)
+__device__ __forceinline__ uint32_t or_rows_tail(const uint32_t (&T)[32]) {
+  uint32_t o = 0;
+#pragma unroll
+  for (int i = 1; i < 32; ++i) o |= T[i ^ 7];
+  return o;
+}
+// sign-magnitude deltas -> the block's code; d_0 of an outlier block is taken out of the planes
+template <int MODE>
+__device__ __forceinline__ BlockCode code_of(uint32_t (&d)[32], uint32_t or_tail) {
+  BlockCode c;
+  c.sign = 0;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) c.sign = __funnelshift_l(d[i], c.sign, 1);
+  c.a0 = d[0] & 0x7fffffffu;
+  c.rate = choose_rate(or_tail | c.a0, or_tail, c.a0, MODE != kModePlain);
+  c.len = payload_len(c.rate);
+  if (c.rate & 0x80u) d[0] = 0;
+  return c;
+}
+
+// Packs one block per lane into the ring at `base` (shared address, 16-byte aligned), the lane's payload at byte `rel`:
+// outlier bytes, sign map, planes T[0..W-1] (those at and above F are zero).  Only whole words are stored.  The
+// word in which a block starts is shared with the block before it: every lane first stores all its words behind
+// that one, the last of them padded with zeros, then merges its first bytes into what the lane in front left.
+// The ring must have 4 bytes behind the warp's payload.
+template <int W>
+__device__ __forceinline__ void pack_block(uint32_t base, uint32_t rel, const BlockCode& c, const uint32_t (&T)[32]) {
+  const uint32_t F = c.rate & 31u;
+  const bool outl = (c.rate & 0x80u) != 0;
+  const uint32_t nout = outl ? ((c.rate >> 5) & 3u) + 1u : 0u;
+  const uint32_t a0 = outl ? c.a0 : 0u;
+  const uint32_t p2 = rel + nout;
+  const uint32_t s0 = 8u * (rel & 3u), s = 8u * (p2 & 3u);
+  const uint32_t first = base + (rel & ~3u), at = base + (p2 & ~3u);  // words of the first byte, of the sign map
+  const uint32_t sign = __byte_perm(c.sign, 0, 0x0123);
+  uint32_t head = a0 << s0;
+  if (c.len) {
+    const uint32_t x = sign << s;
+    if (at == first) head |= x;
+    else sts32(at, __funnelshift_l(a0, 0u, s0) | x);
+    uint32_t prev = sign;
+#pragma unroll
+    for (int j = 1; j <= W + 1; ++j) {
+      const uint32_t next = j <= W ? T[j - 1] : 0u;
+      sts32_upto(at + 4 * j, __funnelshift_l(prev, next, s), (uint32_t)j, F + 1u);
+      prev = next;
+    }
+  }
+  __syncwarp();
+  if (c.len) sts32(first, (rel ? lds32(first) : 0u) | head);
+  __syncwarp();
+}
+template <int W>
+__device__ __forceinline__ void pack_w(uint32_t base, uint32_t rel, const BlockCode& c, const uint32_t (&d)[32]) {
+  uint32_t T[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) T[i ^ 7] = W == 32 ? d[i] & 0x7fffffffu : d[i];  // (W <= 16: the sign bits drop out)
+  if (W) planes_from_rows<W ? W : 4>(T);
+  pack_block<W>(base, rel, c, T);
+}
+// W: plane_width of the largest F of the warp
+__device__ __forceinline__ void pack_blocks(uint32_t base, uint32_t rel, const BlockCode& c, const uint32_t (&d)[32], int W) {
+  switch (W) {
+    case 0: pack_w<0>(base, rel, c, d); break;  // outlier blocks with F = 0 carry bytes
+    case 4: pack_w<4>(base, rel, c, d); break;
+    case 8: pack_w<8>(base, rel, c, d); break;
+    case 12: pack_w<12>(base, rel, c, d); break;
+    case 16: pack_w<16>(base, rel, c, d); break;
+    default: pack_w<32>(base, rel, c, d); break;
+  }
+}
+
+// 16-byte units of copy_ring: source bytes start K words and sh bits into 16-byte aligned shared memory
+template <int K>
+__device__ __forceinline__ void copy_units(uint32_t src, uint8_t* out, uint32_t units, uint32_t sh) {
+  for (uint32_t u = threadIdx.x & 31u; u < units; u += 32u) {
+    uint32_t a[8];
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(src + 16u * u) : "memory");
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]) : "r"(src + 16u * u + 16u) : "memory");
+    *reinterpret_cast<uint4*>(out + 16u * u) =
+        make_uint4(__funnelshift_r(a[K], a[K + 1], sh), __funnelshift_r(a[K + 1], a[K + 2], sh),
+                   __funnelshift_r(a[K + 2], a[K + 3], sh), __funnelshift_r(a[K + 3], a[K + 4], sh));
+  }
+}
+// Moves the `tot` bytes at ring address `src` (16-byte aligned) to `dst` in global memory, one warp: 16-byte stores
+// for whole units, the bytes of the first and last partial unit one per lane.  The shift between the alignments of
+// source and destination is the same for every unit: whole words by choosing registers, the rest by funnel shifts.
+// Reads up to 16 bytes behind the payload.
+__device__ __forceinline__ void copy_ring(uint32_t src, uint8_t* dst, uint32_t tot) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t head = (16u - ((uint32_t)reinterpret_cast<uintptr_t>(dst) & 15u)) & 15u;
+  if (head > tot) head = tot;
+  const uint32_t units = (tot - head) >> 4, tail = (tot - head) & 15u;
+  if (lane < 16u ? lane < head : lane - 16u < tail) {
+    const uint32_t at = lane < 16u ? lane : head + 16u * units + lane - 16u;
+    uint32_t b;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(b) : "r"(src + at) : "memory");
+    dst[at] = (uint8_t)b;
+  }
+  switch (head >> 2) {
+    case 0: copy_units<0>(src, dst + head, units, 8u * (head & 3u)); break;
+    case 1: copy_units<1>(src, dst + head, units, 8u * (head & 3u)); break;
+    case 2: copy_units<2>(src, dst + head, units, 8u * (head & 3u)); break;
+    default: copy_units<3>(src, dst + head, units, 8u * (head & 3u)); break;
+  }
+}
 
 }  // namespace dev
 }  // namespace hc

@@ -27,31 +27,12 @@ namespace dev {
 // while the CTAs of the step before leave it.
 __host__ __device__ constexpr int dec_max_warps(bool sum, bool runs) { return !runs ? 4 : sum ? 16 : 20; }
 __host__ __device__ constexpr int dec_ctas(bool sum, bool runs) { return runs ? 1 : sum ? 4 : 5; }
-constexpr int kSubBlocks = 32;
-constexpr int kSubValues = kSubBlocks * kBlock;
-constexpr int kSubBytes = kSubValues * 4;  // 4096
 // payload ring of a warp: the largest payload of corrupt rate bytes (32 x 132) with its 16-byte phase, and in
 // front of the ring's end what read_planes may look at behind a payload
 constexpr int kDecRing = 6144;
 constexpr int kDecRingUsable = kDecRing - 160;
 constexpr int kDecWarpBytes = kSubBytes + kDecRing;
 static_assert(32 * 132 + 32 <= kDecRingUsable, "one payload must fit");
-
-// rate bytes [16 l, 16 l + 16) of the sub-tiles [a, b) of a stream; 0 past b and past the end of the stream
-__device__ __forceinline__ uint4 rates16(const DecSegment& sg, uint32_t a, uint32_t b, uint32_t l) {
-  const uint64_t at = (uint64_t)a * kSubBlocks + 16u * l;
-  uint4 v = make_uint4(0, 0, 0, 0);
-  if (at >= (uint64_t)b * kSubBlocks) return v;
-  if ((reinterpret_cast<uintptr_t>(sg.in) & 15u) == 0 && at + 16u <= sg.in_size) return ld_cg_u4(sg.in + at);
-  v.x = load_rates4(sg.in, sg.in_size, at);
-  v.y = load_rates4(sg.in, sg.in_size, at + 4u);
-  v.z = load_rates4(sg.in, sg.in_size, at + 8u);
-  v.w = load_rates4(sg.in, sg.in_size, at + 12u);
-  return v;
-}
-__device__ __forceinline__ uint32_t payload_len16(const uint4& v) {
-  return payload_len4(v.x) + payload_len4(v.y) + payload_len4(v.z) + payload_len4(v.w);
-}
 
 // SUM: the n_seg streams hold contributions to ONE array; a warp stages the same sub-tile of every stream in
 // turn, adds the signed deltas in registers and writes seg[0].out once.
@@ -129,7 +110,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     run_end = (uint32_t)((uint64_t)subs * (gw + 1) / nw);
     it_end = run_end - pool;
 #pragma unroll
-    for (uint32_t qq = 0; qq < (SUM ? kMaxDst : 1); ++qq) rates[qq] = qq < Q ? rates16(p.seg[qq], it, run_end, lane) : make_uint4(0, 0, 0, 0);
+    for (uint32_t qq = 0; qq < (SUM ? kMaxDst : 1); ++qq) rates[qq] = qq < Q ? rates16(p.seg[qq].in, p.seg[qq].in_size, it, run_end, lane) : make_uint4(0, 0, 0, 0);
   }
   const uint32_t run_begin = it;
   // ---- tickets: sub-tiles of the pools (RUNS), tiles or quarters (!RUNS) -----------------------------------------------
@@ -213,7 +194,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
       if (qq >= Q) break;
       uint32_t sum = payload_len16(rates[qq]);
       for (uint32_t l = lane + 32u; run_begin * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u)
-        sum += payload_len16(rates16(p.seg[qq], run_begin, run_end, l));
+        sum += payload_len16(rates16(p.seg[qq].in, p.seg[qq].in_size, run_begin, run_end, l));
       sum = __reduce_add_sync(0xffffffffu, sum);
       if (lane == 0) s_tot[warp][qq] = sum;
     }

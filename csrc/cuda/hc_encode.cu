@@ -1,0 +1,602 @@
+// fp32 (+ streams) -> stream (compress and the homomorphic adds, stand-alone): kernel and launcher.
+//
+// A unit of work is a SUB-TILE, 32 consecutive blocks (1024 values, 4 KB of fp32), one block per lane.  A CHUNK of nc
+// sub-tiles, one per compute warp, is what a CTA takes at a time; one CTA per SM.  The compute warps of a CTA do not
+// wait for each other: each has a stage for its fp32 rows (TMA tiled load, 128-byte swizzle), for the adds a byte ring
+// for incoming payloads (bulk copies up to two jobs ahead), and a byte ring for packed payloads, in which several of
+// them wait for their place in the output while the warp goes on.
+//
+// Where payloads go: the total of every chunk is published as one word; one warp per CTA (the CLERK) adds up the words
+// between its CTA's previous chunk and the current one (at most about 150, five loads a lane, one round trip once they
+// are there) and hands every compute warp its byte offset.  A clerk only ever waits for chunk totals, never for another
+// clerk, so there is no chain of hops as in a decoupled look-back.
+// Where payloads come from (adds): the same sums over the rate bytes of the input streams, four chunks ahead of the
+// compute warps.
+#include "hc_host.cuh"
+#include "hc_launch.h"
+#include "hc_warp.cuh"
+
+namespace hc {
+namespace dev {
+
+constexpr int kSlots = 8;    // chunks of a CTA between "total known" and "payload copied out"
+constexpr int kInSlots = 4;  // chunks whose input offsets are known
+
+// compute warps of a CTA at most: 16 warps with the clerk, 128 registers each (19 + 1 at 96 registers spilled: 84 us
+// against 77 at 256 MB)
+constexpr int kEncWarps = 15;
+// packed payloads: a payload of 4096 bytes, 4 bytes pack_block adds, 16 copy_ring looks ahead
+__host__ __device__ constexpr int enc_out_ring(int op) { return op == kOpCompress ? 8192 : 5120; }
+// incoming payloads: see hc_decode.cu
+__host__ __device__ constexpr int enc_in_ring(int op) { return op == kOpCompress ? 0 : 4864; }
+__host__ __device__ constexpr int enc_warp_bytes(int op) { return kSubBytes + enc_out_ring(op) + enc_in_ring(op); }
+constexpr int kInUsable = 4864 - 160;
+static_assert(kEncWarps * 4096 < (1 << 24), "EncShared::sum");
+static_assert(32 * 132 + 32 <= kInUsable, "one payload must fit");
+
+struct EncShared {
+  uint64_t stage_full[kEncWarps];
+  uint64_t in_full[kEncWarps][4];
+  uint64_t placed[kSlots];                      // out_at[] of the chunk is valid
+  uint64_t in_known[kInSlots];                  // in_at[] of the chunk is valid (one arrival per stream)
+  uint64_t out_at[kSlots][kEncWarps];           // byte offset of the warp's payload; ~0: not to be stored
+  uint64_t in_at[kInSlots][kMaxIn][kEncWarps];  // byte offsets of the incoming payloads
+  uint64_t in_run[kMaxIn];                      // streams: payload bytes before the CTA's next chunk
+  uint32_t tot[kSlots][kEncWarps];
+  uint32_t sum[kSlots];  // running total of the chunk [23:0] and number of warps that have added theirs [31:24]
+  uint32_t dead;         // an earlier launch timed out and nobody has cleared it: no output
+};
+
+// chunk number -> segment and chunk inside it
+struct Chunk {
+  uint32_t seg, lc;
+};
+__device__ __forceinline__ Chunk chunk_of(const SoloParams& p, uint32_t t) {
+  uint32_t g = 0;
+  while (g + 1 < p.n_seg && t >= p.first[g + 1]) ++g;
+  return Chunk{g, t - p.first[g]};
+}
+// Chunk number k of this CTA: dealt out in turn (the CTAs of a launch keep the same pace; numbers from a counter went
+// unevenly to CTAs whose first warp ran ahead of the others: 21 to 26 of 23 chunks at 256 MB).  kNoTile: none left
+__device__ __forceinline__ uint32_t ticket(const SoloParams& p, uint32_t k) {
+  const uint32_t t = k * gridDim.x + blockIdx.x;
+  return t < p.first[p.n_seg] ? t : kNoTile;
+}
+
+// Running sum over the totals of consecutive chunks of a launch: brings `base` from chunk `next` to chunk t (one warp)
+__device__ __forceinline__ void advance_base(const uint64_t* words, uint32_t& next, uint64_t& base, uint32_t t, const Workspace& ws) {
+  while (next < t) {
+    const uint32_t n = t - next < (uint32_t)kMaxCtas ? t - next : (uint32_t)kMaxCtas;
+    base += sum_status_words<kMaxCtas / 32>(words + next, n, ws);
+    next += n;
+  }
+}
+
+// "All compute warps have put down their total of chunk k": hardware barrier 1 + k % kSlots; they arrive, the clerk
+// waits (polling an mbarrier instead it took up to half of the issue slots of its scheduler).  A warp comes to chunk
+// k + kSlots only after chunk k has been placed, so no barrier is entered twice.  The wait has no time limit of its
+// own: it ends because every compute warp arrives once for every chunk of its CTA, one that gave up on something
+// included.
+__device__ __forceinline__ void totals_arrive(uint32_t k, uint32_t nc) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(1u + k % kSlots), "r"(32u * nc + 32u) : "memory");
+}
+__device__ __forceinline__ void totals_wait(uint32_t k, uint32_t nc) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1u + k % kSlots), "r"(32u * nc + 32u) : "memory");
+}
+
+// ---- the clerk ---------------------------------------------------------------------------------------------------
+// Payload bytes of chunk t in the input streams q0, q0 + dq, ..., published for everybody; one warp
+__device__ __forceinline__ void publish_inputs(const SoloParams& p, uint32_t nc, uint32_t subs, uint32_t t, uint32_t q0, uint32_t dq) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t a = t * nc, b = a + nc < subs ? a + nc : subs;
+  for (uint32_t q = q0; q < p.n_in; q += dq) {
+    const uint32_t all = __reduce_add_sync(0xffffffffu, payload_len16(rates16(p.in[q], p.in_size[q], a, b, lane)));
+    if (lane == 0) st_relaxed_gpu_u64(p.in_words + (size_t)q * p.first[1] + t, st_pack(kStAgg, p.ws.epoch, all));
+  }
+}
+// Payload offsets of the sub-tiles of chunk t in input stream q (slot r of in_at); one warp.  `next`: chunks before it
+// are in sh.in_run[q]
+__device__ __forceinline__ void input_offsets(const SoloParams& p, EncShared& sh, uint32_t nc, uint32_t subs, uint32_t t,
+                                              uint32_t q, uint32_t r, uint32_t next) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t a = t * nc, b = a + nc < subs ? a + nc : subs;
+  const uint32_t sum = payload_len16(rates16(p.in[q], p.in_size[q], a, b, lane));  // half a sub-tile per lane
+  const uint32_t inc = warp_inclusive_scan(sum, (int)lane);
+  const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
+  uint64_t base = sh.in_run[q];
+  advance_base(p.in_words + (size_t)q * p.first[1], next, base, t, p.ws);
+  if (!(lane & 1u) && (lane >> 1) < nc) sh.in_at[r][q][lane >> 1] = rate_bytes(p.n[0]) + base + inc - sum;
+  __syncwarp();
+  if (lane == 0) {
+    sh.in_run[q] = base + all;
+    mbar_arrive(&sh.in_known[r]);
+  }
+}
+
+// Adds up the chunk totals, places the payloads; keeps the input offsets kInSlots chunks ahead of the compute warps and
+// the published input totals two chunks ahead of that (the first chunk's inputs are the compute warps' work).
+__device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32_t nc, uint32_t subs) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const Workspace& ws = p.ws;
+  constexpr uint32_t kLead = 2;
+  auto inputs_ahead = [&](uint32_t k) {  // offsets of chunk k, totals of chunk k + kLead
+    const uint32_t lead = ticket(p, k + kLead), t = ticket(p, k);
+    if (lead != kNoTile) publish_inputs(p, nc, subs, lead, 0u, 1u);
+    if (t == kNoTile) return;
+    for (uint32_t q = 0; q < p.n_in; ++q) input_offsets(p, sh, nc, subs, t, q, k % kInSlots, ticket(p, k - 1) + 1u);
+  };
+  if (p.n_in) {
+    for (uint32_t k = 1; k <= kLead; ++k)
+      if (ticket(p, k) != kNoTile) publish_inputs(p, nc, subs, ticket(p, k), 0u, 1u);
+    warp_wait(&sh.in_known[0], 0u, ws, kSiteLoaderInFree);  // in_run is the compute warps' until then
+    for (uint32_t k = 1; k < (uint32_t)kInSlots; ++k) inputs_ahead(k);
+  }
+  uint32_t next = 0;  // chunks [first of the segment, next) are in base
+  uint64_t base = 0;
+  uint32_t seg = 0;
+  for (uint32_t k = 0;; ++k) {
+    const uint32_t t = ticket(p, k);
+    if (t == kNoTile) break;
+    const uint32_t r = k % kSlots;
+    totals_wait(k, nc);
+    const uint32_t tot = lane < nc ? sh.tot[r][lane] : 0u;
+    const uint32_t inc = warp_inclusive_scan(tot, (int)lane);
+    const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
+    const Chunk c = chunk_of(p, t);
+    if (c.seg != seg) {  // every segment is a stream of its own
+      seg = c.seg;
+      base = 0;
+      next = p.first[seg];
+    }
+    advance_base(p.out_words, next, base, t, ws);
+    const uint64_t start = rate_bytes(p.n[seg]) + base;
+    const uint64_t at = start + inc - tot;
+    const bool fits = at + tot <= p.out_cap && !fatal_error(ws.ctrl);
+    if (tot && !fits) note_error(ws.ctrl, kErrCapacity);
+    if (lane < nc) sh.out_at[r][lane] = tot && fits ? at : ~0ull;
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(&sh.placed[r]);
+      // the last chunk ends where the stream ends: no size for a stream that did not fit
+      if (p.size_out && t + 1 == p.first[seg + 1] && start + all <= p.out_cap && !fatal_error(ws.ctrl)) p.size_out[seg] = start + all;
+    }
+    base += all;
+    next = t + 1;
+    if (p.n_in) inputs_ahead(k + kInSlots);  // every compute warp has taken the inputs of chunk k out of the slot
+  }
+}
+
+// ---- blocks beyond the reach of the subnormal form ------------------------------------------------------------------
+// Out of line and on copies in local memory: kept inline, the int32 arithmetic of these blocks took registers and
+// instruction cache from the common path (64 MB add: 56 us inline, 52 this way).
+struct Row {
+  uint32_t v[32];
+};
+// the deltas of row `row` of the stage in int32
+template <int MODE>
+__device__ __noinline__ void cold_local(Row* d, const uint8_t* stage, int row, float recip) {
+  uint32_t x[32];
+  load_row_swizzled(stage, row, x);
+  deltas_int<MODE>(x, recip);
+#pragma unroll
+  for (int i = 0; i < 32; ++i) d->v[i] = x[i];
+}
+// d += the deltas of a decoded block (rows as decode_rows leaves them), in int32; `subs`: d_1 .. d_31 still are subnormals
+__device__ __noinline__ void cold_add_block(Row* d, const Row* T, uint32_t sign, bool subs) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const uint32_t m = (uint32_t)((int32_t)(sign << i) >> 31);
+    const uint32_t b = d->v[i];
+    d->v[i] = (subs && i ? sub_to_int(b) : b) + (T->v[i ^ 7] ^ m) - m;
+  }
+}
+__device__ __noinline__ void cold_sign_magnitude(Row* d) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) d->v[i] = sign_magnitude(d->v[i]);
+}
+__device__ __forceinline__ Row row_of(const uint32_t (&d)[32]) {
+  Row r;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) r.v[i] = d[i];
+  return r;
+}
+__device__ __forceinline__ void from_row(uint32_t (&d)[32], const Row& r) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) d[i] = r.v[i];
+}
+
+// ---- the kernel --------------------------------------------------------------------------------------------------
+template <int OP, int MODE>
+__global__ void __launch_bounds__((kEncWarps + 1) * 32, 1)
+hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ SoloParams p) {
+  constexpr bool kHasLocal = OP != kOpAddStream;
+  constexpr bool kHasIn = OP != kOpCompress;
+  constexpr bool kFloat = OP != kOpAddI32;  // the subnormal form may apply
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ EncShared sh;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t nc = (blockDim.x >> 5) - 1u;  // compute warps
+  uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const Workspace& ws = p.ws;
+  const uint32_t Q = kHasIn ? p.n_in : 0u;
+
+  if (tid < nc) {
+    mbar_init(&sh.stage_full[tid], 1);
+    if (kHasIn)
+      for (int i = 0; i < 4; ++i) mbar_init(&sh.in_full[tid][i], 1);
+  } else if (warp == 1u) {
+    if (lane < (uint32_t)kSlots) {
+      mbar_init(&sh.placed[lane], 1);
+      sh.sum[lane] = 0;
+    }
+    if (kHasIn && lane < (uint32_t)kInSlots) mbar_init(&sh.in_known[lane], Q);
+    if (kHasIn && lane < (uint32_t)kMaxIn) sh.in_run[lane] = 0;
+  }
+  fence_mbar_init();
+  if (tid == 0) {
+    launch_dependents();
+    sh.dead = fatal_error(ws.ctrl) ? 1u : 0u;
+  }
+  __syncthreads();
+  if (sh.dead) return;  // (one answer for all warps)
+  const uint32_t subs0 = (uint32_t)((p.n[0] + kSubValues - 1) / kSubValues);
+  if (warp == nc) {
+    clerk(p, sh, nc, subs0);
+    return;
+  }
+
+  // ============================================ compute warps ==========================================================
+  uint8_t* const stage = smem + warp * kSubBytes;
+  uint8_t* const inring = smem + nc * kSubBytes + warp * enc_in_ring(OP);
+  const uint32_t oring = smem_u32(smem + nc * (kSubBytes + enc_in_ring(OP)) + warp * enc_out_ring(OP));
+  constexpr uint32_t kOutBytes = (uint32_t)enc_out_ring(OP);
+  struct Where {
+    uint32_t seg, sub;  // segment, sub-tile inside it
+  };
+  auto where = [&](uint32_t t) -> Where {
+    if (kHasIn) return Where{0u, t * nc + warp};
+    const Chunk c = chunk_of(p, t);
+    return Where{c.seg, c.lc * nc + warp};
+  };
+  auto n_local = [&](uint32_t g) -> uint64_t { return OP == kOpAddI32 ? num_blocks(p.n[g]) * kBlock : p.n[g]; };
+  // whole sub-tiles of an aligned operand come through the TMA unit; the rest is loaded by the warp itself
+  auto by_tma = [&](const Where& w) -> bool { return p.use_tma[w.seg] && (uint64_t)(w.sub + 1) * kSubValues <= n_local(w.seg); };
+  auto fetch_stage = [&](uint32_t t) {
+    if (!kHasLocal || t == kNoTile) return;
+    const Where w = where(t);
+    if (lane == 0) {
+      if (by_tma(w)) {
+        fence_proxy_async();
+        mbar_expect_tx(&sh.stage_full[warp], kSubBytes);
+        tma_load_2d(stage, &tmaps.m[w.seg], 0, (int)(w.sub * kSubBlocks), &sh.stage_full[warp]);
+      } else {
+        mbar_arrive(&sh.stage_full[warp]);
+      }
+    }
+  };
+
+  // ---- incoming payloads: jobs (chunk k, stream q) --------------------------------------------------------------------
+  uint32_t pk = 0, pq = 0, pt = kNoTile;  // next job to be staged
+  uint32_t praw = 0;                      // rate byte of the lane's block in it
+  uint32_t live_at = 0, live_end = 0, jobs = 0, staged = 0;
+  uint32_t cur_rate = 0, cur_pos = 0, nxt_rate = 0, nxt_pos = 0;
+  auto load_rate = [&]() {
+    const uint64_t b = ((uint64_t)pt * nc + warp) * kSubBlocks + lane;
+    praw = pt != kNoTile && b < (uint64_t)subs0 * kSubBlocks && b < p.in_size[pq] ? ld_cg_u8(p.in[pq] + b) : 0u;
+  };
+  // stages the next job unless the ring has no room for it
+  auto produce = [&]() {
+    if (pq == 0 && !warp_wait(&sh.in_known[pk % kInSlots], (pk / kInSlots) & 1u, ws, kSiteLoaderInFree)) {
+      pt = kNoTile;
+      return;
+    }
+    const uint32_t len = payload_len(praw);
+    const uint32_t inc = warp_inclusive_scan(len, (int)lane);
+    uint32_t tot = __shfl_sync(0xffffffffu, inc, 31), rate = praw;
+    uint32_t at = staged ? live_end : 0u;
+    if (tot && at + tot + 31u > (uint32_t)kInUsable) {
+      at = 0;
+      if (tot + 31u > (staged ? live_at : (uint32_t)kInUsable)) return;
+    }
+    const uint64_t off = sh.in_at[pk % kInSlots][pq][warp];
+    if (tot && off + tot > p.in_size[pq]) {  // stream shorter than its rate bytes imply
+      if (lane == 0) note_error(ws.ctrl, kErrTruncated);
+      tot = 0;
+      rate = 0;
+    }
+    const uint8_t* const src = p.in[pq] + off;
+    const uint32_t phase = (uint32_t)reinterpret_cast<uintptr_t>(src) & 15u;
+    const uint32_t bytes = tot ? (phase + tot + 15u) & ~15u : 0u;
+    live_at = at;
+    live_end = at + bytes;
+    uint64_t* const bar = &sh.in_full[warp][jobs & 3u];
+    if (lane == 0) {
+      if (tot) {
+        fence_proxy_async();
+        mbar_expect_tx(bar, bytes);
+        bulk_load(inring + at, src - phase, bytes, bar);
+      } else {
+        mbar_arrive(bar);
+      }
+    }
+    ++jobs;
+    const uint32_t pos = at + phase + inc - len;
+    if (staged) nxt_rate = rate, nxt_pos = pos;
+    else cur_rate = rate, cur_pos = pos;
+    ++staged;
+    if (++pq == Q) {
+      pq = 0;
+      ++pk;
+      pt = ticket(p, pk);
+    }
+    load_rate();
+  };
+
+  uint32_t t = ticket(p, 0);
+  fetch_stage(t);
+  if (kHasIn) {
+    pt = t;
+    load_rate();
+    if (t != kNoTile) {
+      publish_inputs(p, nc, subs0, t, warp, nc);
+      for (uint32_t q = warp; q < Q; q += nc) input_offsets(p, sh, nc, subs0, t, q, 0u, 0u);
+    }
+  }
+
+  // ---- packed payloads waiting for their place: lane k % kSlots keeps those of chunk k --------------------------------
+  uint32_t my_start = 0, my_tot = 0, my_seg = 0;
+  // ring: free is [head, end) and [0, tail), or, once wrapped (head < tail), [head, tail); all of it when taken == 0
+  uint32_t head = 0, tail = 0, taken = 0;
+  uint32_t copied = 0;  // chunks [copied, k) wait
+  auto room_for = [&](uint32_t tot) -> uint32_t { return tot ? (tot + 20u + 15u) & ~15u : 0u; };
+  auto copy_oldest = [&]() {
+    const uint32_t r = copied % kSlots;
+    const uint32_t start = __shfl_sync(0xffffffffu, my_start, (int)r), tot = __shfl_sync(0xffffffffu, my_tot, (int)r);
+    const uint64_t at = sh.out_at[r][warp];
+    if (tot) {
+      if (at != ~0ull) copy_ring(oring + start, p.out[__shfl_sync(0xffffffffu, my_seg, (int)r)] + at, tot);
+      tail = start + room_for(tot);
+      if (--taken == 0) head = tail = 0;
+    }
+    ++copied;
+  };
+  auto placed = [&](uint32_t k) -> bool { return __all_sync(0xffffffffu, mbar_test(&sh.placed[k % kSlots], (k / kSlots) & 1u)); };
+
+  bool failed = false;  // a wait ran out (recorded)
+  for (uint32_t k = 0;; ++k) {
+    if (t == kNoTile) {
+      for (; copied < k && !failed;) {
+        if (!warp_wait(&sh.placed[copied % kSlots], (copied / kSlots) & 1u, ws, kSiteCopierBase)) break;
+        copy_oldest();
+      }
+      break;
+    }
+    if (failed) {  // nothing more from this warp, but the clerk counts on it
+      totals_arrive(k, nc);
+      t = ticket(p, k + 1);
+      continue;
+    }
+    const Where w = where(t);
+    const uint32_t t_next = ticket(p, k + 1);
+    uint32_t d[32];
+    bool ints = !kFloat;  // d holds int32 deltas instead of subnormals (d[0] is an int32 with inputs in any case)
+    uint32_t or_tail = 0;
+    // ---- local operand: first, because it needs nothing but its rows --------------------------------------------------
+    if (kHasLocal) {
+      if (!warp_wait(&sh.stage_full[warp], k & 1u, ws, kSiteComputeTile)) failed = true;
+      if (!by_tma(w)) {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(p.local[w.seg]);
+        const uint64_t first = (uint64_t)w.sub * kSubValues, n = n_local(w.seg);
+#pragma unroll 4
+        for (int r = 0; r < kSubBlocks; ++r) {
+          const uint64_t i = first + r * kBlock + lane;
+          sts32((swizzled_row(stage, r) ^ ((lane >> 2) << 4)) | ((lane & 3u) << 2), i < n ? __ldg(src + i) : 0u);
+        }
+        __syncwarp();
+      }
+      load_row_swizzled(stage, (int)lane, d);
+      if (kFloat) {
+        deltas_sub<MODE>(d, p.recip);
+        // exact when no quantised value of the block reaches 2^24: |q_0| below 2^23 and 31 differences below 2^18
+        or_tail = or_tail_of(d);
+        if (!__all_sync(0xffffffffu, or_tail < (1u << 18) && (d[0] & 0x7fffffffu) < (1u << 23))) {
+          Row c;
+          cold_local<MODE>(&c, stage, (int)lane, p.recip);
+          if (!kHasIn) {
+            cold_sign_magnitude(&c);
+            from_row(d, c);
+            or_tail = or_tail_of(d);
+          } else {
+            from_row(d, c);
+            ints = true;
+          }
+        } else if (kHasIn) {
+          d[0] = sub_to_int(d[0]);
+        }
+      }
+      __syncwarp();
+      fetch_stage(t_next);  // every lane holds its row
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) d[i] = 0;
+    }
+    // ---- incoming streams ----------------------------------------------------------------------------------------------
+    if (kHasIn) {
+      for (uint32_t q = 0; q < Q; ++q) {
+        while (staged < 2u && pt != kNoTile) {
+          const uint32_t before = staged;
+          produce();
+          if (staged == before) break;
+        }
+        const uint32_t v = k * Q + q;
+        if (!warp_wait(&sh.in_full[warp][v & 3u], (v >> 2) & 1u, ws, kSiteComputeInFull)) cur_rate = 0, failed = true;
+        uint32_t T[32], sign, a0;
+        decode_rows(inring, cur_pos, cur_rate, plane_width(__reduce_max_sync(0xffffffffu, cur_rate & 31u)), sign, a0, T);
+        __syncwarp();
+        // |d_1| .. |d_31| small enough for sums of eight such streams: so with up to 16 planes, else to be looked at (a
+        // plain block may have many planes for the sake of d_0 alone, which is summed in int32)
+        bool fits = (cur_rate & 31u) <= 16u;
+        if (kFloat && !__all_sync(0xffffffffu, fits)) fits = fits || or_rows_tail(T) < (1u << 20);
+        cur_rate = nxt_rate;
+        cur_pos = nxt_pos;
+        --staged;
+        if (!kFloat) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const uint32_t m = (uint32_t)((int32_t)(sign << i) >> 31);
+            d[i] += (T[i ^ 7] ^ m) - m;
+          }
+        } else if (__all_sync(0xffffffffu, fits) && !ints) {
+          const uint32_t m = (uint32_t)((int32_t)sign >> 31);
+          d[0] += (T[7] ^ m) - m;
+#pragma unroll
+          for (int i = 1; i < 32; ++i) d[i] = as_u(__fadd_rn(as_f(d[i]), signed_sub(T[i ^ 7], sign, i)));
+        } else {
+          Row c = row_of(d);
+          const Row tr = row_of(T);
+          cold_add_block(&c, &tr, sign, !ints);
+          from_row(d, c);
+          ints = true;
+        }
+      }
+      if (!kFloat) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
+      } else if (ints) {
+        Row c = row_of(d);
+        cold_sign_magnitude(&c);
+        from_row(d, c);
+      } else {
+        d[0] = sign_magnitude(d[0]);
+      }
+      or_tail = or_tail_of(d);
+    }
+
+    // ---- encode -----------------------------------------------------------------------------------------------------------
+    const BlockCode code = code_of<MODE>(d, or_tail);
+    const uint32_t inc = warp_inclusive_scan(code.len, (int)lane);
+    const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
+    if (lane == 0) {
+      const uint32_t r = k % kSlots;
+      sh.tot[r][warp] = tot;
+      // the last warp publishes the chunk's total, not the clerk: other CTAs wait for it, whatever this one's clerk
+      // is waiting for (published by the clerks, the totals moved on in lock step, 4 us a chunk)
+      const uint32_t before = atomicAdd(&sh.sum[r], (1u << 24) | tot);
+      if (before >> 24 == nc - 1u) {
+        st_relaxed_gpu_u64(p.out_words + t, st_pack(kStAgg, ws.epoch, (before & 0xffffffu) + tot));
+        sh.sum[r] = 0;
+      }
+    }
+    __syncwarp();
+    totals_arrive(k, nc);
+    const uint32_t subs = (uint32_t)((p.n[w.seg] + kSubValues - 1) / kSubValues);
+    uint8_t* const rates = p.out[w.seg];
+    if (w.sub < subs) rates[(uint64_t)w.sub * kSubBlocks + lane] = (uint8_t)code.rate;
+    if (w.sub + 1 == subs)  // section A covers whole chunks of 32768 values
+      for (uint64_t b = (uint64_t)subs * kSubBlocks + lane; b < rate_bytes(p.n[w.seg]); b += 32u) rates[b] = 0;
+
+    // payloads whose place is known leave; the oldest ones have to where this one needs their room
+    while (copied < k && placed(copied)) copy_oldest();
+    const uint32_t need = room_for(tot);
+    uint32_t start = head;
+    while (true) {
+      bool room = true;
+      start = head;
+      if (need && taken) {
+        if (head >= tail && head + need > kOutBytes) {
+          start = 0;
+          room = need < tail;
+        } else if (head < tail) {
+          room = head + need < tail;
+        }
+      }
+      if (room && k - copied < (uint32_t)kSlots - 1u) break;
+      if (!warp_wait(&sh.placed[copied % kSlots], (copied / kSlots) & 1u, ws, kSiteComputeRing)) {
+        failed = true;
+        break;
+      }
+      copy_oldest();
+    }
+    t = t_next;
+    if (failed) continue;
+    __syncwarp();
+    pack_blocks(oring + start, inc - code.len, code, d, plane_width(__reduce_max_sync(0xffffffffu, code.rate & 31u)));
+    if (lane == k % kSlots) {
+      my_start = start;
+      my_tot = tot;
+      my_seg = w.seg;
+    }
+    if (need) {
+      head = start + need;
+      ++taken;
+    }
+  }
+}
+
+}  // namespace dev
+
+// ---- host side ---------------------------------------------------------------------------------------------------
+
+namespace {
+
+template <int OP, int MODE>
+cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t stream) {
+  constexpr int kWarps = dev::kEncWarps;
+  auto smem = [](int nc) { return nc * dev::enc_warp_bytes(OP) + 1024; };
+  static thread_local int cache[64] = {};
+  const int cap = resident_ctas(dev::hc_encode_solo_kernel<OP, MODE>, 32 * (kWarps + 1), smem(kWarps), cache);
+  if (cap <= 0) return cudaErrorLaunchOutOfResources;
+  const uint64_t sms = (uint64_t)(cap < dev::kMaxCtas ? cap : dev::kMaxCtas);
+  // Compute warps per CTA: as many rounds of chunks as the largest CTA needs, then no more warps than fill them (where
+  // the last round would be half empty, all rounds are narrower instead); at least four at a time.
+  uint64_t subs = 0;
+  for (uint32_t g = 0; g < p.n_seg; ++g) subs += (p.n[g] + dev::kSubValues - 1) / dev::kSubValues;
+  const uint64_t rounds = (subs + sms * kWarps - 1) / (sms * kWarps);
+  uint64_t nc = (subs + sms * rounds - 1) / (sms * rounds);
+  if (nc < 4) nc = 4;
+  p.first[0] = 0;
+  for (uint32_t g = 0; g < p.n_seg; ++g)
+    p.first[g + 1] = p.first[g] + (uint32_t)(((p.n[g] + dev::kSubValues - 1) / dev::kSubValues + nc - 1) / nc);
+  const uint32_t chunks = p.first[p.n_seg];
+  const int grid = (int)(chunks < sms ? chunks : sms);
+  p.out_words = p.ws.st_a;
+  p.in_words = p.ws.st_a + chunks;
+  dev::hc_encode_solo_kernel<OP, MODE><<<grid, 32 * ((int)nc + 1), smem((int)nc), stream>>>(maps, p);
+  return cudaGetLastError();
+}
+
+template <int OP>
+cudaError_t launch_solo_m(int mode, const TensorMaps& maps, const SoloParams& p, cudaStream_t stream) {
+  switch (mode) {
+    case kModeOutlier: return launch_solo_t<OP, kModeOutlier>(maps, p, stream);
+    case kModePlain: return launch_solo_t<OP, kModePlain>(maps, p, stream);
+    case kModeVec: return launch_solo_t<OP, kModeVec>(maps, p, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_encode_solo(int op, int mode, SoloParams p, cudaStream_t stream) {
+  if (p.n_seg == 0 || p.n_seg > (uint32_t)kMaxDst || p.n_in > (uint32_t)kMaxIn) return cudaErrorInvalidValue;
+  if ((p.n_seg > 1 && op != kOpCompress) || (op == kOpCompress) != (p.n_in == 0)) return cudaErrorInvalidValue;
+  TensorMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  uint64_t total = 0;
+  for (uint32_t g = 0; g < p.n_seg; ++g) {
+    total += p.n[g];
+    p.use_tma[g] = 0;
+    if (op != kOpAddStream && p.n[g])  // int32 deltas are stored in whole blocks; fp32 data may end in a ragged row
+      p.use_tma[g] = make_rows_map(&maps.m[g], p.local[g], op == kOpAddI32 ? num_blocks(p.n[g]) : p.n[g] / kBlock, dev::kSubBlocks) ? 1u : 0u;
+  }
+  if (total == 0) return cudaSuccess;
+  switch (op) {
+    case kOpCompress: return launch_solo_m<kOpCompress>(mode, maps, p, stream);
+    case kOpAddF32: return launch_solo_m<kOpAddF32>(mode, maps, p, stream);
+    case kOpAddI32: return launch_solo_m<kOpAddI32>(mode, maps, p, stream);
+    case kOpAddStream: return launch_solo_m<kOpAddStream>(mode, maps, p, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace hc

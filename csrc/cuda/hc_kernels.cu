@@ -574,7 +574,7 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
       // ---- encode ----------------------------------------------------------------------------------
       if (tid == 0) HC_PH(3);
       uint32_t A[32];
-      BlockCode code = analyse_block<MODE>(d, A);
+      TileCode code = analyse_block<MODE>(d, A);
       uint32_t tot;
       if (tid == 0) {
         HC_PH(4);

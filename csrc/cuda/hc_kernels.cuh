@@ -98,6 +98,26 @@ struct EncParams {
   Workspace ws;
 };
 
+// A stand-alone stream-producing launch (hc_encode.cu): either n_seg independent compressions, or one segment with up
+// to kMaxIn input streams summed into it.
+struct SoloParams {
+  const void* local[kMaxDst];  // fp32 values or int32 deltas, per segment
+  uint64_t n[kMaxDst];         // values per segment
+  uint8_t* out[kMaxDst];
+  uint32_t use_tma[kMaxDst];
+  uint32_t first[kMaxDst + 1];  // chunk numbers at which the segments start; [n_seg]: number of chunks (set by the launcher)
+  uint32_t n_seg;
+  uint32_t n_in;
+  float recip;  // 0.5f / eb
+  const uint8_t* in[kMaxIn];
+  uint64_t in_size[kMaxIn];
+  uint64_t out_cap;
+  uint64_t* size_out;   // device words receiving the exact stream length of each segment (or null)
+  uint64_t* out_words;  // one word per chunk: its payload bytes (set by the launcher)
+  uint64_t* in_words;   // n_in rows of such words
+  Workspace ws;
+};
+
 // One decode launch can take several independent streams ("segments"): the all-gather phase of a
 // collective decodes the P reduced chunks with one kernel.  Every segment owns tiles_per_seg
 // consecutive tile tickets and its own look-back chain.
@@ -162,7 +182,7 @@ __device__ __forceinline__ void lorenzo_inverse(int32_t (&d)[32]) {
   for (int i = S; i < 32; ++i) d[i] += d[i - S];
 }
 
-struct BlockCode {
+struct TileCode {
   uint32_t rate;      // rate byte
   uint32_t len;       // payload bytes
   uint32_t a0;        // |d0| when outlier mode
@@ -171,7 +191,7 @@ struct BlockCode {
 
 // signed deltas -> rows A[j] = |d[j ^ 7]| plus the block's code
 template <int MODE>
-__device__ __forceinline__ BlockCode analyse_block(const int32_t (&d)[32], uint32_t (&A)[32]) {
+__device__ __forceinline__ TileCode analyse_block(const int32_t (&d)[32], uint32_t (&A)[32]) {
   uint32_t sign = 0, or_tail = 0;
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
@@ -191,7 +211,7 @@ __device__ __forceinline__ BlockCode analyse_block(const int32_t (&d)[32], uint3
     }
     or_all = or_tail | A[7];
   }
-  BlockCode c;
+  TileCode c;
   c.a0 = A[7];
   c.rate = choose_rate(or_all, or_tail, c.a0, MODE != kModePlain);
   c.len = payload_len(c.rate);
@@ -214,7 +234,7 @@ __device__ __forceinline__ void transpose_forward(uint32_t (&A)[32], int W) {
 // Writes the block's payload at byte `pos` of the staging buffer.  T[0..W-1] hold the planes
 // (planes at and above F are zero because every magnitude is below 2^F).
 template <int W>
-__device__ __forceinline__ void write_payload_w(uint8_t* obuf, uint32_t pos, const BlockCode& c, const uint32_t (&T)[32]) {
+__device__ __forceinline__ void write_payload_w(uint8_t* obuf, uint32_t pos, const TileCode& c, const uint32_t (&T)[32]) {
   const uint32_t F = c.rate & 31u;
   const bool outl = (c.rate & 0x80u) != 0;
   if (!outl && F == 0) return;
@@ -255,7 +275,7 @@ __device__ __forceinline__ void write_payload_w(uint8_t* obuf, uint32_t pos, con
       if (b < s) tb[b] = (uint8_t)(tail >> (8 * b));
   }
 }
-__device__ __forceinline__ void write_payload(uint8_t* obuf, uint32_t pos, const BlockCode& c, const uint32_t (&T)[32],
+__device__ __forceinline__ void write_payload(uint8_t* obuf, uint32_t pos, const TileCode& c, const uint32_t (&T)[32],
                                               int W) {
   switch (W) {
     case 0: {  // only "outlier with F = 0" blocks carry bytes here

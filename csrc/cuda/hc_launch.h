@@ -23,6 +23,8 @@ int device_sm_count();
 // kernel on the stream is running, and fills the SMs as that kernel's CTAs leave.  Only for launches
 // whose inputs are ordered by arrival flags, with a workspace view of their own set.
 cudaError_t launch_encode(int op, int mode, EncParams p, cudaStream_t stream, bool overlap = false);
+// Stand-alone compression of n_seg arrays, or sum of n_in streams and a local operand (hc_encode.cu).
+cudaError_t launch_encode_solo(int op, int mode, SoloParams p, cudaStream_t stream);
 cudaError_t launch_decode(int mode, DecParams p, cudaStream_t stream, bool overlap = false);
 // Per-tile payload offsets of stand-alone input streams as arrival flags (see OffsetParams);
 // offsets_fit says whether the workspace of a handle sized for max_elems has room for the flags of

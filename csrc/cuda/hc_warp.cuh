@@ -6,6 +6,10 @@ namespace hc {
 namespace dev {
 
 constexpr uint32_t kNoTile = 0xffffffffu;
+// sub-tile: 32 consecutive blocks, one per lane; what a warp works on at a time
+constexpr int kSubBlocks = 32;
+constexpr int kSubValues = kSubBlocks * kBlock;
+constexpr int kSubBytes = kSubValues * 4;  // 4096
 
 __device__ __forceinline__ void note_error(uint32_t* ctrl, uint32_t code) { atomicMax(ctrl + 2, code); }
 // timeouts and peer failures end the launch early; capacity / truncation errors only skip data
@@ -78,6 +82,22 @@ __device__ __forceinline__ uint32_t load_rates4(const uint8_t* in, uint64_t in_s
   for (int k = 0; k < 4; ++k)
     if (b + k < in_size) r |= ld_cg_u8(in + b + k) << (8 * k);
   return r;
+}
+
+// rate bytes [16 l, 16 l + 16) of the sub-tiles [a, b) of a stream; 0 past b and past the end of the stream
+__device__ __forceinline__ uint4 rates16(const uint8_t* in, uint64_t in_size, uint32_t a, uint32_t b, uint32_t l) {
+  const uint64_t at = (uint64_t)a * kSubBlocks + 16u * l;
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (at >= (uint64_t)b * kSubBlocks) return v;
+  if ((reinterpret_cast<uintptr_t>(in) & 15u) == 0 && at + 16u <= in_size) return ld_cg_u4(in + at);
+  v.x = load_rates4(in, in_size, at);
+  v.y = load_rates4(in, in_size, at + 4u);
+  v.z = load_rates4(in, in_size, at + 8u);
+  v.w = load_rates4(in, in_size, at + 12u);
+  return v;
+}
+__device__ __forceinline__ uint32_t payload_len16(const uint4& v) {
+  return payload_len4(v.x) + payload_len4(v.y) + payload_len4(v.z) + payload_len4(v.w);
 }
 
 constexpr int kMaxCtas = 160;  // CTAs of a launch with one CTA per SM
