@@ -452,7 +452,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
     p.variant = (uint32_t)c->reduce_variant;
     p.sparse = c->sparse ? 1u : 0u;
     p.ws = next_ws(c, stream);
-    if (hc::launch_encode(P > 1 ? hc::kOpAddF32 : hc::kOpCompress, hc::kModeOutlier, p, stream, overlap && launched) !=
+    if (hc::launch_encode(hc::kOpAddF32, hc::kModeOutlier, p, stream, overlap && launched) !=
         cudaSuccess)
       return hc::kErrCuda;
     launched = true;
@@ -478,6 +478,50 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
   }
   d.ws = next_ws(c, stream);
   if (hc::launch_decode(hc::kModeOutlier, d, stream, overlap && launched) != cudaSuccess) return hc::kErrCuda;
+  mark();
+  return hc::kOk;
+}
+
+// A communicator of one rank: the message is compressed and decoded by the stand-alone kernels, one after the other
+// (64 MB: 42 us, against 62 us with the kernels of the collective steps, whose tiles sit at fixed offsets behind
+// arrival flags so that other ranks can follow).
+static int allreduce_single(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t count, float eb, hc_stream_t stream) {
+  const Layout& L = c->lay;
+  c->call += 1;
+  if ((c->call & 0xffffffu) == 0) c->call += 1;
+  uint8_t* const slot = c->peer[0] + L.data_off(L.ag_slot((int)(c->call & 1u), 0));
+  c->n_ev = 0;
+  auto mark = [&]() {
+    if (c->trace) cudaEventRecord(c->ev[c->n_ev++], stream);
+  };
+  mark();
+  if (c->algorithm != 0) mark();  // the direct form's scatter step, which has nothing to do
+  {
+    NvtxRange step_range("hc single: compress");
+    hc::SoloParams p;
+    memset(&p, 0, sizeof(p));
+    p.n_seg = 1;
+    p.local[0] = d_sbuf;
+    p.n[0] = count;
+    p.recip = 0.5f / eb;
+    p.out[0] = slot;
+    p.out_cap = L.slot_bytes;
+    p.size_out = c->sizes;
+    p.ws = next_ws(c, stream);
+    if (hc::launch_encode_solo(hc::kOpCompress, hc::kModeOutlier, p, stream) != cudaSuccess) return hc::kErrCuda;
+  }
+  mark();
+  NvtxRange decode_range("hc single: decode");
+  hc::DecParams d;
+  memset(&d, 0, sizeof(d));
+  d.eb = eb;
+  d.n_seg = 1;
+  d.seg[0].in = slot;
+  d.seg[0].in_size = L.slot_bytes;
+  d.seg[0].out = d_rbuf;
+  d.seg[0].n = count;
+  d.ws = next_ws(c, stream);
+  if (hc::launch_decode(hc::kModeOutlier, d, stream) != cudaSuccess) return hc::kErrCuda;
   mark();
   return hc::kOk;
 }
@@ -633,6 +677,7 @@ extern "C" int hc_allreduce(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
   if (count == 0) return hc::kOk;
   NvtxRange call_range("hc_allreduce");
   c->last_form = c->algorithm == 0 ? 0 : 1;
+  if (c->world == 1) return allreduce_single(c, d_sbuf, d_rbuf, count, eb, stream);
   if (c->algorithm == 0) return allreduce_ring(c, d_sbuf, d_rbuf, count, eb, stream);
   // one step for every message that fits (algorithm 2), or for those up to the small-message limit
   if (c->world > 1 && count <= onestep_capacity(c) && (c->algorithm == 2 || count <= c->small_count)) {
