@@ -12,6 +12,7 @@ import torch
 import torch.distributed as dist
 
 from .. import _lib
+from ..ops.codec import _current_device, _raw_stream
 
 
 class CompressedAllreduce:
@@ -43,6 +44,7 @@ class CompressedAllreduce:
         self.rank = dist.get_rank(group)
         self.world = dist.get_world_size(group)
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+        self._index = torch.cuda.current_device() if self.device.index is None else self.device.index
         self.max_count = int(max_count)
         self.lib = _lib.cuda()
         self._peers = {}
@@ -118,6 +120,16 @@ class CompressedAllreduce:
             torch.cuda.synchronize()
         dist.barrier(group=group)  # every region is zeroed and mapped before the first store
 
+    def _call(self, what, fn, *args):
+        """``fn(*args, stream)`` with this handle's device current (see ``ops.codec``)."""
+        if _current_device() == self._index:
+            st = fn(*args, _raw_stream(self._index))
+        else:
+            with torch.cuda.device(self.device):
+                st = fn(*args, _raw_stream(self._index))
+        if st:
+            _lib.check(st, what)
+
     def allreduce(self, send: torch.Tensor, recv: torch.Tensor | None = None, eb: float = 1e-4) -> torch.Tensor:
         if send.dtype != torch.float32 or not send.is_cuda or not send.is_contiguous():
             raise ValueError("expected a contiguous float32 CUDA tensor")
@@ -127,9 +139,7 @@ class CompressedAllreduce:
         if n > self.max_count or recv.numel() != n or recv.dtype != torch.float32 or not recv.is_cuda \
                 or not recv.is_contiguous():
             raise ValueError("recv must be a contiguous float32 CUDA tensor of send's size, at most max_count values")
-        with torch.cuda.device(self.device):
-            _lib.check(self.lib.hc_allreduce(self._h, send.data_ptr(), recv.data_ptr(), n, eb,
-                                             torch.cuda.current_stream().cuda_stream), "allreduce")
+        self._call("allreduce", self.lib.hc_allreduce, self._h, send.data_ptr(), recv.data_ptr(), n, eb)
         self._last = (n, eb)
         return recv
 
@@ -147,9 +157,8 @@ class CompressedAllreduce:
         if n > self.max_count or recv.numel() != n or recv.dtype != torch.float32 or recv.is_cuda \
                 or not recv.is_contiguous():
             raise ValueError("recv must be a contiguous float32 host tensor of send's size, at most max_count values")
-        with torch.cuda.device(self.device):
-            _lib.check(self.lib.hc_allreduce_host(self._h, send.data_ptr(), recv.data_ptr(), n, eb, int(pieces),
-                                                  torch.cuda.current_stream().cuda_stream), "allreduce_host")
+        self._call("allreduce_host", self.lib.hc_allreduce_host, self._h, send.data_ptr(), recv.data_ptr(), n, eb,
+                   int(pieces))
         self._last = (min(n, -(-n // max(1, pieces))), eb)
         return recv
 
@@ -161,9 +170,7 @@ class CompressedAllreduce:
             recv = send
         if recv.numel() != send.numel() or recv.dtype != torch.float32 or not recv.is_cuda or not recv.is_contiguous():
             raise ValueError("recv must be a contiguous float32 CUDA tensor of send's size")
-        with torch.cuda.device(self.device):
-            _lib.check(self.lib.hc_allreduce_raw(self._h, send.data_ptr(), recv.data_ptr(), send.numel(),
-                                                 torch.cuda.current_stream().cuda_stream), "allreduce_raw")
+        self._call("allreduce_raw", self.lib.hc_allreduce_raw, self._h, send.data_ptr(), recv.data_ptr(), send.numel())
         return recv
 
     def status(self, clear: bool = True) -> int:
