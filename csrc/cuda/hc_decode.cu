@@ -52,6 +52,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   if (lane < 4u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
+  if (RUNS) grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   __syncwarp();
 
   const uint32_t Q = SUM ? p.n_seg : 1u;  // streams per sub-tile
@@ -476,7 +477,7 @@ cudaError_t launch_t(const TensorMaps& maps, DecParams p, cudaStream_t stream, b
     if (p.grid_limit && (int)p.grid_limit < grid) grid = (int)p.grid_limit;
   }
   const int block = 32 * (int)warps, smem = dec_smem((int)warps);
-  if (overlap) return launch_overlapped(dev::hc_decode_kernel<MODE, SUM, RUNS>, grid, block, smem, stream, maps, p);
+  if (overlap || RUNS) return launch_overlapped(dev::hc_decode_kernel<MODE, SUM, RUNS>, grid, block, smem, stream, maps, p);
   dev::hc_decode_kernel<MODE, SUM, RUNS><<<grid, block, smem, stream>>>(maps, p);
   return cudaGetLastError();
 }

@@ -165,6 +165,9 @@ __device__ __forceinline__ void multimem_st_f32(void* mc_addr, float v) {
 // programmatic dependent launch: lets the runtime schedule the next kernel of the stream (if it was
 // launched with programmatic serialisation) once every CTA of this grid has got here or has left
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// waits until the kernels this one was launched behind with programmatic serialisation have completed and their
+// memory is visible (at once in an ordinary launch)
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void fence_acq_rel_sys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
 __device__ __forceinline__ uint4 ld_cg_u4(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ uint32_t ld_cg_u8(const uint8_t* p) { return (uint32_t)__ldcg(p); }

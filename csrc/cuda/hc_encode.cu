@@ -233,8 +233,9 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     if (kHasIn && lane < (uint32_t)kMaxIn) sh.in_run[lane] = 0;
   }
   fence_mbar_init();
+  if (tid == 0) launch_dependents();
+  grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   if (tid == 0) {
-    launch_dependents();
     sh.dead = fatal_error(ws.ctrl) ? 1u : 0u;
   }
   __syncthreads();
@@ -561,8 +562,7 @@ cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t str
   const int grid = (int)(chunks < sms ? chunks : sms);
   p.out_words = p.ws.st_a;
   p.in_words = p.ws.st_a + chunks;
-  dev::hc_encode_solo_kernel<OP, MODE><<<grid, 32 * ((int)nc + 1), smem((int)nc), stream>>>(maps, p);
-  return cudaGetLastError();
+  return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE>, grid, 32 * ((int)nc + 1), smem((int)nc), stream, maps, p);
 }
 
 template <int OP>

@@ -59,7 +59,10 @@ cudaError_t set_smem(K kernel, int bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-// launch with programmatic stream serialisation (see launch_encode in hc_launch.h)
+// Launch with programmatic stream serialisation: the kernel may start while the one before it drains.  The steps of a
+// collective order their data by arrival flags; every other kernel launched this way executes griddepcontrol.wait
+// before it touches global memory, and only its launch and set-up overlap (a 4 KB compress back to back: 6.1 us a call
+// without).
 template <typename... Params, typename... Args>
 cudaError_t launch_overlapped(void (*kernel)(Params...), int grid, int block, int smem, cudaStream_t stream,
                               const Args&... args) {
