@@ -697,9 +697,12 @@ extern "C" int hc_allreduce_host(hc_comm* c, const float* h_sbuf, float* h_rbuf,
                                  hc_stream_t stream) {
   if (!c || !h_sbuf || !h_rbuf || !(eb > 0.0f) || count > c->max_count) return hc::kErrArgument;
   if (count == 0) return hc::kOk;
-  if (pieces < 1) {  // default: pieces of 4 MiB, at most 16 (fill and drain of the pipeline cost one piece each)
-    const size_t want = count / ((size_t)1 << 20);
-    pieces = want < 1 ? 1 : (want > 16 ? 16 : (int)want);
+  if (pieces < 1) {
+    // Filling and draining the pipeline costs one piece, and every piece costs about 25 us of its own (two copies that
+    // start and end while the other direction is busy, the events between the streams), so the best number grows
+    // with the square root of the message: 64 MB on one GPU 1731 us in 6 pieces, 1762 in 4, 1908 in 16.
+    const size_t unit = 400000;
+    for (pieces = 1; pieces < 16 && (size_t)(pieces + 1) * (size_t)(pieces + 1) * unit <= count + (size_t)pieces * unit; ++pieces) {}
   }
   if (pieces > kMaxHostPieces) pieces = kMaxHostPieces;
   if (!c->host_in) {  // first use: staging buffers, streams and events (set-up, not the call path)

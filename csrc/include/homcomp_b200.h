@@ -143,7 +143,7 @@ int hc_comm_status_site(hc_comm* c);        // after a time-out: the wait that r
 // synchronises.
 int hc_allreduce(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t count, float eb, hc_stream_t stream);
 // The same sum for buffers in (pinned) host memory: the message crosses PCIe in `pieces` pieces
-// (0 = default: pieces of 4 MiB, at most 16; never more than 32) on two copy streams of the handle while earlier pieces are reduced on
+// (0 = default: 1 to 16, growing with the square root of the message; never more than 32) on two copy streams of the handle while earlier pieces are reduced on
 // `stream` and still earlier ones travel back, so the call costs about one direction of the
 // transfer.  `stream` ends behind the last copy down.  The first call allocates the device staging
 // (2 x max_count floats).  Pageable host memory works but serialises the copies.

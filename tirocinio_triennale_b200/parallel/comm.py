@@ -146,7 +146,7 @@ class CompressedAllreduce:
     def allreduce_host(self, send: torch.Tensor, recv: torch.Tensor | None = None, eb: float = 1e-4,
                        pieces: int = 0) -> torch.Tensor:
         """The same sum for float32 tensors in host memory (pin them: ``.pin_memory()``).  The message
-        crosses PCIe in ``pieces`` pieces (0: pieces of 4 MiB, at most 16) while earlier pieces are being reduced and still earlier ones
+        crosses PCIe in ``pieces`` pieces (0: 1 to 16, growing with the square root of the message) while earlier pieces are being reduced and still earlier ones
         travel back, so a call costs about one direction of the transfer.  Asynchronous: the result is
         on the host once the current CUDA stream has been synchronised."""
         if send.dtype != torch.float32 or send.is_cuda or not send.is_contiguous():
