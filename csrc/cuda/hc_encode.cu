@@ -22,11 +22,12 @@ namespace dev {
 constexpr int kSlots = 8;    // chunks of a CTA between "total known" and "payload copied out"
 constexpr int kInSlots = 4;  // chunks whose input offsets are known
 
-// compute warps of a CTA at most: 16 warps with the clerk, 128 registers each (19 + 1 at 96 registers spilled: 84 us
-// against 77 at 256 MB)
-constexpr int kEncWarps = 15;
+// Compute warps of a CTA at most.  Compress: 24 warps with the clerk, 80 registers each (256 MB: 63 us; 68 with 20
+// warps at 96 registers, 73 with 16 at 128).  Adds: 16 warps, which is what the shared memory holds.
+constexpr int kEncWarps = 23;
+__host__ __device__ constexpr int enc_warps(int op) { return op == kOpCompress ? kEncWarps : 15; }
 // packed payloads: a payload of 4096 bytes, 4 bytes pack_block adds, 16 copy_ring looks ahead
-__host__ __device__ constexpr int enc_out_ring(int op) { return op == kOpCompress ? 8192 : 5120; }
+__host__ __device__ constexpr int enc_out_ring(int op) { return op == kOpCompress ? 5376 : 5120; }
 // incoming payloads: see hc_decode.cu
 __host__ __device__ constexpr int enc_in_ring(int op) { return op == kOpCompress ? 0 : 4864; }
 __host__ __device__ constexpr int enc_warp_bytes(int op) { return kSubBytes + enc_out_ring(op) + enc_in_ring(op); }
@@ -36,11 +37,11 @@ static_assert(32 * 132 + 32 <= kInUsable, "one payload must fit");
 
 struct EncShared {
   uint64_t stage_full[kEncWarps];
-  uint64_t in_full[kEncWarps][4];
+  uint64_t in_full[enc_warps(kOpAddF32)][4];
   uint64_t placed[kSlots];                      // out_at[] of the chunk is valid
   uint64_t in_known[kInSlots];                  // in_at[] of the chunk is valid (one arrival per stream)
   uint64_t out_at[kSlots][kEncWarps];           // byte offset of the warp's payload; ~0: not to be stored
-  uint64_t in_at[kInSlots][kMaxIn][kEncWarps];  // byte offsets of the incoming payloads
+  uint64_t in_at[kInSlots][kMaxIn][enc_warps(kOpAddF32)];  // byte offsets of the incoming payloads
   uint64_t in_run[kMaxIn];                      // streams: payload bytes before the CTA's next chunk
   uint32_t tot[kSlots][kEncWarps];
   uint32_t sum[kSlots];  // running total of the chunk [23:0] and number of warps that have added theirs [31:24]
@@ -52,6 +53,7 @@ struct Chunk {
   uint32_t seg, lc;
 };
 __device__ __forceinline__ Chunk chunk_of(const SoloParams& p, uint32_t t) {
+  if (p.n_seg == 1u) return Chunk{0u, t};
   uint32_t g = 0;
   while (g + 1 < p.n_seg && t >= p.first[g + 1]) ++g;
   return Chunk{g, t - p.first[g]};
@@ -207,7 +209,7 @@ __device__ __forceinline__ void from_row(uint32_t (&d)[32], const Row& r) {
 
 // ---- the kernel --------------------------------------------------------------------------------------------------
 template <int OP, int MODE>
-__global__ void __launch_bounds__((kEncWarps + 1) * 32, 1)
+__global__ void __launch_bounds__((enc_warps(OP) + 1) * 32, 1)
 hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ SoloParams p) {
   constexpr bool kHasLocal = OP != kOpAddStream;
   constexpr bool kHasIn = OP != kOpCompress;
@@ -240,7 +242,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   }
   __syncthreads();
   if (sh.dead) return;  // (one answer for all warps)
-  const uint32_t subs0 = (uint32_t)((p.n[0] + kSubValues - 1) / kSubValues);
+  const uint32_t subs0 = p.subs[0];
   if (warp == nc) {
     clerk(p, sh, nc, subs0);
     return;
@@ -261,7 +263,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   };
   auto n_local = [&](uint32_t g) -> uint64_t { return OP == kOpAddI32 ? num_blocks(p.n[g]) * kBlock : p.n[g]; };
   // whole sub-tiles of an aligned operand come through the TMA unit; the rest is loaded by the warp itself
-  auto by_tma = [&](const Where& w) -> bool { return p.use_tma[w.seg] && (uint64_t)(w.sub + 1) * kSubValues <= n_local(w.seg); };
+  auto by_tma = [&](const Where& w) -> bool { return w.sub < p.by_tma[w.seg]; };
   auto fetch_stage = [&](uint32_t t) {
     if (!kHasLocal || t == kNoTile) return;
     const Where w = where(t);
@@ -490,7 +492,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     }
     __syncwarp();
     totals_arrive(k, nc);
-    const uint32_t subs = (uint32_t)((p.n[w.seg] + kSubValues - 1) / kSubValues);
+    const uint32_t subs = p.subs[w.seg];
     uint8_t* const rates = p.out[w.seg];
     if (w.sub < subs) rates[(uint64_t)w.sub * kSubBlocks + lane] = (uint8_t)code.rate;
     if (w.sub + 1 == subs)  // section A covers whole chunks of 32768 values
@@ -542,7 +544,7 @@ namespace {
 
 template <int OP, int MODE>
 cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t stream) {
-  constexpr int kWarps = dev::kEncWarps;
+  constexpr int kWarps = dev::enc_warps(OP);
   auto smem = [](int nc) { return nc * dev::enc_warp_bytes(OP) + 1024; };
   static thread_local int cache[64] = {};
   const int cap = resident_ctas(dev::hc_encode_solo_kernel<OP, MODE>, 32 * (kWarps + 1), smem(kWarps), cache);
@@ -551,13 +553,13 @@ cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t str
   // Compute warps per CTA: as many rounds of chunks as the largest CTA needs, then no more warps than fill them (where
   // the last round would be half empty, all rounds are narrower instead); at least four at a time.
   uint64_t subs = 0;
-  for (uint32_t g = 0; g < p.n_seg; ++g) subs += (p.n[g] + dev::kSubValues - 1) / dev::kSubValues;
+  for (uint32_t g = 0; g < p.n_seg; ++g) subs += p.subs[g];
   const uint64_t rounds = (subs + sms * kWarps - 1) / (sms * kWarps);
   uint64_t nc = (subs + sms * rounds - 1) / (sms * rounds);
   if (nc < 4) nc = 4;
   p.first[0] = 0;
   for (uint32_t g = 0; g < p.n_seg; ++g)
-    p.first[g + 1] = p.first[g] + (uint32_t)(((p.n[g] + dev::kSubValues - 1) / dev::kSubValues + nc - 1) / nc);
+    p.first[g + 1] = p.first[g] + (uint32_t)((p.subs[g] + nc - 1) / nc);
   const uint32_t chunks = p.first[p.n_seg];
   const int grid = (int)(chunks < sms ? chunks : sms);
   p.out_words = p.ws.st_a;
@@ -585,9 +587,12 @@ cudaError_t launch_encode_solo(int op, int mode, SoloParams p, cudaStream_t stre
   uint64_t total = 0;
   for (uint32_t g = 0; g < p.n_seg; ++g) {
     total += p.n[g];
-    p.use_tma[g] = 0;
-    if (op != kOpAddStream && p.n[g])  // int32 deltas are stored in whole blocks; fp32 data may end in a ragged row
-      p.use_tma[g] = make_rows_map(&maps.m[g], p.local[g], op == kOpAddI32 ? num_blocks(p.n[g]) : p.n[g] / kBlock, dev::kSubBlocks) ? 1u : 0u;
+    p.subs[g] = (uint32_t)((p.n[g] + dev::kSubValues - 1) / dev::kSubValues);
+    p.by_tma[g] = 0;
+    if (op == kOpAddStream) continue;
+    // int32 deltas are stored in whole blocks; fp32 data may end in a ragged row
+    const uint64_t whole = (op == kOpAddI32 ? num_blocks(p.n[g]) * kBlock : p.n[g]) / dev::kSubValues;
+    if (whole && make_rows_map(&maps.m[g], p.local[g], whole * dev::kSubBlocks, dev::kSubBlocks)) p.by_tma[g] = (uint32_t)whole;
   }
   if (total == 0) return cudaSuccess;
   switch (op) {

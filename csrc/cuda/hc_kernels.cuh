@@ -104,8 +104,9 @@ struct SoloParams {
   const void* local[kMaxDst];  // fp32 values or int32 deltas, per segment
   uint64_t n[kMaxDst];         // values per segment
   uint8_t* out[kMaxDst];
-  uint32_t use_tma[kMaxDst];
-  uint32_t first[kMaxDst + 1];  // chunk numbers at which the segments start; [n_seg]: number of chunks (set by the launcher)
+  uint32_t subs[kMaxDst];    // sub-tiles of 1024 values, the last one perhaps ragged (this and the next two: set by the launcher)
+  uint32_t by_tma[kMaxDst];  // those of them that the TMA unit can load: whole ones of an aligned operand
+  uint32_t first[kMaxDst + 1];  // chunk numbers at which the segments start; [n_seg]: number of chunks
   uint32_t n_seg;
   uint32_t n_in;
   float recip;  // 0.5f / eb
