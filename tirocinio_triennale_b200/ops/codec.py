@@ -154,13 +154,14 @@ class Codec:
         k = len(xs)
         for x in xs:
             self._check_f32(x)
-        cap = max(max_compressed_bytes(x.numel()) for x in xs) + 16
+        lens = [x.numel() for x in xs]
+        cap = max_compressed_bytes(max(lens)) + 16
         stride = (cap + 511) // 512 * 512  # one allocation for all the streams
         buf = torch.empty((k, stride), dtype=torch.uint8, device=self.device)
         outs = list(buf[:, :cap].unbind(0))
         sizes = self._size_words(k)
         xp = (C.c_void_p * k)(*[x.data_ptr() for x in xs])
-        ns = (C.c_size_t * k)(*[x.numel() for x in xs])
+        ns = (C.c_size_t * k)(*lens)
         at = buf.data_ptr()
         op = (C.c_void_p * k)(*range(at, at + k * stride, stride))
         self._call("compress_batch", self.lib.hc_compress_batch, self._h, k, xp, ns, eb, _mode(mode), op, cap,
