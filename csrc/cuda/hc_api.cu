@@ -132,7 +132,7 @@ int hc_codec_status(hc_codec* c, int clear) {
   uint32_t ctrl[4] = {0, 0, 0, 0};
   if (cudaDeviceSynchronize() != cudaSuccess) return hc::kErrCuda;
   if (cudaMemcpy(ctrl, c->ws_mem, sizeof(ctrl), cudaMemcpyDeviceToHost) != cudaSuccess) return hc::kErrCuda;
-  if (clear && (ctrl[2] != 0 || ctrl[0] != 0 || ctrl[1] != 0)) cudaMemset(c->ws_mem, 0, 64);  // status and ticket counters
+  if (clear && (ctrl[2] != 0 || ctrl[0] != 0 || ctrl[1] != 0)) cudaMemset(c->ws_mem, 0, c->ws_bytes);  // status, ticket counters, sums left behind
   return (int)ctrl[2];
 }
 

@@ -200,12 +200,10 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
       if (lane == 0) s_tot[warp][qq] = sum;
     }
     __syncthreads();
+    for (uint32_t qq = warp; qq < Q; qq += n_warps)
+      give_total(ws.sums + (1u + qq) * kMaxCtas, warp_sum_u64(lane < n_warps ? s_tot[lane][qq] : 0ull));
     for (uint32_t qq = warp; qq < Q; qq += n_warps) {
-      const uint32_t cta = blockIdx.x;
-      const uint64_t tot = warp_sum_u64(lane < n_warps ? s_tot[lane][qq] : 0ull);
-      uint64_t* const words = p.chain + (size_t)qq * gridDim.x;
-      if (lane == 0 && cta + 1 < gridDim.x) st_relaxed_gpu_u64(words + cta, st_pack(kStAgg, ws.epoch, tot));
-      const uint64_t pre = cta ? sum_status_words<kMaxCtas / 32>(words, cta, ws) : 0ull;
+      const uint64_t pre = take_total(ws.sums + (1u + qq) * kMaxCtas, ws);
       if (lane == 0) s_pre[qq] = pre;
     }
     __syncthreads();
@@ -458,15 +456,14 @@ cudaError_t launch_t(const TensorMaps& maps, DecParams p, cudaStream_t stream, b
   if (RUNS) {
     // few sub-tiles are spread over the SMs four at a time (fewer CTAs exchange their totals faster)
     const uint64_t subs = (p.seg[0].n + dev::kSubValues - 1) / dev::kSubValues;
-    const uint64_t sms = (uint64_t)(cap < dev::kMaxCtas ? cap : dev::kMaxCtas);
+    const uint64_t sms = (uint64_t)(cap < kMaxCtas ? cap : kMaxCtas);
     warps = (subs + sms - 1) / sms;
     warps = warps < 4u ? 4u : warps > (uint64_t)kWarps ? (uint64_t)kWarps : warps;
     grid = (int)((subs + warps - 1) / warps < sms ? (subs + warps - 1) / warps : sms);
     // the pool: an eighth of a run; none where a run is a sub-tile or three
     const uint64_t run = subs / (grid * warps);
     p.pool = run < 4 ? 0u : run < 8 ? 1u : (uint32_t)(run / 8);
-    p.chain = p.ws.st_a;
-    p.flags = p.ws.st_a + (size_t)p.n_seg * grid;
+    p.flags = p.ws.st_a;
   } else {
     // tickets are quarters of a tile while there is a warp for each
     const uint32_t tiles = SUM ? p.tiles_per_seg : p.n_tiles;

@@ -94,6 +94,7 @@ __device__ __forceinline__ void publish_inputs(const SoloParams& p, uint32_t nc,
   for (uint32_t q = q0; q < p.n_in; q += dq) {
     const uint32_t all = __reduce_add_sync(0xffffffffu, payload_len16(rates16(p.in[q], p.in_size[q], a, b, lane)));
     if (lane == 0) st_relaxed_gpu_u64(p.in_words + (size_t)q * p.first[1] + t, st_pack(kStAgg, p.ws.epoch, all));
+    if (p.one_round) give_total(p.ws.sums + (1u + q) * kMaxCtas, all);
   }
 }
 // Payload offsets of the sub-tiles of chunk t in input stream q (slot r of in_at); one warp.  `next`: chunks before it
@@ -106,7 +107,8 @@ __device__ __forceinline__ void input_offsets(const SoloParams& p, EncShared& sh
   const uint32_t inc = warp_inclusive_scan(sum, (int)lane);
   const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
   uint64_t base = sh.in_run[q];
-  advance_base(p.in_words + (size_t)q * p.first[1], next, base, t, p.ws);
+  if (p.one_round) base = take_total(p.ws.sums + (1u + q) * kMaxCtas, p.ws);
+  else advance_base(p.in_words + (size_t)q * p.first[1], next, base, t, p.ws);
   if (!(lane & 1u) && (lane >> 1) < nc) sh.in_at[r][q][lane >> 1] = rate_bytes(p.n[0]) + base + inc - sum;
   __syncwarp();
   if (lane == 0) {
@@ -150,7 +152,8 @@ __device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32
       base = 0;
       next = p.first[seg];
     }
-    advance_base(p.out_words, next, base, t, ws);
+    if (p.one_round) base = take_total(ws.sums, ws);
+    else advance_base(p.out_words, next, base, t, ws);
     const uint64_t start = rate_bytes(p.n[seg]) + base;
     const uint64_t at = start + inc - tot;
     const bool fits = at + tot <= p.out_cap && !fatal_error(ws.ctrl);
@@ -479,16 +482,21 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     const BlockCode code = code_of<MODE>(d, or_tail);
     const uint32_t inc = warp_inclusive_scan(code.len, (int)lane);
     const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
+    uint32_t before = 0;
     if (lane == 0) {
       const uint32_t r = k % kSlots;
       sh.tot[r][warp] = tot;
       // the last warp publishes the chunk's total, not the clerk: other CTAs wait for it, whatever this one's clerk
       // is waiting for (published by the clerks, the totals moved on in lock step, 4 us a chunk)
-      const uint32_t before = atomicAdd(&sh.sum[r], (1u << 24) | tot);
+      before = atomicAdd(&sh.sum[r], (1u << 24) | tot);
       if (before >> 24 == nc - 1u) {
         st_relaxed_gpu_u64(p.out_words + t, st_pack(kStAgg, ws.epoch, (before & 0xffffffu) + tot));
         sh.sum[r] = 0;
       }
+    }
+    if (p.one_round) {
+      before = __shfl_sync(0xffffffffu, before, 0);
+      if (before >> 24 == nc - 1u) give_total(ws.sums, (before & 0xffffffu) + tot);
     }
     __syncwarp();
     totals_arrive(k, nc);
@@ -549,7 +557,7 @@ cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t str
   static thread_local int cache[64] = {};
   const int cap = resident_ctas(dev::hc_encode_solo_kernel<OP, MODE>, 32 * (kWarps + 1), smem(kWarps), cache);
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
-  const uint64_t sms = (uint64_t)(cap < dev::kMaxCtas ? cap : dev::kMaxCtas);
+  const uint64_t sms = (uint64_t)(cap < kMaxCtas ? cap : kMaxCtas);
   // Compute warps per CTA: as many rounds of chunks as the largest CTA needs, then no more warps than fill them (where
   // the last round would be half empty, all rounds are narrower instead); at least four at a time.
   uint64_t subs = 0;
@@ -562,6 +570,7 @@ cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t str
     p.first[g + 1] = p.first[g] + (uint32_t)((p.subs[g] + nc - 1) / nc);
   const uint32_t chunks = p.first[p.n_seg];
   const int grid = (int)(chunks < sms ? chunks : sms);
+  p.one_round = p.n_seg == 1 && chunks <= sms;
   p.out_words = p.ws.st_a;
   p.in_words = p.ws.st_a + chunks;
   return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE>, grid, 32 * ((int)nc + 1), smem((int)nc), stream, maps, p);

@@ -832,7 +832,8 @@ size_t workspace_bytes(size_t max_elems, int sets) {
   size_t groups = tiles / 32 + 1 + kMaxDst;
   if (sets < 1) sets = 1;
   if (sets > kMaxWorkspaceSets) sets = kMaxWorkspaceSets;
-  return kWorkspaceHeader + (size_t)sets * 3 * (tiles + groups) * sizeof(uint64_t);
+  // look-back words of all sets, then the exchange words of all sets
+  return kWorkspaceHeader + (size_t)sets * (3 * (tiles + groups) + (1 + kMaxIn) * kMaxCtas) * sizeof(uint64_t);
 }
 
 Workspace workspace_view(void* mem, size_t max_elems, uint32_t epoch, uint64_t spin_limit_ns, int sets) {
@@ -852,6 +853,8 @@ Workspace workspace_view(void* mem, size_t max_elems, uint32_t epoch, uint64_t s
   w.grp_a = w.st_out + tiles;
   w.grp_b = w.grp_a + groups;
   w.grp_out = w.grp_b + groups;
+  w.sums = reinterpret_cast<uint64_t*>(b + kWorkspaceHeader) + (size_t)sets * 3 * (tiles + groups) +
+           set * (1 + kMaxIn) * kMaxCtas;
   w.epoch = epoch;
   w.spin_limit_ns = spin_limit_ns;
   return w;

@@ -43,6 +43,7 @@ constexpr int kTileBytes = kTileElems * 4;        // 16384
 constexpr int kBufBytes = 17 * 1024;              // a tile of stream bytes + alignment slack
 constexpr int kComputeThreads = kTileBlocks;
 constexpr int kMaxDst = 8;
+constexpr int kMaxCtas = 160;  // CTAs of a launch with one CTA per SM
 
 enum Op : int {
   kOpCompress = 0,   // fp32 -> stream
@@ -60,6 +61,7 @@ struct Workspace {
   uint64_t* grp_b;
   uint64_t* grp_out;
   uint32_t* tick;  // [0] tile ticket counter, [1] CTAs that have left; re-armed by the last CTA of a launch
+  uint64_t* sums;      // [1 + kMaxIn][kMaxCtas] exchange of CTA totals (dev::give_total): zero between launches
   uint64_t* size_acc;  // [kMaxDst] payload bytes per segment of a launch with sparse tiles; zeroed by its last CTA
   uint32_t epoch;
   uint64_t spin_limit_ns;
@@ -114,6 +116,7 @@ struct SoloParams {
   uint64_t in_size[kMaxIn];
   uint64_t out_cap;
   uint64_t* size_out;   // device words receiving the exact stream length of each segment (or null)
+  uint32_t one_round;   // one stream, a chunk per CTA: totals are exchanged by give_total (set by the launcher)
   uint64_t* out_words;  // one word per chunk: its payload bytes (set by the launcher)
   uint64_t* in_words;   // n_in rows of such words
   Workspace ws;
@@ -143,9 +146,8 @@ struct DecParams {
   uint32_t sum;         // 1: the n_seg streams are contributions to one array of seg[0].n values; their
                         //    quantised values are added tile by tile and seg[0].out receives the sum
   uint32_t parts;       // flagged segments: tickets per tile, 1 (a warp takes all four quarters) or 4
-  // stand-alone streams (no in_ready; set by the launcher): one word per CTA and stream for the exchange of payload
-  // totals; sub-tiles of every warp's run that are handed out one by one, and their payload offsets as flag words
-  uint64_t* chain;
+  // stand-alone streams (no in_ready; set by the launcher): sub-tiles of every warp's run that are handed out one by
+  // one, and their payload offsets as flag words
   uint64_t* flags;
   uint32_t pool;
   Workspace ws;

@@ -54,7 +54,7 @@ int hc_noalloc_status(int clear) {
   if (cudaDeviceSynchronize() != cudaSuccess) return hc::kErrCuda;
   if (cudaMemcpy(ctrl, d->scratch, sizeof(ctrl), cudaMemcpyDeviceToHost) != cudaSuccess) return hc::kErrCuda;
   // status word, first-time-out site and the ticket counters a failed launch may have left behind
-  if (clear && cudaMemset(d->scratch, 0, 64) != cudaSuccess) return hc::kErrCuda;
+  if (clear && cudaMemset(d->scratch, 0, kScratchBytes) != cudaSuccess) return hc::kErrCuda;
   return (int)ctrl[2];
 }
 

@@ -222,8 +222,7 @@ int hc_comm_status(hc_comm* c, int clear) {
   if (cudaMemcpy(ctrl, c->ws_mem, sizeof(ctrl), cudaMemcpyDeviceToHost) != cudaSuccess) return hc::kErrCuda;
   const uint32_t st = ctrl[2] > ctrl[34] ? ctrl[2] : ctrl[34];
   if (clear && (ctrl[0] | ctrl[1] | ctrl[2] | ctrl[3] | ctrl[33] | ctrl[34])) {
-    cudaMemset(c->ws_mem, 0, 64);                                      // status and ticket counters
-    cudaMemset(static_cast<uint32_t*>(c->ws_mem) + 32, 0, 4 * sizeof(uint32_t));  // raw kernels' counter and status
+    cudaMemset(c->ws_mem, 0, c->ws_bytes);  // status words, ticket counters, sums left behind
   }
   return (int)st;
 }
