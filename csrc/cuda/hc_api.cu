@@ -16,7 +16,6 @@ struct hc_codec {
   bool owns = false;
   uint32_t epoch = 0;
   uint64_t spin_limit_ns = 2000ull * 1000 * 1000;
-  bool prepass = true;  // large stand-alone inputs: tile offsets from a pre-pass instead of an input look-back
 };
 
 namespace {
@@ -123,7 +122,7 @@ int hc_codec_status_site(hc_codec* c) {
 
 int hc_codec_set_prepass(hc_codec* c, int on) {
   if (!c) return hc::kErrArgument;
-  c->prepass = on != 0;
+  (void)on;  // kept for callers: the kernels find the offsets themselves
   return hc::kOk;
 }
 

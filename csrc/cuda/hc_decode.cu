@@ -17,6 +17,7 @@
 // warp, its rate bytes scanned once), or a quarter of a tile while the GPU holds a warp for each.
 #include "hc_host.cuh"
 #include "hc_launch.h"
+#include "hc_timeline.cuh"
 #include "hc_warp.cuh"
 
 namespace hc {
@@ -184,6 +185,12 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
       u.raw_ok = false;
     }
   };
+  HC_TL_DECL(ws.epoch);
+  if (threadIdx.x == 0) {
+    HC_TL_ZERO();
+    HC_STAMP(0);
+    HC_PH_START();
+  }
   if (!RUNS) ask();
   uint32_t tk = dead ? kNoTile : next_item(), tk_next = tk == kNoTile ? kNoTile : next_item();
   Unit un, un_next{0ull, 0u, 0u, true};
@@ -315,6 +322,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   bool ints = false;
   uint32_t bound = 0;  // of |sum of the deltas| of this lane's block
   bool announced = !RUNS || pool == 0u;
+  if (threadIdx.x == 0) HC_PH(0);
   for (uint32_t v = 0;;) {
     if (staged < 2u && tk != kNoTile) {
       Staged st;
@@ -340,14 +348,17 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
         }
       }
     }
+    if (threadIdx.x == 0) HC_PH(1);
     if (staged == 0u) break;
     if (!warp_wait(&full[v & 3u], (v >> 2) & 1u, ws, kSiteDecodeInFull)) break;
     ++v;
+    if (threadIdx.x == 0) HC_PH(2);
     const int W = plane_width(__reduce_max_sync(0xffffffffu, cur.rate & 31u));
     uint32_t T[32], sign, a0;
     decode_rows(ring, cur.pos, cur.rate, W, sign, a0, T);
     __syncwarp();
 
+    if (threadIdx.x == 0) HC_PH(3);
     // ---- signs, sum over the streams, prefix sum, scaling ----------------------------------------------------------
     uint32_t w[32];
     const bool little = (cur.rate & 31u) <= 16u && a0 < (SUM ? 1u << 20 : 1u << 23);
@@ -408,6 +419,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
           w[i] = as_u(__fmul_rn(__fmul_rn((float)qv[i], p.eb), 2.0f));
         }
       }
+      if (threadIdx.x == 0) HC_PH(4);
       // ---- out -------------------------------------------------------------------------------------------------------
       const uint32_t sgo = SUM ? 0u : cur.seg;
       const DecSegment& sg = p.seg[sgo];
@@ -432,8 +444,13 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     }
     cur = nxt;
     --staged;
+    if (threadIdx.x == 0) {
+      HC_PH(5);
+      HC_PH_COUNT();
+    }
   }
   if (lane == 0) tma_wait_group<0>();
+  if (lane == 0) HC_STAMP_MAX(7);
   if (dynamic) cta_epilogue(ws.tick);
 }
 
@@ -523,3 +540,5 @@ cudaError_t launch_decode(int mode, DecParams p, cudaStream_t stream, bool overl
 }
 
 }  // namespace hc
+
+HC_TL_READ(hc_debug_timeline_decode)

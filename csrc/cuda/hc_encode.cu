@@ -10,10 +10,14 @@
 // between its CTA's previous chunk and the current one (at most about 150, five loads a lane, one round trip once they
 // are there) and hands every compute warp its byte offset.  A clerk only ever waits for chunk totals, never for another
 // clerk, so there is no chain of hops as in a decoupled look-back.
+// A launch of one round (a chunk per CTA: up to 2220 sub-tiles for the adds, 3404 for compress) pushes its totals instead
+// (give_total): its time is start-up and drain, 147 reductions a CTA in all cost nothing there (seven streams of 8 MB
+// added and decoded: 31.9 us, 37.1 before).  In longer launches pushing gained nothing for the first chunk alone.
 // Where payloads come from (adds): the same sums over the rate bytes of the input streams, four chunks ahead of the
 // compute warps.
 #include "hc_host.cuh"
 #include "hc_launch.h"
+#include "hc_timeline.cuh"
 #include "hc_warp.cuh"
 
 namespace hc {
@@ -223,6 +227,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   const uint32_t nc = (blockDim.x >> 5) - 1u;  // compute warps
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const Workspace& ws = p.ws;
+  HC_TL_DECL(ws.epoch);
   const uint32_t Q = kHasIn ? p.n_in : 0u;
 
   if (tid < nc) {
@@ -242,6 +247,8 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   if (tid == 0) {
     sh.dead = fatal_error(ws.ctrl) ? 1u : 0u;
+    HC_TL_ZERO();
+    HC_STAMP(0);
   }
   __syncthreads();
   if (sh.dead) return;  // (one answer for all warps)
@@ -369,6 +376,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   auto placed = [&](uint32_t k) -> bool { return __all_sync(0xffffffffu, mbar_test(&sh.placed[k % kSlots], (k / kSlots) & 1u)); };
 
   bool failed = false;  // a wait ran out (recorded)
+  if (tid == 0) HC_PH_START();
   for (uint32_t k = 0;; ++k) {
     if (t == kNoTile) {
       for (; copied < k && !failed;) {
@@ -382,6 +390,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       t = ticket(p, k + 1);
       continue;
     }
+    if (tid == 0) HC_PH(0);
     const Where w = where(t);
     const uint32_t t_next = ticket(p, k + 1);
     uint32_t d[32];
@@ -390,6 +399,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     // ---- local operand: first, because it needs nothing but its rows --------------------------------------------------
     if (kHasLocal) {
       if (!warp_wait(&sh.stage_full[warp], k & 1u, ws, kSiteComputeTile)) failed = true;
+      if (tid == 0) HC_PH(1);
       if (!by_tma(w)) {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(p.local[w.seg]);
         const uint64_t first = (uint64_t)w.sub * kSubValues, n = n_local(w.seg);
@@ -426,6 +436,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
 #pragma unroll
       for (int i = 0; i < 32; ++i) d[i] = 0;
     }
+    if (tid == 0) HC_PH(2);
     // ---- incoming streams ----------------------------------------------------------------------------------------------
     if (kHasIn) {
       for (uint32_t q = 0; q < Q; ++q) {
@@ -436,6 +447,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
         }
         const uint32_t v = k * Q + q;
         if (!warp_wait(&sh.in_full[warp][v & 3u], (v >> 2) & 1u, ws, kSiteComputeInFull)) cur_rate = 0, failed = true;
+        if (tid == 0) HC_PH(3);
         uint32_t T[32], sign, a0;
         decode_rows(inring, cur_pos, cur_rate, plane_width(__reduce_max_sync(0xffffffffu, cur_rate & 31u)), sign, a0, T);
         __syncwarp();
@@ -478,6 +490,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       or_tail = or_tail_of(d);
     }
 
+    if (tid == 0) HC_PH(4);
     // ---- encode -----------------------------------------------------------------------------------------------------------
     const BlockCode code = code_of<MODE>(d, or_tail);
     const uint32_t inc = warp_inclusive_scan(code.len, (int)lane);
@@ -506,6 +519,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     if (w.sub + 1 == subs)  // section A covers whole chunks of 32768 values
       for (uint64_t b = (uint64_t)subs * kSubBlocks + lane; b < rate_bytes(p.n[w.seg]); b += 32u) rates[b] = 0;
 
+    if (tid == 0) HC_PH(5);
     // payloads whose place is known leave; the oldest ones have to where this one needs their room
     while (copied < k && placed(copied)) copy_oldest();
     const uint32_t need = room_for(tot);
@@ -530,6 +544,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     }
     t = t_next;
     if (failed) continue;
+    if (tid == 0) HC_PH(6);
     __syncwarp();
     pack_blocks(oring + start, inc - code.len, code, d, plane_width(__reduce_max_sync(0xffffffffu, code.rate & 31u)));
     if (lane == k % kSlots) {
@@ -541,7 +556,13 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       head = start + need;
       ++taken;
     }
+    if (tid == 0) {
+      HC_PH(7);
+      HC_PH_COUNT();
+    }
   }
+  if (tid == 0) HC_PH(8);
+  if (lane == 0) HC_STAMP_MAX(7);
 }
 
 }  // namespace dev
@@ -614,3 +635,5 @@ cudaError_t launch_encode_solo(int op, int mode, SoloParams p, cudaStream_t stre
 }
 
 }  // namespace hc
+
+HC_TL_READ(hc_debug_timeline_encode)

@@ -5,6 +5,7 @@
 
 #include "hc_launch.h"
 #include "hc_host.cuh"
+#include "hc_timeline.cuh"
 #include "hc_warp.cuh"
 
 namespace hc {
@@ -38,53 +39,6 @@ struct __align__(16) EncShared {
   uint16_t in_rel[2][kTileBlocks];
   uint8_t in_rate[2][kTileBlocks];
 };
-
-// Optional per-CTA timeline (compile with -DHC_TIMELINE): nanosecond stamps of the first tile's way
-// through the roles (slots 0-15) and, for the first compute warp, SM-clock cycles accumulated per
-// phase of the tile loop (slots 16-30) with the number of tiles in slot 31, for finding where a
-// launch spends its time.  Not part of a normal build.
-#ifdef HC_TIMELINE
-constexpr int kTlSlots = 32;
-__device__ unsigned long long g_timeline[4 * 1024 * kTlSlots];  // [launch epoch & 3][CTA][slot]
-__device__ __forceinline__ unsigned long long timeline_now() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-#define HC_TL_DECL(epoch)                                                                                      \
-  unsigned long long* const hc_tl =                                                                            \
-      g_timeline + (((epoch)&3u) * 1024u + (blockIdx.x < 1024u ? blockIdx.x : 1023u)) * (unsigned)kTlSlots;     \
-  long long hc_ph_t = 0
-#define HC_TL_ZERO()                                \
-  do {                                              \
-    hc_tl[7] = hc_tl[14] = hc_tl[15] = 0;           \
-    for (int i_ = 16; i_ < kTlSlots; ++i_) hc_tl[i_] = 0; \
-  } while (0)
-#define HC_STAMP(i) hc_tl[i] = timeline_now()
-#define HC_STAMP_MAX(i) atomicMax(&hc_tl[i], timeline_now())
-#define HC_TIC() const unsigned long long hc_tic = timeline_now()
-#define HC_TOC(i) hc_tl[i] += timeline_now() - hc_tic
-// phase accounting of one thread: HC_PH_START() once, then HC_PH(i) charges the cycles since the
-// previous mark to phase i
-#define HC_PH_START() hc_ph_t = clock64()
-#define HC_PH(i)                                  \
-  do {                                            \
-    const long long now_ = clock64();             \
-    hc_tl[16 + (i)] += (unsigned long long)(now_ - hc_ph_t); \
-    hc_ph_t = now_;                               \
-  } while (0)
-#define HC_PH_COUNT() hc_tl[kTlSlots - 1] += 1
-#else
-#define HC_TL_DECL(epoch)
-#define HC_TL_ZERO()
-#define HC_STAMP(i)
-#define HC_STAMP_MAX(i)
-#define HC_TIC()
-#define HC_TOC(i)
-#define HC_PH_START()
-#define HC_PH(i)
-#define HC_PH_COUNT()
-#endif
 
 // bounded mbarrier wait that records a timeout; `site` says which wait it was
 __device__ __forceinline__ bool wait_or_flag(uint64_t* bar, uint32_t parity, const Workspace& ws, volatile uint32_t* abort,
@@ -191,14 +145,15 @@ __host__ __device__ constexpr int enc_cbuf_off(int op, int ns, bool inplace) {
 }
 static_assert(kRingBytesCompress >= kTileBytes + 32 && kRingBytesAdd >= kTileBytes + 32, "a tile of 128-byte blocks must fit");
 
-template <int OP, int MODE, int NS, bool INPLACE>
+template <int OP, int NS, bool INPLACE>
 __global__ void __launch_bounds__(kEncThreads, (OP == kOpCompress || INPLACE) ? 4 : 3)
 hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
   static_assert(NS <= kMaxStages && (!INPLACE || NS == 1), "stage count");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ EncShared sh;
-  constexpr bool kHasLocal = OP != kOpAddStream;
+  static_assert(OP == kOpCompress || OP == kOpAddF32, "stand-alone calls run hc_encode_solo_kernel");
+  constexpr int MODE = kModeOutlier;
   constexpr bool kHasIn = OP != kOpCompress;
   constexpr uint32_t kRingBytes = (uint32_t)enc_ring_bytes(OP, INPLACE);
   uint8_t* const stage0 = smem + 1024;
@@ -217,8 +172,7 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
   struct Seg {
     uint32_t g, lt;      // segment, tile inside the segment
     uint64_t n, nrate;   // values and rate bytes of the segment
-    uint64_t full_rows;  // rows the tensor map covers (int32 deltas come in whole blocks)
-    uint64_t n_local;    // readable 4-byte values of the local operand
+    uint64_t full_rows;  // rows the tensor map covers
   };
   auto seg_of = [&](uint32_t tile) -> Seg {
     Seg v;
@@ -228,15 +182,14 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
     v.g = p.n_seg > 1 ? tile - v.lt * p.n_seg : 0u;
     v.n = p.n[v.g];
     v.nrate = rate_bytes(v.n);
-    v.full_rows = OP == kOpAddI32 ? num_blocks(v.n) : v.n / kBlock;
-    v.n_local = OP == kOpAddI32 ? num_blocks(v.n) * kBlock : v.n;
+    v.full_rows = v.n / kBlock;
     return v;
   };
   // destinations of a tile: every destination of the single segment, or the segment's own one
   auto dst_first = [&](const Seg& v) -> uint32_t { return p.n_seg > 1 ? v.g : 0u; };
   auto dst_count = [&](const Seg&) -> uint32_t { return p.n_seg > 1 ? 1u : p.n_dst; };
 
-  if (tid == 32 && kHasLocal) {  // descriptor of the segment this CTA's first tile belongs to
+  if (tid == 32) {  // descriptor of the segment this CTA's first tile belongs to
     const uint32_t g0 = p.n_seg > 1 ? blockIdx.x % p.n_seg : 0u;
     if (p.use_tma[g0]) tma_prefetch_map(&tmaps.m[g0]);
   }
@@ -331,7 +284,7 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
         if (lane == 0) {
           sh.tile[slot] = t_stage;
           bool fetch = false;
-          if (kHasLocal && t_stage != kNoTile) {
+          if (t_stage != kNoTile) {
             const Seg v = seg_of(t_stage);
             fetch = p.use_tma[v.g] && (uint64_t)v.lt * kTileBlocks < v.full_rows;
             if (fetch) {
@@ -538,7 +491,7 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
       const Seg v = seg_of(tile);
 
       // ---- local operand -------------------------------------------------------------------------
-      if (kHasLocal) {
+      {
         uint32_t w[32];
         const uint64_t row = (uint64_t)v.lt * kTileBlocks + tid;
         if (p.use_tma[v.g]) {
@@ -548,27 +501,19 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) w[i] = 0;
           }
-          // the ragged last row of fp32 data is not part of the tensor map
-          if (OP != kOpAddI32 && row * kBlock < v.n && (row + 1) * kBlock > v.n)
-            load_row_global((const uint32_t*)p.local[v.g], v.n, row, w);
+          // the ragged last row is not part of the tensor map
+          if (row * kBlock < v.n && (row + 1) * kBlock > v.n) load_row_global((const uint32_t*)p.local[v.g], v.n, row, w);
         } else {
-          load_row_global((const uint32_t*)p.local[v.g], v.n_local, row, w);
+          load_row_global((const uint32_t*)p.local[v.g], v.n, row, w);
         }
         if (!INPLACE) mbar_arrive(&sh.stage_free[s]);  // this thread's row is in registers
-        if (OP == kOpAddI32) {
+        int32_t q[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) d[i] += (int32_t)w[i];
-        } else {
-          int32_t q[32];
+        for (int i = 0; i < 32; ++i) q[i] = quantise(__uint_as_float(w[i]), p.recip);
+        int32_t dl[32];
+        lorenzo_forward<MODE>(q, dl);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) q[i] = quantise(__uint_as_float(w[i]), p.recip);
-          int32_t dl[32];
-          lorenzo_forward<MODE>(q, dl);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) d[i] += dl[i];
-        }
-      } else if (!INPLACE) {
-        mbar_arrive(&sh.stage_free[s]);
+        for (int i = 0; i < 32; ++i) d[i] += dl[i];
       }
 
       // ---- encode ----------------------------------------------------------------------------------
@@ -661,76 +606,6 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
   }
 }
 
-// Pre-pass for the stand-alone stream consumers (decompress and the homomorphic adds on streams that
-// no collective step has flagged): reads the rate bytes of up to kMaxIn streams and writes, for every
-// tile, the byte offset of its payload in the arrival-flag format (dev::flag_pack(tag, offset)), so
-// that the consuming kernel stages each tile straight from its flag word instead of walking a
-// look-back chain over the input tile by tile.  One CTA covers kOffTiles tiles of one stream: each
-// warp sums the payload lengths of 32 tiles (lane j ends up with tile j's total), the CTA scans its
-// totals, warp 0 chains the CTA totals with the two-level look-back, then every thread publishes one
-// flag word.  A 256 MB input has 2 MiB of rate bytes and 64 CTAs here: a few microseconds.
-constexpr int kOffThreads = 256;
-constexpr int kOffTiles = kOffThreads;  // tiles per CTA, one flag word per thread
-__global__ void __launch_bounds__(kOffThreads) hc_offsets_kernel(const OffsetParams p) {
-  __shared__ uint32_t s_wsum[kOffThreads / 32];
-  __shared__ uint64_t s_base;
-  __shared__ uint32_t s_ok;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t q = blockIdx.y, cta = blockIdx.x;
-  const uint8_t* in = p.in[q];
-  const uint64_t in_size = p.in_size[q];
-  if (tid == 0) launch_dependents();  // the consumer may fill the SMs right away; it waits on the flags
-  const uint32_t t0 = cta * kOffTiles + warp * 32;
-  uint32_t mine = 0;
-#pragma unroll 8
-  for (int j = 0; j < 32; ++j) {
-    const uint32_t t = t0 + j;
-    uint32_t sum = 0;
-    if (t < p.tiles_per_seg) {
-      const uint64_t b0 = (uint64_t)t * kTileBlocks + (uint64_t)lane * 4;
-      uint32_t r4 = 0;
-      if (b0 + 4 <= in_size && (reinterpret_cast<uintptr_t>(in) & 3u) == 0) {
-        r4 = __ldcg(reinterpret_cast<const uint32_t*>(in + b0));
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (b0 + k < in_size) r4 |= ld_cg_u8(in + b0 + k) << (8 * k);
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) sum += payload_len((r4 >> (8 * k)) & 0xffu);
-    }
-    sum = __reduce_add_sync(0xffffffffu, sum);
-    if (lane == j) mine = sum;
-  }
-  const uint32_t inc = warp_inclusive_scan(mine, lane);
-  if (lane == 31) s_wsum[warp] = inc;
-  __syncthreads();
-  uint32_t pre = 0, tot = 0;
-#pragma unroll
-  for (int w = 0; w < kOffThreads / 32; ++w) {
-    const uint32_t v = s_wsum[w];
-    if (w < warp) pre += v;
-    tot += v;
-  }
-  if (warp == 0) {
-    const uint32_t n_cta = (p.tiles_per_seg + kOffTiles - 1) / kOffTiles;
-    const uint32_t stride = n_cta + n_cta / 32 + 4;  // CTA words, then the words of their groups of 32
-    const Chain chain{p.ws.grp_a + (size_t)q * stride, p.ws.grp_a + (size_t)q * stride + n_cta + 1};
-    bool ok = true;
-    const uint64_t excl = lookback(chain, cta, p.ws.epoch, tot, p.ws.spin_limit_ns, p.ws.ctrl + 2, &ok);
-    if (lane == 0) {
-      s_base = p.nrate + excl;
-      s_ok = ok ? 1u : 0u;
-    }
-  }
-  __syncthreads();
-  const uint32_t t = cta * kOffTiles + tid;
-  if (t < p.tiles_per_seg) {
-    const uint64_t off = s_ok ? s_base + pre + (inc - mine) : kFlagOffsetMask;
-    st_relaxed_sys_u64(p.flags[q] + t, flag_pack(p.tag, off));
-  }
-}
-
 // fp32 -> int32 Lorenzo deltas of the quantised values, padded with zero deltas to whole blocks.
 // Counterpart of kernel_quant_prediction (HomComp/src/homcomp.cu:1553-1602).
 template <int MODE>
@@ -790,35 +665,25 @@ constexpr int enc_smem_bytes(int op, int ns, bool inplace) {
   return dev::enc_cbuf_off(op, ns, inplace) + (op == kOpCompress ? 0 : 2 * kBufBytes) + 1024;
 }
 
-template <int OP, int MODE, bool INPLACE = false>
+template <int OP, bool INPLACE = false>
 int encode_capacity() {
   constexpr int NS = INPLACE ? 1 : dev::enc_stages(OP);
   static thread_local int cache[64] = {};
-  return resident_ctas(dev::hc_encode_kernel<OP, MODE, NS, INPLACE>, dev::kEncThreads, enc_smem_bytes(OP, NS, INPLACE), cache);
+  return resident_ctas(dev::hc_encode_kernel<OP, NS, INPLACE>, dev::kEncThreads, enc_smem_bytes(OP, NS, INPLACE), cache);
 }
 
-template <int OP, int MODE, bool INPLACE = false>
+template <int OP, bool INPLACE = false>
 cudaError_t launch_encode_t(const TensorMaps& map, const EncParams& p, cudaStream_t stream, bool overlap) {
   constexpr int NS = INPLACE ? 1 : dev::enc_stages(OP);
   constexpr int smem = enc_smem_bytes(OP, NS, INPLACE);
-  const int cap = encode_capacity<OP, MODE, INPLACE>();
+  const int cap = encode_capacity<OP, INPLACE>();
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
   int grid = (int)(p.n_tiles < (uint32_t)cap ? p.n_tiles : (uint32_t)cap);
   if (p.grid_limit && (int)p.grid_limit < grid) grid = (int)p.grid_limit;
   if (overlap)
-    return launch_overlapped(dev::hc_encode_kernel<OP, MODE, NS, INPLACE>, grid, dev::kEncThreads, smem, stream, map, p);
-  dev::hc_encode_kernel<OP, MODE, NS, INPLACE><<<grid, dev::kEncThreads, smem, stream>>>(map, p);
+    return launch_overlapped(dev::hc_encode_kernel<OP, NS, INPLACE>, grid, dev::kEncThreads, smem, stream, map, p);
+  dev::hc_encode_kernel<OP, NS, INPLACE><<<grid, dev::kEncThreads, smem, stream>>>(map, p);
   return cudaGetLastError();
-}
-
-template <int OP>
-cudaError_t launch_encode_m(int mode, const TensorMaps& map, const EncParams& p, cudaStream_t stream, bool overlap) {
-  switch (mode) {
-    case kModeOutlier: return launch_encode_t<OP, kModeOutlier>(map, p, stream, overlap);
-    case kModePlain: return launch_encode_t<OP, kModePlain>(map, p, stream, overlap);
-    case kModeVec: return launch_encode_t<OP, kModeVec>(map, p, stream, overlap);
-    default: return cudaErrorInvalidValue;
-  }
 }
 
 }  // namespace
@@ -862,7 +727,7 @@ Workspace workspace_view(void* mem, size_t max_elems, uint32_t epoch, uint64_t s
 
 int device_sm_count() { return device_info().sms > 0 ? device_info().sms : 148; }
 
-cudaError_t launch_encode(int op, int mode, EncParams p, cudaStream_t stream, bool overlap) {
+cudaError_t launch_encode(int op, EncParams p, cudaStream_t stream, bool overlap) {
   if (p.n_seg == 0 || p.n_seg > (uint32_t)kMaxDst || p.n_in > (uint32_t)kMaxIn) return cudaErrorInvalidValue;
   if (p.n_seg > 1 && (op != kOpCompress || p.n_in != 0)) return cudaErrorInvalidValue;
   if (op == kOpCompress) p.n_in = 0;
@@ -875,45 +740,24 @@ cudaError_t launch_encode(int op, int mode, EncParams p, cudaStream_t stream, bo
   memset(&maps, 0, sizeof(maps));
   for (uint32_t g = 0; g < p.n_seg; ++g) {
     p.use_tma[g] = 0;
-    if (op != kOpAddStream && p.n[g]) {
-      // int32 deltas are stored in whole blocks; fp32 data may end in a ragged row
-      uint64_t rows = op == kOpAddI32 ? num_blocks(p.n[g]) : p.n[g] / kBlock;
-      p.use_tma[g] = make_rows_map(&maps.m[g], p.local[g], rows, kTileBlocks) ? 1u : 0u;
-    }
+    if (p.n[g]) p.use_tma[g] = make_rows_map(&maps.m[g], p.local[g], p.n[g] / kBlock, kTileBlocks) ? 1u : 0u;
   }
-  if (op == kOpAddF32 && mode == kModeOutlier) {
+  if (op == kOpAddF32) {
     // the in-place variant holds a fourth CTA per SM: taken when that saves a whole round of tiles
     // (tiles per CTA, rounded up) and leaves at most two
-    const uint32_t cap3 = (uint32_t)encode_capacity<kOpAddF32, kModeOutlier, false>();
-    const uint32_t cap4 = (uint32_t)encode_capacity<kOpAddF32, kModeOutlier, true>();
+    const uint32_t cap3 = (uint32_t)encode_capacity<kOpAddF32>();
+    const uint32_t cap4 = (uint32_t)encode_capacity<kOpAddF32, true>();
     if (cap3 && cap4) {
       const uint32_t rounds3 = (p.n_tiles + cap3 - 1) / cap3, rounds4 = (p.n_tiles + cap4 - 1) / cap4;
       if (p.variant == 2 || (p.variant == 0 && rounds4 < rounds3 && rounds4 <= 2))
-        return launch_encode_t<kOpAddF32, kModeOutlier, true>(maps, p, stream, overlap);
+        return launch_encode_t<kOpAddF32, true>(maps, p, stream, overlap);
     }
   }
   switch (op) {
-    case kOpCompress: return launch_encode_m<kOpCompress>(mode, maps, p, stream, overlap);
-    case kOpAddF32: return launch_encode_m<kOpAddF32>(mode, maps, p, stream, overlap);
-    case kOpAddI32: return launch_encode_m<kOpAddI32>(mode, maps, p, stream, overlap);
-    case kOpAddStream: return launch_encode_m<kOpAddStream>(mode, maps, p, stream, overlap);
+    case kOpCompress: return launch_encode_t<kOpCompress>(maps, p, stream, overlap);
+    case kOpAddF32: return launch_encode_t<kOpAddF32>(maps, p, stream, overlap);
     default: return cudaErrorInvalidValue;
   }
-}
-
-bool offsets_fit(const Workspace& ws, size_t max_elems, uint32_t n_in, uint32_t tiles_per_seg) {
-  (void)ws;
-  const size_t tiles = workspace_tiles(max_elems);
-  const size_t groups = tiles / 32 + 1 + kMaxDst;
-  const size_t n_cta = (tiles_per_seg + dev::kOffTiles - 1) / dev::kOffTiles;
-  return (size_t)n_in * (n_cta + n_cta / 32 + 4) <= 2 * groups && (size_t)n_in * tiles_per_seg <= 2 * tiles;
-}
-
-cudaError_t launch_offsets(const OffsetParams& p, cudaStream_t stream) {
-  if (p.n_in == 0 || p.n_in > (uint32_t)kMaxIn || p.tiles_per_seg == 0) return cudaErrorInvalidValue;
-  const dim3 grid((p.tiles_per_seg + dev::kOffTiles - 1) / dev::kOffTiles, p.n_in);
-  dev::hc_offsets_kernel<<<grid, dev::kOffThreads, 0, stream>>>(p);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_quant_pred(int mode, const float* x, int32_t* deltas, uint64_t n, float eb, cudaStream_t stream) {
@@ -943,20 +787,11 @@ cudaError_t launch_sum(float* dst, const float* a, const float* b, const float* 
 // in place (the variant for launches of about one tile per CTA)
 extern "C" int hc_resident_ctas(int op) {
   switch (op) {
-    case 0: return hc::encode_capacity<hc::kOpCompress, hc::kModeOutlier, false>();
-    case 1: return hc::encode_capacity<hc::kOpAddF32, hc::kModeOutlier, false>();
-    case 2: return hc::encode_capacity<hc::kOpAddF32, hc::kModeOutlier, true>();
+    case 0: return hc::encode_capacity<hc::kOpCompress>();
+    case 1: return hc::encode_capacity<hc::kOpAddF32>();
+    case 2: return hc::encode_capacity<hc::kOpAddF32, true>();
     default: return 0;
   }
 }
 
-#ifdef HC_TIMELINE
-// copies the stamps of the last four launches (4 x 1024 CTAs x 32 slots) to the host (synchronises) and clears them
-extern "C" int hc_debug_timeline(unsigned long long* host) {
-  if (cudaDeviceSynchronize() != cudaSuccess) return -1;
-  if (cudaMemcpyFromSymbol(host, hc::dev::g_timeline, sizeof(hc::dev::g_timeline)) != cudaSuccess) return -1;
-  void* sym = nullptr;
-  if (cudaGetSymbolAddress(&sym, hc::dev::g_timeline) == cudaSuccess) cudaMemset(sym, 0, sizeof(hc::dev::g_timeline));
-  return 0;
-}
-#endif
+HC_TL_READ(hc_debug_timeline)

@@ -155,18 +155,6 @@ struct DecParams {
 struct TensorMaps {
   CUtensorMap m[kMaxDst];
 };
-// Pre-pass that turns the rate bytes of n_in streams (tiles_per_seg tiles each, nrate rate bytes
-// each) into per-tile arrival flags: flags[q][t] = flag_pack(tag, byte offset of tile t's payload).
-struct OffsetParams {
-  const uint8_t* in[kMaxIn];
-  uint64_t in_size[kMaxIn];
-  uint64_t* flags[kMaxIn];
-  uint32_t n_in;
-  uint32_t tiles_per_seg;
-  uint64_t nrate;
-  uint32_t tag;
-  Workspace ws;  // grp_a / grp_b hold the chain of CTA totals
-};
 
 namespace dev {
 
@@ -177,12 +165,6 @@ __device__ __forceinline__ void lorenzo_forward(const int32_t (&q)[32], int32_t 
   constexpr int S = MODE == kModeVec ? 4 : 1;
 #pragma unroll
   for (int i = 31; i >= 0; --i) d[i] = i >= S ? q[i] - q[i - S] : q[i];
-}
-template <int MODE>
-__device__ __forceinline__ void lorenzo_inverse(int32_t (&d)[32]) {
-  constexpr int S = MODE == kModeVec ? 4 : 1;
-#pragma unroll
-  for (int i = S; i < 32; ++i) d[i] += d[i - S];
 }
 
 struct TileCode {
@@ -364,22 +346,6 @@ __device__ __forceinline__ void decode_block(const uint8_t* cbuf, uint32_t pos, 
   for (int i = 0; i < 32; ++i) {
     const int32_t m = (int32_t)(sign << i) >> 31;
     d[i] = ((int32_t)T[i ^ 7] ^ m) - m;
-  }
-}
-
-// staged payload -> quantised values q[0..31]: sign application and inverse Lorenzo in one pass
-// (q_i = q_{i-S} + (|d_i| ^ m_i) - m_i is a single three-input add per element)
-template <int MODE>
-__device__ __forceinline__ void decode_block_quant(const uint8_t* cbuf, uint32_t pos, uint32_t rate, int W,
-                                                   int32_t (&q)[32]) {
-  constexpr int S = MODE == kModeVec ? 4 : 1;
-  uint32_t T[32];
-  const uint32_t sign = decode_magnitudes(cbuf, pos, rate, W, T);
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int32_t m = (int32_t)(sign << i) >> 31;
-    const int32_t t = (int32_t)T[i ^ 7] ^ m;
-    q[i] = i >= S ? q[i - S] + t - m : t - m;
   }
 }
 

@@ -22,15 +22,11 @@ int device_sm_count();
 // `overlap`: programmatic dependent launch: the kernel may start as soon as every CTA of the previous
 // kernel on the stream is running, and fills the SMs as that kernel's CTAs leave.  Only for launches
 // whose inputs are ordered by arrival flags, with a workspace view of their own set.
-cudaError_t launch_encode(int op, int mode, EncParams p, cudaStream_t stream, bool overlap = false);
+// A step of a collective (mode outlier): kOpCompress or kOpAddF32.
+cudaError_t launch_encode(int op, EncParams p, cudaStream_t stream, bool overlap = false);
 // Stand-alone compression of n_seg arrays, or sum of n_in streams and a local operand (hc_encode.cu).
 cudaError_t launch_encode_solo(int op, int mode, SoloParams p, cudaStream_t stream);
 cudaError_t launch_decode(int mode, DecParams p, cudaStream_t stream, bool overlap = false);
-// Per-tile payload offsets of stand-alone input streams as arrival flags (see OffsetParams);
-// offsets_fit says whether the workspace of a handle sized for max_elems has room for the flags of
-// n_in streams of tiles_per_seg tiles and for the pre-pass's own chain.
-bool offsets_fit(const Workspace& ws, size_t max_elems, uint32_t n_in, uint32_t tiles_per_seg);
-cudaError_t launch_offsets(const OffsetParams& p, cudaStream_t stream);
 cudaError_t launch_quant_pred(int mode, const float* x, int32_t* deltas, uint64_t n, float eb, cudaStream_t stream);
 cudaError_t launch_sum(float* dst, const float* a, const float* b, const float* c, const float* d, uint64_t n,
                        cudaStream_t stream);

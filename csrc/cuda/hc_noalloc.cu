@@ -69,8 +69,7 @@ int hc_compress_noalloc(const float* d_x, size_t n, float eb, uint8_t* d_out, si
     if (d_size && cudaMemsetAsync(d_size, 0, sizeof(uint64_t), stream) != cudaSuccess) return hc::kErrCuda;
     return hc::kOk;
   }
-  // Nothing is cleared here.  The ticket and exit counters (words 8 and 9 of the array) are put back
-  // to zero by the last CTA of every launch, the look-back words behind the header are told apart by
+  // Nothing is cleared here.  The kernel leaves the exchange words zero, its other words are told apart by
   // the call number (epoch), and the status word (word 2) is sticky on purpose: it keeps the first
   // error until hc_noalloc_status(1) has shown it to the caller, and a time-out left there makes
   // later calls return without output until then.
@@ -81,18 +80,17 @@ int hc_compress_noalloc(const float* d_x, size_t n, float eb, uint8_t* d_out, si
       return hc::kErrCuda;
     d->epoch = 1;
   }
-  hc::EncParams p;
+  hc::SoloParams p;
   memset(&p, 0, sizeof(p));
   p.n_seg = 1;
   p.local[0] = d_x;
   p.n[0] = n;
   p.recip = 0.5f / eb;
-  p.n_dst = 1;
   p.out[0] = d_out;
   p.out_cap = cap;
   p.size_out = d_size;
   p.ws = hc::workspace_view(d->scratch, HC_NOALLOC_MAX_ELEMS, d->epoch, g_timeout_ns);
-  return hc::launch_encode(hc::kOpCompress, hc::kModeOutlier, p, stream) == cudaSuccess ? hc::kOk : hc::kErrCuda;
+  return hc::launch_encode_solo(hc::kOpCompress, hc::kModeOutlier, p, stream) == cudaSuccess ? hc::kOk : hc::kErrCuda;
 }
 
 }  // extern "C"

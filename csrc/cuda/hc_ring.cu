@@ -320,7 +320,7 @@ static int allreduce_ring(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t
     }
     p.sparse = c->sparse ? 1u : 0u;
     p.ws = next_ws(c, stream);
-    if (hc::launch_encode(s == 0 ? hc::kOpCompress : hc::kOpAddF32, hc::kModeOutlier, p, stream, overlapped()) !=
+    if (hc::launch_encode(s == 0 ? hc::kOpCompress : hc::kOpAddF32, p, stream, overlapped()) !=
         cudaSuccess)
       return hc::kErrCuda;
     mark();
@@ -415,7 +415,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
       p.sparse = c->sparse ? 1u : 0u;
       if (overlap && c->share_scatter) p.grid_limit = (uint32_t)(hc::device_sm_count() * c->share_scatter);
       p.ws = next_ws(c, stream);
-      if (hc::launch_encode(hc::kOpCompress, hc::kModeOutlier, p, stream) != cudaSuccess) return hc::kErrCuda;
+      if (hc::launch_encode(hc::kOpCompress, p, stream) != cudaSuccess) return hc::kErrCuda;
       launched = true;
     }
   }
@@ -451,7 +451,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
     p.variant = (uint32_t)c->reduce_variant;
     p.sparse = c->sparse ? 1u : 0u;
     p.ws = next_ws(c, stream);
-    if (hc::launch_encode(hc::kOpAddF32, hc::kModeOutlier, p, stream, overlap && launched) !=
+    if (hc::launch_encode(hc::kOpAddF32, p, stream, overlap && launched) !=
         cudaSuccess)
       return hc::kErrCuda;
     launched = true;
@@ -572,7 +572,7 @@ static int allreduce_onestep(hc_comm* c, const float* d_sbuf, float* d_rbuf, siz
     if (c->mc && P > 1) p.out_mc = c->mc + L.data_off(slot);
     p.sparse = c->sparse ? 1u : 0u;
     p.ws = next_ws(c, stream);
-    if (hc::launch_encode(hc::kOpCompress, hc::kModeOutlier, p, stream) != cudaSuccess) return hc::kErrCuda;
+    if (hc::launch_encode(hc::kOpCompress, p, stream) != cudaSuccess) return hc::kErrCuda;
   }
   mark();
   NvtxRange decode_range("hc one-step: decode + sum");

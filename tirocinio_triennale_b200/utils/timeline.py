@@ -3,11 +3,13 @@
     HC_TIMELINE=1 python -m tirocinio_triennale_b200.utils.timeline --n 16777216 --ops compress,decompress,hom_add,reduce7
 
 The instrumented library (``_build.build_cuda(timeline=True)`` -> ``libhomcomp_b200_tl.so``) makes
-every CTA write, for the last four launches, nanosecond stamps of its first tile's way through the
-loader / compute / scanner warps (slots 0-15) and, for its first compute warp, the SM-clock cycles
-spent in each phase of the tile loop (slots 16-30) plus the number of tiles it handled (slot 31).
-``hc_debug_timeline`` copies them to the host.  This module runs one operation at a time and prints
-the device span of the launch (first CTA in to last CTA out) and the share of each phase.
+every CTA write, for the last four launches, nanosecond stamps of its start and end (slots 0 and 7) and,
+for its first compute warp, the SM-clock cycles spent in each phase of the loop (slots 16-30) plus the
+number of sub-tiles it handled (slot 31); the kernels of the collective steps also stamp their first
+tile's way through the loader / compute / scanner warps (slots 1-15).  ``hc_debug_timeline`` (collective
+steps), ``hc_debug_timeline_encode`` and ``hc_debug_timeline_decode`` (stand-alone calls) copy them to
+the host.  This module runs one stand-alone operation at a time and prints the device span of the launch
+(first CTA in to last CTA out) and the share of each phase.
 The reference has no tracing of any kind (its thesis used Nsight Compute by hand).
 """
 from __future__ import annotations
@@ -19,19 +21,18 @@ import os
 import numpy as np
 
 SLOTS = 32
-ENCODE_PHASES = ["wait input stream", "decode input", "wait fp32 tile", "load+quantise+lorenzo", "analyse",
-                 "(unused)", "copy out (+wait for ring space)", "pack", "scan (barrier)", "rate store+transpose",
-                 "S: wait tile total", "S: look-back"]
-N_COMPUTE_PHASES = 10  # "S:" entries are the scanner warp's
-DECODE_PHASES = ["wait input stream", "decode", "dequantise", "wait tma store+barrier", "store tile+barrier"]
+ENCODE_PHASES = ["between turns", "wait fp32 rows", "quantise+lorenzo", "stage+wait input stream", "decode+add",
+                 "code+scan", "copy out (+wait for ring space)", "pack", "drain"]
+DECODE_PHASES = ["offsets", "stage", "wait input stream", "decode", "signs+sum+dequantise", "store"]
 
 
-def read(lib) -> np.ndarray:
-    """(4 launches, 1024 CTAs, 32 slots) int64; clears the device copy."""
-    lib.hc_debug_timeline.restype = C.c_int
-    lib.hc_debug_timeline.argtypes = [C.c_void_p]
+def read(lib, what="") -> np.ndarray:
+    """(4 launches, 1024 CTAs, 32 slots) int64; clears the device copy.  ``what``: "", "_encode" or "_decode"."""
+    fn = getattr(lib, "hc_debug_timeline" + what)
+    fn.restype = C.c_int
+    fn.argtypes = [C.c_void_p]
     a = np.zeros((4, 1024, SLOTS), dtype=np.uint64)
-    if lib.hc_debug_timeline(a.ctypes.data) != 0:
+    if fn(a.ctypes.data) != 0:
         raise RuntimeError("hc_debug_timeline failed")
     return a.astype(np.int64)
 
@@ -45,13 +46,12 @@ def summarise(a: np.ndarray, phases):
         if not len(g):
             continue
         cyc = g[:, 16:16 + len(phases)].sum(axis=0).astype(np.float64)
-        nc = N_COMPUTE_PHASES if len(phases) > N_COMPUTE_PHASES else len(phases)
-        tot = cyc[:nc].sum()
+        tot = cyc.sum()
         out.append({
             "span_us": (g[:, 7].max() - g[:, 0].min()) / 1e3,
             "start_spread_us": (g[:, 0].max() - g[:, 0].min()) / 1e3,
-            "ctas": int(len(g)), "tiles_first_warp": int(g[:, SLOTS - 1].sum()),
-            "cycles_per_tile": tot / max(1, int(g[:, SLOTS - 1].sum())),
+            "ctas": int(len(g)), "subtiles_first_warp": int(g[:, SLOTS - 1].sum()),
+            "cycles_per_subtile": tot / max(1, int(g[:, SLOTS - 1].sum())),
             "phase_share": {p: (c / tot if tot else 0.0) for p, c in zip(phases, cyc)},
         })
     return out
@@ -82,7 +82,7 @@ def main():
     dec = torch.empty_like(x)
     size2 = torch.zeros_like(size)
     flush = torch.empty(64 * 1024 * 1024, dtype=torch.int32, device="cuda")
-    read(lib)
+    read(lib, "_encode")
     parts = None
     for op in args.ops.split(","):
         for rep in range(args.reps):
@@ -103,15 +103,15 @@ def main():
                     chunk = n // 8 // 4096 * 4096
                     parts = codec.compress_batch([x[(k + 1) * chunk: (k + 2) * chunk] for k in range(7)], args.eb)
                     part_bytes = [int(v) for v in parts[1].tolist()]
-                    read(lib)
+                    read(lib, "_encode")
                 codec.hom_add_multi(parts[0], y[:chunk], args.eb, stream_bytes=part_bytes)
                 phases = ENCODE_PHASES
             else:
                 raise SystemExit("unknown op " + op)
-            for s in summarise(read(lib), phases):
+            for s in summarise(read(lib, "_decode" if phases is DECODE_PHASES else "_encode"), phases):
                 shares = ", ".join("%s %.0f%%" % (k, 100 * v) for k, v in s["phase_share"].items())
-                print("%s rep %d: span %.1f us, %d CTAs (start spread %.1f us), %.0f cycles/tile of the first compute "
-                      "warp: %s" % (op, rep, s["span_us"], s["ctas"], s["start_spread_us"], s["cycles_per_tile"],
+                print("%s rep %d: span %.1f us, %d CTAs (start spread %.1f us), %.0f cycles/sub-tile of the first compute "
+                      "warp: %s" % (op, rep, s["span_us"], s["ctas"], s["start_spread_us"], s["cycles_per_subtile"],
                                     shares), flush=True)
     assert codec.status() == 0
 
