@@ -476,6 +476,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
           from_row(d, c);
           ints = true;
         }
+        if (tid == 0) HC_PH(4);
       }
       if (!kFloat) {
 #pragma unroll
