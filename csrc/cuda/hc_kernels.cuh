@@ -1,16 +1,15 @@
-// The sm_100a codec kernels: one persistent, warp-specialised kernel family for everything that
-// produces a stream (compress, and the three homomorphic adds) and one for everything that
-// consumes a stream into fp32 (decompress).
+// The kernel that produces the streams of collective steps (compress into the peers' slots, sum of received
+// streams and the local chunk): persistent and warp-specialised.  Also here: the parameters of all codec kernels,
+// the look-back, and the workspace.  Stand-alone calls run hc_encode.cu; every decode runs hc_decode.cu.
 //
 // Geometry.  A tile is 128 consecutive 32-element blocks (4096 values, 16 KB of fp32).  A CTA has
 // four COMPUTE warps in which thread t owns block t of the tile, i.e. one thread per block with
 // the whole block in registers, plus a LOADER warp and a SCANNER warp:
 //   loader   starts with tile blockIdx.x and takes further tiles from a ticket counter two turns
 //            ahead, issues the 2-D TMA tiled load of the fp32 tile ({32, 128} box, 128-byte
-//            swizzle; 3 stages for compress, 2 for the adds, 1 in the add variant that runs four
-//            CTAs per SM); for the homomorphic adds it also reads the rate bytes of every input
+//            swizzle; 2 stages for compress, 1 for the add); for the add it also reads the rate bytes of every input
 //            stream's tile one turn ahead, scans them, learns the payload offset (from the tile's
-//            arrival flag in a collective step, from a look-back over the INPUT stream otherwise)
+//            arrival flag)
 //            and brings the payload bytes into shared memory with one bulk copy (up to 8 streams
 //            per tile through two staging buffers);
 //   compute  decodes the staged payloads to deltas and sums them, moves the PREVIOUS tile's packed

@@ -70,15 +70,13 @@ int hc_codec_set_timeout_ms(hc_codec* c, unsigned ms);
 // Synchronises the device, returns the sticky hc::Status of the handle and clears it when asked.
 int hc_codec_status(hc_codec* c, int clear);
 // After a status 3 (time-out): which wait ran out FIRST in the launch that failed (call it before
-// clearing the status).  1 loader: fp32 stage not released, 2 loader: input buffer not released,
-// 3 compute: input stream not staged, 4 compute: fp32 tile not landed, 5 compute: no room in the
-// payload ring, 6 scanner: tile total missing, 7 copier: look-back result missing, 8 copier: tile not
-// packed, 9 / 10 the decoder's loader / compute warps, 11 a look-back over tile totals; 0 none.
+// clearing the status).  1 loader: fp32 stage not released, 2 input buffer not released or input offsets
+// missing, 3 compute: input stream not staged, 4 compute: fp32 rows not landed, 5 compute: no room in the
+// payload ring, 6 scanner: tile total missing, 7 place of a packed payload missing, 8 copier: tile not
+// packed, 10 decoder: payload not landed, 11 totals of other CTAs; 0 none.
 int hc_codec_status_site(hc_codec* c);
-// Stand-alone decompress / homomorphic adds on large streams (16 MiB of values and up) first run a
-// small kernel that turns the input's rate bytes into per-tile payload offsets, so the main kernel
-// stages every tile without a look-back over the input (two launches instead of one; on by
-// default).  0 turns it off: one launch, input offsets by decoupled look-back.  Same output bytes.
+// Kept for callers of earlier versions, which ran a small kernel for the payload offsets of large streams
+// or did without: every call is one launch now, whatever was set here.
 int hc_codec_set_prepass(hc_codec* c, int on);
 
 int hc_compress(hc_codec* c, const float* d_x, size_t n, float eb, int mode, uint8_t* d_out, size_t cap,

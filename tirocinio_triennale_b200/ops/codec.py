@@ -60,8 +60,8 @@ class Codec:
             return int(self.lib.hc_codec_status_site(self._h))
 
     def set_prepass(self, on: bool = True):
-        """Large stand-alone inputs: tile offsets from a small pre-pass kernel (default) or from a
-        look-back inside the consuming kernel (``False``).  Same bytes either way."""
+        """Kept for callers of earlier versions (a choice between two ways to the payload offsets of large
+        inputs); without effect."""
         _lib.check(self.lib.hc_codec_set_prepass(self._h, 1 if on else 0), "set_prepass")
 
     def status(self, clear: bool = True) -> int:
