@@ -537,10 +537,12 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
         }
       }
       if (room && k - copied < (uint32_t)kSlots - 1u) break;
+      if (tid == 0) HC_PH(6);
       if (!warp_wait(&sh.placed[copied % kSlots], (copied / kSlots) & 1u, ws, kSiteComputeRing)) {
         failed = true;
         break;
       }
+      if (tid == 0) HC_PH(9);
       copy_oldest();
     }
     t = t_next;

@@ -22,7 +22,8 @@ import numpy as np
 
 SLOTS = 32
 ENCODE_PHASES = ["between turns", "wait fp32 rows", "quantise+lorenzo", "stage+wait input stream", "decode+add",
-                 "code+scan", "copy out (+wait for ring space)", "pack", "drain"]
+                 "code+scan", "copy out", "pack", "drain",
+                 "wait for the place of the oldest payload"]
 DECODE_PHASES = ["offsets", "stage", "wait input stream", "decode", "signs+sum+dequantise", "store"]
 
 
