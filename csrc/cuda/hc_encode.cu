@@ -367,7 +367,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     const uint32_t start = __shfl_sync(0xffffffffu, my_start, (int)r), tot = __shfl_sync(0xffffffffu, my_tot, (int)r);
     const uint64_t at = sh.out_at[r][warp];
     if (tot) {
-      if (at != ~0ull) copy_ring(oring + start, p.out[__shfl_sync(0xffffffffu, my_seg, (int)r)] + at, tot);
+      if (at != ~0ull) copy_ring(oring + start, (p.n_seg == 1u ? p.out[0] : p.out[__shfl_sync(0xffffffffu, my_seg, (int)r)]) + at, tot);
       tail = start + room_for(tot);
       if (--taken == 0) head = tail = 0;
     }
@@ -522,7 +522,11 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
 
     if (tid == 0) HC_PH(5);
     // payloads whose place is known leave; the oldest ones have to where this one needs their room
-    while (copied < k && placed(copied)) copy_oldest();
+    // (one a turn keeps the pace; a second look pays only where they pile up)
+    if (copied < k && placed(copied)) {
+      copy_oldest();
+      while (copied + 2u < k && placed(copied)) copy_oldest();
+    }
     const uint32_t need = room_for(tot);
     uint32_t start = head;
     while (true) {
