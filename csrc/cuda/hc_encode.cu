@@ -176,42 +176,20 @@ __device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32
 }
 
 // ---- blocks beyond the reach of the subnormal form ------------------------------------------------------------------
-// Out of line and on copies in local memory: kept inline, the int32 arithmetic of these blocks took registers and
-// instruction cache from the common path (64 MB add: 56 us inline, 52 this way).
-struct Row {
-  uint32_t v[32];
-};
-// the deltas of row `row` of the stage in int32
-template <int MODE>
-__device__ __noinline__ void cold_local(Row* d, const uint8_t* stage, int row, float recip) {
+// Row `row` of the stage: fp32 values -> deltas in int32, or their sign and magnitude.  Out of line, and through the stage:
+// kept inline it took registers and instruction cache from the common path (64 MB add: 56 us inline, 52 out of line), and
+// handed over in local memory it went to L2 and back (32 M values of a random walk with most blocks of this kind, add of
+// a stream: 236 us, 126 this way; compress 80, 65).
+template <int MODE, bool SIGN>
+__device__ __noinline__ void cold_local(uint8_t* stage, int row, float recip) {
   uint32_t x[32];
   load_row_swizzled(stage, row, x);
   deltas_int<MODE>(x, recip);
+  if (SIGN) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) d->v[i] = x[i];
-}
-// d += the deltas of a decoded block (rows as decode_rows leaves them), in int32; `subs`: d_1 .. d_31 still are subnormals
-__device__ __noinline__ void cold_add_block(Row* d, const Row* T, uint32_t sign, bool subs) {
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const uint32_t m = (uint32_t)((int32_t)(sign << i) >> 31);
-    const uint32_t b = d->v[i];
-    d->v[i] = (subs && i ? sub_to_int(b) : b) + (T->v[i ^ 7] ^ m) - m;
+    for (int i = 0; i < 32; ++i) x[i] = sign_magnitude(x[i]);
   }
-}
-__device__ __noinline__ void cold_sign_magnitude(Row* d) {
-#pragma unroll
-  for (int i = 0; i < 32; ++i) d->v[i] = sign_magnitude(d->v[i]);
-}
-__device__ __forceinline__ Row row_of(const uint32_t (&d)[32]) {
-  Row r;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) r.v[i] = d[i];
-  return r;
-}
-__device__ __forceinline__ void from_row(uint32_t (&d)[32], const Row& r) {
-#pragma unroll
-  for (int i = 0; i < 32; ++i) d[i] = r.v[i];
+  store_row_swizzled(stage, row, x);
 }
 
 // ---- the kernel --------------------------------------------------------------------------------------------------
@@ -416,16 +394,10 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
         // exact when no quantised value of the block reaches 2^24: |q_0| below 2^23 and 31 differences below 2^18
         or_tail = or_tail_of(d);
         if (!__all_sync(0xffffffffu, or_tail < (1u << 18) && (d[0] & 0x7fffffffu) < (1u << 23))) {
-          Row c;
-          cold_local<MODE>(&c, stage, (int)lane, p.recip);
-          if (!kHasIn) {
-            cold_sign_magnitude(&c);
-            from_row(d, c);
-            or_tail = or_tail_of(d);
-          } else {
-            from_row(d, c);
-            ints = true;
-          }
+          cold_local<MODE, !kHasIn>(stage, (int)lane, p.recip);
+          load_row_swizzled(stage, (int)lane, d);
+          if (!kHasIn) or_tail = or_tail_of(d);
+          else ints = true;
         } else if (kHasIn) {
           d[0] = sub_to_int(d[0]);
         }
@@ -470,11 +442,16 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
 #pragma unroll
           for (int i = 1; i < 32; ++i) d[i] = as_u(__fadd_rn(as_f(d[i]), signed_sub(T[i ^ 7], sign, i)));
         } else {
-          Row c = row_of(d);
-          const Row tr = row_of(T);
-          cold_add_block(&c, &tr, sign, !ints);
-          from_row(d, c);
-          ints = true;
+          if (!ints) {
+#pragma unroll
+            for (int i = 1; i < 32; ++i) d[i] = sub_to_int(d[i]);
+            ints = true;
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const uint32_t m = (uint32_t)((int32_t)(sign << i) >> 31);
+            d[i] += (T[i ^ 7] ^ m) - m;
+          }
         }
         if (tid == 0) HC_PH(4);
       }
@@ -482,9 +459,8 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
 #pragma unroll
         for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
       } else if (ints) {
-        Row c = row_of(d);
-        cold_sign_magnitude(&c);
-        from_row(d, c);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
       } else {
         d[0] = sign_magnitude(d[0]);
       }
