@@ -42,6 +42,7 @@ static_assert(32 * 132 + 32 <= kInUsable, "one payload must fit");
 struct EncShared {
   uint64_t stage_full[kEncWarps];
   uint64_t in_full[enc_warps(kOpAddF32)][4];
+  uint64_t totals[kSlots];                      // tot[] of the chunk is complete (one arrival per compute warp)
   uint64_t placed[kSlots];                      // out_at[] of the chunk is valid
   uint64_t in_known[kInSlots];                  // in_at[] of the chunk is valid (one arrival per stream)
   uint64_t out_at[kSlots][kEncWarps];           // byte offset of the warp's payload; ~0: not to be stored
@@ -78,16 +79,23 @@ __device__ __forceinline__ void advance_base(const uint64_t* words, uint32_t& ne
   }
 }
 
-// "All compute warps have put down their total of chunk k": hardware barrier 1 + k % kSlots; they arrive, the clerk
-// waits (polling an mbarrier instead it took up to half of the issue slots of its scheduler).  A warp comes to chunk
-// k + kSlots only after chunk k has been placed, so no barrier is entered twice.  The wait has no time limit of its
-// own: it ends because every compute warp arrives once for every chunk of its CTA, one that gave up on something
-// included.
-__device__ __forceinline__ void totals_arrive(uint32_t k, uint32_t nc) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(1u + k % kSlots), "r"(32u * nc + 32u) : "memory");
-}
-__device__ __forceinline__ void totals_wait(uint32_t k, uint32_t nc) {
-  asm volatile("bar.sync %0, %1;" ::"r"(1u + k % kSlots), "r"(32u * nc + 32u) : "memory");
+// The clerk's wait for the totals of chunk k.  The hardware suspends the warp for up to kTotalsNap ns a try, so that
+// polling does not take issue slots from the compute warps (100 ns to 20 us measure the same).  False: it ran out, or another wait of the launch
+// has (recorded).  A hardware barrier (bar.sync) will not do here: it has no time limit, and a warp that gave up
+// would have to go on arriving, in step with the others, for the clerk ever to come back.
+constexpr uint32_t kTotalsNap = 2000;
+__device__ __forceinline__ bool totals_wait(EncShared& sh, uint32_t k, const Workspace& ws) {
+  uint64_t* const bar = &sh.totals[k % kSlots];
+  const uint32_t parity = (k / kSlots) & 1u;
+  if (__all_sync(0xffffffffu, mbar_try_wait_for(bar, parity, kTotalsNap))) return true;
+  const long long t0 = clock64();
+  const long long limit_clk = (long long)ws.spin_limit_ns * 2;
+  for (uint32_t it = 0; it < (1u << 26); ++it) {
+    if (__all_sync(0xffffffffu, mbar_try_wait_for(bar, parity, kTotalsNap))) return true;
+    if ((it & 15u) == 15u && __any_sync(0xffffffffu, clock64() - t0 > limit_clk || fatal_error(ws.ctrl))) break;
+  }
+  if ((threadIdx.x & 31u) == 0u) note_timeout(ws, kSiteScannerTotal);
+  return false;
 }
 
 // ---- the clerk ---------------------------------------------------------------------------------------------------
@@ -122,7 +130,8 @@ __device__ __forceinline__ void input_offsets(const SoloParams& p, EncShared& sh
 }
 
 // Adds up the chunk totals, places the payloads; keeps the input offsets kInSlots chunks ahead of the compute warps and
-// the published input totals two chunks ahead of that (the first chunk's inputs are the compute warps' work).
+// the published input totals two chunks ahead of that (the first chunk's inputs are the compute warps' work).  Leaves when
+// a compute warp has given up; what that leaves unplaced runs out in the others' waits.
 __device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32_t nc, uint32_t subs) {
   const uint32_t lane = threadIdx.x & 31u;
   const Workspace& ws = p.ws;
@@ -136,7 +145,7 @@ __device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32
   if (p.n_in) {
     for (uint32_t k = 1; k <= kLead; ++k)
       if (ticket(p, k) != kNoTile) publish_inputs(p, nc, subs, ticket(p, k), 0u, 1u);
-    warp_wait(&sh.in_known[0], 0u, ws, kSiteLoaderInFree);  // in_run is the compute warps' until then
+    if (!warp_wait(&sh.in_known[0], 0u, ws, kSiteLoaderInFree)) return;  // in_run is the compute warps' until then
     for (uint32_t k = 1; k < (uint32_t)kInSlots; ++k) inputs_ahead(k);
   }
   uint32_t next = 0;  // chunks [first of the segment, next) are in base
@@ -146,7 +155,7 @@ __device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32
     const uint32_t t = ticket(p, k);
     if (t == kNoTile) break;
     const uint32_t r = k % kSlots;
-    totals_wait(k, nc);
+    if (!totals_wait(sh, k, ws)) return;
     const uint32_t tot = lane < nc ? sh.tot[r][lane] : 0u;
     const uint32_t inc = warp_inclusive_scan(tot, (int)lane);
     const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
@@ -214,6 +223,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       for (int i = 0; i < 4; ++i) mbar_init(&sh.in_full[tid][i], 1);
   } else if (warp == 1u) {
     if (lane < (uint32_t)kSlots) {
+      mbar_init(&sh.totals[lane], nc);
       mbar_init(&sh.placed[lane], 1);
       sh.sum[lane] = 0;
     }
@@ -353,20 +363,17 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   };
   auto placed = [&](uint32_t k) -> bool { return __all_sync(0xffffffffu, mbar_test(&sh.placed[k % kSlots], (k / kSlots) & 1u)); };
 
-  bool failed = false;  // a wait ran out (recorded)
+  // A warp whose wait ran out (recorded) leaves.  Every wait of the others has a limit of its own, so they follow.
+  bool failed = false;
+  uint32_t k = 0, rows = 0, read = 0;  // failed: the chunk whose rows, the input job that may still be on their way
   if (tid == 0) HC_PH_START();
-  for (uint32_t k = 0;; ++k) {
+  for (;; ++k) {
     if (t == kNoTile) {
-      for (; copied < k && !failed;) {
+      while (copied < k) {
         if (!warp_wait(&sh.placed[copied % kSlots], (copied / kSlots) & 1u, ws, kSiteCopierBase)) break;
         copy_oldest();
       }
       break;
-    }
-    if (failed) {  // nothing more from this warp, but the clerk counts on it
-      totals_arrive(k, nc);
-      t = ticket(p, k + 1);
-      continue;
     }
     if (tid == 0) HC_PH(0);
     const Where w = where(t);
@@ -376,7 +383,12 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     uint32_t or_tail = 0;
     // ---- local operand: first, because it needs nothing but its rows --------------------------------------------------
     if (kHasLocal) {
-      if (!warp_wait(&sh.stage_full[warp], k & 1u, ws, kSiteComputeTile)) failed = true;
+      if (!warp_wait(&sh.stage_full[warp], k & 1u, ws, kSiteComputeTile)) {
+        failed = true;
+        rows = k;
+        read = k * Q;
+        break;
+      }
       if (tid == 0) HC_PH(1);
       if (!by_tma(w)) {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(p.local[w.seg]);
@@ -418,7 +430,12 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
           if (staged == before) break;
         }
         const uint32_t v = k * Q + q;
-        if (!warp_wait(&sh.in_full[warp][v & 3u], (v >> 2) & 1u, ws, kSiteComputeInFull)) cur_rate = 0, failed = true;
+        if (!warp_wait(&sh.in_full[warp][v & 3u], (v >> 2) & 1u, ws, kSiteComputeInFull)) {
+          failed = true;
+          rows = k + 1u;
+          read = v;
+          break;
+        }
         if (tid == 0) HC_PH(3);
         uint32_t T[32], sign, a0;
         decode_rows(inring, cur_pos, cur_rate, plane_width(__reduce_max_sync(0xffffffffu, cur_rate & 31u)), sign, a0, T);
@@ -455,6 +472,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
         }
         if (tid == 0) HC_PH(4);
       }
+      if (failed) break;
       if (!kFloat) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
@@ -488,8 +506,8 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       before = __shfl_sync(0xffffffffu, before, 0);
       if (before >> 24 == nc - 1u) give_total(ws.sums, (before & 0xffffffu) + tot);
     }
+    if (lane == 0) mbar_arrive(&sh.totals[k % kSlots]);
     __syncwarp();
-    totals_arrive(k, nc);
     const uint32_t subs = p.subs[w.seg];
     uint8_t* const rates = p.out[w.seg];
     if (w.sub < subs) rates[(uint64_t)w.sub * kSubBlocks + lane] = (uint8_t)code.rate;
@@ -520,13 +538,15 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       if (tid == 0) HC_PH(6);
       if (!warp_wait(&sh.placed[copied % kSlots], (copied / kSlots) & 1u, ws, kSiteComputeRing)) {
         failed = true;
+        rows = k + 1u;
+        read = rows * Q;
         break;
       }
       if (tid == 0) HC_PH(9);
       copy_oldest();
     }
     t = t_next;
-    if (failed) continue;
+    if (failed) break;
     if (tid == 0) HC_PH(6);
     __syncwarp();
     pack_blocks(oring + start, inc - code.len, code, d, plane_width(__reduce_max_sync(0xffffffffu, code.rate & 31u)));
@@ -543,6 +563,10 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       HC_PH(7);
       HC_PH_COUNT();
     }
+  }
+  if (failed) {  // nothing may land in shared memory once the CTA has left it
+    if (kHasLocal && ticket(p, rows) != kNoTile) mbar_wait_bounded(&sh.stage_full[warp], rows & 1u, ws.spin_limit_ns);
+    for (; kHasIn && read < jobs; ++read) mbar_wait_bounded(&sh.in_full[warp][read & 3u], (read >> 2) & 1u, ws.spin_limit_ns);
   }
   if (tid == 0) HC_PH(8);
   if (lane == 0) HC_STAMP_MAX(7);

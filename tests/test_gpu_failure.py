@@ -58,6 +58,43 @@ def test_corrupted_rate_bytes_are_contained():
     assert codec.status() == 0
 
 
+@pytest.mark.parametrize("op", ["compress", "hom_add"])
+def test_grid_that_is_not_resident_as_a_whole_gives_up(op):
+    """Another kernel keeps half of the SMs for longer than the waits may take, so half of the CTAs of a launch with ten
+    chunks and more a CTA never publish a total: the others' waits run out in every role, the launch ends with
+    status 3, and the handle works again once that has been read."""
+    n, eb, held = 30_000_000, 1e-4, 74
+    x = torch.randn(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)) * 0.01
+    codec = ops.Codec(2 * n)
+
+    def call():
+        return codec.compress(x, eb) if op == "compress" else codec.hom_add(s, x, eb, stream_bytes=s_bytes)
+
+    s, size = codec.compress(x, eb)
+    s_bytes = int(size)
+    want, size = call()
+    want = want[:int(size)].clone()
+    # the holder: a decode whose flags nothing raises, one CTA a tile, gone after its own 400 ms
+    holder = ops.Codec(held * codec.tile_elems, timeout_ms=400)
+    flags = torch.zeros(held, dtype=torch.int64, device="cuda")
+    y = torch.empty(held * codec.tile_elems, device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        holder.decompress_flagged(s, y.numel(), eb, flags, want=5, out=y, stream_bytes=s_bytes)
+    time.sleep(0.02)
+    codec.set_timeout_ms(20)
+    t0 = time.time()
+    call()
+    assert codec.status() == 3
+    assert time.time() - t0 < 5
+    assert holder.status() == 6
+    codec.set_timeout_ms(2000)
+    got, size = call()
+    assert codec.status() == 0 and int(size) == want.numel()
+    assert torch.equal(got[:want.numel()], want)
+
+
 def _missing_peer(rank, world):
     """A rank that is alive but sits one call out.  Host-made failure: no kernel faults or hangs; the
     other rank's bounded waits run out, it reads status 6, the ranks realign their call numbers over
