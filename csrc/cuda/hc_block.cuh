@@ -78,11 +78,12 @@ __device__ __forceinline__ void store_row_swizzled(uint8_t* rows, int row, const
                  "r"(w[4 * c + 3]), "r"(r ^ (c << 4))
                  : "memory");
 }
-// plain-load path (unaligned base, tiny inputs) and the ragged last row
+// plain-load path (unaligned base, tiny inputs) and the ragged last row.  Coherent loads, not __ldg: in an allreduce in
+// place a step that is already running writes to the array that this one reads.
 __device__ __forceinline__ void load_row_global(const uint32_t* base, uint64_t n, uint64_t row, uint32_t (&w)[32]) {
   uint64_t o = row * kBlock;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) w[i] = (o + i < n) ? __ldg(base + o + i) : 0u;
+  for (int i = 0; i < 32; ++i) w[i] = (o + i < n) ? base[o + i] : 0u;
 }
 
 // ---- payload lengths ----------------------------------------------------------------------------------

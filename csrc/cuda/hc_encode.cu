@@ -80,9 +80,9 @@ __device__ __forceinline__ void advance_base(const uint64_t* words, uint32_t& ne
 }
 
 // The clerk's wait for the totals of chunk k.  The hardware suspends the warp for up to kTotalsNap ns a try, so that
-// polling does not take issue slots from the compute warps (100 ns to 20 us measure the same).  False: it ran out, or another wait of the launch
-// has (recorded).  A hardware barrier (bar.sync) will not do here: it has no time limit, and a warp that gave up
-// would have to go on arriving, in step with the others, for the clerk ever to come back.
+// polling does not take issue slots from the compute warps (100 ns to 20 us measure the same).  False: it ran out, or
+// another wait of the launch has (recorded).  A hardware barrier (bar.sync) will not do here: it has no time limit, and
+// a warp that gave up would have to go on arriving, in step with the others, for the clerk ever to come back.
 constexpr uint32_t kTotalsNap = 2000;
 __device__ __forceinline__ bool totals_wait(EncShared& sh, uint32_t k, const Workspace& ws) {
   uint64_t* const bar = &sh.totals[k % kSlots];
@@ -393,10 +393,11 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       if (!by_tma(w)) {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(p.local[w.seg]);
         const uint64_t first = (uint64_t)w.sub * kSubValues, n = n_local(w.seg);
+        // (coherent loads: the kernel may have started while the one that writes the operand was still at work)
 #pragma unroll 4
         for (int r = 0; r < kSubBlocks; ++r) {
           const uint64_t i = first + r * kBlock + lane;
-          sts32((swizzled_row(stage, r) ^ ((lane >> 2) << 4)) | ((lane & 3u) << 2), i < n ? __ldg(src + i) : 0u);
+          sts32((swizzled_row(stage, r) ^ ((lane >> 2) << 4)) | ((lane & 3u) << 2), i < n ? __ldcg(src + i) : 0u);
         }
         __syncwarp();
       }

@@ -82,3 +82,23 @@ def test_batch_of_very_different_sizes_in_a_codec_for_their_sum():
         assert size == want.size
         np.testing.assert_array_equal(out[:size].cpu().numpy(), want)
     assert c.status() == 0
+
+
+@pytest.mark.parametrize("n,shift", [(1023, 0), (4099, 1), (70_001, 3)])
+def test_chain_through_one_ragged_operand(n, shift):
+    """Every call reads what the call before it has just written into the same buffer, past the TMA unit (ragged, or
+    off the 16-byte boundary); small enough that several of the launches are on an SM at the same time."""
+    c = ops.Codec(2 * 32768 * (n // 32768 + 1))
+    refs = [ops.cpu_compress(_data(n, s), EB) for s in range(24)]
+    gs = [_gpu(r) for r in refs]
+    x = _gpu(np.zeros(n, np.float32), shift)
+    got = []
+    for i, r in enumerate(refs):
+        c.decompress(gs[i], n, EB, out=x, stream_bytes=r.size)
+        got.append((c.compress(x, EB), c.hom_add(gs[0], x, EB, stream_bytes=refs[0].size)))
+    assert c.status() == 0
+    for r, ((out, size), (added, added_size)) in zip(refs, got):
+        y = ops.cpu_decompress(r, n, EB)
+        for o, k, want in ((out, size, ops.cpu_compress(y, EB)), (added, added_size, ops.cpu_hom_add(refs[0], y, EB))):
+            assert int(k) == want.size
+            np.testing.assert_array_equal(o[:want.size].cpu().numpy(), want)
