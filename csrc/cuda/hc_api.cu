@@ -91,6 +91,12 @@ int hc_codec_create(hc_codec** out, size_t max_elems) {
   size_t bytes = hc::workspace_bytes(max_elems);
   if (cudaMalloc(&mem, bytes) != cudaSuccess) return hc::kErrCuda;
   int rc = hc_codec_create_in(out, mem, bytes, max_elems, nullptr);
+  // the first call may come on a stream that does not order itself behind the default one
+  if (rc == hc::kOk && cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    delete *out;
+    *out = nullptr;
+    rc = hc::kErrCuda;
+  }
   if (rc != hc::kOk) {
     cudaFree(mem);
     return rc;
@@ -131,7 +137,11 @@ int hc_codec_status(hc_codec* c, int clear) {
   uint32_t ctrl[4] = {0, 0, 0, 0};
   if (cudaDeviceSynchronize() != cudaSuccess) return hc::kErrCuda;
   if (cudaMemcpy(ctrl, c->ws_mem, sizeof(ctrl), cudaMemcpyDeviceToHost) != cudaSuccess) return hc::kErrCuda;
-  if (clear && (ctrl[2] != 0 || ctrl[0] != 0 || ctrl[1] != 0)) cudaMemset(c->ws_mem, 0, c->ws_bytes);  // status, ticket counters, sums left behind
+  // status, ticket counters, sums left behind; done before this returns, because the next call may come on a stream
+  // that does not order itself behind the default one
+  if (clear && (ctrl[2] != 0 || ctrl[0] != 0 || ctrl[1] != 0) &&
+      (cudaMemset(c->ws_mem, 0, c->ws_bytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess))
+    return hc::kErrCuda;
   return (int)ctrl[2];
 }
 

@@ -53,8 +53,10 @@ int hc_noalloc_status(int clear) {
   uint32_t ctrl[4] = {0, 0, 0, 0};
   if (cudaDeviceSynchronize() != cudaSuccess) return hc::kErrCuda;
   if (cudaMemcpy(ctrl, d->scratch, sizeof(ctrl), cudaMemcpyDeviceToHost) != cudaSuccess) return hc::kErrCuda;
-  // status word, first-time-out site and the ticket counters a failed launch may have left behind
-  if (clear && cudaMemset(d->scratch, 0, kScratchBytes) != cudaSuccess) return hc::kErrCuda;
+  // status word, first-time-out site and the ticket counters a failed launch may have left behind; done before this
+  // returns (see hc_codec_status)
+  if (clear && (cudaMemset(d->scratch, 0, kScratchBytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess))
+    return hc::kErrCuda;
   return (int)ctrl[2];
 }
 

@@ -155,7 +155,7 @@ int hc_comm_create(hc_comm** out, int rank, int world, size_t max_count, void* c
   c->ws_bytes = hc::workspace_bytes(max_count, hc::kMaxWorkspaceSets);
   if (cudaMalloc(&c->ws_mem, c->ws_bytes) != cudaSuccess || cudaMemset(c->ws_mem, 0, c->ws_bytes) != cudaSuccess ||
       cudaMalloc(&c->sizes, 16 * sizeof(uint64_t)) != cudaSuccess ||
-      cudaMemset(c->sizes, 0, 16 * sizeof(uint64_t)) != cudaSuccess) {
+      cudaMemset(c->sizes, 0, 16 * sizeof(uint64_t)) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
     hc_comm_destroy(c);
     return hc::kErrCuda;
   }
@@ -221,9 +221,10 @@ int hc_comm_status(hc_comm* c, int clear) {
   if (cudaDeviceSynchronize() != cudaSuccess) return hc::kErrCuda;
   if (cudaMemcpy(ctrl, c->ws_mem, sizeof(ctrl), cudaMemcpyDeviceToHost) != cudaSuccess) return hc::kErrCuda;
   const uint32_t st = ctrl[2] > ctrl[34] ? ctrl[2] : ctrl[34];
-  if (clear && (ctrl[0] | ctrl[1] | ctrl[2] | ctrl[3] | ctrl[33] | ctrl[34])) {
-    cudaMemset(c->ws_mem, 0, c->ws_bytes);  // status words, ticket counters, sums left behind
-  }
+  // status words, ticket counters, sums left behind; done before this returns (see hc_codec_status)
+  if (clear && (ctrl[0] | ctrl[1] | ctrl[2] | ctrl[3] | ctrl[33] | ctrl[34]) &&
+      (cudaMemset(c->ws_mem, 0, c->ws_bytes) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess))
+    return hc::kErrCuda;
   return (int)st;
 }
 
