@@ -40,14 +40,20 @@ struct __align__(16) EncShared {
   uint8_t in_rate[2][kTileBlocks];
 };
 
-// bounded mbarrier wait that records a timeout; `site` says which wait it was
-__device__ __forceinline__ bool wait_or_flag(uint64_t* bar, uint32_t parity, const Workspace& ws, volatile uint32_t* abort,
-                                             uint32_t site) {
+// bounded mbarrier wait that records a timeout; `site` says which wait it was.  The answer is this lane's: a warp whose
+// lanes go on together has to agree on it first (the compute warps in an operation that they do anyway).
+__device__ __forceinline__ bool lane_wait(uint64_t* bar, uint32_t parity, const Workspace& ws, volatile uint32_t* abort,
+                                          uint32_t site) {
   if (mbar_wait_bounded(bar, parity, ws.spin_limit_ns)) return true;
   if (!*abort) atomicCAS(ws.ctrl + 3, 0u, site);
   note_error(ws.ctrl, kErrTimeout);
   *abort = 1;
   return false;
+}
+// the same with one answer for the warp
+__device__ __forceinline__ bool wait_or_flag(uint64_t* bar, uint32_t parity, const Workspace& ws, volatile uint32_t* abort,
+                                             uint32_t site) {
+  return __all_sync(0xffffffffu, lane_wait(bar, parity, ws, abort, site));
 }
 
 // Loader-warp work for one input stream, in two parts so that the rate bytes of the NEXT tile are
@@ -424,12 +430,12 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
     // blocking: tiles [copied, upto) out, whatever their look-backs take
     auto drain_to = [&](uint32_t upto) {
       for (uint32_t j = copied; j < upto; ++j) {
-        wait_or_flag(&sh.base_ready[j % kRing], (j / kRing) & 1, ws, abort, kSiteComputeRing);
-        copy_tile(j);
+        if (lane_wait(&sh.base_ready[j % kRing], (j / kRing) & 1, ws, abort, kSiteComputeRing)) copy_tile(j);
       }
       copied = upto > copied ? upto : copied;
     };
-    for (uint32_t k = 0;; ++k) {
+    uint32_t k = 0;
+    for (;; ++k) {
       const int s = k % NS, slot = k & 7, r = k % kRing;
       uint8_t* const stage_s = stage0 + s * kTileBytes;
       int32_t d[32];
@@ -437,20 +443,20 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
       for (int i = 0; i < 32; ++i) d[i] = 0;
 
       // ---- incoming stream(s) -> signed deltas, summed -------------------------------------------
-      bool end = false;
+      bool leave = false;  // no tile this turn, or a wait ran out; not known to be the same in all compute warps
       if (kHasIn) {
         for (uint32_t q = 0; q < Q; ++q) {
           const uint32_t vv = k * Q + q, b = vv & 1u;
-          const bool staged = wait_or_flag(&sh.in_full[b], (vv >> 1) & 1, ws, abort, kSiteComputeInFull);
+          const bool staged = lane_wait(&sh.in_full[b], (vv >> 1) & 1, ws, abort, kSiteComputeInFull);
           if (tid == 0) HC_PH(0);
-          if (q == 0 && (!staged || sh.in_end[b])) {
-            end = true;  // no tile this turn (or the loader gave up)
+          const uint32_t rate_in = sh.in_rate[b][tid];
+          const uint32_t pos = sh.in_phase[b] + sh.in_rel[b][tid];
+          int W = staged && !(q == 0 && sh.in_end[b]) ? plane_width(rate_in & 31u) : 64;
+          W = __reduce_max_sync(0xffffffffu, W);
+          if (W == 64) {
+            leave = true;
             break;
           }
-          const uint32_t rate_in = staged ? sh.in_rate[b][tid] : 0u;
-          const uint32_t pos = sh.in_phase[b] + sh.in_rel[b][tid];
-          int W = plane_width(rate_in & 31u);
-          W = __reduce_max_sync(0xffffffffu, W);
           if (__any_sync(0xffffffffu, rate_in != 0)) {
             int32_t d2[32];
             decode_block(cbuf[b], pos, rate_in, W, d2);
@@ -462,30 +468,21 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
           if (k == 0 && tid == 0 && q < 8) HC_STAMP(8 + q);
         }
       }
-      if (INPLACE && k >= 1 && !end) {
+      if (INPLACE && k >= 1) {
         // the tile packed over the fp32 stage has to leave before the next fp32 tile can come in
-        compute_barrier();  // every thread has packed tile k-1
-        drain_to(k);
-        mbar_arrive(&sh.stage_free[0]);
+        leave = compute_barrier_or(leave);  // every thread has packed tile k-1
+        if (!leave) {
+          drain_to(k);
+          mbar_arrive(&sh.stage_free[0]);
+        }
       }
-      const bool alive = !end && wait_or_flag(&sh.tma_full[s], (k / NS) & 1, ws, abort, kSiteComputeTile);
+      const bool alive = !leave && wait_or_flag(&sh.tma_full[s], (k / NS) & 1, ws, abort, kSiteComputeTile);
       if (tid == 0) HC_PH(2);
       if (k == 0 && tid == 0) HC_STAMP(2);
       const uint32_t tile = alive ? sh.tile[slot] : kNoTile;
       if (tile == kNoTile) {
-        // end of work: everything still in the ring leaves, then the scanner hears of the end through
-        // the same barrier as of a tile
+        if (lane == 31) sh.wsum[k & 1][warp] = kLeaveTotal;
         compute_barrier();  // every thread has packed the last tile
-        if (tid == 0) HC_STAMP(5);
-        drain_to(k);
-        if (tid == 0) HC_STAMP(12);
-        if (INPLACE && k >= 1) mbar_arrive(&sh.stage_free[0]);  // the loader's last hand-over waits for it
-        compute_barrier();  // every thread's stores are issued before the scanner announces them
-        if (tid == 0) {
-          sh.stored_upto = k;
-          sh.out_tile[r] = kNoTile;
-          mbar_arrive(&sh.scan_done[r]);
-        }
         break;
       }
       const Seg v = seg_of(tile);
@@ -553,7 +550,7 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
           if (j > dep && j >= 0 && sh.ring_start[j % kRing] < end_b && start < sh.ring_end[j % kRing]) dep = j;
         }
       }
-      if (tid == 0) {
+      if (tid == 0 && tot < kLeaveTotal) {
         // publish the tile aggregate right away: successors can look back through this tile
         if (v.lt != 0 && !p.sparse)
           st_relaxed_gpu_u64(ws.st_out + (size_t)v.g * p.tiles_per_seg + v.lt, st_pack(kStAgg, ws.epoch, tot));
@@ -580,6 +577,8 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
       W = __reduce_max_sync(0xffffffffu, W);
       transpose_forward(A, W);
       if (tid == 0) HC_PH(9);
+      // some warp leaves, and this one with it (looked at only here: the transposition does not need the total)
+      if (tot >= kLeaveTotal) break;
       if (!INPLACE) {
         // packed tiles whose offset is known leave now; the ones this tile needs the room of leave
         // whatever their look-back takes
@@ -594,6 +593,18 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
         HC_PH(7);
         HC_PH_COUNT();
       }
+    }
+    // end of work: everything still in the ring leaves, then the scanner hears of the end through the same barrier as
+    // of a tile
+    if (tid == 0) HC_STAMP(5);
+    drain_to(k);
+    if (tid == 0) HC_STAMP(12);
+    if (INPLACE && k >= 1) mbar_arrive(&sh.stage_free[0]);  // the loader's last hand-over waits for it
+    compute_barrier();  // every thread's stores are issued before the scanner announces them
+    if (tid == 0) {
+      sh.stored_upto = k;
+      sh.out_tile[k % kRing] = kNoTile;
+      mbar_arrive(&sh.scan_done[k % kRing]);
     }
   }
   if (lane == 0) HC_STAMP_MAX(7);

@@ -82,6 +82,7 @@ struct hc_comm {
   uint32_t raw_call = 0;
   int algorithm = 1;              // 0 ring (P + 1 kernels), 1 direct (3 kernels), 2 one step (2 kernels) where it fits
   size_t small_count = 0;         // direct: messages of at most this many values take the one-step form
+  int step_first = 0, step_last = 1 << 30;  // launches of a call that hc_allreduce enqueues (hc_comm_set_steps)
   int last_form = 1;              // the form the last hc_allreduce took (0 ring, 1 direct, 2 one step)
   bool trace = false;             // record one CUDA event per step of hc_allreduce
   bool overlap = true;            // direct algorithm: steps 2 and 3 start while their predecessor drains
@@ -114,6 +115,16 @@ struct NvtxRange {
   NvtxRange(const NvtxRange&) = delete;
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
+
+// number of the call that a launch belongs to
+uint32_t begin_call(hc_comm* c) {
+  if (c->step_first == 0) {
+    c->call += 1;
+    if ((c->call & 0xffffffu) == 0) c->call += 1;  // flags carry 24 bits of it; 0 means "never written"
+  }
+  return c->call;
+}
+bool wanted(const hc_comm* c, int step) { return step >= c->step_first && step < c->step_last; }
 
 hc::Workspace next_ws(hc_comm* c, cudaStream_t stream) {
   c->ws_epoch = (c->ws_epoch + 1) & hc::dev::kEpochMask;
@@ -255,9 +266,7 @@ static int allreduce_ring(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t
     size_t hi = lo + B;
     return (hi > count ? count : hi) - lo;
   };
-  c->call += 1;
-  if ((c->call & 0xffffffu) == 0) c->call += 1;  // flags carry 24 bits of it; 0 means "never written"
-  const uint32_t call = c->call;
+  const uint32_t call = begin_call(c);
   const int parity = (int)(call & 1u);
   const int next = (r + 1) % P;
   uint8_t* self = c->peer[r];
@@ -285,7 +294,7 @@ static int allreduce_ring(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t
   for (int s = 0; s < P; ++s) {
     const int ch = ((r - s) % P + P) % P;
     const size_t n = chunk_len(ch);
-    if (n == 0) continue;
+    if (n == 0 || !wanted(c, s)) continue;
     NvtxRange step_range(s == 0 ? "hc ring: compress" : (s < P - 1 ? "hc ring: hop" : "hc ring: last hop + all-gather"));
     hc::EncParams p;
     memset(&p, 0, sizeof(p));
@@ -328,6 +337,7 @@ static int allreduce_ring(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t
   }
 
   // ---- all-gather side: one kernel decodes the P reduced chunks as their tiles arrive ------------
+  if (!wanted(c, P)) return hc::kOk;
   NvtxRange decode_range("hc ring: decode");
   hc::DecParams d;
   memset(&d, 0, sizeof(d));
@@ -375,9 +385,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
     size_t hi = lo + B;
     return (hi > count ? count : hi) - lo;
   };
-  c->call += 1;
-  if ((c->call & 0xffffffu) == 0) c->call += 1;  // flags carry 24 bits of it; 0 means "never written"
-  const uint32_t call = c->call;
+  const uint32_t call = begin_call(c);
   const int parity = (int)(call & 1u);
   uint8_t* self = c->peer[r];
   c->n_ev = 0;
@@ -392,7 +400,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
   bool launched = false;  // a kernel of this call is already on the stream
   mark();
   // ---- 1. scatter: chunk d -> rank d's slot for source r ------------------------------------------
-  if (P > 1) {
+  if (P > 1 && wanted(c, 0)) {
     NvtxRange step_range("hc direct: scatter-compress");
     hc::EncParams p;
     memset(&p, 0, sizeof(p));
@@ -422,7 +430,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
   }
   mark();
   // ---- 2. reduce the own chunk and push the result to everybody -----------------------------------
-  if (const size_t n = chunk_len(r)) {
+  if (const size_t n = wanted(c, 1) ? chunk_len(r) : 0) {
     NvtxRange step_range("hc direct: reduce + all-gather");
     hc::EncParams p;
     memset(&p, 0, sizeof(p));
@@ -459,6 +467,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
   }
   mark();
   // ---- 3. decode the P reduced chunks as their tiles arrive ----------------------------------------
+  if (!wanted(c, 2)) return hc::kOk;
   NvtxRange decode_range("hc direct: decode");
   hc::DecParams d;
   memset(&d, 0, sizeof(d));
@@ -487,9 +496,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
 // arrival flags so that other ranks can follow).
 static int allreduce_single(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t count, float eb, hc_stream_t stream) {
   const Layout& L = c->lay;
-  c->call += 1;
-  if ((c->call & 0xffffffu) == 0) c->call += 1;
-  uint8_t* const slot = c->peer[0] + L.data_off(L.ag_slot((int)(c->call & 1u), 0));
+  uint8_t* const slot = c->peer[0] + L.data_off(L.ag_slot((int)(begin_call(c) & 1u), 0));
   c->n_ev = 0;
   auto mark = [&]() {
     if (c->trace) cudaEventRecord(c->ev[c->n_ev++], stream);
@@ -541,18 +548,16 @@ static int allreduce_single(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
 static int allreduce_onestep(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t count, float eb, hc_stream_t stream) {
   const int P = c->world, r = c->rank;
   const Layout& L = c->lay;
-  c->call += 1;
-  if ((c->call & 0xffffffu) == 0) c->call += 1;
-  const uint32_t call = c->call;
+  const uint32_t call = begin_call(c);
   const int parity = (int)(call & 1u);
   uint8_t* self = c->peer[r];
   c->n_ev = 0;
   auto mark = [&]() {
     if (c->trace) cudaEventRecord(c->ev[c->n_ev++], stream);
   };
-  const bool overlap = c->overlap && !c->trace;
+  const bool overlap = c->overlap && !c->trace && wanted(c, 0);  // step 1 of the same call is right in front
   mark();
-  {
+  if (wanted(c, 0)) {
     NvtxRange step_range("hc one-step: compress + broadcast");
     hc::EncParams p;
     memset(&p, 0, sizeof(p));
@@ -576,6 +581,7 @@ static int allreduce_onestep(hc_comm* c, const float* d_sbuf, float* d_rbuf, siz
     if (hc::launch_encode(hc::kOpCompress, p, stream) != cudaSuccess) return hc::kErrCuda;
   }
   mark();
+  if (!wanted(c, 1)) return hc::kOk;
   NvtxRange decode_range("hc one-step: decode + sum");
   hc::DecParams d;
   memset(&d, 0, sizeof(d));
@@ -663,6 +669,13 @@ extern "C" int hc_comm_resync(hc_comm* c, uint32_t call, uint32_t raw_call) {
   if (cudaDeviceSynchronize() != cudaSuccess) return hc::kErrCuda;              // nothing of an old call in flight
   c->call = call;
   c->raw_call = raw_call;
+  return hc::kOk;
+}
+
+extern "C" int hc_comm_set_steps(hc_comm* c, int first, int last) {
+  if (!c || first < 0 || last <= first) return hc::kErrArgument;
+  c->step_first = first;
+  c->step_last = last;
   return hc::kOk;
 }
 

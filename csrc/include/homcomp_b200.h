@@ -176,6 +176,12 @@ int hc_comm_set_shares(hc_comm* c, int scatter_ctas_per_sm, int reduce_ctas_per_
 // either way, only the bytes of the payload are ever written or read, and consumers take each tile's
 // offset from its arrival flag.  Results and hc_comm_last_stream_bytes do not depend on it.
 int hc_comm_set_sparse_tiles(hc_comm* c, int on);
+// Launches of a call that the following hc_allreduce calls enqueue: first .. last - 1 of them (ring: 0 .. world - 1
+// the hops, world the decode; direct: scatter, reduce, decode; one step: compress, decode; default: all).  For ranks
+// that share one GPU: they take turns, step by step (every rank makes the call with steps 0..1, then every rank with
+// 1..2, and so on, on one stream), and no kernel ever waits for another one that has not finished.  Ignored by a
+// communicator of one rank.
+int hc_comm_set_steps(hc_comm* c, int first, int last);
 // Uncompressed sum over the same peer mappings (two-shot direct algorithm, three kernels); the
 // compressed and the uncompressed collective of one handle must not be in flight together.
 int hc_allreduce_raw(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t count, hc_stream_t stream);

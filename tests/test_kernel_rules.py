@@ -30,6 +30,20 @@ def test_block_wide_barriers_of_encode_stand_before_the_roles_part():
     assert "__syncthreads" not in kernel.split("clerk(p, sh", 1)[1]
 
 
+def test_compute_warps_of_the_collective_kernel_leave_together():
+    """They meet at hardware barriers, so a wait that ran out in one of them is no reason to go before all know: lanes
+    agree within the warp, the warp tells the others at a barrier that it comes to itself."""
+    code = _code("hc_kernels.cu")
+    wait = code.split("bool wait_or_flag(", 1)[1].split("\n}", 1)[0]
+    assert "__all_sync" in wait
+    loop = code.split("int32_t d[32];", 1)[1].split("write_payload(", 1)[0]
+    # the ways out of the tile loop: told and through the barrier, or told by it
+    told = re.findall(r"kLeaveTotal;\s*compute_barrier\(\);\s*break;", loop)
+    tellers = re.findall(r"if \(tot >= kLeaveTotal\) break;", loop)
+    streams = re.findall(r"if \(W == 64\) \{\s*leave = true;\s*break;", loop)  # out of the loop over the streams
+    assert (len(told), len(tellers), len(streams)) == (1, 1, 1) and loop.count("break;") == 3
+
+
 @pytest.mark.parametrize("name", sorted(p.name for p in CUDA.glob("hc_*.cu*")))
 def test_no_non_coherent_loads(name):
     code = _code(name)
