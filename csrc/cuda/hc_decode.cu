@@ -323,7 +323,8 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   uint32_t bound = 0;  // of |sum of the deltas| of this lane's block
   bool announced = !RUNS || pool == 0u;
   if (threadIdx.x == 0) HC_PH(0);
-  for (uint32_t v = 0;;) {
+  uint32_t v = 0;  // jobs whose payload has landed
+  for (;;) {
     if (staged < 2u && tk != kNoTile) {
       Staged st;
       if (produce(st, staged != 0u, staged == 0u)) {
@@ -449,6 +450,8 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
       HC_PH_COUNT();
     }
   }
+  // after a wait that ran out: nothing may land in shared memory once the CTA has left it
+  for (; v < jobs; ++v) mbar_wait_bounded(&full[v & 3u], (v >> 2) & 1u, ws.spin_limit_ns);
   if (lane == 0) tma_wait_group<0>();
   if (lane == 0) HC_STAMP_MAX(7);
   if (dynamic) cta_epilogue(ws.tick);

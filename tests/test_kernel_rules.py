@@ -52,3 +52,11 @@ def test_no_non_coherent_loads(name):
     overlapped = re.findall(r"launch_overlapped\(dev::(\w+)", code)
     for kernel in overlapped:
         assert "__restrict__" not in code.split(kernel + "(", 1)[1].split("{", 1)[0]
+
+
+@pytest.mark.parametrize("name", ["hc_encode.cu", "hc_decode.cu"])
+def test_a_warp_that_gives_up_waits_for_its_copies(name):
+    """Bulk copies land in shared memory; the CTA does not leave it while one may be on its way."""
+    kernel = _code(name).split("__global__", 1)[1].split("\n}\n", 1)[0]
+    after_the_loop = kernel.rsplit("HC_PH_COUNT();", 1)[1]
+    assert re.search(r"for \(;[^;]*< jobs; [^)]*\)\s*mbar_wait_bounded\(", after_the_loop)
