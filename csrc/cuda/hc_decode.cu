@@ -471,23 +471,20 @@ cudaError_t launch_t(const TensorMaps& maps, DecParams p, cudaStream_t stream, b
   static thread_local int cache[64] = {};
   const int cap = resident_ctas(dev::hc_decode_kernel<MODE, SUM, RUNS>, 32 * kWarps, dec_smem(kWarps), cache);
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
-  uint64_t warps;
+  uint32_t warps;
   int grid;
   if (RUNS) {
-    // few sub-tiles are spread over the SMs four at a time (fewer CTAs exchange their totals faster)
     const uint64_t subs = (p.seg[0].n + dev::kSubValues - 1) / dev::kSubValues;
-    const uint64_t sms = (uint64_t)(cap < kMaxCtas ? cap : kMaxCtas);
-    warps = (subs + sms - 1) / sms;
-    warps = warps < 4u ? 4u : warps > (uint64_t)kWarps ? (uint64_t)kWarps : warps;
-    grid = (int)((subs + warps - 1) / warps < sms ? (subs + warps - 1) / warps : sms);
-    // the pool: an eighth of a run; none where a run is a sub-tile or three
-    const uint64_t run = subs / (grid * warps);
-    p.pool = run < 4 ? 0u : run < 8 ? 1u : (uint32_t)(run / 8);
+    const RunSplit split = split_runs(subs, (uint32_t)(cap < kMaxCtas ? cap : kMaxCtas), (uint32_t)kWarps);
+    if (run_words(split, p.n_seg) > p.ws.words) return cudaErrorInvalidValue;
+    warps = split.warps;
+    grid = (int)split.grid;
+    p.pool = split.pool;
     p.flags = p.ws.st_a;
   } else {
     // tickets are quarters of a tile while there is a warp for each
     const uint32_t tiles = SUM ? p.tiles_per_seg : p.n_tiles;
-    warps = kWarps;
+    warps = (uint32_t)kWarps;
     p.parts = tiles <= (uint32_t)cap ? 4u : 1u;
     const uint32_t ctas = p.parts == 4u ? tiles : (tiles + 3u) / 4u;
     grid = (int)(ctas < (uint32_t)cap ? ctas : (uint32_t)cap);

@@ -586,23 +586,14 @@ cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t str
   static thread_local int cache[64] = {};
   const int cap = resident_ctas(dev::hc_encode_solo_kernel<OP, MODE>, 32 * (kWarps + 1), smem(kWarps), cache);
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
-  const uint64_t sms = (uint64_t)(cap < kMaxCtas ? cap : kMaxCtas);
-  // Compute warps per CTA: as many rounds of chunks as the largest CTA needs, then no more warps than fill them (where
-  // the last round would be half empty, all rounds are narrower instead); at least four at a time.
-  uint64_t subs = 0;
-  for (uint32_t g = 0; g < p.n_seg; ++g) subs += p.subs[g];
-  const uint64_t rounds = (subs + sms * kWarps - 1) / (sms * kWarps);
-  uint64_t nc = (subs + sms * rounds - 1) / (sms * rounds);
-  if (nc < 4) nc = 4;
-  p.first[0] = 0;
-  for (uint32_t g = 0; g < p.n_seg; ++g)
-    p.first[g + 1] = p.first[g] + (uint32_t)((p.subs[g] + nc - 1) / nc);
-  const uint32_t chunks = p.first[p.n_seg];
-  const int grid = (int)(chunks < sms ? chunks : sms);
-  p.one_round = p.n_seg == 1 && chunks <= sms;
+  const EncodeSplit split = split_encode(p.subs, p.n_seg, (uint32_t)(cap < kMaxCtas ? cap : kMaxCtas), (uint32_t)kWarps);
+  if (encode_words(split, p.n_seg, p.n_in) > p.ws.words) return cudaErrorInvalidValue;
+  const int nc = (int)split.warps;
+  memcpy(p.first, split.first, sizeof(p.first));
+  p.one_round = split.one_round;
   p.out_words = p.ws.st_a;
-  p.in_words = p.ws.st_a + chunks;
-  return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE>, grid, 32 * ((int)nc + 1), smem((int)nc), stream, maps, p);
+  p.in_words = p.ws.st_a + p.first[p.n_seg];
+  return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE>, (int)split.grid, 32 * (nc + 1), smem(nc), stream, maps, p);
 }
 
 template <int OP>

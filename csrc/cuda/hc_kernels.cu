@@ -699,38 +699,31 @@ cudaError_t launch_encode_t(const TensorMaps& map, const EncParams& p, cudaStrea
 
 }  // namespace
 
-// sized for max_elems values split over up to kMaxDst segments (each rounded up to whole chunks)
-static size_t workspace_tiles(size_t max_elems) {
-  return rate_bytes(max_elems) / kTileBlocks + (size_t)kMaxDst * (kBlocksPerChunk / kTileBlocks) + 1;
-}
 size_t workspace_bytes(size_t max_elems, int sets) {
-  size_t tiles = workspace_tiles(max_elems);
-  size_t groups = tiles / 32 + 1 + kMaxDst;
   if (sets < 1) sets = 1;
   if (sets > kMaxWorkspaceSets) sets = kMaxWorkspaceSets;
-  // look-back words of all sets, then the exchange words of all sets
-  return kWorkspaceHeader + (size_t)sets * (3 * (tiles + groups) + (1 + kMaxIn) * kMaxCtas) * sizeof(uint64_t);
+  // words of all sets, then the exchange words of all sets
+  return kWorkspaceHeader + (size_t)sets * (workspace_words(max_elems) + (1 + kMaxIn) * kMaxCtas) * sizeof(uint64_t);
 }
 
 Workspace workspace_view(void* mem, size_t max_elems, uint32_t epoch, uint64_t spin_limit_ns, int sets) {
-  size_t tiles = workspace_tiles(max_elems);
+  const size_t tiles = workspace_tiles(max_elems), groups = workspace_groups(max_elems), words = workspace_words(max_elems);
   Workspace w;
   uint8_t* b = static_cast<uint8_t*>(mem);
   w.ctrl = reinterpret_cast<uint32_t*>(b);
-  size_t groups = tiles / 32 + 1 + kMaxDst;
   if (sets < 1) sets = 1;
   if (sets > kMaxWorkspaceSets) sets = kMaxWorkspaceSets;
   const size_t set = epoch % (uint32_t)sets;
   w.tick = w.ctrl + 8 + 2 * set;  // words 8..15 of the header
   w.size_acc = reinterpret_cast<uint64_t*>(b + 256) + set * kMaxDst;  // second half of the header
-  w.st_a = reinterpret_cast<uint64_t*>(b + kWorkspaceHeader) + set * 3 * (tiles + groups);
+  w.st_a = reinterpret_cast<uint64_t*>(b + kWorkspaceHeader) + set * words;
   w.st_b = w.st_a + tiles;
   w.st_out = w.st_b + tiles;
   w.grp_a = w.st_out + tiles;
   w.grp_b = w.grp_a + groups;
   w.grp_out = w.grp_b + groups;
-  w.sums = reinterpret_cast<uint64_t*>(b + kWorkspaceHeader) + (size_t)sets * 3 * (tiles + groups) +
-           set * (1 + kMaxIn) * kMaxCtas;
+  w.words = words;
+  w.sums = reinterpret_cast<uint64_t*>(b + kWorkspaceHeader) + (size_t)sets * words + set * (1 + kMaxIn) * kMaxCtas;
   w.epoch = epoch;
   w.spin_limit_ns = spin_limit_ns;
   return w;

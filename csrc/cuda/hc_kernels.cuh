@@ -33,16 +33,13 @@
 // (HomComp/src/GSZ.cu:33-756, HomComp/src/GSZ_entry.cu:263-301).
 #pragma once
 #include "hc_block.cuh"
+#include "hc_split.h"
 
 namespace hc {
 
-constexpr int kTileBlocks = 128;
-constexpr int kTileElems = kTileBlocks * kBlock;  // 4096
 constexpr int kTileBytes = kTileElems * 4;        // 16384
 constexpr int kBufBytes = 17 * 1024;              // a tile of stream bytes + alignment slack
 constexpr int kComputeThreads = kTileBlocks;
-constexpr int kMaxDst = 8;
-constexpr int kMaxCtas = 160;  // CTAs of a launch with one CTA per SM
 
 enum Op : int {
   kOpCompress = 0,   // fp32 -> stream
@@ -53,13 +50,17 @@ enum Op : int {
 
 struct Workspace {
   uint32_t* ctrl;    // [2] sticky error (hc::Status); the other words of the 256-byte header hold the tick sets
-  uint64_t* st_a;    // look-back chain of the first input stream (tile words, then group words)
-  uint64_t* st_b;    // look-back chain of the second input stream
-  uint64_t* st_out;  // look-back chain of the output stream
+  // steps of a collective: look-back chains (tile words, then group words) of two input streams and the output
+  uint64_t* st_a;
+  uint64_t* st_b;
+  uint64_t* st_out;
   uint64_t* grp_a;
   uint64_t* grp_b;
   uint64_t* grp_out;
-  uint32_t* tick;  // [0] tile ticket counter, [1] CTAs that have left; re-armed by the last CTA of a launch
+  // stand-alone launches: all of the above as one array from st_a on, of so many words (the launchers check that they
+  // do with them: encode_words, run_words)
+  uint64_t words;
+  uint32_t* tick;      // [0] tile ticket counter, [1] CTAs that have left; re-armed by the last CTA of a launch
   uint64_t* sums;      // [1 + kMaxIn][kMaxCtas] exchange of CTA totals (dev::give_total): zero between launches
   uint64_t* size_acc;  // [kMaxDst] payload bytes per segment of a launch with sparse tiles; zeroed by its last CTA
   uint32_t epoch;
@@ -72,7 +73,6 @@ struct Workspace {
 //     a ring step, or the reduced chunk pushed to every rank), or, for compress only, to n_seg
 //     independent streams ("segments": segment g compresses local[g] of n[g] values into out[g]);
 //     tickets go round the segments, each of which has its own look-back chain.
-constexpr int kMaxIn = kMaxDst;
 struct EncParams {
   const void* local[kMaxDst];  // fp32 values or int32 deltas, per segment
   uint64_t n[kMaxDst];         // values per segment
