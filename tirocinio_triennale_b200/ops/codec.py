@@ -15,9 +15,11 @@ from .. import _lib, MODES
 from .cpu_codec import max_compressed_bytes
 
 # Small calls cost what the host spends on them, so the two torch front ends that took 4.6 of 11 us a call
-# (torch.cuda.current_stream() 3.2 us, the torch.cuda.device context 1.4 us) are replaced by what they end in.
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-_current_device = getattr(torch._C, "_cuda_getDevice", None)
+# (torch.cuda.current_stream() 3.2 us, the torch.cuda.device context 1.4 us) are replaced by what they end in.  Those are
+# private functions: where a version of torch does not have them, the public ones do the same.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or (lambda: torch.cuda.current_device())
 
 
 def _mode(mode) -> int:
