@@ -84,10 +84,13 @@ class Codec:
 
     def _size_words(self, k):
         """``k`` zeroed int64 words that nobody else uses.  Blocks of 256 are zeroed at a time on the stream that
-        will use them (a fill kernel per call took 5.7 us); at most 16 streams keep a block."""
+        will use them (a fill kernel per call took 5.7 us); at most 16 streams keep a block.  A block made during a
+        stream capture belongs to the graph, which would zero it again in every replay: none is kept then."""
         key = _raw_stream(self._index)
         block = self._sizes.get(key)
         if block is None or block[1] + k > 256:
+            if torch.cuda.is_current_stream_capturing():
+                return torch.zeros(k, dtype=torch.int64, device=self.device)
             if len(self._sizes) >= 16:
                 self._sizes.clear()
             block = self._sizes[key] = [torch.zeros(256, dtype=torch.int64, device=self.device), 0]
