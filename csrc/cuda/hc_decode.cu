@@ -488,7 +488,6 @@ cudaError_t launch_t(const TensorMaps& maps, DecParams p, cudaStream_t stream, b
     p.parts = tiles <= (uint32_t)cap ? 4u : 1u;
     const uint32_t ctas = p.parts == 4u ? tiles : (tiles + 3u) / 4u;
     grid = (int)(ctas < (uint32_t)cap ? ctas : (uint32_t)cap);
-    if (p.grid_limit && (int)p.grid_limit < grid) grid = (int)p.grid_limit;
   }
   const int block = 32 * (int)warps, smem = dec_smem((int)warps);
   if (overlap || RUNS) return launch_overlapped(dev::hc_decode_kernel<MODE, SUM, RUNS>, grid, block, smem, stream, maps, p);

@@ -159,7 +159,6 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ EncShared sh;
   static_assert(OP == kOpCompress || OP == kOpAddF32, "stand-alone calls run hc_encode_solo_kernel");
-  constexpr int MODE = kModeOutlier;
   constexpr bool kHasIn = OP != kOpCompress;
   constexpr uint32_t kRingBytes = (uint32_t)enc_ring_bytes(OP, INPLACE);
   uint8_t* const stage0 = smem + 1024;
@@ -508,7 +507,7 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) q[i] = quantise(__uint_as_float(w[i]), p.recip);
         int32_t dl[32];
-        lorenzo_forward<MODE>(q, dl);
+        lorenzo_forward(q, dl);
 #pragma unroll
         for (int i = 0; i < 32; ++i) d[i] += dl[i];
       }
@@ -516,7 +515,7 @@ hc_encode_kernel(const __grid_constant__ TensorMaps tmaps, const EncParams p) {
       // ---- encode ----------------------------------------------------------------------------------
       if (tid == 0) HC_PH(3);
       uint32_t A[32];
-      TileCode code = analyse_block<MODE>(d, A);
+      TileCode code = analyse_block(d, A);
       uint32_t tot;
       if (tid == 0) {
         HC_PH(4);

@@ -141,7 +141,6 @@ struct DecParams {
   uint32_t ring_epoch;
   float eb;
   float scale;          // 2 eb * 2^23 where one multiplication by it gives the bits of (q * eb) * 2; else 0
-  uint32_t grid_limit;  // at most this many CTAs (0: as many as the GPU holds)
   uint32_t sum;         // 1: the n_seg streams are contributions to one array of seg[0].n values; their
                         //    quantised values are added tile by tile and seg[0].out receives the sum
   uint32_t parts;       // flagged segments: tickets per tile, 1 (a warp takes all four quarters) or 4
@@ -157,13 +156,14 @@ struct TensorMaps {
 
 namespace dev {
 
-// ---- per-thread block arithmetic ------------------------------------------------------------
+// ---- per-thread block arithmetic of the collective steps (mode outlier) -----------------------------
+// In int32 and with a path of its own for aligned payloads, unlike that of the stand-alone kernels (hc_block.cuh): a
+// thread shares its registers with the tile pipeline (80 to 96 a thread), and what the other form would do here
+// has not been measured on several GPUs.
 
-template <int MODE>
 __device__ __forceinline__ void lorenzo_forward(const int32_t (&q)[32], int32_t (&d)[32]) {
-  constexpr int S = MODE == kModeVec ? 4 : 1;
 #pragma unroll
-  for (int i = 31; i >= 0; --i) d[i] = i >= S ? q[i] - q[i - S] : q[i];
+  for (int i = 31; i >= 0; --i) d[i] = i >= 1 ? q[i] - q[i - 1] : q[i];
 }
 
 struct TileCode {
@@ -174,7 +174,6 @@ struct TileCode {
 };
 
 // signed deltas -> rows A[j] = |d[j ^ 7]| plus the block's code
-template <int MODE>
 __device__ __forceinline__ TileCode analyse_block(const int32_t (&d)[32], uint32_t (&A)[32]) {
   uint32_t sign = 0, or_tail = 0;
 #pragma unroll
@@ -197,7 +196,7 @@ __device__ __forceinline__ TileCode analyse_block(const int32_t (&d)[32], uint32
   }
   TileCode c;
   c.a0 = A[7];
-  c.rate = choose_rate(or_all, or_tail, c.a0, MODE != kModePlain);
+  c.rate = choose_rate(or_all, or_tail, c.a0, true);
   c.len = payload_len(c.rate);
   c.sign_mem = __byte_perm(sign, 0, 0x0123);
   if (c.rate & 0x80u) A[7] = 0;

@@ -21,8 +21,7 @@ __device__ __forceinline__ bool fatal_error(const uint32_t* ctrl) {
 // the launch is only a consequence of it
 enum WaitSite : uint32_t {
   kSiteLoaderStageFree = 1, kSiteLoaderInFree = 2, kSiteComputeInFull = 3, kSiteComputeTile = 4, kSiteComputeRing = 5,
-  kSiteScannerTotal = 6, kSiteCopierBase = 7, kSiteCopierPacked = 8, kSiteDecodeInFree = 9, kSiteDecodeInFull = 10,
-  kSiteLookBack = 11,
+  kSiteScannerTotal = 6, kSiteCopierBase = 7, kSiteDecodeInFull = 10, kSiteLookBack = 11,  // (8 and 9 belonged to roles that no longer exist)
 };
 __device__ __forceinline__ void note_timeout(const Workspace& ws, uint32_t site) {
   if (!fatal_error(ws.ctrl)) atomicCAS(ws.ctrl + 3, 0u, site);

@@ -69,11 +69,10 @@ void hc_codec_destroy(hc_codec* c);
 int hc_codec_set_timeout_ms(hc_codec* c, unsigned ms);
 // Synchronises the device, returns the sticky hc::Status of the handle and clears it when asked.
 int hc_codec_status(hc_codec* c, int clear);
-// After a status 3 (time-out): which wait ran out FIRST in the launch that failed (call it before
-// clearing the status).  1 loader: fp32 stage not released, 2 input buffer not released or input offsets
-// missing, 3 compute: input stream not staged, 4 compute: fp32 rows not landed, 5 compute: no room in the
-// payload ring, 6 total of a tile or chunk missing, 7 place of a packed payload missing, 8 copier: tile not
-// packed, 10 decoder: payload not landed, 11 totals of other CTAs; 0 none.
+// After a status 3 (time-out): which wait ran out FIRST in the launch that failed (call it before clearing the status).
+// 1 loader: fp32 stage not released, 2 input buffer not released or input offsets missing, 3 compute: input stream not
+// staged, 4 compute: fp32 rows not landed, 5 compute: no room in the payload ring, 6 total of a tile or chunk
+// missing, 7 place of a packed payload missing, 10 decoder: payload not landed, 11 totals of other CTAs; 0 none.
 int hc_codec_status_site(hc_codec* c);
 // Kept for callers of earlier versions, which ran a small kernel for the payload offsets of large streams
 // or did without: every call is one launch now, whatever was set here.
