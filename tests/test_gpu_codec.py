@@ -177,9 +177,9 @@ def test_multi_stream_add_matches_oracle(k, n):
 @pytest.mark.parametrize("n", [1, 33, 8193, 300000, 1100 * 4096 + 7])
 def test_decode_and_sum_of_streams_matches_oracle(k, n):
     """One kernel decodes k streams and adds their quantised values: the oracle's chain of stream adds
-    followed by one decompress, bit for bit (1100 tiles and more go through the offsets pre-pass)."""
+    followed by one decompress, bit for bit (the largest size: runs of one or two sub-tiles a warp)."""
     eb = 1e-4
-    codec = ops.Codec(max_elems=8 * n + 8 * 32768)  # room for eight look-back chains of whole chunks
+    codec = ops.Codec(max_elems=8 * n + 8 * 32768)  # room for the words of eight streams of whole chunks
     xs = [ALL["gradient" if i % 2 else "smooth"](n, seed=40 + i) for i in range(k)]
     streams = [ops.cpu_compress(x, eb) for x in xs]
     acc = streams[0]
@@ -196,8 +196,8 @@ def test_decode_and_sum_of_streams_matches_oracle(k, n):
 
 @pytest.mark.parametrize("k,n", [(1, 500 * 4096 + 77), (3, 520 * 4096), (7, 1000 * 4096 + 5)])
 def test_multi_stream_add_about_one_tile_per_cta(k, n):
-    """Tile counts for which the launcher picks the single-stage, four-CTAs-per-SM variant of the
-    add kernel (one round of tiles fewer than with three CTAs per SM)."""
+    """2001 to 4001 sub-tiles: one and two rounds of chunks over the CTAs.  (What these sizes were chosen for, the shapes
+    of the collective steps' kernel, runs in ``test_gpu_ranks_in_turn.py``.)"""
     eb = 1e-4
     codec = ops.Codec(max_elems=8 * n)
     xs = [ALL["gradient"](n, seed=20 + i) for i in range(k)]
@@ -271,9 +271,8 @@ def test_stream_files_cross_between_device_and_host(tmp_path):
 
 
 @pytest.mark.parametrize("name", ["gradient", "sparse"])
-def test_prepass_offsets_give_the_same_bytes(name):
-    """Streams of 1024 tiles and more get their tile offsets from the pre-pass kernel: decode and all
-    homomorphic adds must give the bytes of the look-back path and of the oracle, ragged tail included."""
+def test_streams_of_a_thousand_tiles_match_the_oracle(name):
+    """Adds of two rounds of chunks, decode of one or two sub-tiles a warp, ragged tail included."""
     n, eb = 1024 * 4096 + 4096 * 3 + 77, 1e-4
     c = ops.Codec(max_elems=2 * n + 65536)  # two input streams, each rounded up to whole chunks
     x, y = ALL[name](n, seed=11), ALL[name](n, seed=12)
@@ -282,19 +281,17 @@ def test_prepass_offsets_give_the_same_bytes(name):
     gsy = _gpu(np.concatenate([sy, np.zeros(32, np.uint8)]))
     ref_add = ops.cpu_hom_add(sx, y, eb)
     ref_dec = ops.cpu_decompress(sx, n, eb)
-    for on in (True, False):
-        c.set_prepass(on)
-        d = torch.full((n,), 3.0, device="cuda")
-        c.decompress(gsx, n, eb, out=d, stream_bytes=sx.size)
-        np.testing.assert_array_equal(d.cpu().numpy(), ref_dec)
-        out, size = c.hom_add(gsx, _gpu(y), eb, stream_bytes=sx.size)
-        np.testing.assert_array_equal(_stream(out, size), ref_add)
-        out, size = c.hom_add_streams(gsx, gsy, n, a_bytes=sx.size, b_bytes=sy.size)
-        np.testing.assert_array_equal(_stream(out, size), ref_add)
-        out, size = c.hom_add_multi([gsx, gsy], torch.zeros(n, device="cuda"), eb, stream_bytes=[sx.size, sy.size])
-        np.testing.assert_array_equal(_stream(out, size), ref_add)
-        assert c.status() == 0
+    c.set_prepass(True)  # accepted, without effect
+    d = torch.full((n,), 3.0, device="cuda")
+    c.decompress(gsx, n, eb, out=d, stream_bytes=sx.size)
+    np.testing.assert_array_equal(d.cpu().numpy(), ref_dec)
+    out, size = c.hom_add(gsx, _gpu(y), eb, stream_bytes=sx.size)
+    np.testing.assert_array_equal(_stream(out, size), ref_add)
+    out, size = c.hom_add_streams(gsx, gsy, n, a_bytes=sx.size, b_bytes=sy.size)
+    np.testing.assert_array_equal(_stream(out, size), ref_add)
+    out, size = c.hom_add_multi([gsx, gsy], torch.zeros(n, device="cuda"), eb, stream_bytes=[sx.size, sy.size])
+    np.testing.assert_array_equal(_stream(out, size), ref_add)
+    assert c.status() == 0
     # a truncated stream is still reported, not read past its end
-    c.set_prepass(True)
     c.decompress(gsx, n, eb, stream_bytes=sx.size - 5000)
     assert c.status() == 2
