@@ -492,7 +492,7 @@ static int allreduce_direct(hc_comm* c, const float* d_sbuf, float* d_rbuf, size
 }
 
 // A communicator of one rank: the message is compressed and decoded by the stand-alone kernels, one after the other
-// (64 MB: 42 us, against 62 us with the kernels of the collective steps, whose tiles sit at fixed offsets behind
+// (64 MB: 52 us a call, against 62 us with the kernels of the collective steps, whose tiles sit at fixed offsets behind
 // arrival flags so that other ranks can follow).
 static int allreduce_single(hc_comm* c, const float* d_sbuf, float* d_rbuf, size_t count, float eb, hc_stream_t stream) {
   const Layout& L = c->lay;
@@ -711,9 +711,11 @@ extern "C" int hc_allreduce_host(hc_comm* c, const float* h_sbuf, float* h_rbuf,
   if (!c || !h_sbuf || !h_rbuf || !(eb > 0.0f) || count > c->max_count) return hc::kErrArgument;
   if (count == 0) return hc::kOk;
   if (pieces < 1) {
-    // Filling and draining the pipeline costs one piece, and every piece costs about 25 us of its own (two copies that
+    // Filling and draining the pipeline costs one piece, and every piece costs about 23 us of its own (two copies that
     // start and end while the other direction is busy, the events between the streams), so the best number grows
-    // with the square root of the message: 64 MB on one GPU 1731 us in 6 pieces, 1762 in 4, 1908 in 16.
+    // with the square root of the message.  Measured on one GPU, this rule's choice and the best one in us: 1 MB 75 in
+    // one piece (65 in 2), 4 MB 182 in 1 (170 in 3), 16 MB 512 in 3 (the best), 64 MB 1694 in 6 (1687 in 7), 256 MB
+    // 6097 in 14 (the best; 6286 in 6, 6196 in 24).
     const size_t unit = 400000;
     for (pieces = 1; pieces < 16 && (size_t)(pieces + 1) * (size_t)(pieces + 1) * unit <= count + (size_t)pieces * unit; ++pieces) {}
   }

@@ -125,8 +125,8 @@ __device__ __forceinline__ uint64_t sum_status_words(const uint64_t* words, uint
 // Exclusive sum over one total per CTA, by pushing: each CTA adds its total to a word of every later CTA (at most 147
 // reductions, five a lane; sum in [47:0], number of totals in [63:48]), and polls nothing but its own word until it is
 // complete.  Everybody reading everybody's published word instead costs 2.7 us from the last store to the last reader
-// at 148 CTAs, because the polls of all of them queue up on ten L2 lines; this way decode of 256 MB takes 63.3 us (67.4
-// before), a sum of four 4 MB streams 14.4 (16.9).  It is right for one exchange per launch only: with a push for every
+// at 148 CTAs, because the polls of all of them queue up on ten L2 lines; this way decode of 256 MB went from 67.4 us to
+// 63.3, a sum of four 4 MB streams from 16.9 to 14.4.  It is right for one exchange per launch only: with a push for every
 // chunk of a compress of 256 MB the reductions themselves are the queue (70 us, 63 with published words).
 __device__ __forceinline__ void give_total(uint64_t* sums, uint64_t total) {
   for (uint32_t j = blockIdx.x + 1u + (threadIdx.x & 31u); j < gridDim.x; j += 32u)

@@ -52,6 +52,8 @@ size_t hc_chunk_elems(size_t count, int P);
 // `stream`: they never allocate, never synchronise and never copy to the host.  The exact stream
 // length is written to the device word d_size.  One codec handle serialises on one stream at a
 // time (its workspace holds the look-back state of the launch in flight).
+// Calls are not meant to be replayed from a CUDA graph: every launch carries a number of its own that tells its words in
+// the workspace from those of earlier launches, and a replay would repeat it.
 // Input streams are read with 16-byte aligned bulk copies: the buffer that holds a stream must be
 // readable up to the next 16-byte boundary past its last byte (true of any device allocation whose
 // size is a multiple of 16, e.g. one of hc_max_compressed_bytes(n) rounded up).

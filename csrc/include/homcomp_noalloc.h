@@ -18,8 +18,8 @@
 //   * n may not exceed HC_NOALLOC_MAX_ELEMS values; larger calls fail with status 4 (argument)
 //     and do nothing.
 //   * The FIRST call on each device looks up the array's device address (cudaGetSymbolAddress,
-//     with that device current) and registers the kernel's shared-memory size.  Make that first
-//     call before any stream capture begins.
+//     with that device current) and registers the kernel's shared-memory size.  As everywhere in the
+//     library, calls are not meant to be replayed from a CUDA graph (see homcomp_b200.h).
 //   * Every call on a device uses the same array, which keeps what the last call left in it.  The
 //     counters that must start from zero are put back by the kernel itself when its last block
 //     leaves, and everything else is tagged with a call number, so stale contents are ignored.
