@@ -12,14 +12,14 @@
 //            arrival flag)
 //            and brings the payload bytes into shared memory with one bulk copy (up to 8 streams
 //            per tile through two staging buffers);
-//   compute  decodes the staged payloads to deltas and sums them, moves the PREVIOUS tile's packed
-//            payload to its byte offset in global or peer memory (16-byte stores, or one multimem
-//            store for all ranks), then quantises the local values, adds, chooses the block mode,
+//   compute  decodes the staged payloads to deltas and sums them, quantises the local values, adds,
+//            chooses the block mode, moves packed tiles whose place is known to their byte offset in
+//            global or peer memory (16-byte stores, or one multimem store for all ranks),
 //            transposes the magnitudes to bit planes in registers (hc_bitplane.h) and packs the
-//            tile's payload into the stage the fp32 tile came in;
-//   scanner  runs the two-level decoupled look-back of the OUTPUT stream as soon as the tile total
-//            is known and hands the compute warps the tile's global offset; when the launch is a
-//            step of a collective it raises the consumers' arrival flags (call number and payload
+//            tile's payload into a byte ring (in place: into the stage the fp32 tile came in);
+//   scanner  finds a tile's offset in the OUTPUT stream as soon as its total is known (fixed offsets, or
+//            the two-level decoupled look-back where tiles are packed back to back), hands it to the
+//            compute warps and raises the consumers' arrival flags (call number and payload
 //            offset in one 64-bit word), one system-scope fence per four stored tiles.
 // The roles hand tiles to each other through mbarriers, so the compute warps never wait on a
 // global-memory round trip of their own.  Look-back status words are 64-bit and epoch-tagged:
@@ -122,8 +122,7 @@ struct SoloParams {
 };
 
 // One decode launch can take several independent streams ("segments"): the all-gather phase of a
-// collective decodes the P reduced chunks with one kernel.  Every segment owns tiles_per_seg
-// consecutive tile tickets and its own look-back chain.
+// collective decodes the P reduced chunks with one kernel, whose tickets go round the segments.
 struct DecSegment {
   const uint8_t* in;
   uint64_t in_size;
