@@ -27,11 +27,6 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
 __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
   asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-// stores v when j <= limit, as a predicated store (no branch)
-__device__ __forceinline__ void sts32_upto(uint32_t addr, uint32_t v, uint32_t j, uint32_t limit) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.le.u32 p, %2, %3;\n\t@p st.shared.u32 [%0], %1;\n\t}" ::"r"(addr), "r"(v), "r"(j), "r"(limit)
-               : "memory");
-}
 // (a & b) | c in one operation, with b and c kept from being split into two immediates
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
@@ -168,6 +163,7 @@ __host__ __device__ constexpr int lorenzo_stride() { return MODE == kModeVec ? 4
 struct BlockCode {
   uint32_t rate;  // rate byte
   uint32_t len;   // payload bytes
+  uint32_t nout;  // outlier bytes (0: plain layout)
   uint32_t a0;    // |d_0|
   uint32_t sign;  // sign map, element i at bit 31 - i
 };
@@ -212,7 +208,11 @@ __device__ __forceinline__ uint32_t or_rows_tail(const uint32_t (&T)[32]) {
   for (int i = 1; i < 32; ++i) o |= T[i ^ 7];
   return o;
 }
-// sign-magnitude deltas -> the block's code; d_0 of an outlier block is taken out of the planes
+// sign-magnitude deltas -> the block's code; d_0 of an outlier block is taken out of the planes.
+// choose_rate() and payload_len() in fewer operations.  With f and w the bit widths of or_tail and |d_0| and o the
+// bytes that w bits take, the plain layout has 4 + 4 max(f, w) bytes (none if that maximum is 0), the outlier layout
+// 4 + 4 f + o, and the smaller one is taken, plain if equal.  For w <= f that is plain; for w > f it is the outlier layout if
+// 4 w > 4 f + o, which w <= f never meets.
 template <int MODE>
 __device__ __forceinline__ BlockCode code_of(uint32_t (&d)[32], uint32_t or_tail) {
   BlockCode c;
@@ -220,9 +220,17 @@ __device__ __forceinline__ BlockCode code_of(uint32_t (&d)[32], uint32_t or_tail
 #pragma unroll
   for (int i = 0; i < 32; ++i) c.sign = __funnelshift_l(d[i], c.sign, 1);
   c.a0 = d[0] & 0x7fffffffu;
-  c.rate = choose_rate(or_tail | c.a0, or_tail, c.a0, MODE != kModePlain);
-  c.len = payload_len(c.rate);
-  if (c.rate & 0x80u) d[0] = 0;
+  const uint32_t f = 32u - (uint32_t)__clz((int)or_tail), w = 32u - (uint32_t)__clz((int)c.a0), o = (w + 7u) >> 3;
+  const uint32_t top = f > w ? f : w;
+  c.rate = top;
+  c.len = top ? 4u * top + 4u : 0u;
+  c.nout = 0;
+  if (MODE != kModePlain && 4u * w > 4u * f + o) {
+    c.rate = f + 32u * o + 96u;  // 0x80 | (o - 1) << 5 | f
+    c.len = 4u * f + 4u + o;
+    c.nout = o;
+    d[0] = 0;
+  }
   return c;
 }
 
@@ -234,25 +242,26 @@ __device__ __forceinline__ BlockCode code_of(uint32_t (&d)[32], uint32_t or_tail
 template <int W>
 __device__ __forceinline__ void pack_block(uint32_t base, uint32_t rel, const BlockCode& c, const uint32_t (&T)[32]) {
   const uint32_t F = c.rate & 31u;
-  const bool outl = (c.rate & 0x80u) != 0;
-  const uint32_t nout = outl ? ((c.rate >> 5) & 3u) + 1u : 0u;
-  const uint32_t a0 = outl ? c.a0 : 0u;
-  const uint32_t p2 = rel + nout;
-  const uint32_t s0 = 8u * (rel & 3u), s = 8u * (p2 & 3u);
+  const uint32_t a0 = c.nout ? c.a0 : 0u;
+  const uint32_t p2 = rel + c.nout;
+  const uint32_t s0 = 8u * rel, s = 8u * p2;  // (funnel shifts take them modulo 32)
   const uint32_t first = base + (rel & ~3u), at = base + (p2 & ~3u);  // words of the first byte, of the sign map
   const uint32_t sign = __byte_perm(c.sign, 0, 0x0123);
-  uint32_t head = a0 << s0;
+  uint32_t head = __funnelshift_l(0u, a0, s0);
   if (c.len) {
-    const uint32_t x = sign << s;
-    if (at == first) head |= x;
-    else sts32(at, __funnelshift_l(a0, 0u, s0) | x);
+    // words 1 .. F + 1 hold payload; as bits of a register seven comparisons turn into one instruction
+    const uint32_t live = (4u << F) - 1u;
     uint32_t prev = sign;
 #pragma unroll
     for (int j = 1; j <= W + 1; ++j) {
       const uint32_t next = j <= W ? T[j - 1] : 0u;
-      sts32_upto(at + 4 * j, __funnelshift_l(prev, next, s), (uint32_t)j, F + 1u);
+      const uint32_t v = __funnelshift_l(prev, next, s);
+      if (W <= 16 ? (live & (1u << (j & 31))) != 0 : (uint32_t)j <= F + 1u) sts32(at + 4 * j, v);
       prev = next;
     }
+    const uint32_t x = __funnelshift_l(0u, sign, s);
+    if (at == first) head |= x;
+    else sts32(at, __funnelshift_l(a0, 0u, s0) | x);
   }
   __syncwarp();
   if (c.len) sts32(first, (rel ? lds32(first) : 0u) | head);

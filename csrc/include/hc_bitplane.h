@@ -9,8 +9,8 @@
 // index with bit s of the column index.  Stages 16 and 8 are byte permutes (PRMT), stages 4, 2, 1
 // are shift-xor swaps.  When every magnitude of the block fits W bits (W = 4, 8, 12, 16) the upper rows
 // of the result are known zero and most of the network disappears, which is what makes the
-// thread-per-block layout cheaper than one warp ballot per plane: cost is ~2.6 (W=8) to ~9.5 (W=32)
-// integer instructions per element, independent of F.
+// thread-per-block layout cheaper than one warp ballot per plane: 114 instructions a block at W = 12, 140 at W = 16 (150 and 188 before the
+// bit selects were single instructions; isolated loops, counted), independent of F.
 //
 // The reference packs planes with 32 shift/or pairs per output byte (HomComp/src/GSZ.cu:1698-1735).
 #pragma once
@@ -18,14 +18,33 @@
 
 namespace hc {
 
+// byte permute; selector bit 3 gives the chosen byte's sign bit in all eight places (which __byte_perm leaves out)
 HC_HD uint32_t perm(uint32_t a, uint32_t b, uint32_t sel) {
 #if defined(__CUDA_ARCH__)
-  return __byte_perm(a, b, sel);
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
 #else
   uint64_t v = ((uint64_t)b << 32) | a;
   uint32_t r = 0;
-  for (int k = 0; k < 4; ++k) r |= (uint32_t)((v >> (8 * ((sel >> (4 * k)) & 7))) & 0xff) << (8 * k);
+  for (int k = 0; k < 4; ++k) {
+    uint32_t byte = (uint32_t)(v >> (8 * ((sel >> (4 * k)) & 7))) & 0xffu;
+    if ((sel >> (4 * k)) & 8u) byte = byte & 0x80u ? 0xffu : 0u;
+    r |= byte << (8 * k);
+  }
   return r;
+#endif
+}
+
+// bits of a where m has ones, of b where it has zeros.  One 3-input operation; written as plain C, two constant masks
+// (m and ~m) each take an operation of their own, because an instruction holds one immediate
+HC_HD uint32_t bit_select(uint32_t a, uint32_t b, uint32_t m) {
+#if defined(__CUDA_ARCH__)
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xe4;" : "=r"(d) : "r"(a), "r"(b), "r"(m));
+  return d;
+#else
+  return (a & m) | (b & ~m);
 #endif
 }
 
@@ -35,8 +54,8 @@ template <int S>
 HC_HD void swap_stage(uint32_t& lo, uint32_t& hi) {
   constexpr uint32_t m = S == 4 ? 0x0f0f0f0fu : (S == 2 ? 0x33333333u : 0x55555555u);
   const uint32_t l = lo, h = hi;
-  lo = (l & m) | ((h << S) & ~m);
-  hi = ((l >> S) & m) | (h & ~m);
+  lo = bit_select(l, h << S, m);
+  hi = bit_select(l >> S, h, m);
 }
 
 // Forward: rows A[0..31] hold values below 2^W; on return A[0..W-1] hold planes 0..W-1.
@@ -66,14 +85,14 @@ HC_HD void planes_from_rows(uint32_t (&A)[32]) {
   // stage 4
   if (W == 4) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) A[k] = (A[k] & 0x0f0f0f0fu) | ((A[k + 4] << 4) & 0xf0f0f0f0u);
+    for (int k = 0; k < 4; ++k) A[k] = bit_select(A[k], A[k + 4] << 4, 0x0f0f0f0fu);
   } else {
 #pragma unroll
     for (int k = 0; k < R; ++k)
       if ((k & 4) == 0) swap_stage<4>(A[k], A[k + 4]);
     if (W == 12) {
 #pragma unroll
-      for (int k = 8; k < 12; ++k) A[k] = (A[k] & 0x0f0f0f0fu) | ((A[k + 4] << 4) & 0xf0f0f0f0u);
+      for (int k = 8; k < 12; ++k) A[k] = bit_select(A[k], A[k + 4] << 4, 0x0f0f0f0fu);
     }
   }
 #pragma unroll
@@ -117,6 +136,17 @@ HC_HD void rows_from_planes(uint32_t (&A)[32]) {
       A[k + 8] = perm(v, 0u, 0x4441);
       A[k + 16] = perm(v, 0u, 0x4442);
       A[k + 24] = perm(v, 0u, 0x4443);
+    }
+    return;
+  }
+  if (W == 12) {  // the same: two bytes a row, the upper one below 16, so that its sign (selectors 8 and up) fills the rest
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t lo = A[k], hi = A[k + 8];
+      A[k] = perm(lo, hi, 0xcc40);
+      A[k + 8] = perm(lo, hi, 0xdd51);
+      A[k + 16] = perm(lo, hi, 0xee62);
+      A[k + 24] = perm(lo, hi, 0xff73);
     }
     return;
   }
