@@ -405,7 +405,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       }
       load_row_swizzled(stage, (int)lane, d);
       if (kFloat) {
-        deltas_sub<MODE>(d, p.recip);
+        deltas_sub<MODE>(d, p.recip, p.one);
         // exact when no quantised value of the block reaches 2^24: |q_0| below 2^23 and 31 differences below 2^18
         or_tail = or_tail_of(d);
         if (!__all_sync(0xffffffffu, or_tail < (1u << 18) && (d[0] & 0x7fffffffu) < (1u << 23))) {
@@ -459,8 +459,10 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
         } else if (__all_sync(0xffffffffu, fits) && !ints) {
           const uint32_t m = (uint32_t)((int32_t)sign >> 31);
           d[0] += (T[7] ^ m) - m;
+          d[1] = as_u(__fadd_rn(as_f(d[1]), as_f(signed_sub(T[6], sign, 1))));
 #pragma unroll
-          for (int i = 1; i < 32; ++i) d[i] = as_u(__fadd_rn(as_f(d[i]), signed_sub(T[i ^ 7], sign, i)));
+          for (int i = 2; i < 32; i += 2)
+            unpack2(add2(pack2(d[i], d[i + 1]), pack2(signed_sub(T[i ^ 7], sign, i), signed_sub(T[(i + 1) ^ 7], sign, i + 1))), d[i], d[i + 1]);
         } else {
           if (!ints) {
 #pragma unroll
@@ -593,6 +595,7 @@ cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t str
   const int nc = (int)split.warps;
   memcpy(p.first, split.first, sizeof(p.first));
   p.one_round = split.one_round;
+  p.one = 1.0f;
   p.out_words = p.ws.st_a;
   p.in_words = p.ws.st_a + p.first[p.n_seg];
   return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE>, (int)split.grid, 32 * (nc + 1), smem(nc), stream, maps, p);

@@ -111,6 +111,7 @@ struct SoloParams {
   uint32_t n_seg;
   uint32_t n_in;
   float recip;  // 0.5f / eb
+  float one;    // 1.0f (dev::quantise_sub2)
   const uint8_t* in[kMaxIn];
   uint64_t in_size[kMaxIn];
   uint64_t out_cap;
