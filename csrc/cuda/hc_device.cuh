@@ -62,14 +62,16 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 }
 // bounded wait; false = gave up
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  const long long limit_clk = (long long)limit_ns * 2;  // SM clock is at most ~2 GHz
-  for (uint32_t it = 0; it < (1u << 26); ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 63u) == 63u && clock64() - t0 > limit_clk) return false;
+  long long t0 = 0;
+#pragma unroll 1
+  for (uint32_t it = 0; !mbar_try_wait(bar, parity); ++it) {
+    if ((it & 63u) == 0u) {
+      const long long now = clock64();
+      if (it == 0u) t0 = now;
+      else if (now - t0 > (long long)limit_ns * 2 || it >= (1u << 26)) return false;  // SM clock is at most ~2 GHz
+    }
   }
-  return false;
+  return true;
 }
 
 // ---- TMA (tiled, 2-D, no cluster features) -------------------------------------------------------

@@ -60,6 +60,7 @@ struct Chunk {
 __device__ __forceinline__ Chunk chunk_of(const SoloParams& p, uint32_t t) {
   if (p.n_seg == 1u) return Chunk{0u, t};
   uint32_t g = 0;
+#pragma unroll 1
   while (g + 1 < p.n_seg && t >= p.first[g + 1]) ++g;
   return Chunk{g, t - p.first[g]};
 }
@@ -105,6 +106,7 @@ __device__ __forceinline__ bool totals_wait(EncShared& sh, uint32_t k, const Wor
 __device__ __forceinline__ void publish_inputs(const SoloParams& p, uint32_t nc, uint32_t subs, uint32_t t, uint32_t q0, uint32_t dq) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t a = t * nc, b = a + nc < subs ? a + nc : subs;
+#pragma unroll 1
   for (uint32_t q = q0; q < p.n_in; q += dq) {
     const uint32_t all = __reduce_add_sync(0xffffffffu, payload_len16(rates16(p.in[q], p.in_size[q], a, b, lane)));
     if (lane == 0) st_relaxed_gpu_u64(p.in_words + (size_t)q * p.first[1] + t, st_pack(kStAgg, p.ws.epoch, all));
@@ -134,20 +136,27 @@ __device__ __forceinline__ void input_offsets(const SoloParams& p, EncShared& sh
 // Adds up the chunk totals, places the payloads; keeps the input offsets kInSlots chunks ahead of the compute warps and
 // the published input totals two chunks ahead of that (the first chunk's inputs are the compute warps' work).  Leaves when
 // a compute warp has given up; what that leaves unplaced runs out in the others' waits.
-__device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32_t nc, uint32_t subs) {
+__device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32_t nc, uint32_t subs, bool has_in) {
   const uint32_t lane = threadIdx.x & 31u;
   const Workspace& ws = p.ws;
+  // section A covers whole chunks of 32768 values: what is behind the blocks
+  for (uint32_t g = blockIdx.x; g < p.n_seg; g += gridDim.x)
+#pragma unroll 1
+    for (uint64_t b = (uint64_t)p.subs[g] * kSubBlocks + lane; b < rate_bytes(p.n[g]); b += 32u) p.out[g][b] = 0;
   constexpr uint32_t kLead = 2;
   auto inputs_ahead = [&](uint32_t k) {  // offsets of chunk k, totals of chunk k + kLead
     const uint32_t lead = ticket(p, k + kLead), t = ticket(p, k);
     if (lead != kNoTile) publish_inputs(p, nc, subs, lead, 0u, 1u);
     if (t == kNoTile) return;
+#pragma unroll 1
     for (uint32_t q = 0; q < p.n_in; ++q) input_offsets(p, sh, nc, subs, t, q, k % kInSlots, ticket(p, k - 1) + 1u);
   };
-  if (p.n_in) {
+  if (has_in) {
+#pragma unroll 1
     for (uint32_t k = 1; k <= kLead; ++k)
       if (ticket(p, k) != kNoTile) publish_inputs(p, nc, subs, ticket(p, k), 0u, 1u);
     if (!warp_wait(&sh.in_known[0], 0u, ws, kSiteLoaderInFree)) return;  // in_run is the compute warps' until then
+#pragma unroll 1
     for (uint32_t k = 1; k < (uint32_t)kInSlots; ++k) inputs_ahead(k);
   }
   uint32_t next = 0;  // chunks [first of the segment, next) are in base
@@ -182,7 +191,7 @@ __device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32
     }
     base += all;
     next = t + 1;
-    if (p.n_in) inputs_ahead(k + kInSlots);  // every compute warp has taken the inputs of chunk k out of the slot
+    if (has_in) inputs_ahead(k + kInSlots);  // every compute warp has taken the inputs of chunk k out of the slot
   }
 }
 
@@ -201,6 +210,17 @@ __device__ __noinline__ void cold_local(uint8_t* stage, int row, float recip) {
     for (int i = 0; i < 32; ++i) x[i] = sign_magnitude(x[i]);
   }
   store_row_swizzled(stage, row, x);
+}
+
+// Rows that the TMA unit cannot bring (a ragged end, an operand off the 16-byte boundary), past `n` zeros.  Coherent loads: the
+// kernel may have started while the one that writes the operand was still at work.
+static __device__ __noinline__ void load_rows(uint8_t* stage, const uint32_t* src, uint64_t first, uint64_t n) {
+  const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll 4
+  for (int r = 0; r < kSubBlocks; ++r) {
+    const uint64_t i = first + r * kBlock + lane;
+    sts32((swizzled_row(stage, r) ^ ((lane >> 2) << 4)) | ((lane & 3u) << 2), i < n ? __ldcg(src + i) : 0u);
+  }
 }
 
 // ---- the kernel --------------------------------------------------------------------------------------------------
@@ -244,7 +264,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   if (sh.dead) return;  // (one answer for all warps)
   const uint32_t subs0 = p.subs[0];
   if (warp == nc) {
-    clerk(p, sh, nc, subs0);
+    clerk(p, sh, nc, subs0, kHasIn);
     return;
   }
 
@@ -342,6 +362,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     load_rate();
     if (t != kNoTile) {
       publish_inputs(p, nc, subs0, t, warp, nc);
+#pragma unroll 1
       for (uint32_t q = warp; q < Q; q += nc) input_offsets(p, sh, nc, subs0, t, q, 0u, 0u);
     }
   }
@@ -371,6 +392,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   if (tid == 0) HC_PH_START();
   for (;; ++k) {
     if (t == kNoTile) {
+#pragma unroll 1
       while (copied < k) {
         if (!warp_wait(&sh.placed[copied % kSlots], (copied / kSlots) & 1u, ws, kSiteCopierBase)) break;
         copy_oldest();
@@ -393,14 +415,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       }
       if (tid == 0) HC_PH(1);
       if (!by_tma(w)) {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(p.local[w.seg]);
-        const uint64_t first = (uint64_t)w.sub * kSubValues, n = n_local(w.seg);
-        // (coherent loads: the kernel may have started while the one that writes the operand was still at work)
-#pragma unroll 4
-        for (int r = 0; r < kSubBlocks; ++r) {
-          const uint64_t i = first + r * kBlock + lane;
-          sts32((swizzled_row(stage, r) ^ ((lane >> 2) << 4)) | ((lane & 3u) << 2), i < n ? __ldcg(src + i) : 0u);
-        }
+        load_rows(stage, reinterpret_cast<const uint32_t*>(p.local[w.seg]), (uint64_t)w.sub * kSubValues, n_local(w.seg));
         __syncwarp();
       }
       load_row_swizzled(stage, (int)lane, d);
@@ -426,7 +441,9 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     if (tid == 0) HC_PH(2);
     // ---- incoming streams ----------------------------------------------------------------------------------------------
     if (kHasIn) {
+#pragma unroll 1
       for (uint32_t q = 0; q < Q; ++q) {
+#pragma unroll 1
         while (staged < 2u && pt != kNoTile) {
           const uint32_t before = staged;
           produce();
@@ -516,18 +533,18 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     const uint32_t subs = p.subs[w.seg];
     uint8_t* const rates = p.out[w.seg];
     if (w.sub < subs) rates[(uint64_t)w.sub * kSubBlocks + lane] = (uint8_t)code.rate;
-    if (w.sub + 1 == subs)  // section A covers whole chunks of 32768 values
-      for (uint64_t b = (uint64_t)subs * kSubBlocks + lane; b < rate_bytes(p.n[w.seg]); b += 32u) rates[b] = 0;
 
     if (tid == 0) HC_PH(5);
     // payloads whose place is known leave; the oldest ones have to where this one needs their room
     // (one a turn keeps the pace; a second look pays only where they pile up)
     if (copied < k && placed(copied)) {
       copy_oldest();
+#pragma unroll 1
       while (copied + 2u < k && placed(copied)) copy_oldest();
     }
     const uint32_t need = room_for(tot);
     uint32_t start = head;
+#pragma unroll 1
     while (true) {
       bool room = true;
       start = head;

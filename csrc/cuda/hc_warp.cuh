@@ -83,17 +83,18 @@ __device__ __forceinline__ uint32_t load_rates4(const uint8_t* in, uint64_t in_s
   return r;
 }
 
+// the 16 rate bytes at `at` of a stream that is not aligned, or that ends among them (out of line: every caller has the code
+// for aligned ones next to the call)
+static __device__ __noinline__ uint4 rates16_any(const uint8_t* in, uint64_t in_size, uint64_t at) {
+  return make_uint4(load_rates4(in, in_size, at), load_rates4(in, in_size, at + 4u), load_rates4(in, in_size, at + 8u),
+                    load_rates4(in, in_size, at + 12u));
+}
 // rate bytes [16 l, 16 l + 16) of the sub-tiles [a, b) of a stream; 0 past b and past the end of the stream
 __device__ __forceinline__ uint4 rates16(const uint8_t* in, uint64_t in_size, uint32_t a, uint32_t b, uint32_t l) {
   const uint64_t at = (uint64_t)a * kSubBlocks + 16u * l;
-  uint4 v = make_uint4(0, 0, 0, 0);
-  if (at >= (uint64_t)b * kSubBlocks) return v;
+  if (at >= (uint64_t)b * kSubBlocks) return make_uint4(0, 0, 0, 0);
   if ((reinterpret_cast<uintptr_t>(in) & 15u) == 0 && at + 16u <= in_size) return ld_cg_u4(in + at);
-  v.x = load_rates4(in, in_size, at);
-  v.y = load_rates4(in, in_size, at + 4u);
-  v.z = load_rates4(in, in_size, at + 8u);
-  v.w = load_rates4(in, in_size, at + 12u);
-  return v;
+  return rates16_any(in, in_size, at);
 }
 __device__ __forceinline__ uint32_t payload_len16(const uint4& v) {
   return payload_len4(v.x) + payload_len4(v.y) + payload_len4(v.z) + payload_len4(v.w);
