@@ -73,9 +73,10 @@ __device__ __forceinline__ uint32_t ticket(const SoloParams& p, uint32_t k) {
 
 // Running sum over the totals of consecutive chunks of a launch: brings `base` from chunk `next` to chunk t (one warp)
 __device__ __forceinline__ void advance_base(const uint64_t* words, uint32_t& next, uint64_t& base, uint32_t t, const Workspace& ws) {
+#pragma unroll 1
   while (next < t) {
     const uint32_t n = t - next < (uint32_t)kMaxCtas ? t - next : (uint32_t)kMaxCtas;
-    base += sum_status_words<kMaxCtas / 32>(words + next, n, ws);
+    base += sum_totals(words + next, n, ws);
     next += n;
   }
 }

@@ -100,24 +100,27 @@ __device__ __forceinline__ uint32_t payload_len16(const uint4& v) {
   return payload_len4(v.x) + payload_len4(v.y) + payload_len4(v.z) + payload_len4(v.w);
 }
 
-// Sum of the status words words[0 .. n) of this launch (n <= 32 * U), one warp; polls until all are there (bounded)
-template <int U>
-__device__ __forceinline__ uint64_t sum_status_words(const uint64_t* words, uint32_t n, const Workspace& ws) {
+// Sum of the totals words[0 .. n) of chunks of this launch (n <= kMaxCtas, a total below 2^24 each), one warp; polls until all
+// are there (bounded).  Out of line, because it is the clerk's in more than one place and compute warps share its cache.
+static __device__ __noinline__ uint32_t sum_totals(const uint64_t* words, uint32_t n, const Workspace& ws) {
   const uint32_t lane = threadIdx.x & 31;
-  const long long t0 = clock64();
-  const long long limit_clk = (long long)ws.spin_limit_ns * 2;
+  const uint32_t tag = (uint32_t)(st_pack(kStAgg, ws.epoch, 0) >> 32);
+  long long t0 = 0;
+#pragma unroll 1
   for (uint32_t it = 0; it < (1u << 24); ++it) {
-    uint64_t w[U], sum = 0;
+    uint64_t w[kMaxCtas / 32];
+    uint32_t sum = 0;
     bool ready = true;
 #pragma unroll
-    for (int u = 0; u < U; ++u) w[u] = lane + 32u * u < n ? ld_relaxed_gpu_u64(words + lane + 32u * u) : st_pack(kStAgg, ws.epoch, 0);
+    for (int u = 0; u < kMaxCtas / 32; ++u) w[u] = lane + 32u * u < n ? ld_relaxed_gpu_u64(words + lane + 32u * u) : (uint64_t)tag << 32;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      ready = ready && st_state(w[u], ws.epoch) != 0;
-      sum += st_value(w[u]);
+    for (int u = 0; u < kMaxCtas / 32; ++u) {
+      ready = ready && (uint32_t)(w[u] >> 32) == tag;
+      sum += (uint32_t)w[u];
     }
-    if (__all_sync(0xffffffffu, ready)) return warp_sum_u64(sum);
-    if ((it & 15u) == 15u && __any_sync(0xffffffffu, clock64() - t0 > limit_clk || fatal_error(ws.ctrl))) break;
+    if (__all_sync(0xffffffffu, ready)) return __reduce_add_sync(0xffffffffu, sum);
+    if (it == 0u) t0 = clock64();
+    if ((it & 15u) == 15u && __any_sync(0xffffffffu, clock64() - t0 > (long long)ws.spin_limit_ns * 2 || fatal_error(ws.ctrl))) break;
   }
   if (lane == 0) note_timeout(ws, kSiteLookBack);
   return 0;
