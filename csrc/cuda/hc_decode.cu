@@ -1,16 +1,18 @@
 // stream -> fp32 (decompress, its flagged and multi-stream forms): kernel and launcher.
 //
 // A unit of work is a SUB-TILE: 32 consecutive blocks (1024 values, 4 KB of fp32), one block per lane, a quarter
-// of a tile.  Every warp works alone: payloads come by bulk copy into a byte ring of its own (two or three
-// typical payloads fit, one of the worst kind), up to two sub-tiles ahead; the decoded 4 KB go to an output
+// of a tile.  Every warp works alone: payloads come by bulk copy into a byte ring of its own; the decoded 4 KB go to an output
 // buffer (128-byte swizzle) and leave through a TMA tiled store.  Inside the loop no warp waits for another one.
 //
-// Stand-alone streams (RUNS): every warp of the grid owns a contiguous run of sub-tiles.  It sums the payload lengths
-// of its run from the rate bytes (700 bytes for a 256 MB array), the CTAs (one per SM, so at most 148) exchange their
-// totals once through the workspace (about 2 us), and from there on a warp carries its own running offset: no
+// Stand-alone streams (hc_decode_run_kernel; RUNS, the sum of several): every warp of the grid owns a contiguous run of
+// sub-tiles.  It sums the payload lengths of its run from the rate bytes (700 bytes for a 256 MB array), the CTAs (one per SM, so
+// at most 148) exchange their totals once through the workspace, and from there on a warp carries its own running offset: no
 // look-back, no second kernel.  The SMs do not run at the same pace (with equal static shares the first warp of a 256 MB launch
 // finished at 42 us, the last at 70), so the last eighth of every run goes to whoever is free first; the payload
-// offsets of those sub-tiles are written to the workspace at the start.
+// offsets of those sub-tiles are written to the workspace after the first one has been decoded.
+// What bounds them: arrays of 64 MB and more the memory (256 MB: 62 us; 63 with the arithmetic left out, and 34 without the
+// stores), smaller ones the way to the first payload: rate bytes, exchange, payload, one trip to L2 after the other (8 MB: of 6.1 us
+// on the device 3.3; 5.1 of 7.5 when 64-bit divisions, the status and the offsets of the pool stood in between).
 //
 // Steps of a collective (!RUNS): the producer raises one flag word per tile, carrying the tile's payload offset.
 // Tickets are dealt in the order in which the flags rise, round the segments: a tile (all four quarters by one
@@ -23,10 +25,10 @@
 namespace hc {
 namespace dev {
 
-// Warps of a CTA at most, 20 (96 registers a thread) or 16 (128) on an SM.  RUNS: one CTA per SM, so that the totals
+// Warps of a CTA at most, 20 (96 registers a thread) or 16 (128) on an SM.  Stand-alone: one CTA per SM, so that the totals
 // of at most 148 CTAs are exchanged.  Steps of a collective: CTAs of four warps, which slip into an SM one by one
 // while the CTAs of the step before leave it.
-__host__ __device__ constexpr int dec_max_warps(bool sum, bool runs) { return !runs ? 4 : sum ? 16 : 20; }
+__host__ __device__ constexpr int dec_max_warps(bool runs) { return runs ? 16 : 4; }
 __host__ __device__ constexpr int dec_ctas(bool sum, bool runs) { return runs ? 1 : sum ? 4 : 5; }
 // payload ring of a warp: the largest payload of corrupt rate bytes (32 x 132) with its 16-byte phase, and in
 // front of the ring's end what read_planes may look at behind a payload
@@ -35,14 +37,24 @@ constexpr int kDecRingUsable = kDecRing - 160;
 constexpr int kDecWarpBytes = kSubBytes + kDecRing;
 static_assert(32 * 132 + 32 <= kDecRingUsable, "one payload must fit");
 
+// What the TMA unit cannot store of a sub-tile: the ragged last row (not part of the tensor map), or everything when the array is
+// not 16-byte aligned
+static __device__ __noinline__ void store_rows(const uint8_t* rows, const DecSegment& sg, uint64_t first) {
+  const uint32_t len = sg.n - first < kSubValues ? (uint32_t)(sg.n - first) : (uint32_t)kSubValues;
+#pragma unroll 1
+  for (uint32_t e = (sg.use_tma ? len / kBlock * kBlock : 0u) + (threadIdx.x & 31u); e < len; e += 32u)
+    sg.out[first + e] = as_f(lds32((swizzled_row(rows, (int)(e >> 5)) ^ ((e & 28u) << 2)) | ((e & 3u) << 2)));
+  __syncwarp();
+}
+
 // SUM: the n_seg streams hold contributions to ONE array; a warp stages the same sub-tile of every stream in
 // turn, adds the signed deltas in registers and writes seg[0].out once.
 template <int MODE, bool SUM, bool RUNS>
-__global__ void __launch_bounds__(dec_max_warps(SUM, RUNS) * 32, dec_ctas(SUM, RUNS))
+__global__ void __launch_bounds__(dec_max_warps(RUNS) * 32, dec_ctas(SUM, RUNS))
 hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ uint64_t s_full[dec_max_warps(SUM, RUNS)][4];
-  __shared__ uint64_t s_tot[dec_max_warps(SUM, RUNS)][SUM ? kMaxDst : 1];
+  __shared__ uint64_t s_full[dec_max_warps(RUNS)][4];
+  __shared__ uint32_t s_tot[dec_max_warps(RUNS)][kMaxDst];  // payload bytes of a run; RUNS
   __shared__ uint64_t s_pre[kMaxDst];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -58,7 +70,8 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
 
   const uint32_t Q = SUM ? p.n_seg : 1u;  // streams per sub-tile
   const uint32_t gw = blockIdx.x * n_warps + warp, nw = gridDim.x * n_warps;
-  const bool dead = fatal_error(ws.ctrl);  // an earlier launch timed out and nobody has cleared it: no output
+  static_assert(SUM || !RUNS, "one stand-alone stream: hc_decode_run_kernel");
+  const uint32_t status = *((volatile const uint32_t*)(ws.ctrl + 2));
 
   // A job is a sub-tile of one stream.  Its ITEM is a sub-tile (RUNS) or a tile; items are known one ahead, so that
   // the next one's rate bytes and flag are asked for a job or more before they are looked at.
@@ -101,20 +114,42 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   };
 
   // ---- RUNS: shares, offsets -----------------------------------------------------------------------------------------
-  const uint32_t subs = (uint32_t)((p.seg[0].n + kSubValues - 1) / kSubValues);
+  auto run_of = [&](uint32_t w) -> uint32_t { return p.run_all * w + (w < p.run_more ? w : p.run_more); };
   const uint32_t pool = p.pool;  // sub-tiles at the end of every run that are handed out one by one
   uint32_t it = 0, it_end = 0;   // this warp's own sub-tiles still to be staged
   uint64_t run_base = 0;         // lane q: payload offset of the next one in stream q
   uint32_t run_end = 0;
-  uint4 rates[SUM && RUNS ? kMaxDst : 1];
   if (RUNS) {
-    it = (uint32_t)((uint64_t)subs * gw / nw);
-    run_end = (uint32_t)((uint64_t)subs * (gw + 1) / nw);
+    it = run_of(gw);
+    run_end = run_of(gw + 1u);
     it_end = run_end - pool;
+    // Payload bytes of the run in every stream.  Runs of up to four sub-tiles: eight lanes a stream, four streams at a time (a
+    // load per stream, its code eight times over, took 0.5 us more where all is start-up)
+    if (p.run_all + (p.run_more ? 1u : 0u) <= 4u) {
+      const uint32_t l = lane & 7u, q0 = lane >> 3, q1 = q0 + 4u;
+      uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
+      if (q0 < Q) v0 = rates16(p.seg[q0].in, p.seg[q0].in_size, it, run_end, l);
+      if (q1 < Q) v1 = rates16(p.seg[q1].in, p.seg[q1].in_size, it, run_end, l);
+      uint32_t s0 = payload_len16(v0), s1 = payload_len16(v1);  // below 2^16 each: 4 * 32 * 132 at most
+      s0 |= s1 << 16;
 #pragma unroll
-    for (uint32_t qq = 0; qq < (SUM ? kMaxDst : 1); ++qq) rates[qq] = qq < Q ? rates16(p.seg[qq].in, p.seg[qq].in_size, it, run_end, lane) : make_uint4(0, 0, 0, 0);
+      for (int o = 1; o < 8; o <<= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      if (l == 0) {
+        s_tot[warp][q0] = s0 & 0xffffu;
+        s_tot[warp][q1] = s0 >> 16;
+      }
+    } else {
+#pragma unroll 1
+      for (uint32_t qq = 0; qq < Q; ++qq) {
+        uint32_t sum = 0;
+#pragma unroll 1
+        for (uint32_t l = lane; it * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u)
+          sum += payload_len16(rates16(p.seg[qq].in, p.seg[qq].in_size, it, run_end, l));
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0) s_tot[warp][qq] = sum;
+      }
+    }
   }
-  const uint32_t run_begin = it;
   // ---- tickets: sub-tiles of the pools (RUNS), tiles or quarters (!RUNS) -----------------------------------------------
   const bool small = p.parts == 4u;
   const uint32_t n_tickets = RUNS ? pool * nw : (SUM ? p.tiles_per_seg : p.n_tiles) * p.parts;
@@ -147,12 +182,12 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     return RUNS ? t | kPool : t;
   };
   auto tile_at = [&](uint32_t t) -> uint32_t { return small ? t >> 2 : t; };
-  auto seg_at = [&](uint32_t t, uint32_t qq) -> uint32_t { return SUM ? qq : (RUNS ? 0u : tile_at(t) % p.n_seg); };
+  auto seg_at = [&](uint32_t t, uint32_t qq) -> uint32_t { return SUM ? qq : tile_at(t) % p.n_seg; };
   auto local_tile = [&](uint32_t t) -> uint32_t { return SUM ? tile_at(t) : tile_at(t) / p.n_seg; };
   // RUNS: sub-tile and flag word of pool ticket t: the (t / nw)-th pool sub-tile of warp t % nw
   auto pool_sub = [&](uint32_t t) -> uint32_t {
     const uint32_t w = (t & ~kPool) % nw, k = (t & ~kPool) / nw;
-    return (uint32_t)((uint64_t)subs * (w + 1) / nw) - pool + k;
+    return run_of(w + 1u) - pool + k;
   };
   auto pool_flag = [&](uint32_t t, uint32_t qq) -> uint64_t* { return p.flags + (size_t)qq * pool * nw + (t & ~kPool); };
 
@@ -192,25 +227,17 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     HC_PH_START();
   }
   if (!RUNS) ask();
-  uint32_t tk = dead ? kNoTile : next_item(), tk_next = tk == kNoTile ? kNoTile : next_item();
+  // (an earlier launch that timed out, and nobody has cleared its status: no output)
+  uint32_t tk = status >= (uint32_t)kErrTimeout ? kNoTile : next_item(), tk_next = tk == kNoTile ? kNoTile : next_item();
   Unit un, un_next{0ull, 0u, 0u, true};
   uint32_t r = small ? tk & 3u : 0u, q = 0;  // !RUNS: quarter; stream of the next job
   prime(un, tk, 0u);
   if (RUNS) {
-#pragma unroll
-    for (uint32_t qq = 0; qq < (SUM ? kMaxDst : 1); ++qq) {
-      if (qq >= Q) break;
-      uint32_t sum = payload_len16(rates[qq]);
-      for (uint32_t l = lane + 32u; run_begin * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u)
-        sum += payload_len16(rates16(p.seg[qq].in, p.seg[qq].in_size, run_begin, run_end, l));
-      sum = __reduce_add_sync(0xffffffffu, sum);
-      if (lane == 0) s_tot[warp][qq] = sum;
-    }
     __syncthreads();
     for (uint32_t qq = warp; qq < Q; qq += n_warps)
-      give_total(ws.sums + (1u + qq) * kMaxCtas, warp_sum_u64(lane < n_warps ? s_tot[lane][qq] : 0ull));
+      give_total_of(ws.sums + (1u + qq) * kSumWords, warp_sum_u64(lane < n_warps ? s_tot[lane][qq] : 0ull));
     for (uint32_t qq = warp; qq < Q; qq += n_warps) {
-      const uint64_t pre = take_total(ws.sums + (1u + qq) * kMaxCtas, ws);
+      const uint64_t pre = take_total_of(ws.sums + (1u + qq) * kSumWords, ws);
       if (lane == 0) s_pre[qq] = pre;
     }
     __syncthreads();
@@ -457,6 +484,265 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   if (dynamic) cta_epilogue(ws.tick);
 }
 
+
+// ---- one stand-alone stream ----------------------------------------------------------------------------------------
+// The payloads of a warp's run lie behind one another in the stream, so they are staged as what they are: one sequence of bytes,
+// in pieces of kPiece through a ring of four, whatever the sub-tiles in it are.  Staging sub-tile by sub-tile took half of the
+// 700 instructions that a sub-tile cost (its own copy, barrier, room in the ring and bounds).  A sub-tile of a pool is a
+// sequence of its own and begins at a piece.  Bytes are counted through the ring from 0 on (a "place"), place modulo kRing is
+// where they are; the first kMirror bytes of the ring stand once more behind its end, so that a block reads on across it.
+constexpr uint32_t kPiece = 1536, kRing = 4 * kPiece, kMirror = 160;
+constexpr int kRunWarpBytes = kSubBytes + (int)(kRing + kMirror);
+constexpr int kRunWarps = 20;
+static_assert(32 * 132 + 15 <= 1 + 3 * kPiece, "a payload touches four pieces at most");
+static_assert(132 + 8 <= kMirror, "a block and what read_planes looks at behind it");
+
+template <int MODE>
+__global__ void __launch_bounds__(kRunWarps * 32, 1)
+hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ uint64_t s_full[kRunWarps][4];
+  __shared__ uint32_t s_tot[kRunWarps];
+  __shared__ uint64_t s_pre;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
+  uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* const obuf = smem + warp * kSubBytes;
+  uint8_t* const ring = smem + n_warps * kSubBytes + warp * (kRing + kMirror);
+  const Workspace& ws = p.ws;
+  uint64_t* const full = s_full[warp];
+  if (lane < 4u) mbar_init(&full[lane], 1);
+  fence_mbar_init();
+  if (tid == 0) launch_dependents();
+  grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
+  __syncwarp();
+  const DecSegment& sg = p.seg[0];
+  const uint8_t* const in = sg.in;
+  const uint32_t gw = blockIdx.x * n_warps + warp, nw = gridDim.x * n_warps;
+  HC_TL_DECL(ws.epoch);
+  if (tid == 0) {
+    HC_TL_ZERO();
+    HC_STAMP(0);
+    HC_PH_START();
+  }
+
+  // ---- shares, offsets -----------------------------------------------------------------------------------------------
+  // What the first payload waits for, one after the other: rate bytes, total of the CTA, exchange.  Nothing else stands in
+  // between: a 64-bit division by the number of warps, a look at the status and the sums of the pool did, and the first payload of
+  // a 64 MB array was asked for after 6.1 us
+  const uint32_t pool = p.pool;  // sub-tiles at the end of every run that are handed out one by one
+  auto run_of = [&](uint32_t w) -> uint32_t { return p.run_all * w + (w < p.run_more ? w : p.run_more); };
+  const uint32_t run_begin = run_of(gw), run_end = run_of(gw + 1u);
+  const uint32_t own_end = run_end - pool;
+  const uint4 rates = rates16(in, sg.in_size, run_begin, run_end, lane);  // of 16 sub-tiles, and of the next 16
+  const uint4 rates_2 = run_end - run_begin > 16u ? rates16(in, sg.in_size, run_begin, run_end, lane + 32u) : make_uint4(0, 0, 0, 0);
+  const uint32_t status = *((volatile const uint32_t*)(ws.ctrl + 2));
+  auto rate_of = [&](uint32_t sub) -> uint32_t {
+    const uint64_t b = (uint64_t)sub * kSubBlocks + lane;
+    return b < sg.in_size ? ld_cg_u8(in + b) : 0u;
+  };
+  // items: own sub-tiles, then tickets of the pools (kPool set)
+  constexpr uint32_t kPool = 0x80000000u;
+  uint32_t it = run_begin, tk_raw = kNoTile;
+  const uint32_t n_tickets = pool * nw;
+  auto ask = [&]() {
+    if (lane == 0) tk_raw = atomicAdd(ws.tick, 1u);
+  };
+  auto next_item = [&]() -> uint32_t {
+    if (it < own_end) {
+      const uint32_t i = it++;
+      if (it == own_end && pool) ask();
+      return i;
+    }
+    if (!pool) return kNoTile;
+    const uint32_t t = __shfl_sync(0xffffffffu, tk_raw, 0);
+    if (t >= n_tickets) return kNoTile;
+    ask();
+    return t | kPool;
+  };
+  // ticket t is the (t / nw)-th pool sub-tile of warp t % nw
+  auto sub_of = [&](uint32_t item) -> uint32_t {
+    if (!(item & kPool)) return item;
+    const uint32_t w = (item & ~kPool) % nw, k = (item & ~kPool) / nw;
+    return run_of(w + 1u) - pool + k;
+  };
+  uint32_t sub = run_begin, rate = run_begin < run_end ? rate_of(run_begin) : 0u;  // (a pool is smaller than its run)
+  uint32_t sum = payload_len16(rates), own = run_begin + (lane >> 1) < own_end ? sum : 0u;
+#pragma unroll 1
+  for (uint32_t l = lane + 64u; run_begin * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u) {
+    const uint32_t s = payload_len16(rates16(in, sg.in_size, run_begin, run_end, l));
+    sum += s;
+    if (run_begin + (l >> 1) < own_end) own += s;
+  }
+  const uint32_t sum_2 = payload_len16(rates_2);
+  sum += sum_2;
+  if (run_begin + 16u + (lane >> 1) < own_end) own += sum_2;
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (lane == 0) s_tot[warp] = sum;
+  __syncthreads();
+  const uint32_t tot_of = lane < n_warps ? s_tot[lane] : 0u;  // of warp `lane`; sums in two halves of 16 bits
+  auto sum64 = [&](uint32_t v) -> uint64_t {
+    return __reduce_add_sync(0xffffffffu, v & 0xffffu) + ((uint64_t)__reduce_add_sync(0xffffffffu, v >> 16) << 16);
+  };
+  if (warp == 0) {
+    give_total_of(ws.sums + kSumWords, sum64(tot_of));
+    const uint64_t pre = take_total_of(ws.sums + kSumWords, ws);
+    if (lane == 0) s_pre = pre;
+  }
+  uint64_t own_base = rate_bytes(sg.n) + sum64(lane < warp ? tot_of : 0u);  // byte of the stream where this warp's run begins
+  const uint32_t own_bytes = __reduce_add_sync(0xffffffffu, own);           // payload bytes of its own sub-tiles
+  __syncthreads();
+  own_base += s_pre;
+  // (an earlier launch that timed out, and nobody has cleared its status: no output)
+  uint32_t item = status >= (uint32_t)kErrTimeout ? kNoTile : next_item();
+
+  // ---- staging -------------------------------------------------------------------------------------------------------
+  const uint8_t* f_src = in;  // the next bytes to be staged, 16-byte aligned
+  uint32_t f_left = 0;        // of the sequence that is being staged
+  uint32_t issued = 0, landed = 0, freed = 0;  // pieces asked for, waited for, and read
+  auto pump = [&]() {
+    if (lane == 0) fence_proxy_async();  // what used to be in the bytes has been read
+#pragma unroll 1
+    while (f_left && issued - freed < 4u) {
+      const uint32_t bytes = f_left < kPiece ? f_left : kPiece;
+      if (lane == 0) {
+        uint64_t* const bar = &full[issued & 3u];
+        uint8_t* const dst = ring + (issued & 3u) * kPiece;
+        const uint32_t again = issued & 3u ? 0u : bytes < kMirror ? bytes : kMirror;
+        mbar_expect_tx(bar, bytes + again);
+        bulk_load(dst, f_src, bytes, bar);
+        if (again) bulk_load(ring + kRing, f_src, again, bar);
+      }
+      f_src += bytes;
+      f_left -= bytes;
+      ++issued;
+    }
+  };
+  uint32_t limit = 0;  // place up to which the sequence has bytes (the stream may end before its rate bytes say so)
+  // a sequence of `bytes` bytes from byte `off` of the stream: place of its first byte
+  auto begin = [&](uint64_t off, uint32_t bytes) -> uint32_t {
+    const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(in) + off) & 15u;
+    const uint32_t place = issued * kPiece + phase;
+    const uint32_t there = off >= sg.in_size ? 0u : sg.in_size - off < bytes ? (uint32_t)(sg.in_size - off) : bytes;
+    f_src = in + off - phase;
+    f_left = there ? (phase + there + 15u) & ~15u : 0u;
+    limit = place + there;
+    return place;
+  };
+  uint32_t at = item == kNoTile ? 0u : begin(own_base, own_bytes);  // place of the current item's payload
+  pump();
+  uint32_t next = item == kNoTile ? kNoTile : next_item(), next_sub = 0, next_rate = 0;
+  uint64_t next_flag = 0;  // lane 0's look at the payload offset of a pool item
+  auto look = [&]() {
+    if (next == kNoTile) return;
+    next_sub = sub_of(next);
+    next_rate = rate_of(next_sub);
+    if (next & kPool && lane == 0) next_flag = ld_relaxed_gpu_u64(p.flags + (next & ~kPool));
+  };
+  look();
+  bool announced = pool == 0u;
+  if (tid == 0) HC_PH(0);
+
+  while (item != kNoTile) {
+    const uint32_t len = payload_len(rate);
+    const uint32_t inc = warp_inclusive_scan(len, (int)lane);
+    const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
+    if (tot && at + tot > limit) {  // stream shorter than its rate bytes imply
+      if (lane == 0) note_error(ws.ctrl, kErrTruncated);
+      rate = 0;
+    } else {
+      bool gave_up = false;
+      while (landed * kPiece < at + tot && landed < issued) {
+        gave_up = !warp_wait(&full[landed & 3u], (landed >> 2) & 1u, ws, kSiteDecodeInFull);
+        if (gave_up) break;
+        ++landed;
+      }
+      if (gave_up) break;
+    }
+    if (tid == 0) HC_PH(2);
+    uint32_t pos = at % kRing + inc - len;
+    if (pos >= kRing) pos -= kRing;
+    uint32_t T[32], sign, a0;
+    decode_rows(ring, pos, rate, plane_width(__reduce_max_sync(0xffffffffu, rate & 31u)), sign, a0, T);
+    const bool little = (rate & 31u) <= 16u && a0 < (1u << 23);
+    const uint32_t cur = sub;
+    __syncwarp();
+    if (tid == 0) HC_PH(3);
+    // ---- what comes next: its payload begins here, or is a sequence of its own
+    item = next;
+    if (item != kNoTile) {
+      sub = next_sub;
+      rate = next_rate;
+      if (item & kPool) {
+        while (landed < issued && warp_wait(&full[landed & 3u], (landed >> 2) & 1u, ws, kSiteDecodeInFull)) ++landed;
+        freed = landed;
+        uint64_t fw = __shfl_sync(0xffffffffu, next_flag, 0);
+        if (!flag_matches(fw, p.ring_epoch)) fw = own_flag_wait(p.flags + (item & ~kPool), p.ring_epoch, ws);
+        at = begin(fw & kFlagOffsetMask, __reduce_add_sync(0xffffffffu, payload_len(rate)));
+      } else {
+        at += tot;
+        freed = at / kPiece;
+      }
+      pump();
+      next = next_item();
+      look();
+    }
+    if (tid == 0) HC_PH(1);
+
+    // ---- signs, prefix sum, scaling --------------------------------------------------------------------------------
+    uint32_t w[32];
+    constexpr int S = MODE == kModeVec ? 4 : 1;
+    if (p.scale != 0.0f && __all_sync(0xffffffffu, little)) {
+      float qv[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        qv[i] = __fmaf_rn(as_f(T[i ^ 7]), sign_scale(sign, i), i >= S ? qv[i - S] : 0.0f);
+        w[i] = as_u(__fmul_rn(qv[i], p.scale));
+      }
+    } else {
+      int32_t qv[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int32_t m = (int32_t)(sign << i) >> 31;
+        qv[i] = (i >= S ? qv[i - S] : 0) + ((int32_t)T[i ^ 7] ^ m) - m;
+        w[i] = as_u(__fmul_rn(__fmul_rn((float)qv[i], p.eb), 2.0f));
+      }
+    }
+    if (tid == 0) HC_PH(4);
+    // ---- out -------------------------------------------------------------------------------------------------------
+    if (lane == 0) tma_wait_group_read<0>();  // the rows of a turn ago have left the buffer
+    __syncwarp();
+    store_row_swizzled(obuf, (int)lane, w);
+    fence_proxy_async();
+    __syncwarp();
+    const uint64_t first = (uint64_t)cur * kSubValues;
+    if (lane == 0 && sg.use_tma && first + kBlock <= sg.n) {
+      tma_store_2d(&tmaps.m[0], 0, (int)(cur * kSubBlocks), obuf);
+      tma_commit_group();
+    }
+    if (!(sg.use_tma && first + kSubValues <= sg.n) && first < sg.n) store_rows(obuf, sg, first);
+    if (!announced) {
+      // offsets of the sub-tiles of this run that others may take, counted back from its end; after the first own one, so that it
+      // delays nothing (in front of it, 2.3 us at 256 MB)
+      announced = true;
+      uint64_t off = own_base + sum;
+#pragma unroll 1
+      for (uint32_t k = pool; k-- > 0u;) {
+        off -= __reduce_add_sync(0xffffffffu, payload_len(rate_of(own_end + k)));
+        if (lane == 0) st_relaxed_gpu_u64(p.flags + (k * nw + gw), flag_pack(p.ring_epoch, off));
+      }
+    }
+    if (tid == 0) {
+      HC_PH(5);
+      HC_PH_COUNT();
+    }
+  }
+  // after a wait that ran out: nothing may land in shared memory once the CTA has left it
+  for (; landed < issued; ++landed) mbar_wait_bounded(&full[landed & 3u], (landed >> 2) & 1u, ws.spin_limit_ns);
+  if (lane == 0) tma_wait_group<0>();
+  if (lane == 0) HC_STAMP_MAX(7);
+  if (pool) cta_epilogue(ws.tick);
+}
+
 }  // namespace dev
 
 // ---- host side ---------------------------------------------------------------------------------------------
@@ -467,7 +753,7 @@ constexpr int dec_smem(int warps) { return warps * dev::kDecWarpBytes + 1024; }
 
 template <int MODE, bool SUM, bool RUNS>
 cudaError_t launch_t(const TensorMaps& maps, DecParams p, cudaStream_t stream, bool overlap) {
-  constexpr int kWarps = dev::dec_max_warps(SUM, RUNS);
+  constexpr int kWarps = dev::dec_max_warps(RUNS);
   static thread_local int cache[64] = {};
   const int cap = resident_ctas(dev::hc_decode_kernel<MODE, SUM, RUNS>, 32 * kWarps, dec_smem(kWarps), cache);
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
@@ -479,6 +765,8 @@ cudaError_t launch_t(const TensorMaps& maps, DecParams p, cudaStream_t stream, b
     if (run_words(split, p.n_seg) > p.ws.words) return cudaErrorInvalidValue;
     warps = split.warps;
     grid = (int)split.grid;
+    p.run_all = (uint32_t)(subs / (split.grid * split.warps));
+    p.run_more = (uint32_t)(subs % (split.grid * split.warps));
     p.pool = split.pool;
     p.flags = p.ws.st_a;
   } else {
@@ -495,10 +783,31 @@ cudaError_t launch_t(const TensorMaps& maps, DecParams p, cudaStream_t stream, b
   return cudaGetLastError();
 }
 
+template <int MODE>
+cudaError_t launch_run(const TensorMaps& maps, DecParams p, cudaStream_t stream) {
+  static thread_local int cache[64] = {};
+  auto smem = [](int warps) { return warps * dev::kRunWarpBytes + 1024; };
+  const int cap = resident_ctas(dev::hc_decode_run_kernel<MODE>, 32 * dev::kRunWarps, smem(dev::kRunWarps), cache);
+  if (cap <= 0) return cudaErrorLaunchOutOfResources;
+  const uint64_t subs = (p.seg[0].n + dev::kSubValues - 1) / dev::kSubValues;
+  const RunSplit split = split_runs(subs, (uint32_t)(cap < kMaxCtas ? cap : kMaxCtas), (uint32_t)dev::kRunWarps);
+  if (run_words(split, 1) > p.ws.words) return cudaErrorInvalidValue;
+  p.pool = split.pool;
+  p.flags = p.ws.st_a;
+  p.run_all = (uint32_t)(subs / (split.grid * split.warps));
+  p.run_more = (uint32_t)(subs % (split.grid * split.warps));
+  return launch_overlapped(dev::hc_decode_run_kernel<MODE>, (int)split.grid, 32 * (int)split.warps, smem((int)split.warps), stream, maps, p);
+}
+
+template <int MODE, bool SUM>
+cudaError_t launch_solo(const TensorMaps& maps, const DecParams& p, cudaStream_t stream) {
+  if constexpr (SUM) return launch_t<MODE, true, true>(maps, p, stream, false);
+  else return launch_run<MODE>(maps, p, stream);
+}
 template <int MODE, bool SUM>
 cudaError_t launch_f(const TensorMaps& maps, const DecParams& p, cudaStream_t stream, bool overlap) {
   return p.seg[0].in_ready ? launch_t<MODE, SUM, false>(maps, p, stream, overlap)
-                           : launch_t<MODE, SUM, true>(maps, p, stream, false);
+                           : launch_solo<MODE, SUM>(maps, p, stream);
 }
 
 }  // namespace

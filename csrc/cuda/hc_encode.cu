@@ -111,7 +111,7 @@ __device__ __forceinline__ void publish_inputs(const SoloParams& p, uint32_t nc,
   for (uint32_t q = q0; q < p.n_in; q += dq) {
     const uint32_t all = __reduce_add_sync(0xffffffffu, payload_len16(rates16(p.in[q], p.in_size[q], a, b, lane)));
     if (lane == 0) st_relaxed_gpu_u64(p.in_words + (size_t)q * p.first[1] + t, st_pack(kStAgg, p.ws.epoch, all));
-    if (p.one_round) give_total(p.ws.sums + (1u + q) * kMaxCtas, all);
+    if (p.one_round) give_total(p.ws.sums + (1u + q) * kSumWords, all);
   }
 }
 // Payload offsets of the sub-tiles of chunk t in input stream q (slot r of in_at); one warp.  `next`: chunks before it
@@ -124,7 +124,7 @@ __device__ __forceinline__ void input_offsets(const SoloParams& p, EncShared& sh
   const uint32_t inc = warp_inclusive_scan(sum, (int)lane);
   const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
   uint64_t base = sh.in_run[q];
-  if (p.one_round) base = take_total(p.ws.sums + (1u + q) * kMaxCtas, p.ws);
+  if (p.one_round) base = take_total(p.ws.sums + (1u + q) * kSumWords, p.ws);
   else advance_base(p.in_words + (size_t)q * p.first[1], next, base, t, p.ws);
   if (!(lane & 1u) && (lane >> 1) < nc) sh.in_at[r][q][lane >> 1] = rate_bytes(p.n[0]) + base + inc - sum;
   __syncwarp();

@@ -702,7 +702,7 @@ size_t workspace_bytes(size_t max_elems, int sets) {
   if (sets < 1) sets = 1;
   if (sets > kMaxWorkspaceSets) sets = kMaxWorkspaceSets;
   // words of all sets, then the exchange words of all sets
-  return kWorkspaceHeader + (size_t)sets * (workspace_words(max_elems) + (1 + kMaxIn) * kMaxCtas) * sizeof(uint64_t);
+  return kWorkspaceHeader + (size_t)sets * (workspace_words(max_elems) + (1 + kMaxIn) * kSumWords) * sizeof(uint64_t);
 }
 
 Workspace workspace_view(void* mem, size_t max_elems, uint32_t epoch, uint64_t spin_limit_ns, int sets) {
@@ -722,7 +722,7 @@ Workspace workspace_view(void* mem, size_t max_elems, uint32_t epoch, uint64_t s
   w.grp_b = w.grp_a + groups;
   w.grp_out = w.grp_b + groups;
   w.words = words;
-  w.sums = reinterpret_cast<uint64_t*>(b + kWorkspaceHeader) + (size_t)sets * words + set * (1 + kMaxIn) * kMaxCtas;
+  w.sums = reinterpret_cast<uint64_t*>(b + kWorkspaceHeader) + (size_t)sets * words + set * (1 + kMaxIn) * kSumWords;
   w.epoch = epoch;
   w.spin_limit_ns = spin_limit_ns;
   return w;

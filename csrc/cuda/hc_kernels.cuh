@@ -61,7 +61,7 @@ struct Workspace {
   // do with them: encode_words, run_words)
   uint64_t words;
   uint32_t* tick;      // [0] tile ticket counter, [1] CTAs that have left; re-armed by the last CTA of a launch
-  uint64_t* sums;      // [1 + kMaxIn][kMaxCtas] exchange of CTA totals (dev::give_total): zero between launches
+  uint64_t* sums;      // [1 + kMaxIn][kSumWords] exchange of CTA totals (dev::give_total): zero between launches
   uint64_t* size_acc;  // [kMaxDst] payload bytes per segment of a launch with sparse tiles; zeroed by its last CTA
   uint32_t epoch;
   uint64_t spin_limit_ns;
@@ -148,6 +148,7 @@ struct DecParams {
   // one, and their payload offsets as flag words
   uint64_t* flags;
   uint32_t pool;
+  uint32_t run_all, run_more;  // every run has run_all sub-tiles, the first run_more one more
   Workspace ws;
 };
 struct TensorMaps {

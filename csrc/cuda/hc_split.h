@@ -10,6 +10,10 @@ constexpr int kTileElems = kTileBlocks * kBlock;  // 4096
 constexpr int kMaxDst = 8;
 constexpr int kMaxIn = kMaxDst;
 constexpr int kMaxCtas = 160;  // CTAs of a launch with one CTA per SM
+// exchange of CTA totals (dev::give_total): a word per CTA, a word per group of CTAs, and per CTA what its group's word was
+constexpr int kSumGroup = 13, kSumGroups = (kMaxCtas + kSumGroup - 1) / kSumGroup;
+constexpr int kSumWords = kMaxCtas + 16 + kMaxCtas;
+static_assert(kSumGroups <= 16 && kSumGroup <= 16, "one reduction a lane");
 
 // ---- workspace -----------------------------------------------------------------------------------------------------
 // Words in front of the exchange of CTA totals, for calls of up to max_elems values split over up to kMaxDst segments

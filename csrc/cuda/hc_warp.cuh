@@ -159,6 +159,59 @@ __device__ __forceinline__ uint64_t take_total(uint64_t* sums, const Workspace& 
   return __shfl_sync(0xffffffffu, w & ((1ull << 48) - 1), 0);
 }
 
+// The same for more than kDirect CTAs, in groups of kSumGroup: a total goes to the later CTAs of its group and to one word for
+// each later group, at most one reduction a lane where the direct form has up to 147 words to add to, whose 10900 reductions a
+// launch queue up (148 CTAs: the last one had given 1.5 us after it knew its total, 0.4 us this way; decode of 8 MB 7.2 us and
+// 6.4, sum of four 4 MB streams 13.4 and 12.7).  In a launch of few CTAs, and in the one-round launches of the encode kernel, it
+// is no faster and its longer code costs 0.2 to 0.4 us (seven streams of 8 MB added 18.7 us, 19.5 this way).
+// The word of a group has several readers and is never reset: what counts is by how much it has grown since the launch
+// before, whose end every CTA notes for itself (the last one of a launch also for those of its group that the launch does not have).
+constexpr uint32_t kDirect = 33;
+__device__ __forceinline__ void give_total_grouped(uint64_t* sums, uint64_t total) {
+  const uint32_t lane = threadIdx.x & 31u, g = blockIdx.x / kSumGroup;
+  const uint32_t cta = blockIdx.x + 1u + lane, group = lane - 16u;
+  uint64_t* const to = lane < 16u ? sums + cta : sums + kMaxCtas + group;
+  if (lane < 16u ? cta < (g + 1u) * kSumGroup && cta < gridDim.x : group > g && group * kSumGroup < gridDim.x)
+    atomicAdd(reinterpret_cast<unsigned long long*>(to), (1ull << 48) | total);
+}
+__device__ __forceinline__ uint64_t take_total_grouped(uint64_t* sums, const Workspace& ws) {
+  const uint32_t lane = threadIdx.x & 31u, g = blockIdx.x / kSumGroup;
+  uint64_t* const word = lane ? sums + kMaxCtas + g : sums + blockIdx.x;
+  uint64_t* const noted = sums + kMaxCtas + 16;
+  const uint32_t want = lane == 0u ? blockIdx.x - g * kSumGroup : lane == 1u ? g * kSumGroup : 0u;
+  const uint64_t before = lane == 1u ? ld_relaxed_gpu_u64(noted + blockIdx.x) : 0ull;
+  uint64_t w = before;
+  if (want) {
+    long long t0 = 0;
+#pragma unroll 1
+    for (uint32_t it = 0;; ++it) {
+      w = ld_relaxed_gpu_u64(word);
+      if ((w - before) >> 48 == want) break;
+      if (it == 0u) t0 = clock64();
+      if ((it & 15u) == 15u && (clock64() - t0 > (long long)ws.spin_limit_ns * 2 || it >= (1u << 26) || fatal_error(ws.ctrl))) {
+        note_timeout(ws, kSiteLookBack);
+        break;
+      }
+    }
+    st_relaxed_gpu_u64(lane ? noted + blockIdx.x : word, lane ? w : 0ull);
+  }
+  const uint64_t all = (w - before) & ((1ull << 48) - 1);
+  if (blockIdx.x + 1u == gridDim.x) {
+    const uint64_t group = __shfl_sync(0xffffffffu, w, 1);
+    const uint32_t cta = blockIdx.x + 1u + lane;
+    if (g && cta < (g + 1u) * kSumGroup && cta < (uint32_t)kMaxCtas) st_relaxed_gpu_u64(noted + cta, group);
+  }
+  return __shfl_sync(0xffffffffu, all, 0) + __shfl_sync(0xffffffffu, all, 1);
+}
+// decode: by the number of CTAs
+__device__ __forceinline__ void give_total_of(uint64_t* sums, uint64_t total) {
+  if (gridDim.x <= kDirect) give_total(sums, total);
+  else give_total_grouped(sums, total);
+}
+__device__ __forceinline__ uint64_t take_total_of(uint64_t* sums, const Workspace& ws) {
+  return gridDim.x <= kDirect ? take_total(sums, ws) : take_total_grouped(sums, ws);
+}
+
 // the last CTA to leave re-arms the ticket counter for the next launch (true in thread 0 of that CTA)
 __device__ __forceinline__ bool cta_epilogue(uint32_t* tick) {
   __syncthreads();

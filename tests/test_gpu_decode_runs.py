@@ -1,0 +1,107 @@
+"""Decode of stand-alone streams: payloads staged as a sequence of bytes through a ring, runs and pools, and the exchange of
+totals whose words outlive a launch."""
+import numpy as np
+import pytest
+import torch
+
+from tirocinio_triennale_b200 import ops
+
+pytestmark = pytest.mark.gpu
+EB = 0.5  # quantised values are the values themselves
+
+
+def _values(n, kind, seed):
+    rng = np.random.default_rng(seed)
+    if kind == "wide":  # 31 planes: the longest payloads, none of whose sub-tiles ends where a staged piece does
+        x = rng.integers(-2 ** 29, 2 ** 29, n)
+    elif kind == "mixed":  # from no payload to the longest, block by block
+        bits = np.repeat(rng.integers(0, 30, (n + 31) // 32), 32)[:n]
+        x = rng.integers(-2 ** 29, 2 ** 29, n) >> (29 - bits)
+    else:
+        x = rng.integers(-300, 300, n)
+    return x.astype(np.float32)
+
+
+def _on_gpu(stream, shift):
+    t = torch.zeros(stream.size + 64, dtype=torch.uint8, device="cuda")
+    t[shift:shift + stream.size] = torch.from_numpy(stream)
+    return t[shift:shift + stream.size]
+
+
+@pytest.mark.parametrize("mode", ["outlier", "plain", "vec"])
+@pytest.mark.parametrize("kind,n", [("wide", 5_000_003), ("mixed", 3_333_333), ("narrow", 148 * 20 * 1024 * 4), ("mixed", 33 * 1024 * 4 + 1)])
+def test_payloads_of_all_lengths(kind, n, mode):
+    x = _values(n, kind, n)
+    ref = ops.cpu_compress(x, EB, mode)
+    want = ops.cpu_decompress(ref, n, EB, mode)
+    c = ops.Codec(n)
+    got = [c.decompress(_on_gpu(ref, shift), n, EB, mode, stream_bytes=ref.size) for shift in (0, 1, 15)]
+    for g in got:
+        np.testing.assert_array_equal(g.cpu().numpy(), want)
+    assert c.status() == 0
+
+
+def test_runs_of_more_than_32_sub_tiles():
+    n, eb = 148 * 20 * 1024 * 34 + 5, 1e-3
+    x = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    c = ops.Codec(n)
+    s, size = c.compress(x, eb)
+    y = c.decompress(s, n, eb, stream_bytes=int(size))
+    t = x * (torch.tensor(0.5) / torch.tensor(eb)).item()
+    q = (t + 0.5).trunc() - (t < -0.5).float()
+    assert torch.equal(y, q * np.float32(eb) * 2)
+    assert c.status() == 0
+
+
+@pytest.mark.parametrize("n,cut", [(200_000, 3), (200_000, 200_000), (6_000_000, 1), (6_000_000, 7_000_001)])
+def test_stream_that_ends_early(n, cut):
+    x = _values(n, "mixed", 5)
+    ref = ops.cpu_compress(x, EB)
+    want = ops.cpu_decompress(ref, n, EB)
+    c = ops.Codec(n)
+    got = c.decompress(_on_gpu(ref, 0), n, EB, stream_bytes=ref.size - cut).cpu().numpy()
+    assert c.status() == 2
+    rates = ref[:(n + 31) // 32].astype(np.int64)
+    planes = rates & 31
+    lens = np.where(rates & 128, 5 + 4 * planes + (rates >> 5 & 3), np.where(planes, 4 + 4 * planes, 0))
+    lens = np.append(lens, np.zeros(-lens.size % 32, np.int64)).reshape(-1, 32).sum(1)
+    there = (n + 32767) // 32768 * 1024 + np.cumsum(lens) <= ref.size - cut  # sub-tiles whose payload is complete
+    mask = np.repeat(there | (lens == 0), 1024)[:n]
+    np.testing.assert_array_equal(got, np.where(mask, want, 0))
+
+
+@pytest.mark.parametrize("k", [1, 2, 4, 5, 8])
+def test_sums_by_length_of_the_runs(k):
+    sizes = (1, 1024 * 4 * 148, 1024 * 16 * 148 + 1, 1024 * 16 * 148 * 4, 1024 * 16 * 148 * 4 + 1024)
+    c = ops.Codec(k * ((max(sizes) + 32767) // 32768 * 32768))
+    for n in sizes:
+        refs = [ops.cpu_compress(_values(n, "narrow", n + i), EB) for i in range(k)]
+        got = c.decompress_sum([_on_gpu(r, i) for i, r in enumerate(refs)], n, EB, stream_bytes=[r.size for r in refs])
+        want = refs[0]
+        for r in refs[1:]:
+            want = ops.cpu_hom_add_streams(want, r, n)
+        np.testing.assert_array_equal(got.cpu().numpy(), ops.cpu_decompress(want, n, EB))
+    assert c.status() == 0
+
+
+def test_launches_of_all_grids_behind_one_another():
+    """A launch leaves words of the exchange as they are; the next one, with more CTAs or fewer, starts from there."""
+    rng = np.random.default_rng(3)
+    grids = [148, 1, 34, 33, 147, 14, 35, 148, 39, 40, 52, 53, 146, 2] + list(rng.integers(1, 149, 40))
+    most = 148 * 4 * 1024
+    c = ops.Codec(2 * (most + 32768))
+    x = _values(most, "narrow", 9)
+    runs = []
+    for g in grids:
+        n = int(g) * 4 * 1024 - int(rng.integers(0, 4096))
+        ref = ops.cpu_compress(x[:n], EB)
+        runs.append((n, ref, _on_gpu(ref, 0)))
+    torch.cuda.synchronize()
+    got = []
+    for n, ref, s in runs:  # one launch right behind the other
+        got.append((c.decompress(s, n, EB, stream_bytes=ref.size), c.decompress_sum([s, s], n, EB, stream_bytes=[ref.size] * 2)))
+    for (n, ref, _), (one, two) in zip(runs, got):
+        want = ops.cpu_decompress(ref, n, EB)
+        np.testing.assert_array_equal(one.cpu().numpy(), want)
+        np.testing.assert_array_equal(two.cpu().numpy(), 2 * want)
+    assert c.status() == 0
