@@ -164,18 +164,18 @@ __device__ __forceinline__ void rows_of_block(uint32_t (&T)[32], uint32_t rate, 
   if (rate & 0x80u) T[7] = a0 & 0x7fffffffu;
 }
 
-// staged payload -> rows; W (plane_width of the largest F of the warp) is warp-uniform
+// staged payload -> rows; W (plane_width of the largest F of the warp) is warp-uniform.  The widths that data at the usual error
+// bounds has come first and in line, so that the loop's instructions lie together (as a switch, with the longest
+// variants in between: add of 64 MB 41.7 us, 40.3 this way; decode of 64 MB 22.4, 21.6)
 __device__ __forceinline__ void decode_rows(const uint8_t* buf, uint32_t pos, uint32_t rate, int W, uint32_t& sign,
                                             uint32_t& a0, uint32_t (&T)[32]) {
   const bool outl = __any_sync(0xffffffffu, rate & 0x80u);
-  switch (W) {
-    case 0: read_planes<0>(buf, pos, rate, outl, sign, a0, T); rows_of_block<0>(T, rate, a0); break;
-    case 4: read_planes<4>(buf, pos, rate, outl, sign, a0, T); rows_of_block<4>(T, rate, a0); break;
-    case 8: read_planes<8>(buf, pos, rate, outl, sign, a0, T); rows_of_block<8>(T, rate, a0); break;
-    case 12: read_planes<12>(buf, pos, rate, outl, sign, a0, T); rows_of_block<12>(T, rate, a0); break;
-    case 16: read_planes<16>(buf, pos, rate, outl, sign, a0, T); rows_of_block<16>(T, rate, a0); break;
-    default: read_planes<32>(buf, pos, rate, outl, sign, a0, T); rows_of_block<32>(T, rate, a0); break;
-  }
+  if (__builtin_expect(W == 12, 1)) { read_planes<12>(buf, pos, rate, outl, sign, a0, T); rows_of_block<12>(T, rate, a0); }
+  else if (__builtin_expect(W == 8, 1)) { read_planes<8>(buf, pos, rate, outl, sign, a0, T); rows_of_block<8>(T, rate, a0); }
+  else if (__builtin_expect(W == 16, 1)) { read_planes<16>(buf, pos, rate, outl, sign, a0, T); rows_of_block<16>(T, rate, a0); }
+  else if (W == 4) { read_planes<4>(buf, pos, rate, outl, sign, a0, T); rows_of_block<4>(T, rate, a0); }
+  else if (__builtin_expect(W == 0, 0)) { read_planes<0>(buf, pos, rate, outl, sign, a0, T); rows_of_block<0>(T, rate, a0); }
+  else { read_planes<32>(buf, pos, rate, outl, sign, a0, T); rows_of_block<32>(T, rate, a0); }
 }
 
 // 2^126 with the sign of element i: |d_i| * 2^-149 (the row as it stands, read as a float) times this is
@@ -307,14 +307,12 @@ __device__ __forceinline__ void pack_w(uint32_t base, uint32_t rel, const BlockC
 }
 // W: plane_width of the largest F of the warp
 __device__ __forceinline__ void pack_blocks(uint32_t base, uint32_t rel, const BlockCode& c, const uint32_t (&d)[32], int W) {
-  switch (W) {
-    case 0: pack_w<0>(base, rel, c, d); break;  // outlier blocks with F = 0 carry bytes
-    case 4: pack_w<4>(base, rel, c, d); break;
-    case 8: pack_w<8>(base, rel, c, d); break;
-    case 12: pack_w<12>(base, rel, c, d); break;
-    case 16: pack_w<16>(base, rel, c, d); break;
-    default: pack_w<32>(base, rel, c, d); break;
-  }
+  if (__builtin_expect(W == 12, 1)) pack_w<12>(base, rel, c, d);
+  else if (__builtin_expect(W == 8, 1)) pack_w<8>(base, rel, c, d);
+  else if (__builtin_expect(W == 16, 1)) pack_w<16>(base, rel, c, d);
+  else if (W == 4) pack_w<4>(base, rel, c, d);
+  else if (__builtin_expect(W == 0, 0)) pack_w<0>(base, rel, c, d);
+  else pack_w<32>(base, rel, c, d);
 }
 
 // 16-byte units of copy_ring: source bytes start K words and sh bits into 16-byte aligned shared memory.  Not unrolled: a

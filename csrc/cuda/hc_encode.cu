@@ -415,7 +415,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
         break;
       }
       if (tid == 0) HC_PH(1);
-      if (!by_tma(w)) {
+      if (__builtin_expect(!by_tma(w), 0)) {
         load_rows(stage, reinterpret_cast<const uint32_t*>(p.local[w.seg]), (uint64_t)w.sub * kSubValues, n_local(w.seg));
         __syncwarp();
       }
@@ -424,7 +424,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
         deltas_sub<MODE>(d, p.recip, p.one);
         // exact when no quantised value of the block reaches 2^24: |q_0| below 2^23 and 31 differences below 2^18
         or_tail = or_tail_of(d);
-        if (!__all_sync(0xffffffffu, or_tail < (1u << 18) && (d[0] & 0x7fffffffu) < (1u << 23))) {
+        if (__builtin_expect(!__all_sync(0xffffffffu, or_tail < (1u << 18) && (d[0] & 0x7fffffffu) < (1u << 23)), 0)) {
           cold_local<MODE, !kHasIn>(stage, (int)lane, p.recip);
           load_row_swizzled(stage, (int)lane, d);
           if (!kHasIn) or_tail = or_tail_of(d);
@@ -464,7 +464,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
         // |d_1| .. |d_31| small enough for sums of eight such streams: so with up to 16 planes, else to be looked at (a
         // plain block may have many planes for the sake of d_0 alone, which is summed in int32)
         bool fits = (cur_rate & 31u) <= 16u;
-        if (kFloat && !__all_sync(0xffffffffu, fits)) fits = fits || or_rows_tail(T) < (1u << 20);
+        if (kFloat && __builtin_expect(!__all_sync(0xffffffffu, fits), 0)) fits = fits || or_rows_tail(T) < (1u << 20);
         cur_rate = nxt_rate;
         cur_pos = nxt_pos;
         --staged;
@@ -474,7 +474,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
             const uint32_t m = (uint32_t)((int32_t)(sign << i) >> 31);
             d[i] += (T[i ^ 7] ^ m) - m;
           }
-        } else if (__all_sync(0xffffffffu, fits) && !ints) {
+        } else if (__builtin_expect(__all_sync(0xffffffffu, fits) && !ints, 1)) {
           const uint32_t m = (uint32_t)((int32_t)sign >> 31);
           d[0] += (T[7] ^ m) - m;
           d[1] = as_u(__fadd_rn(as_f(d[1]), as_f(signed_sub(T[6], sign, 1))));
@@ -499,7 +499,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       if (!kFloat) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
-      } else if (ints) {
+      } else if (__builtin_expect(ints, 0)) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
       } else {

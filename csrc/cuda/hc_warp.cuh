@@ -30,7 +30,7 @@ __device__ __forceinline__ void note_timeout(const Workspace& ws, uint32_t site)
 // bounded mbarrier wait of a whole warp; false: gave up (recorded)
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const Workspace& ws, uint32_t site) {
   const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, ws.spin_limit_ns));
-  if (!ok && (threadIdx.x & 31) == 0) note_timeout(ws, site);
+  if (__builtin_expect(!ok, 0) && (threadIdx.x & 31) == 0) note_timeout(ws, site);
   return ok;
 }
 
