@@ -26,8 +26,9 @@ namespace dev {
 constexpr int kSlots = 8;    // chunks of a CTA between "total known" and "payload copied out"
 constexpr int kInSlots = 4;  // chunks whose input offsets are known
 
-// Compute warps of a CTA at most.  Compress: 24 warps with the clerk, 80 registers each (256 MB: 62 us; when it was 63,
-// 68 with 20 warps at 96 registers, 73 with 16 at 128).  Adds: 16 warps, which is what the shared memory holds.
+// Compute warps of a CTA at most.  Compress: 24 warps with the clerk, 80 registers each (256 MB 51.4 us; 57.1 with 20 at 96
+// registers, 64.6 with 25 at 72, which spill).  Adds: 16 warps, which is what the shared memory holds (more would not help: 18 and
+// 20 with smaller rings took 47.6 and 44.5 us for 64 MB where 16 took 42.9).
 constexpr int kEncWarps = 23;
 __host__ __device__ constexpr int enc_warps(int op) { return op == kOpCompress ? kEncWarps : 15; }
 // packed payloads: a payload of 4096 bytes, 4 bytes pack_block adds, 16 copy_ring looks ahead
@@ -57,8 +58,9 @@ struct EncShared {
 struct Chunk {
   uint32_t seg, lc;
 };
+template <bool SEGS>
 __device__ __forceinline__ Chunk chunk_of(const SoloParams& p, uint32_t t) {
-  if (p.n_seg == 1u) return Chunk{0u, t};
+  if (!SEGS) return Chunk{0u, t};
   uint32_t g = 0;
 #pragma unroll 1
   while (g + 1 < p.n_seg && t >= p.first[g + 1]) ++g;
@@ -68,7 +70,7 @@ __device__ __forceinline__ Chunk chunk_of(const SoloParams& p, uint32_t t) {
 // unevenly to CTAs whose first warp ran ahead of the others: 21 to 26 of 23 chunks at 256 MB).  kNoTile: none left
 __device__ __forceinline__ uint32_t ticket(const SoloParams& p, uint32_t k) {
   const uint32_t t = k * gridDim.x + blockIdx.x;
-  return t < p.first[p.n_seg] ? t : kNoTile;
+  return t < p.chunks ? t : kNoTile;
 }
 
 // Running sum over the totals of consecutive chunks of a launch: brings `base` from chunk `next` to chunk t (one warp)
@@ -85,8 +87,8 @@ __device__ __forceinline__ void advance_base(const uint64_t* words, uint32_t& ne
 // polling does not take issue slots from the compute warps (100 ns to 20 us measure the same).  False: it ran out, or
 // another wait of the launch has (recorded).  A hardware barrier (bar.sync) will not do here: it has no time limit, and
 // a warp that gave up would have to go on arriving, in step with the others, for the clerk ever to come back.  It answers
-// 0.2 us sooner (compress of 4 KB back to back, on the device: 4.0 us, 4.2 this way); in longer launches this is
-// no slower (256 MB 63.3 us and 62.3, 64 MB add 47.7 and 47.3).
+// 0.2 us sooner (compress of 4 KB back to back, on the device, when this took its place: 4.0 us, 4.2 this way); in longer
+// launches this was no slower (256 MB 63.3 us and 62.3, 64 MB add 47.7 and 47.3).
 constexpr uint32_t kTotalsNap = 2000;
 __device__ __forceinline__ bool totals_wait(EncShared& sh, uint32_t k, const Workspace& ws) {
   uint64_t* const bar = &sh.totals[k % kSlots];
@@ -137,7 +139,7 @@ __device__ __forceinline__ void input_offsets(const SoloParams& p, EncShared& sh
 // Adds up the chunk totals, places the payloads; keeps the input offsets kInSlots chunks ahead of the compute warps and
 // the published input totals two chunks ahead of that (the first chunk's inputs are the compute warps' work).  Leaves when
 // a compute warp has given up; what that leaves unplaced runs out in the others' waits.
-__device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32_t nc, uint32_t subs, bool has_in) {
+__device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32_t nc, uint32_t subs, bool has_in, bool segs) {
   const uint32_t lane = threadIdx.x & 31u;
   const Workspace& ws = p.ws;
   // section A covers whole chunks of 32768 values: what is behind the blocks
@@ -171,7 +173,7 @@ __device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32
     const uint32_t tot = lane < nc ? sh.tot[r][lane] : 0u;
     const uint32_t inc = warp_inclusive_scan(tot, (int)lane);
     const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
-    const Chunk c = chunk_of(p, t);
+    const Chunk c = segs ? chunk_of<true>(p, t) : Chunk{0u, t};
     if (c.seg != seg) {  // every segment is a stream of its own
       seg = c.seg;
       base = 0;
@@ -225,7 +227,9 @@ static __device__ __noinline__ void load_rows(uint8_t* stage, const uint32_t* sr
 }
 
 // ---- the kernel --------------------------------------------------------------------------------------------------
-template <int OP, int MODE>
+// SEGS: several segments in the launch.  A kernel of its own: what finding the segment of a chunk takes in registers, a single array
+// had in spills (80 registers a thread; compress of 256 MB 54.4 us, 51.4 without)
+template <int OP, int MODE, bool SEGS>
 __global__ void __launch_bounds__((enc_warps(OP) + 1) * 32, 1)
 hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ SoloParams p) {
   constexpr bool kHasLocal = OP != kOpAddStream;
@@ -265,7 +269,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   if (sh.dead) return;  // (one answer for all warps)
   const uint32_t subs0 = p.subs[0];
   if (warp == nc) {
-    clerk(p, sh, nc, subs0, kHasIn);
+    clerk(p, sh, nc, subs0, kHasIn, SEGS);
     return;
   }
 
@@ -279,7 +283,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   };
   auto where = [&](uint32_t t) -> Where {
     if (kHasIn) return Where{0u, t * nc + warp};
-    const Chunk c = chunk_of(p, t);
+    const Chunk c = chunk_of<SEGS>(p, t);
     return Where{c.seg, c.lc * nc + warp};
   };
   auto n_local = [&](uint32_t g) -> uint64_t { return OP == kOpAddI32 ? num_blocks(p.n[g]) * kBlock : p.n[g]; };
@@ -379,7 +383,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     const uint32_t start = __shfl_sync(0xffffffffu, my_start, (int)r), tot = __shfl_sync(0xffffffffu, my_tot, (int)r);
     const uint64_t at = sh.out_at[r][warp];
     if (tot) {
-      if (at != ~0ull) copy_ring(oring + start, (p.n_seg == 1u ? p.out[0] : p.out[__shfl_sync(0xffffffffu, my_seg, (int)r)]) + at, tot);
+      if (at != ~0ull) copy_ring(oring + start, (SEGS ? p.out[__shfl_sync(0xffffffffu, my_seg, (int)r)] : p.out[0]) + at, tot);
       tail = start + room_for(tot);
       if (--taken == 0) head = tail = 0;
     }
@@ -601,30 +605,31 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
 
 namespace {
 
-template <int OP, int MODE>
+template <int OP, int MODE, bool SEGS>
 cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t stream) {
   constexpr int kWarps = dev::enc_warps(OP);
   auto smem = [](int nc) { return nc * dev::enc_warp_bytes(OP) + 1024; };
   static thread_local int cache[64] = {};
-  const int cap = resident_ctas(dev::hc_encode_solo_kernel<OP, MODE>, 32 * (kWarps + 1), smem(kWarps), cache);
+  const int cap = resident_ctas(dev::hc_encode_solo_kernel<OP, MODE, SEGS>, 32 * (kWarps + 1), smem(kWarps), cache);
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
   const EncodeSplit split = split_encode(p.subs, p.n_seg, (uint32_t)(cap < kMaxCtas ? cap : kMaxCtas), (uint32_t)kWarps);
   if (encode_words(split, p.n_seg, p.n_in) > p.ws.words) return cudaErrorInvalidValue;
   const int nc = (int)split.warps;
   memcpy(p.first, split.first, sizeof(p.first));
+  p.chunks = p.first[p.n_seg];
   p.one_round = split.one_round;
   p.one = 1.0f;
   p.out_words = p.ws.st_a;
   p.in_words = p.ws.st_a + p.first[p.n_seg];
-  return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE>, (int)split.grid, 32 * (nc + 1), smem(nc), stream, maps, p);
+  return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE, SEGS>, (int)split.grid, 32 * (nc + 1), smem(nc), stream, maps, p);
 }
 
-template <int OP>
+template <int OP, bool SEGS = false>
 cudaError_t launch_solo_m(int mode, const TensorMaps& maps, const SoloParams& p, cudaStream_t stream) {
   switch (mode) {
-    case kModeOutlier: return launch_solo_t<OP, kModeOutlier>(maps, p, stream);
-    case kModePlain: return launch_solo_t<OP, kModePlain>(maps, p, stream);
-    case kModeVec: return launch_solo_t<OP, kModeVec>(maps, p, stream);
+    case kModeOutlier: return launch_solo_t<OP, kModeOutlier, SEGS>(maps, p, stream);
+    case kModePlain: return launch_solo_t<OP, kModePlain, SEGS>(maps, p, stream);
+    case kModeVec: return launch_solo_t<OP, kModeVec, SEGS>(maps, p, stream);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -648,7 +653,8 @@ cudaError_t launch_encode_solo(int op, int mode, SoloParams p, cudaStream_t stre
   }
   if (total == 0) return cudaSuccess;
   switch (op) {
-    case kOpCompress: return launch_solo_m<kOpCompress>(mode, maps, p, stream);
+    case kOpCompress:
+      return p.n_seg > 1 ? launch_solo_m<kOpCompress, true>(mode, maps, p, stream) : launch_solo_m<kOpCompress>(mode, maps, p, stream);
     case kOpAddF32: return launch_solo_m<kOpAddF32>(mode, maps, p, stream);
     case kOpAddI32: return launch_solo_m<kOpAddI32>(mode, maps, p, stream);
     case kOpAddStream: return launch_solo_m<kOpAddStream>(mode, maps, p, stream);

@@ -108,6 +108,7 @@ struct SoloParams {
   uint32_t subs[kMaxDst];    // sub-tiles of 1024 values, the last one perhaps ragged (this and the next two: set by the launcher)
   uint32_t by_tma[kMaxDst];  // those of them that the TMA unit can load: whole ones of an aligned operand
   uint32_t first[kMaxDst + 1];  // chunk numbers at which the segments start; [n_seg]: number of chunks
+  uint32_t chunks;
   uint32_t n_seg;
   uint32_t n_in;
   float recip;  // 0.5f / eb
