@@ -229,7 +229,9 @@ static __device__ __noinline__ void load_rows(uint8_t* stage, const uint32_t* sr
 // ---- the kernel --------------------------------------------------------------------------------------------------
 // SEGS: several segments in the launch.  A kernel of its own: what finding the segment of a chunk takes in registers, a single array
 // had in spills (80 registers a thread; compress of 256 MB 54.4 us, 51.4 without)
-template <int OP, int MODE, bool SEGS>
+// ONE: one input stream.  Its kernel has no loop over streams (add of 64 MB 40.3 us, 38.8 this way; for the two of
+// stream + stream a constant number gained nothing)
+template <int OP, int MODE, bool SEGS, bool ONE>
 __global__ void __launch_bounds__((enc_warps(OP) + 1) * 32, 1)
 hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ SoloParams p) {
   constexpr bool kHasLocal = OP != kOpAddStream;
@@ -242,7 +244,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const Workspace& ws = p.ws;
   HC_TL_DECL(ws.epoch);
-  const uint32_t Q = kHasIn ? p.n_in : 0u;
+  const uint32_t Q = !kHasIn ? 0u : ONE ? 1u : p.n_in;
 
   if (tid < nc) {
     mbar_init(&sh.stage_full[tid], 1);
@@ -605,12 +607,12 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
 
 namespace {
 
-template <int OP, int MODE, bool SEGS>
+template <int OP, int MODE, bool SEGS, bool ONE>
 cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t stream) {
   constexpr int kWarps = dev::enc_warps(OP);
   auto smem = [](int nc) { return nc * dev::enc_warp_bytes(OP) + 1024; };
   static thread_local int cache[64] = {};
-  const int cap = resident_ctas(dev::hc_encode_solo_kernel<OP, MODE, SEGS>, 32 * (kWarps + 1), smem(kWarps), cache);
+  const int cap = resident_ctas(dev::hc_encode_solo_kernel<OP, MODE, SEGS, ONE>, 32 * (kWarps + 1), smem(kWarps), cache);
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
   const EncodeSplit split = split_encode(p.subs, p.n_seg, (uint32_t)(cap < kMaxCtas ? cap : kMaxCtas), (uint32_t)kWarps);
   if (encode_words(split, p.n_seg, p.n_in) > p.ws.words) return cudaErrorInvalidValue;
@@ -621,15 +623,15 @@ cudaError_t launch_solo_t(const TensorMaps& maps, SoloParams p, cudaStream_t str
   p.one = 1.0f;
   p.out_words = p.ws.st_a;
   p.in_words = p.ws.st_a + p.first[p.n_seg];
-  return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE, SEGS>, (int)split.grid, 32 * (nc + 1), smem(nc), stream, maps, p);
+  return launch_overlapped(dev::hc_encode_solo_kernel<OP, MODE, SEGS, ONE>, (int)split.grid, 32 * (nc + 1), smem(nc), stream, maps, p);
 }
 
-template <int OP, bool SEGS = false>
+template <int OP, bool SEGS = false, bool ONE = false>
 cudaError_t launch_solo_m(int mode, const TensorMaps& maps, const SoloParams& p, cudaStream_t stream) {
   switch (mode) {
-    case kModeOutlier: return launch_solo_t<OP, kModeOutlier, SEGS>(maps, p, stream);
-    case kModePlain: return launch_solo_t<OP, kModePlain, SEGS>(maps, p, stream);
-    case kModeVec: return launch_solo_t<OP, kModeVec, SEGS>(maps, p, stream);
+    case kModeOutlier: return launch_solo_t<OP, kModeOutlier, SEGS, ONE>(maps, p, stream);
+    case kModePlain: return launch_solo_t<OP, kModePlain, SEGS, ONE>(maps, p, stream);
+    case kModeVec: return launch_solo_t<OP, kModeVec, SEGS, ONE>(maps, p, stream);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -655,8 +657,9 @@ cudaError_t launch_encode_solo(int op, int mode, SoloParams p, cudaStream_t stre
   switch (op) {
     case kOpCompress:
       return p.n_seg > 1 ? launch_solo_m<kOpCompress, true>(mode, maps, p, stream) : launch_solo_m<kOpCompress>(mode, maps, p, stream);
-    case kOpAddF32: return launch_solo_m<kOpAddF32>(mode, maps, p, stream);
-    case kOpAddI32: return launch_solo_m<kOpAddI32>(mode, maps, p, stream);
+    case kOpAddF32:
+      return p.n_in == 1 ? launch_solo_m<kOpAddF32, false, true>(mode, maps, p, stream) : launch_solo_m<kOpAddF32>(mode, maps, p, stream);
+    case kOpAddI32: return p.n_in == 1 ? launch_solo_m<kOpAddI32, false, true>(mode, maps, p, stream) : cudaErrorInvalidValue;
     case kOpAddStream: return launch_solo_m<kOpAddStream>(mode, maps, p, stream);
     default: return cudaErrorInvalidValue;
   }
