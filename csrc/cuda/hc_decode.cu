@@ -607,7 +607,8 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
       if (lane == 0) {
         uint64_t* const bar = &full[issued & 3u];
         uint8_t* const dst = ring + (issued & 3u) * kPiece;
-        const uint32_t again = issued & 3u ? 0u : bytes < kMirror ? bytes : kMirror;
+        // (nothing lies in front of the very first piece that could read on into it)
+        const uint32_t again = (issued & 3u) || !issued ? 0u : bytes < kMirror ? bytes : kMirror;
         mbar_expect_tx(bar, bytes + again);
         bulk_load(dst, f_src, bytes, bar);
         if (again) bulk_load(ring + kRing, f_src, again, bar);
