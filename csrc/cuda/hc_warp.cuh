@@ -163,10 +163,11 @@ __device__ __forceinline__ uint64_t take_total(uint64_t* sums, const Workspace& 
 // each later group, at most one reduction a lane where the direct form has up to 147 words to add to, whose 10900 reductions a
 // launch queue up (148 CTAs: the last one had given 1.5 us after it knew its total, 0.4 us this way; decode of 8 MB 7.2 us and
 // 6.4, sum of four 4 MB streams 13.4 and 12.7).  In a launch of few CTAs, and in the one-round launches of the encode kernel, it
-// is no faster and its longer code costs 0.2 to 0.4 us (seven streams of 8 MB added 18.7 us, 19.5 this way).
+// is no faster and its longer code costs 0.2 to 0.4 us (seven streams of 8 MB added 18.7 us, 19.5 this way; sum of two streams
+// in 56 CTAs 6.7 us, 7.3 this way; in 123 CTAs 9.2 and 7.9).
 // The word of a group has several readers and is never reset: what counts is by how much it has grown since the launch
 // before, whose end every CTA notes for itself (the last one of a launch also for those of its group that the launch does not have).
-constexpr uint32_t kDirect = 33;
+constexpr uint32_t kDirect = 64;
 __device__ __forceinline__ void give_total_grouped(uint64_t* sums, uint64_t total) {
   const uint32_t lane = threadIdx.x & 31u, g = blockIdx.x / kSumGroup;
   const uint32_t cta = blockIdx.x + 1u + lane, group = lane - 16u;

@@ -87,7 +87,7 @@ def test_sums_by_length_of_the_runs(k):
 def test_launches_of_all_grids_behind_one_another():
     """A launch leaves words of the exchange as they are; the next one, with more CTAs or fewer, starts from there."""
     rng = np.random.default_rng(3)
-    grids = [148, 1, 34, 33, 147, 14, 35, 148, 39, 40, 52, 53, 146, 2] + list(rng.integers(1, 149, 40))
+    grids = [148, 1, 65, 64, 147, 14, 66, 148, 78, 79, 91, 92, 146, 2] + list(rng.integers(1, 149, 40))
     most = 148 * 4 * 1024
     c = ops.Codec(2 * (most + 32768))
     x = _values(most, "narrow", 9)
