@@ -139,14 +139,25 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
         s_tot[warp][q1] = s0 >> 16;
       }
     } else {
+      // Longer runs: 16 sub-tiles of four streams are asked for before the first is added (one stream after the other: eight of
+      // 40 MB 96.0 us, 92.6 this way; four of 256 MB 240.9 and 237.1; two of 128 MB 70.4 and 70.0)
 #pragma unroll 1
-      for (uint32_t qq = 0; qq < Q; ++qq) {
-        uint32_t sum = 0;
+      for (uint32_t q4 = 0; q4 < Q; q4 += 4u) {
+        uint32_t sum[4] = {0, 0, 0, 0};
 #pragma unroll 1
-        for (uint32_t l = lane; it * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u)
-          sum += payload_len16(rates16(p.seg[qq].in, p.seg[qq].in_size, it, run_end, l));
-        sum = __reduce_add_sync(0xffffffffu, sum);
-        if (lane == 0) s_tot[warp][qq] = sum;
+        for (uint32_t l = lane; it * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u) {
+          uint4 v[4];
+#pragma unroll
+          for (uint32_t u = 0; u < 4u; ++u)
+            v[u] = q4 + u < Q ? rates16(p.seg[q4 + u].in, p.seg[q4 + u].in_size, it, run_end, l) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+          for (uint32_t u = 0; u < 4u; ++u) sum[u] += payload_len16(v[u]);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u) {
+          sum[u] = __reduce_add_sync(0xffffffffu, sum[u]);
+          if (lane == 0) s_tot[warp][q4 + u] = sum[u];  // (room for kMaxDst streams, a multiple of four)
+        }
       }
     }
   }

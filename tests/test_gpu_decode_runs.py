@@ -84,6 +84,23 @@ def test_sums_by_length_of_the_runs(k):
     assert c.status() == 0
 
 
+@pytest.mark.parametrize("k,subs", [(3, 17), (5, 5), (5, 33), (8, 18)])
+def test_sums_over_long_runs(k, subs):
+    """Rate bytes are added up 16 sub-tiles of four streams at a time; every stream has payloads of its own lengths."""
+    n = 148 * 16 * 1024 * subs + 1025  # some warps have a sub-tile more
+    g = torch.Generator("cuda").manual_seed(k)
+    c = ops.Codec(k * ((n + 32767) // 32768 * 32768))
+    want, streams, sizes = torch.zeros(n, device="cuda"), [], []
+    for i in range(k):
+        x = torch.randint(-(3 << i), 3 << i, (n,), device="cuda", generator=g).float()
+        want += x
+        s, size = c.compress(x, EB)
+        streams.append(s)
+        sizes.append(int(size))
+    assert torch.equal(c.decompress_sum(streams, n, EB, stream_bytes=sizes), want)
+    assert c.status() == 0
+
+
 def test_launches_of_all_grids_behind_one_another():
     """A launch leaves words of the exchange as they are; the next one, with more CTAs or fewer, starts from there."""
     rng = np.random.default_rng(3)

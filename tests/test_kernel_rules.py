@@ -30,6 +30,13 @@ def test_block_wide_barriers_of_encode_stand_before_the_roles_part():
     assert "__syncthreads" not in kernel.split("clerk(p, sh", 1)[1]
 
 
+def test_sums_ask_for_rate_bytes_of_several_streams_at_once():
+    """Nothing stands between the loads of one stream and those of the next: added up where it is asked for, every further
+    stream is one more trip to memory before the first payload."""
+    kernel = _code("hc_decode.cu").split("hc_decode_kernel(", 1)[1].split("__global__", 1)[0]
+    assert kernel.count("rates16(p.seg[") == 3 and not re.search(r"payload_len16\(\s*rates16\(", kernel)
+
+
 def test_compute_warps_of_the_collective_kernel_leave_together():
     """They meet at hardware barriers, so a wait that ran out in one of them is no reason to go before all know: lanes
     agree within the warp, the warp tells the others at a barrier that it comes to itself."""
