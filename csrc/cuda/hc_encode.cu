@@ -227,8 +227,9 @@ static __device__ __noinline__ void load_rows(uint8_t* stage, const uint32_t* sr
 }
 
 // ---- the kernel --------------------------------------------------------------------------------------------------
-// SEGS: several segments in the launch.  A kernel of its own: what finding the segment of a chunk takes in registers, a single array
-// had in spills (80 registers a thread; compress of 256 MB 54.4 us, 51.4 without)
+// SEGS: several segments in the launch.  A kernel of its own, because a thread has 80 registers and a single array does not pay for
+// those that finding the segment of a chunk takes (one kernel for both, as it then was, had spills: compress of 256 MB 54.4 us with
+// two arrays in turn, 51.4 with one of its own)
 // ONE: one input stream.  Its kernel has no loop over streams (add of 64 MB 40.3 us, 38.8 this way; for the two of
 // stream + stream a constant number gained nothing)
 template <int OP, int MODE, bool SEGS, bool ONE>
@@ -374,18 +375,24 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     }
   }
 
-  // ---- packed payloads waiting for their place: lane k % kSlots keeps those of chunk k --------------------------------
-  uint32_t my_start = 0, my_tot = 0, my_seg = 0;
+  // ---- packed payloads waiting for their place: lane k % kSlots keeps that of chunk k ----------------------------------
+  // SEGS: segment [31:26], length [25:13] and start [12:0] in one register.  In three it had spills (16 bytes stored, 36 loaded;
+  // two arrays of 64 MB 38.2 us, 36.1 this way, gradients of a block of width 1024 18.1 and 17.6).  The other kernels have none to
+  // lose and are slower for the unpacking (compress of 16 MB 7.04 us, 7.22 this way; add of int32 deltas of 128 MB, whose 12 bytes
+  // of spills it would take away, 70.7 and 71.6)
+  uint32_t my_start = 0, my_tot = 0;
+  static_assert(kOutBytes <= 1u << 13 && kSubBlocks * 128 < 1 << 13 && kMaxDst <= 64, "fields of my_start");
   // ring: free is [head, end) and [0, tail), or, once wrapped (head < tail), [head, tail); all of it when taken == 0
   uint32_t head = 0, tail = 0, taken = 0;
   uint32_t copied = 0;  // chunks [copied, k) wait
   auto room_for = [&](uint32_t tot) -> uint32_t { return tot ? (tot + 20u + 15u) & ~15u : 0u; };
   auto copy_oldest = [&]() {
     const uint32_t r = copied % kSlots;
-    const uint32_t start = __shfl_sync(0xffffffffu, my_start, (int)r), tot = __shfl_sync(0xffffffffu, my_tot, (int)r);
+    const uint32_t mine = __shfl_sync(0xffffffffu, my_start, (int)r), start = SEGS ? mine & 0x1fffu : mine;
+    const uint32_t tot = SEGS ? mine >> 13 & 0x1fffu : __shfl_sync(0xffffffffu, my_tot, (int)r);
     const uint64_t at = sh.out_at[r][warp];
     if (tot) {
-      if (at != ~0ull) copy_ring(oring + start, (SEGS ? p.out[__shfl_sync(0xffffffffu, my_seg, (int)r)] : p.out[0]) + at, tot);
+      if (at != ~0ull) copy_ring(oring + start, p.out[SEGS ? mine >> 26 : 0u] + at, tot);
       tail = start + room_for(tot);
       if (--taken == 0) head = tail = 0;
     }
@@ -580,9 +587,8 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     __syncwarp();
     pack_blocks(oring + start, inc - code.len, code, d, plane_width(__reduce_max_sync(0xffffffffu, code.rate & 31u)));
     if (lane == k % kSlots) {
-      my_start = start;
-      my_tot = tot;
-      my_seg = w.seg;
+      my_start = SEGS ? start | tot << 13 | w.seg << 26 : start;
+      if (!SEGS) my_tot = tot;
     }
     if (need) {
       head = start + need;

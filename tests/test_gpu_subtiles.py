@@ -84,6 +84,22 @@ def test_batch_of_very_different_sizes_in_a_codec_for_their_sum():
     assert c.status() == 0
 
 
+@pytest.mark.parametrize("mode", ["outlier", "plain", "vec"])
+def test_batch_of_several_rounds(mode):
+    """Payloads that wait for their place belong to any of eight arrays; some are as long as a payload gets."""
+    rng = np.random.default_rng(8)
+    xs = [_data(1_200_000 + 777 * i, i) for i in range(8)]
+    for i in (3, 7):  # 31 planes in every block
+        xs[i] = rng.integers(-2 ** 29, 2 ** 29, xs[i].size).astype(np.float32) * np.float32(2 * EB)
+    c = ops.Codec(sum((x.size + 32767) // 32768 * 32768 for x in xs))
+    outs, sizes = c.compress_batch([_gpu(x) for x in xs], EB, mode)
+    for out, size, x in zip(outs, sizes.tolist(), xs):
+        want = ops.cpu_compress(x, EB, mode)
+        assert size == want.size
+        np.testing.assert_array_equal(out[:size].cpu().numpy(), want)
+    assert c.status() == 0
+
+
 @pytest.mark.parametrize("n,shift", [(1023, 0), (4099, 1), (70_001, 3)])
 def test_chain_through_one_ragged_operand(n, shift):
     """Every call reads what the call before it has just written into the same buffer, past the TMA unit (ragged, or

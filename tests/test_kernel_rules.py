@@ -8,9 +8,12 @@ out: ``test_gpu_failure.py``.
 A kernel that starts while the one before it is still at work does not read what that one writes by non-coherent
 loads, which are for memory that nobody writes while the kernel runs."""
 import re
+import subprocess
 from pathlib import Path
 
 import pytest
+
+from tirocinio_triennale_b200 import _build
 
 CUDA = Path(__file__).resolve().parent.parent / "csrc" / "cuda"
 
@@ -67,3 +70,19 @@ def test_a_warp_that_gives_up_waits_for_its_copies(name):
     kernel = _code(name).split("__global__", 1)[1].split("\n}\n", 1)[0]
     after_the_loop = kernel.rsplit("HC_PH_COUNT();", 1)[1]
     assert re.search(r"for \(;[^;]*< jobs; [^)]*\)\s*mbar_wait_bounded\(", after_the_loop)
+
+
+@pytest.mark.skipif(_build.nvcc_path() is None, reason="needs nvcc")
+@pytest.mark.parametrize("name", ["hc_encode.cu", "hc_decode.cu"])
+def test_no_spills(name, tmp_path):
+    """As the assembler reports them.  The add of int32 deltas (operation 2) is left out: it keeps 12 bytes there and is
+    slower in the form that needs none."""
+    flags = [f for f in _build.NVCC_FLAGS if f != "-lineinfo"]
+    out = subprocess.run([_build.nvcc_path(), *flags, "-Xptxas", "-v", "-I", str(CUDA.parent / "include"), "-cubin",
+                          str(CUDA / name), "-o", str(tmp_path / "cubin")], capture_output=True, text=True, check=True).stderr
+    entries = [e for e in out.split("Compiling entry function ")[1:] if "hc_encode_solo_kernelILi2E" not in e]
+    assert len(entries) >= 6
+    for e in entries:
+        name = e.split("'")[1]
+        assert re.findall(r"(\d+) bytes spill stores, (\d+) bytes spill loads", e.split("Function properties for " + name)[1])[0] == (
+            "0", "0"), name
