@@ -58,17 +58,22 @@ def test_corrupted_rate_bytes_are_contained():
     assert codec.status() == 0
 
 
-@pytest.mark.parametrize("op", ["compress", "hom_add"])
+@pytest.mark.parametrize("op", ["compress", "hom_add", "decompress", "decompress_sum"])
 def test_grid_that_is_not_resident_as_a_whole_gives_up(op):
     """Another kernel keeps half of the SMs for longer than the waits may take, so half of the CTAs of a launch with ten
     chunks and more a CTA never publish a total: the others' waits run out in every role, the launch ends with
-    status 3, and the handle works again once that has been read."""
+    status 3, and the handle works again once that has been read.  The exchange of totals of a decode is left half done by
+    that, with words that no launch resets; launches before the status has been read end without touching the output."""
     n, eb, held = 30_000_000, 1e-4, 74
     x = torch.randn(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)) * 0.01
     codec = ops.Codec(2 * n)
 
-    def call():
-        return codec.compress(x, eb) if op == "compress" else codec.hom_add(s, x, eb, stream_bytes=s_bytes)
+    def call(out=None):
+        if op == "decompress":
+            return codec.decompress(s, n, eb, out=out, stream_bytes=s_bytes), n
+        if op == "decompress_sum":
+            return codec.decompress_sum([s, s], n, eb, out=out, stream_bytes=[s_bytes] * 2), n
+        return codec.compress(x, eb, out=out) if op == "compress" else codec.hom_add(s, x, eb, out=out, stream_bytes=s_bytes)
 
     s, size = codec.compress(x, eb)
     s_bytes = int(size)
@@ -86,8 +91,12 @@ def test_grid_that_is_not_resident_as_a_whole_gives_up(op):
     codec.set_timeout_ms(20)
     t0 = time.time()
     call()
+    again = torch.full_like(want, 7)
+    if op in ("decompress", "decompress_sum"):
+        call(again)
     assert codec.status() == 3
     assert time.time() - t0 < 5
+    assert bool((again == 7).all())
     assert holder.status() == 6
     codec.set_timeout_ms(2000)
     got, size = call()
