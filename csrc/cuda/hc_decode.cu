@@ -10,9 +10,10 @@
 // look-back, no second kernel.  The SMs do not run at the same pace (with equal static shares the first warp of a 256 MB launch
 // finished at 42 us, the last at 70), so the last eighth of every run goes to whoever is free first; the payload
 // offsets of those sub-tiles are written to the workspace after the first one has been decoded.
-// What bounds them: arrays of 64 MB and more the memory (256 MB: 62 us; 63 with the arithmetic left out, and 34 without the
-// stores), smaller ones the way to the first payload: rate bytes, exchange, payload, one trip to L2 after the other (8 MB: of 6.1 us
-// on the device 3.3; 5.1 of 7.5 when 64-bit divisions, the status and the offsets of the pool stood in between).
+// What bounds the decode of one stream: 256 MB the memory (62.1 us; 61.9 with the arithmetic left out, 50.4 without the stores), 64 MB
+// the memory and the start (22.8; 20.8, 19.0), smaller ones the way to the first payload: rate bytes, exchange, payload, one trip to
+// L2 after the other (8 MB: of 6.1 us on the device 3.3; 5.1 of 7.5 when 64-bit divisions, the status and the offsets of the pool
+// stood in between).  Sums take their streams one after the other in every warp (four streams of 256 MB 237 us).
 //
 // Steps of a collective (!RUNS): the producer raises one flag word per tile, carrying the tile's payload offset.
 // Tickets are dealt in the order in which the flags rise, round the segments: a tile (all four quarters by one

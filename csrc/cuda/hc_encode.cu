@@ -26,8 +26,8 @@ namespace dev {
 constexpr int kSlots = 8;    // chunks of a CTA between "total known" and "payload copied out"
 constexpr int kInSlots = 4;  // chunks whose input offsets are known
 
-// Compute warps of a CTA at most.  Compress: 24 warps with the clerk, 80 registers each (256 MB 51.4 us; 57.1 with 20 at 96
-// registers, 64.6 with 25 at 72, which spill).  Adds: 16 warps, which is what the shared memory holds (more would not help: 18 and
+// Compute warps of a CTA at most.  Compress: 24 warps with the clerk, 80 registers each (256 MB, two arrays in turn, 51.4 us; 57.1
+// with 20 at 96 registers, 64.6 with 25 at 72, which spill; one array again and again takes 54 to 58).  Adds: 16 warps, which is what the shared memory holds (more would not help: 18 and
 // 20 with smaller rings took 47.6 and 44.5 us for 64 MB where 16 took 42.9).
 constexpr int kEncWarps = 23;
 __host__ __device__ constexpr int enc_warps(int op) { return op == kOpCompress ? kEncWarps : 15; }
