@@ -187,12 +187,16 @@ __device__ __forceinline__ uint32_t st_state(uint64_t w, uint32_t epoch) {
 __device__ __forceinline__ uint64_t st_value(uint64_t w) { return w & ((1ull << 40) - 1); }
 
 // ---- warp / block scans ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, int lane) {
+// (the shuffle itself says whether there is a lane to add)
+__device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, int) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += t;
-  }
+  for (int o = 1; o < 32; o <<= 1)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .u32 t;\n\t"
+        "shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n\t"
+        "@p add.u32 %0, %0, t;\n\t}"
+        : "+r"(v)
+        : "r"(o));
   return v;
 }
 

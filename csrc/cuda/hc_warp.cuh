@@ -27,11 +27,24 @@ __device__ __forceinline__ void note_timeout(const Workspace& ws, uint32_t site)
   if (!fatal_error(ws.ctrl)) atomicCAS(ws.ctrl + 3, 0u, site);
   note_error(ws.ctrl, kErrTimeout);
 }
-// bounded mbarrier wait of a whole warp; false: gave up (recorded)
+// Bounded mbarrier wait of a whole warp; false: gave up (recorded).  The lanes try together and vote, so that the loop is the same
+// for all of them: as a loop per lane every wait carried the code for lanes that leave it apart (a sub-tile of an add 1237 warp
+// instructions, 1206 this way; compress of 4 KB 3.45 us and 3.38, decode of 64 MB 22.8 and 22.4).
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const Workspace& ws, uint32_t site) {
-  const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, ws.spin_limit_ns));
-  if (__builtin_expect(!ok, 0) && (threadIdx.x & 31) == 0) note_timeout(ws, site);
-  return ok;
+  if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
+  long long t0 = 0;
+#pragma unroll 1
+  for (uint32_t it = 0; !__all_sync(0xffffffffu, mbar_try_wait(bar, parity)); ++it) {
+    if ((it & 63u) == 0u) {
+      const long long now = clock64();
+      if (it == 0u) t0 = now;
+      else if (__any_sync(0xffffffffu, now - t0 > (long long)ws.spin_limit_ns * 2) || it >= (1u << 26)) {
+        if ((threadIdx.x & 31) == 0) note_timeout(ws, site);
+        return false;
+      }
+    }
+  }
+  return true;
 }
 
 // collective steps: one non-blocking look at the tile's arrival flag; 0 = not raised yet
