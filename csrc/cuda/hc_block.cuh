@@ -121,7 +121,7 @@ __device__ __forceinline__ uint32_t payload_len4(uint32_t r4) {
 
 // ---- stream -> block --------------------------------------------------------------------------------
 // Reads the payload of the block with rate byte `rate` at byte `pos` of a staged stream: planes into T[0..W-1]
-// (zero at and above F), the sign map with element i at bit 31 - i, |d0| of an outlier block (else 0).  Every
+// (zero at and above F), the sign map in the planes' bit order, |d0| of an outlier block (else 0).  Every
 // word is rebuilt from two neighbours by a funnel shift, whatever the block's alignment: with outlier blocks
 // about, the lanes of a warp have all four alignments, and a second path for aligned blocks ran on top.
 // Blocks without payload give zeros; up to 4 W + 8 bytes behind the payload are read (and ignored).
@@ -144,13 +144,18 @@ __device__ __forceinline__ void read_planes(const uint8_t* buf, uint32_t pos, ui
   uint32_t word[W + 2];
 #pragma unroll
   for (int j = 0; j < W + 2; ++j) word[j] = lds32(wp + 4 * j);
-  sign = __byte_perm(__funnelshift_r(word[0], word[1], sh), 0, 0x0123);
+  sign = __funnelshift_r(word[0], word[1], sh);
 #pragma unroll
   for (int j = 1; j <= W; ++j) {
     const uint32_t x = __funnelshift_r(word[j], word[j + 1], sh);
     T[j - 1] = (uint32_t)j <= F ? x : 0u;
   }
 }
+
+// sign map in the order of the stream's words <-> element i at bit 31 - i
+__device__ __forceinline__ uint32_t swap_order(uint32_t sign) { return __byte_perm(sign, 0, 0x0123); }
+// element 0 of a block in the order of the stream's words
+constexpr uint32_t kFirst = 0x80u;
 
 // planes -> rows: on return T[i ^ 7] = |d_i|
 template <int W>
@@ -164,7 +169,7 @@ __device__ __forceinline__ void rows_of_block(uint32_t (&T)[32], uint32_t rate, 
   if (rate & 0x80u) T[7] = a0 & 0x7fffffffu;
 }
 
-// staged payload -> rows; W (plane_width of the largest F of the warp) is warp-uniform.  The widths that data at the usual error
+// staged payload -> rows, sign map with element i at bit 31 - i; W (plane_width of the largest F of the warp) is warp-uniform.  The widths that data at the usual error
 // bounds has come first and in line, so that the loop's instructions lie together (as a switch, with the longest
 // variants in between: add of 64 MB 41.7 us, 40.3 this way; decode of 64 MB 22.4, 21.6)
 __device__ __forceinline__ void decode_rows(const uint8_t* buf, uint32_t pos, uint32_t rate, int W, uint32_t& sign,
@@ -176,6 +181,7 @@ __device__ __forceinline__ void decode_rows(const uint8_t* buf, uint32_t pos, ui
   else if (W == 4) { read_planes<4>(buf, pos, rate, outl, sign, a0, T); rows_of_block<4>(T, rate, a0); }
   else if (__builtin_expect(W == 0, 0)) { read_planes<0>(buf, pos, rate, outl, sign, a0, T); rows_of_block<0>(T, rate, a0); }
   else { read_planes<32>(buf, pos, rate, outl, sign, a0, T); rows_of_block<32>(T, rate, a0); }
+  sign = swap_order(sign);
 }
 
 // 2^126 with the sign of element i: |d_i| * 2^-149 (the row as it stands, read as a float) times this is
@@ -194,7 +200,7 @@ struct BlockCode {
   uint32_t len;   // payload bytes
   uint32_t nout;  // outlier bytes (0: plain layout)
   uint32_t a0;    // |d_0|
-  uint32_t sign;  // sign map, element i at bit 31 - i
+  uint32_t sign;  // sign map in the order of the stream's words
 };
 
 // values (float bits) -> deltas of the quantised values as subnormals, in place
@@ -238,19 +244,21 @@ __device__ __forceinline__ uint32_t or_rows_tail(const uint32_t (&T)[32]) {
   for (int i = 1; i < 32; ++i) o |= T[i ^ 7];
   return o;
 }
-// sign-magnitude deltas -> the block's code; d_0 of an outlier block is taken out of the planes.
+// sign bits of the rows -> sign map in the order of the stream's words
+__device__ __forceinline__ uint32_t signs_of(const uint32_t (&d)[32]) {
+  uint32_t s = 0;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) s = __funnelshift_l(d[i], s, 1);
+  return swap_order(s);
+}
+// rate byte and length of a block with |d_0| = c.a0 and magnitudes of f bits behind it:
 // choose_rate() and payload_len() in fewer operations.  With f and w the bit widths of or_tail and |d_0| and o the
 // bytes that w bits take, the plain layout has 4 + 4 max(f, w) bytes (none if that maximum is 0), the outlier layout
 // 4 + 4 f + o, and the smaller one is taken, plain if equal.  For w <= f that is plain; for w > f it is the outlier layout if
 // 4 w > 4 f + o, which w <= f never meets.
 template <int MODE>
-__device__ __forceinline__ BlockCode code_of(uint32_t (&d)[32], uint32_t or_tail) {
-  BlockCode c;
-  c.sign = 0;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) c.sign = __funnelshift_l(d[i], c.sign, 1);
-  c.a0 = d[0] & 0x7fffffffu;
-  const uint32_t f = 32u - (uint32_t)__clz((int)or_tail), w = 32u - (uint32_t)__clz((int)c.a0), o = (w + 7u) >> 3;
+__device__ __forceinline__ void choose_code(BlockCode& c, uint32_t f) {
+  const uint32_t w = 32u - (uint32_t)__clz((int)c.a0), o = (w + 7u) >> 3;
   const uint32_t top = f > w ? f : w;
   c.rate = top;
   c.len = top ? 4u * top + 4u : 0u;
@@ -259,8 +267,16 @@ __device__ __forceinline__ BlockCode code_of(uint32_t (&d)[32], uint32_t or_tail
     c.rate = f + 32u * o + 96u;  // 0x80 | (o - 1) << 5 | f
     c.len = 4u * f + 4u + o;
     c.nout = o;
-    d[0] = 0;
   }
+}
+// sign-magnitude deltas -> the block's code; d_0 of an outlier block is taken out of the planes
+template <int MODE>
+__device__ __forceinline__ BlockCode code_of(uint32_t (&d)[32], uint32_t or_tail) {
+  BlockCode c;
+  c.sign = signs_of(d);
+  c.a0 = d[0] & 0x7fffffffu;
+  choose_code<MODE>(c, 32u - (uint32_t)__clz((int)or_tail));
+  if (c.nout) d[0] = 0;
   return c;
 }
 
@@ -276,7 +292,7 @@ __device__ __forceinline__ void pack_block(uint32_t base, uint32_t rel, const Bl
   const uint32_t p2 = rel + c.nout;
   const uint32_t s0 = 8u * rel, s = 8u * p2;  // (funnel shifts take them modulo 32)
   const uint32_t first = base + (rel & ~3u), at = base + (p2 & ~3u);  // words of the first byte, of the sign map
-  const uint32_t sign = __byte_perm(c.sign, 0, 0x0123);
+  const uint32_t sign = c.sign;
   uint32_t head = __funnelshift_l(0u, a0, s0);
   if (c.len) {
     // words 1 .. F + 1 hold payload; as bits of a register seven comparisons turn into one instruction
@@ -313,6 +329,171 @@ __device__ __forceinline__ void pack_blocks(uint32_t base, uint32_t rel, const B
   else if (W == 4) pack_w<4>(base, rel, c, d);
   else if (__builtin_expect(W == 0, 0)) pack_w<0>(base, rel, c, d);
   else pack_w<32>(base, rel, c, d);
+}
+
+// ---- blocks as planes --------------------------------------------------------------------------------
+// Sum of the contributions to one block as two's complement planes (hc_bitplane.h): kNarrow of them while `bound`, which no
+// magnitude of the warp exceeds, fits them, else all 32, which wrap like an int32.
+// |d_0| of outlier blocks, and a local d_0 that does not fit the planes of its warp, are summed apart.
+// What bounds an add of streams is its instructions, at 15 warps an SM, and the latency of each warp's own chain.  A sub-tile of
+// stream + stream takes 1299 warp instructions this way, 1605 by way of rows (gradients; 1478 and 1870 for a random walk), one of seven
+// streams and fp32 3550 and 4380: 16 MB of a random walk 23.8 -> 20.3 us, 64 MB of gradients 49.2 -> 44.5, seven streams of 8 MB and
+// their decode 25.1 -> 23.0.  With ONE stream and fp32 as many instructions are left (the rows of the local operand are there
+// already) and their chain is longer: 64 MB 38.4 us by way of rows, 40.5 this way.
+// Two pieces of code, narrow and wide, not one for each width (44.0 us where this takes 44.5, but 21.6 against 20.3 for the random walk
+// and 44.2 against 37.7 for three of them), and not groups of four planes as far as they are needed (46.4).
+constexpr int kNarrow = 20;
+struct PlaneSum {
+  uint32_t A[32];
+  uint32_t apart, bound;
+};
+__device__ __forceinline__ bool sum_wide(const PlaneSum& s) { return __any_sync(0xffffffffu, s.bound >> (kNarrow - 1)); }
+__device__ __forceinline__ void sum_clear(PlaneSum& s) {
+#pragma unroll
+  for (int j = 0; j < kNarrow; ++j) s.A[j] = 0;
+  s.apart = s.bound = 0;
+}
+// planes 8 B .. 8 B + 7 of a block (zero at and above F); word: the one that plane 8 B begins in
+template <int B>
+__device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F, uint32_t& word, uint32_t (&T)[32]) {
+  uint32_t w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = lds32(wp + 4 * (8 * B + 2 + j));
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t x = __funnelshift_r(j ? w[j - 1] : word, w[j], sh);
+    T[8 * B + j] = (uint32_t)(8 * B + j) < F ? x : 0u;
+  }
+  word = w[7];
+}
+// Adds a staged payload (see read_planes).
+__device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, uint32_t pos, uint32_t rate) {
+  const uint32_t F = rate & 31u, W = __reduce_max_sync(0xffffffffu, F);
+  uint32_t p2 = pos, a0 = 0;
+  if (__any_sync(0xffffffffu, rate & 0x80u)) {
+    if (rate & 0x80u) {
+      const uint32_t nout = ((rate >> 5) & 3u) + 1u;
+      const uint32_t wa = smem_u32(buf) + (pos & ~3u);
+      a0 = __funnelshift_r(lds32(wa), lds32(wa + 4u), 8u * (pos & 3u)) & (0xffffffffu >> (32u - 8u * nout));
+      p2 += nout;
+    }
+  }
+  const uint32_t sh = 8u * (p2 & 3u), wp = smem_u32(buf) + (p2 & ~3u);
+  uint32_t T[32], word0 = lds32(wp), word = lds32(wp + 4u);
+  const uint32_t sign = __funnelshift_r(word0, word, sh);
+  read_eight<0>(wp, sh, F, word, T);
+  if (W > 8u) {
+    read_eight<1>(wp, sh, F, word, T);
+  } else {
+#pragma unroll
+    for (int j = 8; j < 16; ++j) T[j] = 0;
+  }
+  s.apart += sign & kFirst ? 0u - a0 : a0;
+  const bool was_wide = sum_wide(s);
+  s.bound = W > 16u ? 0x7fffffffu : min(s.bound + (1u << W), 0x7fffffffu);
+  if (__builtin_expect(sum_wide(s), 0)) {
+    if (!was_wide) {
+#pragma unroll
+      for (int j = kNarrow; j < 32; ++j) s.A[j] = s.A[kNarrow - 1];
+    }
+    if (W > 16u) {
+      read_eight<2>(wp, sh, F, word, T);
+      read_eight<3>(wp, sh, F, word, T);
+    } else {
+#pragma unroll
+      for (int j = 16; j < 32; ++j) T[j] = 0;
+    }
+    add_planes<32, 32>(s.A, T, sign);
+  } else {
+    add_planes<16, kNarrow>(s.A, T, sign);
+  }
+}
+// Starts a sum with the block's own deltas: subnormals, or int32 (`ints`); or_tail: of the subnormals.
+__device__ __forceinline__ void sum_local(PlaneSum& s, uint32_t (&d)[32], uint32_t or_tail, bool ints) {
+  const uint32_t W = ints ? 32u : __reduce_max_sync(0xffffffffu, 32u - (uint32_t)__clz((int)or_tail));
+  uint32_t (&A)[32] = s.A;
+  s.apart = 0;
+  if (__builtin_expect(W <= 16u, 1)) {
+    if ((d[0] & 0x7fffffffu) >> W) {
+      s.apart = sub_to_int(d[0]);
+      d[0] = 0;
+    }
+    const uint32_t sign = signs_of(d);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) A[i ^ 7] = d[i];
+    planes_up_to_16(A, W);
+    if (W <= 8u) {
+#pragma unroll
+      for (int j = 8; j < 16; ++j) A[j] = 0;
+    } else if (W <= 12u) {
+#pragma unroll
+      for (int j = 12; j < 16; ++j) A[j] = 0;
+    }
+    uint32_t c = sign;
+    negate_planes<16>(A, sign, c);
+#pragma unroll
+    for (int j = 16; j < kNarrow; ++j) A[j] = sign & ~c;
+    s.bound = 1u << W;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) A[i ^ 7] = ints ? d[i] : sub_to_int(d[i]);
+    planes_from_rows<32>(A);
+    s.bound = 0x7fffffffu;
+  }
+}
+// Sum -> magnitude planes in A (zero at and above the planes of the block) and the block's code.
+template <int MODE>
+__device__ __forceinline__ BlockCode sum_code(PlaneSum& s) {
+  BlockCode c;
+  uint32_t (&A)[32] = s.A;
+  const bool wide = sum_wide(s);
+  c.sign = wide ? A[31] : A[kNarrow - 1];
+  // magnitudes, how many planes they take without d_0, and |d_0|
+  uint32_t carry = c.sign, f = 0, v = 0;
+  negate_planes<kNarrow>(A, c.sign, carry);
+  auto look = [&](int g) {
+#pragma unroll
+    for (int j = 4 * g; j < 4 * g + 4; ++j)
+      if (A[j] & ~kFirst) f = j + 1;
+    v |= firsts_of(A[4 * g], A[4 * g + 1], A[4 * g + 2], A[4 * g + 3]) >> 28 << 4 * g;
+  };
+#pragma unroll
+  for (int g = 0; g < kNarrow / 4; ++g) look(g);
+  if (__builtin_expect(wide, 0)) {
+#pragma unroll
+    for (int j = kNarrow; j < 31; ++j) {
+      const uint32_t a = A[j];
+      A[j] = xor3(a, c.sign, carry);
+      carry &= a ^ c.sign;
+    }
+    A[31] = 0;  // 31 bits
+#pragma unroll
+    for (int g = kNarrow / 4; g < 8; ++g) look(g);
+  } else {
+#pragma unroll
+    for (int j = kNarrow; j < 32; ++j) A[j] = 0;
+  }
+  if (c.sign & kFirst) v = v ? 0u - v : kMsb;  // (a sign without a magnitude: the smallest of the 32-bit integers)
+  v += s.apart;
+  c.sign = bit_select(c.sign, v >> 24, ~kFirst);
+  c.a0 = (uint32_t)abs((int32_t)v) & 0x7fffffffu;
+  choose_code<MODE>(c, f);
+  // d_0 in the planes: as it came out of them where the block is a plain one, unless some of it was apart
+  if (__any_sync(0xffffffffu, c.nout | s.apart)) {
+    const uint32_t a0 = c.nout ? 0u : c.a0;
+#pragma unroll
+    for (int j = 0; j < 31; ++j) A[j] = bit_select(A[j], j <= 7 ? a0 << (7 - j) : a0 >> (j - 7), ~kFirst);
+  }
+  return c;
+}
+// packs the planes of a block per lane (see pack_block); W: plane_width of the largest F of the warp
+__device__ __forceinline__ void pack_planes(uint32_t base, uint32_t rel, const BlockCode& c, const uint32_t (&A)[32], int W) {
+  if (__builtin_expect(W == 12, 1)) pack_block<12>(base, rel, c, A);
+  else if (__builtin_expect(W == 8, 1)) pack_block<8>(base, rel, c, A);
+  else if (__builtin_expect(W == 16, 1)) pack_block<16>(base, rel, c, A);
+  else if (W == 4) pack_block<4>(base, rel, c, A);
+  else if (__builtin_expect(W == 0, 0)) pack_block<0>(base, rel, c, A);
+  else pack_block<32>(base, rel, c, A);
 }
 
 // 16-byte units of copy_ring: source bytes start K words and sh bits into 16-byte aligned shared memory.  Not unrolled: a

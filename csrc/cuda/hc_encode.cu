@@ -238,6 +238,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   constexpr bool kHasLocal = OP != kOpAddStream;
   constexpr bool kHasIn = OP != kOpCompress;
   constexpr bool kFloat = OP != kOpAddI32;  // the subnormal form may apply
+  constexpr bool kPlanes = kHasIn && kFloat && !ONE;  // contributions are added as planes (see PlaneSum)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ EncShared sh;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -417,8 +418,9 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     const Where w = where(t);
     const uint32_t t_next = ticket(p, k + 1);
     uint32_t d[32];
-    bool ints = !kFloat;  // d holds int32 deltas instead of subnormals (d[0] is an int32 with inputs in any case)
+    PlaneSum sum;
     uint32_t or_tail = 0;
+    bool ints = false;  // d holds int32 deltas instead of subnormals
     // ---- local operand: first, because it needs nothing but its rows --------------------------------------------------
     if (kHasLocal) {
       if (!warp_wait(&sh.stage_full[warp], k & 1u, ws, kSiteComputeTile)) {
@@ -442,15 +444,15 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
           load_row_swizzled(stage, (int)lane, d);
           if (!kHasIn) or_tail = or_tail_of(d);
           else ints = true;
-        } else if (kHasIn) {
+        } else if (kHasIn && !kPlanes) {
           d[0] = sub_to_int(d[0]);
         }
       }
       __syncwarp();
       fetch_stage(t_next);  // every lane holds its row
+      if (kPlanes) sum_local(sum, d, or_tail, ints);
     } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) d[i] = 0;
+      sum_clear(sum);
     }
     if (tid == 0) HC_PH(2);
     // ---- incoming streams ----------------------------------------------------------------------------------------------
@@ -471,59 +473,60 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
           break;
         }
         if (tid == 0) HC_PH(3);
-        uint32_t T[32], sign, a0;
-        decode_rows(inring, cur_pos, cur_rate, plane_width(__reduce_max_sync(0xffffffffu, cur_rate & 31u)), sign, a0, T);
-        __syncwarp();
-        // |d_1| .. |d_31| small enough for sums of eight such streams: so with up to 16 planes, else to be looked at (a
-        // plain block may have many planes for the sake of d_0 alone, which is summed in int32)
-        bool fits = (cur_rate & 31u) <= 16u;
-        if (kFloat && __builtin_expect(!__all_sync(0xffffffffu, fits), 0)) fits = fits || or_rows_tail(T) < (1u << 20);
+        if (kPlanes) {
+          sum_add(sum, inring, cur_pos, cur_rate);
+          __syncwarp();
+        } else {
+          uint32_t T[32], sign, a0;
+          decode_rows(inring, cur_pos, cur_rate, plane_width(__reduce_max_sync(0xffffffffu, cur_rate & 31u)), sign, a0, T);
+          __syncwarp();
+          // |d_1| .. |d_31| small enough for sums in subnormals: so with up to 16 planes, else to be looked at (a
+          // plain block may have many planes for the sake of d_0 alone, which is summed in int32)
+          bool fits = (cur_rate & 31u) <= 16u;
+          if (kFloat && __builtin_expect(!__all_sync(0xffffffffu, fits), 0)) fits = fits || or_rows_tail(T) < (1u << 20);
+          if (kFloat && __builtin_expect(__all_sync(0xffffffffu, fits) && !ints, 1)) {
+            const uint32_t m = (uint32_t)((int32_t)sign >> 31);
+            d[0] += (T[7] ^ m) - m;
+            d[1] = as_u(__fadd_rn(as_f(d[1]), as_f(signed_sub(T[6], sign, 1))));
+#pragma unroll
+            for (int i = 2; i < 32; i += 2)
+              unpack2(add2(pack2(d[i], d[i + 1]), pack2(signed_sub(T[i ^ 7], sign, i), signed_sub(T[(i + 1) ^ 7], sign, i + 1))), d[i], d[i + 1]);
+          } else {
+            if (kFloat && !ints) {
+#pragma unroll
+              for (int i = 1; i < 32; ++i) d[i] = sub_to_int(d[i]);
+              ints = true;
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const uint32_t m = (uint32_t)((int32_t)(sign << i) >> 31);
+              d[i] += (T[i ^ 7] ^ m) - m;
+            }
+          }
+        }
         cur_rate = nxt_rate;
         cur_pos = nxt_pos;
         --staged;
-        if (!kFloat) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const uint32_t m = (uint32_t)((int32_t)(sign << i) >> 31);
-            d[i] += (T[i ^ 7] ^ m) - m;
-          }
-        } else if (__builtin_expect(__all_sync(0xffffffffu, fits) && !ints, 1)) {
-          const uint32_t m = (uint32_t)((int32_t)sign >> 31);
-          d[0] += (T[7] ^ m) - m;
-          d[1] = as_u(__fadd_rn(as_f(d[1]), as_f(signed_sub(T[6], sign, 1))));
-#pragma unroll
-          for (int i = 2; i < 32; i += 2)
-            unpack2(add2(pack2(d[i], d[i + 1]), pack2(signed_sub(T[i ^ 7], sign, i), signed_sub(T[(i + 1) ^ 7], sign, i + 1))), d[i], d[i + 1]);
-        } else {
-          if (!ints) {
-#pragma unroll
-            for (int i = 1; i < 32; ++i) d[i] = sub_to_int(d[i]);
-            ints = true;
-          }
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const uint32_t m = (uint32_t)((int32_t)(sign << i) >> 31);
-            d[i] += (T[i ^ 7] ^ m) - m;
-          }
-        }
         if (tid == 0) HC_PH(4);
       }
       if (failed) break;
-      if (!kFloat) {
+      if (!kPlanes) {
+        if (!kFloat || __builtin_expect(ints, 0)) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
-      } else if (__builtin_expect(ints, 0)) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
-      } else {
-        d[0] = sign_magnitude(d[0]);
+          for (int i = 0; i < 32; ++i) d[i] = sign_magnitude(d[i]);
+        } else {
+          d[0] = sign_magnitude(d[0]);
+        }
+        or_tail = or_tail_of(d);
       }
-      or_tail = or_tail_of(d);
     }
 
     if (tid == 0) HC_PH(4);
     // ---- encode -----------------------------------------------------------------------------------------------------------
-    const BlockCode code = code_of<MODE>(d, or_tail);
+    const BlockCode code = [&]() -> BlockCode {
+      if constexpr (kPlanes) return sum_code<MODE>(sum);
+      else return code_of<MODE>(d, or_tail);
+    }();
     const uint32_t inc = warp_inclusive_scan(code.len, (int)lane);
     const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
     uint32_t before = 0;
@@ -585,7 +588,9 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     if (failed) break;
     if (tid == 0) HC_PH(6);
     __syncwarp();
-    pack_blocks(oring + start, inc - code.len, code, d, plane_width(__reduce_max_sync(0xffffffffu, code.rate & 31u)));
+    const int W = plane_width(__reduce_max_sync(0xffffffffu, code.rate & 31u));
+    if (kPlanes) pack_planes(oring + start, inc - code.len, code, sum.A, W);
+    else pack_blocks(oring + start, inc - code.len, code, d, W);
     if (lane == k % kSlots) {
       my_start = SEGS ? start | tot << 13 | w.seg << 26 : start;
       if (!SEGS) my_tot = tot;

@@ -103,6 +103,41 @@ HC_HD void planes_from_rows(uint32_t (&A)[32]) {
     if ((k & 1) == 0) swap_stage<1>(A[k], A[k + 1]);
 }
 
+// The same for a width known at run time, at most 16 (a multiple of four): planes 0 .. W-1 in one piece of code for all of them.
+HC_HD void planes_up_to_16(uint32_t (&A)[32], uint32_t W) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) A[k] = perm(A[k], A[k + 16], 0x5410);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const uint32_t lo = A[k], hi = A[k + 8];
+    A[k] = perm(lo, hi, 0x6240);
+    A[k + 8] = perm(lo, hi, 0x7351);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) swap_stage<4>(A[k], A[k + 4]);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if ((k & 2) == 0) swap_stage<2>(A[k], A[k + 2]);
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) swap_stage<1>(A[k], A[k + 1]);
+  if (W <= 8) return;
+  if (W <= 12) {
+#pragma unroll
+    for (int k = 8; k < 12; ++k) A[k] = bit_select(A[k], A[k + 4] << 4, 0x0f0f0f0fu);
+  } else {
+#pragma unroll
+    for (int k = 8; k < 12; ++k) swap_stage<4>(A[k], A[k + 4]);
+    swap_stage<2>(A[12], A[14]);
+    swap_stage<2>(A[13], A[15]);
+    swap_stage<1>(A[12], A[13]);
+    swap_stage<1>(A[14], A[15]);
+  }
+  swap_stage<2>(A[8], A[10]);
+  swap_stage<2>(A[9], A[11]);
+  swap_stage<1>(A[8], A[9]);
+  swap_stage<1>(A[10], A[11]);
+}
+
 // Inverse: A[0..W-1] hold planes 0..W-1 (planes >= F are zero); on return A[0..31] are the rows.
 // Entries A[W..31] are ignored on input.
 template <int W>
@@ -167,6 +202,57 @@ HC_HD void rows_from_planes(uint32_t (&A)[32]) {
     A[k] = perm(lo, hi, 0x5410);
     A[k + 16] = perm(lo, hi, 0x7632);
   }
+}
+
+// ---- sums in bit planes ---------------------------------------------------------------------------------
+// A block's 32 integers as two's complement planes: A[p] holds bit p of every element, A[N - 1] the signs, in the bit order of
+// the stream's words.  Adding a block of a stream, whose planes and sign map stand there already, takes three logic operations a
+// plane; by way of rows it takes the transposition (114 operations at 12 planes) and three a row (96), and a result that goes back
+// into a stream is transposed once more.
+HC_HD uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) {
+#if defined(__CUDA_ARCH__)
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+#else
+  return a ^ b ^ c;
+#endif
+}
+HC_HD uint32_t majority(uint32_t a, uint32_t b, uint32_t c) {
+#if defined(__CUDA_ARCH__)
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xe8;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+#else
+  return (a & b) | (c & (a | b));
+#endif
+}
+// A += the integers with magnitude planes T[0 .. W-1] and sign map `sign`, modulo 2^N
+template <int W, int N>
+HC_HD void add_planes(uint32_t (&A)[32], const uint32_t (&T)[32], uint32_t sign) {
+  static_assert(W <= N && N <= 32, "planes");
+  uint32_t c = sign;  // -m = ~m + 1
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const uint32_t x = j < W ? T[j] ^ sign : sign, a = A[j];
+    A[j] = xor3(a, x, c);
+    if (j + 1 < N) c = majority(a, x, c);
+  }
+}
+// N planes (A ^ sign) + sign: magnitudes into two's complement, or back
+template <int N>
+HC_HD void negate_planes(uint32_t (&A)[32], uint32_t sign, uint32_t& c) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const uint32_t a = A[j];
+    A[j] = xor3(a, sign, c);
+    c &= a ^ sign;
+  }
+}
+// bit 7 of the words a0 .. a3 as bits 31 .. 28 (a3 .. a0), other bits below them
+HC_HD uint32_t firsts_of(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+  const uint32_t v = perm(perm(a0, a1, 0x0040), perm(a2, a3, 0x0040), 0x5410) & 0x80808080u;
+  return v * ((1u << 21) | (1u << 14) | (1u << 7) | 1u);
 }
 
 // smallest supported width that holds F planes (F in 0..31); 0 means "no planes at all"

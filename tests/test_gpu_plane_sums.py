@@ -1,0 +1,43 @@
+"""Sums of streams in bit planes against the oracle: magnitudes at the edges of the planes that the kernel keeps, sums that grow out
+of them and that wrap like an int32, first values inside and outside the planes, blocks without payload among them."""
+import numpy as np
+import pytest
+import torch
+
+from tirocinio_triennale_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _walk(n, bits, seed):
+    """Values (step size 1) whose differences inside a block are of up to `bits` bits, with first values of 0 to 24 bits."""
+    rng = np.random.default_rng(seed)
+    d = rng.integers(-(2 ** bits) + 1, 2 ** bits, n) if bits else np.zeros(n, np.int64)
+    d = d >> rng.integers(0, bits + 1, -(-n // 32)).repeat(32)[:n]  # blocks of fewer planes, and of none
+    d[::32] = rng.integers(-(2 ** 24), 2 ** 24, d[::32].size) >> rng.integers(0, 26, d[::32].size)
+    q = np.concatenate([np.cumsum(b) for b in np.split(d, range(32, n, 32))])
+    return np.clip(q, -(2 ** 29), 2 ** 29).astype(np.float32)
+
+
+def _gpu(a):
+    return torch.from_numpy(np.concatenate([a, np.zeros(32, a.dtype)])).cuda()
+
+
+@pytest.mark.parametrize("mode", ["outlier", "plain", "vec"])
+@pytest.mark.parametrize("bits", [0, 4, 8, 9, 12, 13, 15, 16, 17, 19, 20, 24, 28])
+def test_sums_of_streams(bits, mode):
+    n, eb, k = 5 * 1024 + 77, 0.5, 8
+    codec = ops.Codec((k + 1) * 32768)
+    xs = [_walk(n, max(0, bits - (i % 3 == 1)), 100 * bits + i) for i in range(k + 1)]
+    streams = [ops.cpu_compress(x, eb, mode) for x in xs]
+    gpu = [_gpu(s) for s in streams]
+    want = streams[0]
+    for i in range(1, k):
+        last, want = want, ops.cpu_hom_add_streams(want, streams[i], n, mode)
+        if i in (1, 2, 6, 7):
+            out, size = codec.hom_add_multi(gpu[:i + 1], torch.from_numpy(xs[k]).cuda(), eb, mode,
+                                            stream_bytes=[s.size for s in streams[:i + 1]])
+            np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), ops.cpu_hom_add(want, xs[k], eb, mode))
+        out, size = codec.hom_add_streams(_gpu(last), gpu[i], n, mode, a_bytes=last.size, b_bytes=streams[i].size)
+        np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), want)
+    assert codec.status() == 0
