@@ -13,7 +13,8 @@
 // What bounds the decode of one stream: 256 MB the memory (62.1 us; 61.9 with the arithmetic left out, 50.4 without the stores), 64 MB
 // the memory and the start (22.8; 20.8, 19.0), smaller ones the way to the first payload: rate bytes, exchange, payload, one trip to
 // L2 after the other (8 MB: of 6.1 us on the device 3.3; 5.1 of 7.5 when 64-bit divisions, the status and the offsets of the pool
-// stood in between).  Sums take their streams one after the other in every warp (four streams of 256 MB 237 us).
+// stood in between).  Sums take their streams one after the other in every warp and add them as bit planes (four streams of 256 MB
+// 233 us by way of a row for every stream, 198 this way; seven of 40 MB 80 and 67; four of 4 MB 12.0 and 10.7).
 //
 // Steps of a collective (!RUNS): the producer raises one flag word per tile, carrying the tile's payload offset.
 // Tickets are dealt in the order in which the flags rise, round the segments: a tile (all four quarters by one
@@ -49,7 +50,7 @@ static __device__ __noinline__ void store_rows(const uint8_t* rows, const DecSeg
 }
 
 // SUM: the n_seg streams hold contributions to ONE array; a warp stages the same sub-tile of every stream in
-// turn, adds the signed deltas in registers and writes seg[0].out once.
+// turn, adds the deltas in registers, as bit planes, and writes seg[0].out once.
 template <int MODE, bool SUM, bool RUNS>
 __global__ void __launch_bounds__(dec_max_warps(RUNS) * 32, dec_ctas(SUM, RUNS))
 hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
@@ -357,9 +358,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   // has been read
   Staged cur{}, nxt{};
   uint32_t staged = 0;
-  float acc[32];       // SUM: deltas * 2^-23, or int32 bits once `ints`
-  bool ints = false;
-  uint32_t bound = 0;  // of |sum of the deltas| of this lane's block
+  PlaneSum acc;  // SUM: of this lane's block
   bool announced = !RUNS || pool == 0u;
   if (threadIdx.x == 0) HC_PH(0);
   uint32_t v = 0;  // jobs whose payload has landed
@@ -393,72 +392,42 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     if (!warp_wait(&full[v & 3u], (v >> 2) & 1u, ws, kSiteDecodeInFull)) break;
     ++v;
     if (threadIdx.x == 0) HC_PH(2);
-    const int W = plane_width(__reduce_max_sync(0xffffffffu, cur.rate & 31u));
-    uint32_t T[32], sign, a0;
-    decode_rows(ring, cur.pos, cur.rate, W, sign, a0, T);
-    __syncwarp();
-
-    if (threadIdx.x == 0) HC_PH(3);
-    // ---- signs, sum over the streams, prefix sum, scaling ----------------------------------------------------------
-    uint32_t w[32];
-    const bool little = (cur.rate & 31u) <= 16u && a0 < (SUM ? 1u << 20 : 1u << 23);
-    bool exact = p.scale != 0.0f && __all_sync(0xffffffffu, little);
     constexpr int S = MODE == kModeVec ? 4 : 1;
     bool last = true;
+    uint32_t w[32];
     if (SUM) {
-      if (cur.seg == 0) {
-        ints = !exact;
-        bound = 0;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
-      } else if (!ints && !exact) {
-        ints = true;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = __int_as_float(__float2int_rn(__fmul_rn(acc[i], 8388608.0f)));
-      }
-      if (!ints) {
-        bound += a0 + (31u << (cur.rate & 31u));
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = __fmaf_rn(as_f(T[i ^ 7]), sign_scale(sign, i), acc[i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int32_t m = (int32_t)(sign << i) >> 31;
-          acc[i] = __int_as_float(__float_as_int(acc[i]) + ((int32_t)T[i ^ 7] ^ m) - m);
-        }
-      }
+      if (cur.seg == 0) sum_clear(acc);
+      sum_add(acc, ring, cur.pos, cur.rate);
+      __syncwarp();
+      if (threadIdx.x == 0) HC_PH(3);
       last = cur.seg + 1 == Q;
-      if (last && !ints && !__all_sync(0xffffffffu, bound < (1u << 24))) {
-        ints = true;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = __int_as_float(__float2int_rn(__fmul_rn(acc[i], 8388608.0f)));
-      }
-      exact = !ints;
-    }
-    if (last) {
-      if (exact) {
+      if (last) sum_values<S>(acc, p.scale, p.eb, w);
+    } else {
+      const int W = plane_width(__reduce_max_sync(0xffffffffu, cur.rate & 31u));
+      uint32_t T[32], sign, a0;
+      decode_rows(ring, cur.pos, cur.rate, W, sign, a0, T);
+      __syncwarp();
+      if (threadIdx.x == 0) HC_PH(3);
+      // ---- signs, prefix sum, scaling ------------------------------------------------------------------------------
+      const bool little = (cur.rate & 31u) <= 16u && a0 < (1u << 23);
+      if (p.scale != 0.0f && __all_sync(0xffffffffu, little)) {
         float qv[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const float before = i >= S ? qv[i - S] : 0.0f;
-          if (SUM) qv[i] = i >= S ? __fadd_rn(before, acc[i]) : acc[i];
-          else qv[i] = __fmaf_rn(as_f(T[i ^ 7]), sign_scale(sign, i), before);
+          qv[i] = __fmaf_rn(as_f(T[i ^ 7]), sign_scale(sign, i), i >= S ? qv[i - S] : 0.0f);
           w[i] = as_u(__fmul_rn(qv[i], p.scale));
         }
       } else {
         int32_t qv[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const int32_t before = i >= S ? qv[i - S] : 0;
-          if (SUM) {
-            qv[i] = before + __float_as_int(acc[i]);
-          } else {
-            const int32_t m = (int32_t)(sign << i) >> 31;
-            qv[i] = before + ((int32_t)T[i ^ 7] ^ m) - m;
-          }
+          const int32_t m = (int32_t)(sign << i) >> 31;
+          qv[i] = (i >= S ? qv[i - S] : 0) + ((int32_t)T[i ^ 7] ^ m) - m;
           w[i] = as_u(__fmul_rn(__fmul_rn((float)qv[i], p.eb), 2.0f));
         }
       }
+    }
+    if (last) {
       if (threadIdx.x == 0) HC_PH(4);
       // ---- out -------------------------------------------------------------------------------------------------------
       const uint32_t sgo = SUM ? 0u : cur.seg;

@@ -40,4 +40,27 @@ def test_sums_of_streams(bits, mode):
             np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), ops.cpu_hom_add(want, xs[k], eb, mode))
         out, size = codec.hom_add_streams(_gpu(last), gpu[i], n, mode, a_bytes=last.size, b_bytes=streams[i].size)
         np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), want)
+        if mode != "vec":  # (streams with the stride-1 predictor only)
+            y = codec.decompress_sum(gpu[:i + 1], n, eb, stream_bytes=[s.size for s in streams[:i + 1]])
+            np.testing.assert_array_equal(y.cpu().numpy(), ops.cpu_decompress(want, n, eb, mode))
+    assert codec.status() == 0
+
+
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("k,bits", [(2, 6), (2, 10), (8, 8), (3, 10), (2, 11), (2, 14), (8, 12), (3, 14), (5, 14), (8, 15), (8, 16), (2, 20)])
+def test_decode_of_sums_at_the_edges(k, bits, sign):
+    """Every difference as large as its planes allow, all of one sign, so that the sums reach the bound that the kernel goes by; first
+    values that leave what it adds up in floats, and that just do not."""
+    eb = 0.5
+    firsts = np.array([0, 1, -1, 2 ** 19, 2 ** 22 // k, 2 ** 22 // k - 1, -(2 ** 22) // k, -(2 ** 22) // k - 1, 2 ** 22, -(2 ** 23)])
+    q = firsts.repeat(32) + sign * np.tile(np.arange(32) * (2 ** bits - 1), firsts.size)
+    n = q.size
+    codec = ops.Codec((k + 1) * 32768)
+    stream = ops.cpu_compress(q.astype(np.float32), eb)
+    want = stream
+    for _ in range(k - 1):
+        want = ops.cpu_hom_add_streams(want, stream, n)
+    gpu = _gpu(stream)
+    y = codec.decompress_sum([gpu] * k, n, eb, stream_bytes=[stream.size] * k)
+    np.testing.assert_array_equal(y.cpu().numpy(), ops.cpu_decompress(want, n, eb))
     assert codec.status() == 0
