@@ -101,6 +101,30 @@ def test_sums_over_long_runs(k, subs):
     assert c.status() == 0
 
 
+@pytest.mark.parametrize("k,bits", [(2, 22), (3, 21), (4, 20), (5, 16), (8, 19)])
+def test_sums_of_payloads_that_fill_the_ring(k, bits):
+    """Four payloads of a sub-tile that fit in the ring together, that do not, and some of no bytes, by turns; the last stream ends early."""
+    n = 148 * 16 * 1024 * 5 + 1025
+    g = torch.Generator("cuda").manual_seed(k)
+    c = ops.Codec(k * ((n + 32767) // 32768 * 32768))
+    xs, streams, sizes = [], [], []
+    for i in range(k):
+        x = torch.randint(-2 ** bits, 2 ** bits, (n,), device="cuda", generator=g)
+        less = torch.randint(0, bits + 2, (n // 1024 + 1,), device="cuda", generator=g) * (torch.arange(n // 1024 + 1, device="cuda") % 3 == 0)
+        x = (x * 2 + 1 >> less.repeat_interleave(1024)[:n] + 1).float()
+        s, size = c.compress(x, EB)
+        xs.append(x)
+        streams.append(s)
+        sizes.append(int(size))
+    want = sum(xs)
+    assert torch.equal(c.decompress_sum(streams, n, EB, stream_bytes=sizes), want)
+    assert c.status() == 0
+    sizes[-1] -= 1
+    want[(n - 1) // 1024 * 1024:] -= xs[-1][(n - 1) // 1024 * 1024:]
+    assert torch.equal(c.decompress_sum(streams, n, EB, stream_bytes=sizes), want)
+    assert c.status() == 2
+
+
 def test_launches_of_all_grids_behind_one_another():
     """A launch leaves words of the exchange as they are; the next one, with more CTAs or fewer, starts from there."""
     rng = np.random.default_rng(3)
