@@ -4,7 +4,7 @@
 // of a tile.  Every warp works alone: payloads come by bulk copy into a byte ring of its own; the decoded 4 KB go to an output
 // buffer (128-byte swizzle) and leave through a TMA tiled store.  Inside the loop no warp waits for another one.
 //
-// Stand-alone streams (hc_decode_run_kernel; hc_decode_sum_kernel, the sum of several): every warp of the grid owns a contiguous run of
+// Stand-alone streams (hc_decode_run_kernel; the sum of several: hc_decode_kernel): every warp of the grid owns a contiguous run of
 // sub-tiles.  It sums the payload lengths of its run from the rate bytes (700 bytes for a 256 MB array), the CTAs (one per SM, so
 // at most 148) exchange their totals once through the workspace, and from there on a warp carries its own running offset: no
 // look-back, no second kernel.  The SMs do not run at the same pace (with equal static shares the first warp of a 256 MB launch
@@ -15,9 +15,8 @@
 // L2 after the other (8 MB: of 6.1 us on the device 3.3; 5.1 of 7.5 when 64-bit divisions, the status and the offsets of the pool
 // stood in between).
 //
-// Steps of a collective (hc_decode_kernel): the producer raises one flag word per tile, carrying the tile's payload offset.
-// Tickets are dealt in the order in which the flags rise, round the segments: a tile (all four quarters by one
-// warp, its rate bytes scanned once), or a quarter of a tile while the GPU holds a warp for each.
+// Steps of a collective: hc_decode_step.cuh.
+#include "hc_decode_step.cuh"
 #include "hc_host.cuh"
 #include "hc_launch.h"
 #include "hc_timeline.cuh"
@@ -26,307 +25,350 @@
 namespace hc {
 namespace dev {
 
-// 20 warps (96 registers a thread) or, in sums, 16 (128) on an SM.  Stand-alone: one CTA per SM, so that the totals
-// of at most 148 CTAs are exchanged.  Steps of a collective: CTAs of four warps, which slip into an SM one by one
-// while the CTAs of the step before leave it.
-constexpr int kDecWarps = 4;
-// payload ring of a warp: the largest payload of corrupt rate bytes (32 x 132) with its 16-byte phase, and in
-// front of the ring's end what read_planes may look at behind a payload
-constexpr int kDecRing = 6144;
-constexpr int kDecRingUsable = kDecRing - 160;
-constexpr int kDecWarpBytes = kSubBytes + kDecRing;
-static_assert(32 * 132 + 32 <= kDecRingUsable, "one payload must fit");
+// ---- sum of several stand-alone streams ------------------------------------------------------------------------------
+// As with one stream (below) every warp has a contiguous run of sub-tiles, and its offset in every stream.  What it stages at a time is a
+// BATCH, the payloads of one sub-tile in up to four streams, and everything that goes with one is done for the four at once: lanes
+// 8 s .. 8 s + 7 belong to stream s, each with the rate bytes of four blocks.  Staged one by one, every stream of a sub-tile cost a scan,
+// room in the ring, bounds and a barrier of its own, 300 of its 470 instructions (four streams of 256 MB 198 us, 146 this way; seven
+// of 40 MB 67.6 and 52.1; four of 4 MB 11.0 and 8.7; two of 4 KB 5.2 and 4.9).  A batch whose payloads do not all fit in the ring is
+// staged in parts.  What bounds it: instructions, at 16 warps an SM; short runs the same trips to L2 as one stream's.
+constexpr int kSumWarps = 16;
+constexpr uint32_t kSumRing = 10240, kSumUsable = kSumRing - 160;  // (see kDecRingUsable)
+constexpr int kSumWarpBytes = kSubBytes + (int)kSumRing;
+static_assert(32 * 132 + 32 <= kSumUsable, "one payload must fit");
 
-// What the TMA unit cannot store of a sub-tile: the ragged last row (not part of the tensor map), or everything when the array is
-// not 16-byte aligned
-static __device__ __noinline__ void store_rows(const uint8_t* rows, const DecSegment& sg, uint64_t first) {
-  const uint32_t len = sg.n - first < kSubValues ? (uint32_t)(sg.n - first) : (uint32_t)kSubValues;
-#pragma unroll 1
-  for (uint32_t e = (sg.use_tma ? len / kBlock * kBlock : 0u) + (threadIdx.x & 31u); e < len; e += 32u)
-    sg.out[first + e] = as_f(lds32((swizzled_row(rows, (int)(e >> 5)) ^ ((e & 28u) << 2)) | ((e & 3u) << 2)));
-  __syncwarp();
-}
-
-// Steps of a collective.  SUM: the n_seg streams hold contributions to ONE array; a warp stages the same sub-tile of every stream in
-// turn, adds the deltas in registers, as bit planes, and writes seg[0].out once.
-template <int MODE, bool SUM>
-__global__ void __launch_bounds__(kDecWarps * 32, SUM ? 4 : 5)
+__global__ void __launch_bounds__(kSumWarps * 32, 1)
 hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ uint64_t s_full[kDecWarps][4];
+  __shared__ uint64_t s_full[kSumWarps][2];
+  __shared__ uint32_t s_tot[kSumWarps][kMaxDst];  // payload bytes of a run
+  __shared__ uint64_t s_pre[kMaxDst];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* const obuf = smem + warp * kSubBytes;
-  uint8_t* const ring = smem + n_warps * kSubBytes + warp * kDecRing;
+  uint8_t* const ring = smem + n_warps * kSubBytes + warp * kSumRing;
   const Workspace& ws = p.ws;
   uint64_t* const full = s_full[warp];
-  if (lane < 4u) mbar_init(&full[lane], 1);
+  if (lane < 2u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
+  grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   __syncwarp();
-
-  const uint32_t Q = SUM ? p.n_seg : 1u;  // streams per sub-tile
+  const uint32_t Q = p.n_seg;
   const uint32_t gw = blockIdx.x * n_warps + warp, nw = gridDim.x * n_warps;
   const uint32_t status = *((volatile const uint32_t*)(ws.ctrl + 2));
-
-  // A job is a sub-tile of one stream.  Its ITEM is a tile, or a quarter of one; items are known one ahead, so that
-  // the next one's rate bytes and flag are asked for a job or more before they are looked at.
-  struct Staged {
-    uint32_t rate;  // rate byte of this lane's block (0: nothing staged for it)
-    uint32_t pos;   // its byte position in the ring
-    uint32_t sub;   // sub-tile inside the segment
-    uint32_t seg;   // segment; SUM: number of the stream
-  };
-  uint32_t live_at = 0, live_end = 0;  // ring bytes of the newest staged payload
-  uint32_t jobs = 0;                   // staged so far
-  // room for a payload of `bytes` bytes, `busy`: the newest staged payload has not been read yet
-  auto ring_room = [&](uint32_t bytes, bool busy, uint32_t& at) -> bool {
-    at = busy ? live_end : 0u;
-    if (at + bytes > (uint32_t)kDecRingUsable) {
-      at = 0;
-      if (bytes > live_at) return false;
-    }
-    return true;
-  };
-  // bulk copy of the payload bytes [off, off + tot) of a stream to ring byte `at`; sets rate and pos of the lane's block
-  auto issue = [&](const DecSegment& sg, uint64_t off, uint32_t tot, uint32_t at, Staged& st) {
-    const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(sg.in) + off) & 15u;
-    const uint32_t bytes = tot ? (phase + tot + 15u) & ~15u : 0u;
-    live_at = at;
-    live_end = at + bytes;
-    uint64_t* const bar = &full[jobs & 3u];
-    if (lane == 0) {
-      if (tot) {
-        fence_proxy_async();  // what used to be in these bytes has been read
-        mbar_expect_tx(bar, bytes);
-        bulk_load(ring + at, sg.in + off - phase, bytes, bar);
-      } else {
-        mbar_arrive(bar);
-      }
-    }
-    ++jobs;
-    if (!tot) st.rate = 0;
-    st.pos += at + phase;
-  };
-
-  // ---- tickets: tiles or quarters ---------------------------------------------------------------------------------------
-  const bool small = p.parts == 4u;
-  const uint32_t n_tickets = (SUM ? p.tiles_per_seg : p.n_tiles) * p.parts;
-  const bool dynamic = n_tickets > nw;
-  // the first half of the tickets is dealt out in turn, the rest comes from the counter (one address for all
-  // warps: it answers a request every few cycles)
-  const uint32_t rounds = n_tickets / nw, dealt = rounds > 2u ? rounds / 2u + 1u : rounds;
-  uint32_t asked = 0, tk_raw = kNoTile;  // tickets asked for; lane 0 (all lanes if dealt): the newest answer
-  auto ask = [&]() {
-    if (asked < dealt || !dynamic) tk_raw = asked * nw + gw;
-    else if (lane == 0) tk_raw = dealt * nw + atomicAdd(ws.tick, 1u);
-    ++asked;
-  };
-  auto next_item = [&]() -> uint32_t {
-    const uint32_t t = __shfl_sync(0xffffffffu, tk_raw, 0);
-    if (t >= n_tickets) return kNoTile;
-    ask();
-    return t;
-  };
-  auto tile_at = [&](uint32_t t) -> uint32_t { return small ? t >> 2 : t; };
-  auto seg_at = [&](uint32_t t, uint32_t qq) -> uint32_t { return SUM ? qq : tile_at(t) % p.n_seg; };
-  auto local_tile = [&](uint32_t t) -> uint32_t { return SUM ? tile_at(t) : tile_at(t) / p.n_seg; };
-
-  struct Unit {
-    uint64_t flag;  // lane 0's look at the flag
-    uint32_t raw;   // the rate bytes of four blocks of the tile
-    bool raw_ok;    // raw has been asked for (only once the flag is up)
-  };
-  auto load_raw = [&](uint32_t t, uint32_t qq) -> uint32_t {
-    const DecSegment& sg = p.seg[seg_at(t, qq)];
-    return load_rates4(sg.in, sg.in_size, (uint64_t)local_tile(t) * kTileBlocks + 4u * lane);
-  };
-  auto prime = [&](Unit& u, uint32_t t, uint32_t qq) {
-    u = Unit{0ull, 0u, true};
-    if (t == kNoTile) return;
-    const DecSegment& sg = p.seg[seg_at(t, qq)];
-    if ((uint64_t)local_tile(t) * kTileElems >= sg.n) {
-      u.flag = ~0ull;  // past the end of a segment shorter than the longest one: nothing to read or to wait for
-    } else {
-      if (lane == 0) u.flag = ld_acquire_sys_u64(sg.in_ready + local_tile(t));
-      u.raw_ok = false;
-    }
-  };
   HC_TL_DECL(ws.epoch);
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     HC_TL_ZERO();
     HC_STAMP(0);
     HC_PH_START();
   }
-  ask();
-  // (an earlier launch that timed out, and nobody has cleared its status: no output)
-  uint32_t tk = status >= (uint32_t)kErrTimeout ? kNoTile : next_item(), tk_next = tk == kNoTile ? kNoTile : next_item();
-  Unit un, un_next{0ull, 0u, true};
-  uint32_t r = small ? tk & 3u : 0u, q = 0;  // quarter, stream of the next job
-  prime(un, tk, 0u);
-  uint64_t fw = 0;              // flag word of the current unit (~0: gave up, or nothing there)
-  uint32_t excl = 0, inc = 0;   // scan of the payload lengths of the current tile
-  bool scanned = false;
 
-  // stages the next job; false: flag still down (unless `block`), or no room in the ring
-  auto produce = [&](Staged& st, bool busy, bool block) -> bool {
-    const DecSegment& sg = p.seg[seg_at(tk, q)];
-    if (!scanned) {
-      fw = __shfl_sync(0xffffffffu, un.flag, 0);
-      if (fw != ~0ull && !flag_matches(fw, p.ring_epoch)) {
-        const uint64_t* flag = sg.in_ready + local_tile(tk);
-        fw = block ? flag_wait_warp(flag, p.ring_epoch, ws) : flag_peek(flag, p.ring_epoch);
-        if (fw == 0 && !block) return false;
-        if (fw == 0) {
-          fw = ~0ull;
-          un.raw_ok = true;
+  // ---- shares, offsets -----------------------------------------------------------------------------------------------
+  auto run_of = [&](uint32_t w) -> uint32_t { return p.run_all * w + (w < p.run_more ? w : p.run_more); };
+  const uint32_t pool = p.pool;  // sub-tiles at the end of every run that are handed out one by one
+  uint32_t it = run_of(gw);
+  const uint32_t run_end = run_of(gw + 1u), own_end = run_end - pool;
+  // Payload bytes of the run in every stream.  Runs of up to four sub-tiles: eight lanes a stream, four streams at a time (a
+  // load per stream, its code eight times over, took 0.5 us more where all is start-up)
+  if (p.run_all + (p.run_more ? 1u : 0u) <= 4u) {
+    const uint32_t l = lane & 7u, q0 = lane >> 3, q1 = q0 + 4u;
+    uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
+    if (q0 < Q) v0 = rates16(p.seg[q0].in, p.seg[q0].in_size, it, run_end, l);
+    if (q1 < Q) v1 = rates16(p.seg[q1].in, p.seg[q1].in_size, it, run_end, l);
+    uint32_t s0 = payload_len16(v0), s1 = payload_len16(v1);  // below 2^16 each: 4 * 32 * 132 at most
+    s0 |= s1 << 16;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    if (l == 0) {
+      s_tot[warp][q0] = s0 & 0xffffu;
+      s_tot[warp][q1] = s0 >> 16;
+    }
+  } else {
+    // Longer runs: 16 sub-tiles of four streams are asked for before the first is added (one stream after the other: eight of
+    // 40 MB 96.0 us, 92.6 this way; four of 256 MB 240.9 and 237.1; two of 128 MB 70.4 and 70.0)
+#pragma unroll 1
+    for (uint32_t q4 = 0; q4 < Q; q4 += 4u) {
+      uint32_t sum[4] = {0, 0, 0, 0};
+#pragma unroll 1
+      for (uint32_t l = lane; it * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u) {
+        uint4 v[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u)
+          v[u] = q4 + u < Q ? rates16(p.seg[q4 + u].in, p.seg[q4 + u].in_size, it, run_end, l) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u) sum[u] += payload_len16(v[u]);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < 4u; ++u) {
+        sum[u] = __reduce_add_sync(0xffffffffu, sum[u]);
+        if (lane == 0) s_tot[warp][q4 + u] = sum[u];  // (room for kMaxDst streams, a multiple of four)
+      }
+    }
+  }
+
+  // ---- units: a sub-tile in streams 4 half .. 4 half + 3 ------------------------------------------------------------------
+  // items: own sub-tiles, then tickets of the pools (kPool set)
+  constexpr uint32_t kPool = 0x80000000u;
+  uint32_t tk_raw = kNoTile;
+  const uint32_t n_tickets = pool * nw;
+  auto ask = [&]() {
+    if (lane == 0) tk_raw = atomicAdd(ws.tick, 1u);
+  };
+  auto next_item = [&]() -> uint32_t {
+    if (it < own_end) {
+      const uint32_t i = it++;
+      if (it == own_end && pool) ask();
+      return i;
+    }
+    if (!pool) return kNoTile;
+    const uint32_t t = __shfl_sync(0xffffffffu, tk_raw, 0);
+    if (t >= n_tickets) return kNoTile;
+    ask();
+    return t | kPool;
+  };
+  // ticket t is the (t / nw)-th pool sub-tile of warp t % nw
+  auto sub_of = [&](uint32_t item) -> uint32_t {
+    if (!(item & kPool)) return item;
+    const uint32_t w = (item & ~kPool) % nw, k = (item & ~kPool) / nw;
+    return run_of(w + 1u) - pool + k;
+  };
+  auto pool_flag = [&](uint32_t t, uint32_t q) -> uint64_t* { return p.flags + (size_t)q * pool * nw + (t & ~kPool); };
+  const uint32_t mine = lane >> 3, part = lane & 7u;  // stream of the four, blocks 4 part .. 4 part + 3
+  struct Unit {
+    uint32_t item, half;
+    uint32_t sub;
+    uint32_t rates;  // of the lane's four blocks
+    uint64_t flag;   // pool items: a look at the payload offset
+  };
+  auto look = [&](Unit& u) {
+    const uint32_t q = 4u * u.half + mine;
+    u.rates = 0;
+    u.flag = 0;
+    if (u.item == kNoTile || q >= Q) return;
+    const DecSegment& sg = p.seg[q];
+    u.rates = load_rates4(sg.in, sg.in_size, (uint64_t)u.sub * kSubBlocks + 4u * part);
+    if (u.item & kPool) u.flag = ld_relaxed_gpu_u64(pool_flag(u.item, q));
+  };
+  // (an earlier launch that timed out, and nobody has cleared its status: no output)
+  Unit next{};
+  next.item = status >= (uint32_t)kErrTimeout ? kNoTile : next_item();
+  next.sub = sub_of(next.item);
+  look(next);
+
+  __syncthreads();
+  for (uint32_t q = warp; q < Q; q += n_warps)
+    give_total_of(ws.sums + (1u + q) * kSumWords, warp_sum_u64(lane < n_warps ? s_tot[lane][q] : 0ull));
+  for (uint32_t q = warp; q < Q; q += n_warps) {
+    const uint64_t pre = take_total_of(ws.sums + (1u + q) * kSumWords, ws);
+    if (lane == 0) s_pre[q] = pre;
+  }
+  __syncthreads();
+  uint64_t own_off = 0, own_off_2 = 0;  // of the next own sub-tile's payload in the lane's stream of this half, of the other one
+  if (mine < Q) own_off = rate_bytes(p.seg[0].n) + s_pre[mine];
+  if (mine + 4u < Q) own_off_2 = rate_bytes(p.seg[0].n) + s_pre[mine + 4u];
+#pragma unroll 1
+  for (uint32_t w = 0; w < warp; ++w) {
+    own_off += s_tot[w][mine];
+    own_off_2 += s_tot[w][mine + 4u];
+  }
+
+  // ---- staging -------------------------------------------------------------------------------------------------------
+  struct Batch {
+    uint32_t rates;        // of the lane's four blocks of its stream
+    uint32_t pos;          // ring byte of their payload
+    uint32_t begin, end;   // its streams of the four
+    uint32_t sub;
+    bool first, last;      // of the sub-tile's batches
+  };
+  Batch cur{}, nxt{};
+  uint32_t staged = 0, jobs = 0;  // batches in the ring, and so far
+  uint32_t live_at = 0, live_end = 0;  // ring bytes of the newest batch
+  Unit un{};
+  bool open = false;     // `un` has streams [done, many) still to be staged
+  uint32_t done = 0, many = 0;
+  uint32_t before = 0, bytes = 0;  // payload bytes of the lane's stream in front of its blocks; of the copy
+  uint64_t src = 0;                // address of its payload
+  auto stage = [&](Batch& b) -> bool {
+    if (!open) {
+      un = next;
+      many = Q - 4u * un.half < 4u ? Q - 4u * un.half : 4u;
+      done = 0;
+      open = true;
+      // the next unit's rate bytes and offsets are on their way while this one is worked on
+      if (un.half == 0u && Q > 4u) {
+        next.half = 1u;
+      } else {
+        next.half = 0u;
+        next.item = next_item();
+        if (next.item != kNoTile) next.sub = sub_of(next.item);
+      }
+      look(next);
+      const uint32_t sum = payload_len4(un.rates);
+      uint32_t inc = sum;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o, 8);
+        if (part >= (uint32_t)o) inc += v;
+      }
+      before = inc - sum;
+      const uint32_t tot = __shfl_sync(0xffffffffu, inc, 7, 8);
+      uint64_t off = own_off;
+      if (un.item & kPool) {
+        off = un.flag;
+        const bool there = mine >= many || flag_matches(off, p.ring_epoch);
+        if (__builtin_expect(!__all_sync(0xffffffffu, there), 0)) {
+#pragma unroll 1
+          for (uint32_t s = 0; s < many; ++s) {
+            const uint64_t fw = own_flag_wait(pool_flag(un.item, 4u * un.half + s), p.ring_epoch, ws);
+            if (mine == s) off = fw;
+          }
+        }
+        off &= kFlagOffsetMask;
+      } else {
+        own_off += tot;
+      }
+      if (Q > 4u) {
+        const uint64_t v = own_off;
+        own_off = own_off_2;
+        own_off_2 = v;
+      }
+      bytes = 0;
+      if (tot) {
+        const DecSegment& sg = p.seg[4u * un.half + mine];
+        src = reinterpret_cast<uintptr_t>(sg.in) + off;
+        if (off + tot <= sg.in_size) {
+          bytes = (((uint32_t)src & 15u) + tot + 15u) & ~15u;
+        } else {  // stream shorter than its rate bytes imply (or the offset never came)
+          if (part == 0u && off != kFlagOffsetMask) note_error(ws.ctrl, kErrTruncated);
+          un.rates = 0;
+          before = 0;
         }
       }
-      if (!un.raw_ok) un.raw = load_raw(tk, q);
-      const uint32_t sum = payload_len4(un.raw);
-      inc = warp_inclusive_scan(sum, (int)lane);
-      excl = inc - sum;
-      scanned = true;
-      // the next unit's flag and rate bytes are on their way while this one is worked on
-      if (SUM && q + 1 < Q) prime(un_next, tk, q + 1);
-      else if (SUM && !small && r < 3u) prime(un_next, tk, 0u);
-      else prime(un_next, tk_next, 0u);
-    } else if (!un_next.raw_ok && r >= 2u) {
-      const uint64_t f = __shfl_sync(0xffffffffu, un_next.flag, 0);
-      if (flag_matches(f, p.ring_epoch)) {
-        un_next.raw = load_raw(tk_next, 0u);
-        un_next.raw_ok = true;
-      }
     }
-    const uint32_t before = __shfl_sync(0xffffffffu, excl, 8 * (int)r);
-    const uint32_t tot = __shfl_sync(0xffffffffu, inc, 8 * (int)r + 7) - before;
-    const int src = 8 * (int)r + (int)(lane >> 2);
-    const uint32_t k8 = 8u * (lane & 3u);
-    const uint32_t r4 = __shfl_sync(0xffffffffu, un.raw, src);
-    st.pos = __shfl_sync(0xffffffffu, excl, src) - before + payload_len4(r4 & ((1u << k8) - 1u));
-    st.rate = (r4 >> k8) & 0xffu;
-    st.sub = local_tile(tk) * 4u + r;
-    const uint64_t off = (fw & kFlagOffsetMask) + before;
-    uint32_t at;
-    if (!ring_room(tot ? tot + 31u : 0u, busy, at)) return false;
-    uint32_t take = tot;
-    if ((fw & kFlagOffsetMask) == kFlagOffsetMask) {
-      take = 0;  // the producer gave up on the tile
-    } else if (tot && off + tot > sg.in_size) {  // stream shorter than its rate bytes imply
-      if (lane == 0) note_error(ws.ctrl, kErrTruncated);
-      take = 0;
+    // room: the streams that are left, or as many of them as there is room for
+    uint32_t ends = mine >= done ? bytes : 0u;
+    uint32_t v = __shfl_up_sync(0xffffffffu, ends, 8);
+    if (mine >= 1u) ends += v;
+    v = __shfl_up_sync(0xffffffffu, ends, 16);
+    if (mine >= 2u) ends += v;
+    const uint32_t all = __shfl_sync(0xffffffffu, ends, 31);
+    uint32_t at = staged ? live_end : 0u, space = kSumUsable - at;
+    if (staged && all > space && (all <= live_at || live_at > space)) {
+      at = 0;
+      space = live_at;
     }
-    st.seg = seg_at(tk, q);
-    issue(sg, off, take, at, st);
-    // advance: next stream, next quarter, next item
-    if (SUM && q + 1 < Q) {
-      ++q;
-      scanned = false;
-    } else {
-      q = 0;
-      scanned = !SUM;
-      if (!small && r < 3u) {
-        ++r;
-      } else {
-        scanned = false;
-        tk = tk_next;
-        r = small ? tk & 3u : 0u;
-        if (tk != kNoTile) tk_next = next_item();
-      }
+    uint32_t end = many, used = all;
+    if (__builtin_expect(all > space, 0)) {
+      end = (uint32_t)(__ffs((int)__ballot_sync(0xffffffffu, ends > space)) - 1) >> 3;
+      if (end <= done) return false;  // (not with an empty ring)
+      used = __shfl_sync(0xffffffffu, ends, 8 * (int)end - 1);
     }
-    if (!scanned) un = un_next;
+    uint64_t* const bar = &full[jobs & 1u];
+    fence_proxy_async();  // what used to be in these bytes has been read
+    if (lane == 0) {
+      if (used) mbar_expect_tx(bar, used);
+      else mbar_arrive(bar);
+    }
+    __syncwarp();
+    const uint32_t start = at + ends - bytes;
+    if (part == 0u && bytes && mine >= done && mine < end)
+      bulk_load(ring + start, reinterpret_cast<const uint8_t*>(src & ~uint64_t(15)), bytes, bar);
+    live_at = at;
+    live_end = at + used;
+    ++jobs;
+    b.rates = un.rates;
+    b.pos = start + ((uint32_t)src & 15u) + before;
+    b.begin = done;
+    b.end = end;
+    b.sub = un.sub;
+    b.first = un.half == 0u && done == 0u;
+    b.last = end == many && 4u * un.half + end == Q;
+    done = end;
+    open = end < many;
     return true;
   };
 
-  // ---- consumer side -----------------------------------------------------------------------------------------------
-  // one sub-tile is decoded while the payload of the next one lands; the one after is staged as soon as the first
-  // has been read
-  Staged cur{}, nxt{};
-  uint32_t staged = 0;
-  PlaneSum acc;  // SUM: of this lane's block
-  if (threadIdx.x == 0) HC_PH(0);
-  uint32_t v = 0;  // jobs whose payload has landed
+  // ---- adding up -----------------------------------------------------------------------------------------------------
+  PlaneSum acc;  // of this lane's block
+  bool announced = pool == 0u;
+  if (tid == 0) HC_PH(0);
+  uint32_t landed = 0;  // batches whose payloads have landed
+  const uint32_t ahead = (1u << (8u * (lane & 3u))) - 1u;  // rate bytes of the blocks of a word in front of the lane's
+  const DecSegment& out = p.seg[0];
   for (;;) {
-    if (staged < 2u && tk != kNoTile) {
-      Staged st;
-      if (produce(st, staged != 0u, staged == 0u)) {
-        if (staged == 0u) cur = st;
-        else nxt = st;
+    if (staged < 2u && (open || next.item != kNoTile)) {
+      Batch b;
+      if (stage(b)) {
+        if (staged == 0u) cur = b;
+        else nxt = b;
         ++staged;
         continue;
       }
     }
-    if (threadIdx.x == 0) HC_PH(1);
-    if (staged == 0u) break;
-    if (!warp_wait(&full[v & 3u], (v >> 2) & 1u, ws, kSiteDecodeInFull)) break;
-    ++v;
-    if (threadIdx.x == 0) HC_PH(2);
-    constexpr int S = MODE == kModeVec ? 4 : 1;
-    bool last = true;
-    uint32_t w[32];
-    if (SUM) {
-      if (cur.seg == 0) sum_clear(acc);
-      sum_add(acc, ring, cur.pos, cur.rate);
-      __syncwarp();
-      if (threadIdx.x == 0) HC_PH(3);
-      last = cur.seg + 1 == Q;
-      if (last) sum_values<S>(acc, p.scale, p.eb, w);
-    } else {
-      const int W = plane_width(__reduce_max_sync(0xffffffffu, cur.rate & 31u));
-      uint32_t T[32], sign, a0;
-      decode_rows(ring, cur.pos, cur.rate, W, sign, a0, T);
-      __syncwarp();
-      if (threadIdx.x == 0) HC_PH(3);
-      // ---- signs, prefix sum, scaling ------------------------------------------------------------------------------
-      const bool little = (cur.rate & 31u) <= 16u && a0 < (1u << 23);
-      if (p.scale != 0.0f && __all_sync(0xffffffffu, little)) {
-        float qv[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          qv[i] = __fmaf_rn(as_f(T[i ^ 7]), sign_scale(sign, i), i >= S ? qv[i - S] : 0.0f);
-          w[i] = as_u(__fmul_rn(qv[i], p.scale));
-        }
-      } else {
-        int32_t qv[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int32_t m = (int32_t)(sign << i) >> 31;
-          qv[i] = (i >= S ? qv[i - S] : 0) + ((int32_t)T[i ^ 7] ^ m) - m;
-          w[i] = as_u(__fmul_rn(__fmul_rn((float)qv[i], p.eb), 2.0f));
+    if (!announced) {
+      // offsets of the sub-tiles of this run that others may take, counted back from its end; after the first bulk
+      // copies have been issued, so that it delays nothing
+      announced = true;
+#pragma unroll 1
+      for (uint32_t q = 0; q < Q; ++q) {
+        const DecSegment& sg = p.seg[q];
+        uint64_t off = rate_bytes(sg.n) + s_pre[q];
+        for (uint32_t w = 0; w <= warp; ++w) off += s_tot[w][q];
+#pragma unroll 1
+        for (uint32_t k = pool; k-- > 0u;) {
+          const uint64_t b = (uint64_t)(own_end + k) * kSubBlocks + lane;
+          off -= __reduce_add_sync(0xffffffffu, payload_len(b < sg.in_size ? ld_cg_u8(sg.in + b) : 0u));
+          if (lane == 0) st_relaxed_gpu_u64(pool_flag(k * nw + gw, q), flag_pack(p.ring_epoch, off));
         }
       }
     }
-    if (last) {
-      if (threadIdx.x == 0) HC_PH(4);
-      // ---- out -------------------------------------------------------------------------------------------------------
-      const uint32_t sgo = SUM ? 0u : cur.seg;
-      const DecSegment& sg = p.seg[sgo];
+    if (tid == 0) HC_PH(1);
+    if (staged == 0u) break;
+    uint32_t rates = __shfl_sync(0xffffffffu, cur.rates, (int)(8u * cur.begin + (lane >> 2)));
+    uint32_t pos = __shfl_sync(0xffffffffu, cur.pos, (int)(8u * cur.begin + (lane >> 2)));
+    if (!warp_wait(&full[landed & 1u], (landed >> 1) & 1u, ws, kSiteDecodeInFull)) break;
+    ++landed;
+    if (tid == 0) HC_PH(2);
+    if (cur.first) sum_clear(acc);
+#pragma unroll 1
+    for (uint32_t s = cur.begin; s < cur.end; ++s) {
+      const uint32_t rate = rates >> (8u * (lane & 3u)) & 0xffu, at = pos + payload_len4(rates & ahead);
+      rates = __shfl_sync(0xffffffffu, cur.rates, (int)(8u * s + 8u + (lane >> 2)));  // (past the last one: unused)
+      pos = __shfl_sync(0xffffffffu, cur.pos, (int)(8u * s + 8u + (lane >> 2)));
+      sum_add(acc, ring, at, rate);
+    }
+    __syncwarp();
+    if (tid == 0) HC_PH(3);
+    if (cur.last) {
+      uint32_t w[32];
+      sum_values<1>(acc, p.scale, p.eb, w);
+      if (tid == 0) HC_PH(4);
       const uint64_t first = (uint64_t)cur.sub * kSubValues;
       if (lane == 0) tma_wait_group_read<0>();  // the rows of a turn ago have left the buffer
       __syncwarp();
       store_row_swizzled(obuf, (int)lane, w);
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0 && sg.use_tma && first + kBlock <= sg.n) {
-        tma_store_2d(&tmaps.m[sgo], 0, (int)(cur.sub * kSubBlocks), obuf);
+      if (lane == 0 && out.use_tma && first + kBlock <= out.n) {
+        tma_store_2d(&tmaps.m[0], 0, (int)(cur.sub * kSubBlocks), obuf);
         tma_commit_group();
       }
-      if (!(sg.use_tma && first + kSubValues <= sg.n) && first < sg.n) store_rows(obuf, sg, first);
+      if (!(out.use_tma && first + kSubValues <= out.n) && first < out.n) store_rows(obuf, out, first);
     }
     cur = nxt;
     --staged;
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       HC_PH(5);
       HC_PH_COUNT();
     }
   }
   // after a wait that ran out: nothing may land in shared memory once the CTA has left it
-  for (; v < jobs; ++v) mbar_wait_bounded(&full[v & 3u], (v >> 2) & 1u, ws.spin_limit_ns);
+  for (; landed < jobs; ++landed) mbar_wait_bounded(&full[landed & 1u], (landed >> 1) & 1u, ws.spin_limit_ns);
   if (lane == 0) tma_wait_group<0>();
   if (lane == 0) HC_STAMP_MAX(7);
-  if (dynamic) cta_epilogue(ws.tick);
+  if (pool) cta_epilogue(ws.tick);
 }
-
 
 // ---- one stand-alone stream ----------------------------------------------------------------------------------------
 // The payloads of a warp's run lie behind one another in the stream, so they are staged as what they are: one sequence of bytes,
@@ -587,376 +629,30 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
   if (pool) cta_epilogue(ws.tick);
 }
 
-// ---- sum of several stand-alone streams ------------------------------------------------------------------------------
-// As with one stream every warp has a contiguous run of sub-tiles, and its offset in every stream.  What it stages at a time is a
-// BATCH, the payloads of one sub-tile in up to four streams, and everything that goes with one is done for the four at once: lanes
-// 8 s .. 8 s + 7 belong to stream s, each with the rate bytes of four blocks.  Staged one by one, every stream of a sub-tile cost a scan,
-// room in the ring, bounds and a barrier of its own, 300 of its 470 instructions (four streams of 256 MB 198 us, 146 this way; seven
-// of 40 MB 67.6 and 52.1; four of 4 MB 11.0 and 8.7; two of 4 KB 5.2 and 4.9).  A batch whose payloads do not all fit in the ring is
-// staged in parts.  What bounds it: instructions, at 16 warps an SM; short runs the same trips to L2 as one stream's.
-constexpr int kSumWarps = 16;
-constexpr uint32_t kSumRing = 10240, kSumUsable = kSumRing - 160;  // (see kDecRingUsable)
-constexpr int kSumWarpBytes = kSubBytes + (int)kSumRing;
-static_assert(32 * 132 + 32 <= kSumUsable, "one payload must fit");
-
-__global__ void __launch_bounds__(kSumWarps * 32, 1)
-hc_decode_sum_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ uint64_t s_full[kSumWarps][2];
-  __shared__ uint32_t s_tot[kSumWarps][kMaxDst];  // payload bytes of a run
-  __shared__ uint64_t s_pre[kMaxDst];
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
-  uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* const obuf = smem + warp * kSubBytes;
-  uint8_t* const ring = smem + n_warps * kSubBytes + warp * kSumRing;
-  const Workspace& ws = p.ws;
-  uint64_t* const full = s_full[warp];
-  if (lane < 2u) mbar_init(&full[lane], 1);
-  fence_mbar_init();
-  if (tid == 0) launch_dependents();
-  grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
-  __syncwarp();
-  const uint32_t Q = p.n_seg;
-  const uint32_t gw = blockIdx.x * n_warps + warp, nw = gridDim.x * n_warps;
-  const uint32_t status = *((volatile const uint32_t*)(ws.ctrl + 2));
-  HC_TL_DECL(ws.epoch);
-  if (tid == 0) {
-    HC_TL_ZERO();
-    HC_STAMP(0);
-    HC_PH_START();
-  }
-
-  // ---- shares, offsets -----------------------------------------------------------------------------------------------
-  auto run_of = [&](uint32_t w) -> uint32_t { return p.run_all * w + (w < p.run_more ? w : p.run_more); };
-  const uint32_t pool = p.pool;  // sub-tiles at the end of every run that are handed out one by one
-  uint32_t it = run_of(gw);
-  const uint32_t run_end = run_of(gw + 1u), own_end = run_end - pool;
-  // Payload bytes of the run in every stream.  Runs of up to four sub-tiles: eight lanes a stream, four streams at a time (a
-  // load per stream, its code eight times over, took 0.5 us more where all is start-up)
-  if (p.run_all + (p.run_more ? 1u : 0u) <= 4u) {
-    const uint32_t l = lane & 7u, q0 = lane >> 3, q1 = q0 + 4u;
-    uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
-    if (q0 < Q) v0 = rates16(p.seg[q0].in, p.seg[q0].in_size, it, run_end, l);
-    if (q1 < Q) v1 = rates16(p.seg[q1].in, p.seg[q1].in_size, it, run_end, l);
-    uint32_t s0 = payload_len16(v0), s1 = payload_len16(v1);  // below 2^16 each: 4 * 32 * 132 at most
-    s0 |= s1 << 16;
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    if (l == 0) {
-      s_tot[warp][q0] = s0 & 0xffffu;
-      s_tot[warp][q1] = s0 >> 16;
-    }
-  } else {
-    // Longer runs: 16 sub-tiles of four streams are asked for before the first is added (one stream after the other: eight of
-    // 40 MB 96.0 us, 92.6 this way; four of 256 MB 240.9 and 237.1; two of 128 MB 70.4 and 70.0)
-#pragma unroll 1
-    for (uint32_t q4 = 0; q4 < Q; q4 += 4u) {
-      uint32_t sum[4] = {0, 0, 0, 0};
-#pragma unroll 1
-      for (uint32_t l = lane; it * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u) {
-        uint4 v[4];
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u)
-          v[u] = q4 + u < Q ? rates16(p.seg[q4 + u].in, p.seg[q4 + u].in_size, it, run_end, l) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) sum[u] += payload_len16(v[u]);
-      }
-#pragma unroll
-      for (uint32_t u = 0; u < 4u; ++u) {
-        sum[u] = __reduce_add_sync(0xffffffffu, sum[u]);
-        if (lane == 0) s_tot[warp][q4 + u] = sum[u];  // (room for kMaxDst streams, a multiple of four)
-      }
-    }
-  }
-
-  // ---- units: a sub-tile in streams 4 half .. 4 half + 3 ------------------------------------------------------------------
-  // items: own sub-tiles, then tickets of the pools (kPool set)
-  constexpr uint32_t kPool = 0x80000000u;
-  uint32_t tk_raw = kNoTile;
-  const uint32_t n_tickets = pool * nw;
-  auto ask = [&]() {
-    if (lane == 0) tk_raw = atomicAdd(ws.tick, 1u);
-  };
-  auto next_item = [&]() -> uint32_t {
-    if (it < own_end) {
-      const uint32_t i = it++;
-      if (it == own_end && pool) ask();
-      return i;
-    }
-    if (!pool) return kNoTile;
-    const uint32_t t = __shfl_sync(0xffffffffu, tk_raw, 0);
-    if (t >= n_tickets) return kNoTile;
-    ask();
-    return t | kPool;
-  };
-  // ticket t is the (t / nw)-th pool sub-tile of warp t % nw
-  auto sub_of = [&](uint32_t item) -> uint32_t {
-    if (!(item & kPool)) return item;
-    const uint32_t w = (item & ~kPool) % nw, k = (item & ~kPool) / nw;
-    return run_of(w + 1u) - pool + k;
-  };
-  auto pool_flag = [&](uint32_t t, uint32_t q) -> uint64_t* { return p.flags + (size_t)q * pool * nw + (t & ~kPool); };
-  const uint32_t mine = lane >> 3, part = lane & 7u;  // stream of the four, blocks 4 part .. 4 part + 3
-  struct Unit {
-    uint32_t item, half;
-    uint32_t sub;
-    uint32_t rates;  // of the lane's four blocks
-    uint64_t flag;   // pool items: a look at the payload offset
-  };
-  auto look = [&](Unit& u) {
-    const uint32_t q = 4u * u.half + mine;
-    u.rates = 0;
-    u.flag = 0;
-    if (u.item == kNoTile || q >= Q) return;
-    const DecSegment& sg = p.seg[q];
-    u.rates = load_rates4(sg.in, sg.in_size, (uint64_t)u.sub * kSubBlocks + 4u * part);
-    if (u.item & kPool) u.flag = ld_relaxed_gpu_u64(pool_flag(u.item, q));
-  };
-  // (an earlier launch that timed out, and nobody has cleared its status: no output)
-  Unit next{};
-  next.item = status >= (uint32_t)kErrTimeout ? kNoTile : next_item();
-  next.sub = sub_of(next.item);
-  look(next);
-
-  __syncthreads();
-  for (uint32_t q = warp; q < Q; q += n_warps)
-    give_total_of(ws.sums + (1u + q) * kSumWords, warp_sum_u64(lane < n_warps ? s_tot[lane][q] : 0ull));
-  for (uint32_t q = warp; q < Q; q += n_warps) {
-    const uint64_t pre = take_total_of(ws.sums + (1u + q) * kSumWords, ws);
-    if (lane == 0) s_pre[q] = pre;
-  }
-  __syncthreads();
-  uint64_t own_off = 0, own_off_2 = 0;  // of the next own sub-tile's payload in the lane's stream of this half, of the other one
-  if (mine < Q) own_off = rate_bytes(p.seg[0].n) + s_pre[mine];
-  if (mine + 4u < Q) own_off_2 = rate_bytes(p.seg[0].n) + s_pre[mine + 4u];
-#pragma unroll 1
-  for (uint32_t w = 0; w < warp; ++w) {
-    own_off += s_tot[w][mine];
-    own_off_2 += s_tot[w][mine + 4u];
-  }
-
-  // ---- staging -------------------------------------------------------------------------------------------------------
-  struct Batch {
-    uint32_t rates;        // of the lane's four blocks of its stream
-    uint32_t pos;          // ring byte of their payload
-    uint32_t begin, end;   // its streams of the four
-    uint32_t sub;
-    bool first, last;      // of the sub-tile's batches
-  };
-  Batch cur{}, nxt{};
-  uint32_t staged = 0, batches = 0;
-  uint32_t live_at = 0, live_end = 0;  // ring bytes of the newest batch
-  Unit un{};
-  bool open = false;     // `un` has streams [done, many) still to be staged
-  uint32_t done = 0, many = 0;
-  uint32_t before = 0, bytes = 0;  // payload bytes of the lane's stream in front of its blocks; of the copy
-  uint64_t src = 0;                // address of its payload
-  auto stage = [&](Batch& b) -> bool {
-    if (!open) {
-      un = next;
-      many = Q - 4u * un.half < 4u ? Q - 4u * un.half : 4u;
-      done = 0;
-      open = true;
-      // the next unit's rate bytes and offsets are on their way while this one is worked on
-      if (un.half == 0u && Q > 4u) {
-        next.half = 1u;
-      } else {
-        next.half = 0u;
-        next.item = next_item();
-        if (next.item != kNoTile) next.sub = sub_of(next.item);
-      }
-      look(next);
-      const uint32_t sum = payload_len4(un.rates);
-      uint32_t inc = sum;
-#pragma unroll
-      for (int o = 1; o < 8; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o, 8);
-        if (part >= (uint32_t)o) inc += v;
-      }
-      before = inc - sum;
-      const uint32_t tot = __shfl_sync(0xffffffffu, inc, 7, 8);
-      uint64_t off = own_off;
-      if (un.item & kPool) {
-        off = un.flag;
-        const bool there = mine >= many || flag_matches(off, p.ring_epoch);
-        if (__builtin_expect(!__all_sync(0xffffffffu, there), 0)) {
-#pragma unroll 1
-          for (uint32_t s = 0; s < many; ++s) {
-            const uint64_t fw = own_flag_wait(pool_flag(un.item, 4u * un.half + s), p.ring_epoch, ws);
-            if (mine == s) off = fw;
-          }
-        }
-        off &= kFlagOffsetMask;
-      } else {
-        own_off += tot;
-      }
-      if (Q > 4u) {
-        const uint64_t v = own_off;
-        own_off = own_off_2;
-        own_off_2 = v;
-      }
-      bytes = 0;
-      if (tot) {
-        const DecSegment& sg = p.seg[4u * un.half + mine];
-        src = reinterpret_cast<uintptr_t>(sg.in) + off;
-        if (off + tot <= sg.in_size) {
-          bytes = (((uint32_t)src & 15u) + tot + 15u) & ~15u;
-        } else {  // stream shorter than its rate bytes imply (or the offset never came)
-          if (part == 0u && off != kFlagOffsetMask) note_error(ws.ctrl, kErrTruncated);
-          un.rates = 0;
-          before = 0;
-        }
-      }
-    }
-    // room: the streams that are left, or as many of them as there is room for
-    uint32_t ends = mine >= done ? bytes : 0u;
-    uint32_t v = __shfl_up_sync(0xffffffffu, ends, 8);
-    if (mine >= 1u) ends += v;
-    v = __shfl_up_sync(0xffffffffu, ends, 16);
-    if (mine >= 2u) ends += v;
-    const uint32_t all = __shfl_sync(0xffffffffu, ends, 31);
-    uint32_t at = staged ? live_end : 0u, space = kSumUsable - at;
-    if (staged && all > space && (all <= live_at || live_at > space)) {
-      at = 0;
-      space = live_at;
-    }
-    uint32_t end = many, used = all;
-    if (__builtin_expect(all > space, 0)) {
-      end = (uint32_t)(__ffs((int)__ballot_sync(0xffffffffu, ends > space)) - 1) >> 3;
-      if (end <= done) return false;  // (not with an empty ring)
-      used = __shfl_sync(0xffffffffu, ends, 8 * (int)end - 1);
-    }
-    uint64_t* const bar = &full[batches & 1u];
-    fence_proxy_async();  // what used to be in these bytes has been read
-    if (lane == 0) {
-      if (used) mbar_expect_tx(bar, used);
-      else mbar_arrive(bar);
-    }
-    __syncwarp();
-    const uint32_t start = at + ends - bytes;
-    if (part == 0u && bytes && mine >= done && mine < end)
-      bulk_load(ring + start, reinterpret_cast<const uint8_t*>(src & ~uint64_t(15)), bytes, bar);
-    live_at = at;
-    live_end = at + used;
-    ++batches;
-    b.rates = un.rates;
-    b.pos = start + ((uint32_t)src & 15u) + before;
-    b.begin = done;
-    b.end = end;
-    b.sub = un.sub;
-    b.first = un.half == 0u && done == 0u;
-    b.last = end == many && 4u * un.half + end == Q;
-    done = end;
-    open = end < many;
-    return true;
-  };
-
-  // ---- adding up -----------------------------------------------------------------------------------------------------
-  PlaneSum acc;  // of this lane's block
-  bool announced = pool == 0u;
-  if (tid == 0) HC_PH(0);
-  uint32_t landed = 0;  // batches whose payloads have landed
-  const uint32_t ahead = (1u << (8u * (lane & 3u))) - 1u;  // rate bytes of the blocks of a word in front of the lane's
-  const DecSegment& out = p.seg[0];
-  for (;;) {
-    if (staged < 2u && (open || next.item != kNoTile)) {
-      Batch b;
-      if (stage(b)) {
-        if (staged == 0u) cur = b;
-        else nxt = b;
-        ++staged;
-        continue;
-      }
-    }
-    if (!announced) {
-      // offsets of the sub-tiles of this run that others may take, counted back from its end; after the first bulk
-      // copies have been issued, so that it delays nothing
-      announced = true;
-#pragma unroll 1
-      for (uint32_t q = 0; q < Q; ++q) {
-        const DecSegment& sg = p.seg[q];
-        uint64_t off = rate_bytes(sg.n) + s_pre[q];
-        for (uint32_t w = 0; w <= warp; ++w) off += s_tot[w][q];
-#pragma unroll 1
-        for (uint32_t k = pool; k-- > 0u;) {
-          const uint64_t b = (uint64_t)(own_end + k) * kSubBlocks + lane;
-          off -= __reduce_add_sync(0xffffffffu, payload_len(b < sg.in_size ? ld_cg_u8(sg.in + b) : 0u));
-          if (lane == 0) st_relaxed_gpu_u64(pool_flag(k * nw + gw, q), flag_pack(p.ring_epoch, off));
-        }
-      }
-    }
-    if (tid == 0) HC_PH(1);
-    if (staged == 0u) break;
-    uint32_t rates = __shfl_sync(0xffffffffu, cur.rates, (int)(8u * cur.begin + (lane >> 2)));
-    uint32_t pos = __shfl_sync(0xffffffffu, cur.pos, (int)(8u * cur.begin + (lane >> 2)));
-    if (!warp_wait(&full[landed & 1u], (landed >> 1) & 1u, ws, kSiteDecodeInFull)) break;
-    ++landed;
-    if (tid == 0) HC_PH(2);
-    if (cur.first) sum_clear(acc);
-#pragma unroll 1
-    for (uint32_t s = cur.begin; s < cur.end; ++s) {
-      const uint32_t rate = rates >> (8u * (lane & 3u)) & 0xffu, at = pos + payload_len4(rates & ahead);
-      rates = __shfl_sync(0xffffffffu, cur.rates, (int)(8u * s + 8u + (lane >> 2)));  // (past the last one: unused)
-      pos = __shfl_sync(0xffffffffu, cur.pos, (int)(8u * s + 8u + (lane >> 2)));
-      sum_add(acc, ring, at, rate);
-    }
-    __syncwarp();
-    if (tid == 0) HC_PH(3);
-    if (cur.last) {
-      uint32_t w[32];
-      sum_values<1>(acc, p.scale, p.eb, w);
-      if (tid == 0) HC_PH(4);
-      const uint64_t first = (uint64_t)cur.sub * kSubValues;
-      if (lane == 0) tma_wait_group_read<0>();  // the rows of a turn ago have left the buffer
-      __syncwarp();
-      store_row_swizzled(obuf, (int)lane, w);
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0 && out.use_tma && first + kBlock <= out.n) {
-        tma_store_2d(&tmaps.m[0], 0, (int)(cur.sub * kSubBlocks), obuf);
-        tma_commit_group();
-      }
-      if (!(out.use_tma && first + kSubValues <= out.n) && first < out.n) store_rows(obuf, out, first);
-    }
-    cur = nxt;
-    --staged;
-    if (tid == 0) {
-      HC_PH(5);
-      HC_PH_COUNT();
-    }
-  }
-  // after a wait that ran out: nothing may land in shared memory once the CTA has left it
-  for (; landed < batches; ++landed) mbar_wait_bounded(&full[landed & 1u], (landed >> 1) & 1u, ws.spin_limit_ns);
-  if (lane == 0) tma_wait_group<0>();
-  if (lane == 0) HC_STAMP_MAX(7);
-  if (pool) cta_epilogue(ws.tick);
-}
-
 }  // namespace dev
 
 // ---- host side ---------------------------------------------------------------------------------------------
 
 namespace {
 
-constexpr int dec_smem(int warps) { return warps * dev::kDecWarpBytes + 1024; }
-
 template <int MODE, bool SUM>
 cudaError_t launch_flagged(const TensorMaps& maps, DecParams p, cudaStream_t stream, bool overlap) {
-  constexpr int kWarps = dev::kDecWarps;
+  const auto kernel = dev::hc_decode_step_kernel<MODE, SUM>;
+  constexpr int kWarps = dev::kDecWarps, kSmem = kWarps * dev::kDecWarpBytes + 1024;
   static thread_local int cache[64] = {};
-  const int cap = resident_ctas(dev::hc_decode_kernel<MODE, SUM>, 32 * kWarps, dec_smem(kWarps), cache);
+  const int cap = resident_ctas(kernel, 32 * kWarps, kSmem, cache);
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
   // tickets are quarters of a tile while there is a warp for each
   const uint32_t tiles = SUM ? p.tiles_per_seg : p.n_tiles;
   p.parts = tiles <= (uint32_t)cap ? 4u : 1u;
   const uint32_t ctas = p.parts == 4u ? tiles : (tiles + 3u) / 4u;
   const int grid = (int)(ctas < (uint32_t)cap ? ctas : (uint32_t)cap);
-  if (overlap) return launch_overlapped(dev::hc_decode_kernel<MODE, SUM>, grid, 32 * kWarps, dec_smem(kWarps), stream, maps, p);
-  dev::hc_decode_kernel<MODE, SUM><<<grid, 32 * kWarps, dec_smem(kWarps), stream>>>(maps, p);
+  if (overlap) return launch_overlapped(kernel, grid, 32 * kWarps, kSmem, stream, maps, p);
+  kernel<<<grid, 32 * kWarps, kSmem, stream>>>(maps, p);
   return cudaGetLastError();
 }
 
-// stand-alone: one stream (hc_decode_run_kernel) or the sum of several (hc_decode_sum_kernel)
+// stand-alone: one stream (hc_decode_run_kernel) or the sum of several (hc_decode_kernel)
 template <typename Kernel>
 cudaError_t launch_runs(Kernel kernel, int max_warps, int warp_bytes, int (&cache)[64], const TensorMaps& maps, DecParams p, cudaStream_t stream) {
   auto smem = [&](int warps) { return warps * warp_bytes + 1024; };
@@ -978,7 +674,7 @@ cudaError_t launch_run(const TensorMaps& maps, const DecParams& p, cudaStream_t 
 }
 cudaError_t launch_sum(const TensorMaps& maps, const DecParams& p, cudaStream_t stream) {
   static thread_local int cache[64] = {};
-  return launch_runs(dev::hc_decode_sum_kernel, dev::kSumWarps, dev::kSumWarpBytes, cache, maps, p, stream);
+  return launch_runs(dev::hc_decode_kernel, dev::kSumWarps, dev::kSumWarpBytes, cache, maps, p, stream);
 }
 template <int MODE>
 cudaError_t launch_one(const TensorMaps& maps, const DecParams& p, cudaStream_t stream, bool overlap) {

@@ -1,5 +1,6 @@
 // Warp- and CTA-level helpers of the codec kernels: status words, bounded waits, rate bytes -> payload offsets.
 #pragma once
+#include "hc_block.cuh"
 #include "hc_kernels.cuh"
 
 namespace hc {
@@ -224,6 +225,16 @@ __device__ __forceinline__ void give_total_of(uint64_t* sums, uint64_t total) {
 }
 __device__ __forceinline__ uint64_t take_total_of(uint64_t* sums, const Workspace& ws) {
   return gridDim.x <= kDirect ? take_total(sums, ws) : take_total_grouped(sums, ws);
+}
+
+// What the TMA unit cannot store of a sub-tile: the ragged last row (not part of the tensor map), or everything when the array is
+// not 16-byte aligned
+static __device__ __noinline__ void store_rows(const uint8_t* rows, const DecSegment& sg, uint64_t first) {
+  const uint32_t len = sg.n - first < kSubValues ? (uint32_t)(sg.n - first) : (uint32_t)kSubValues;
+#pragma unroll 1
+  for (uint32_t e = (sg.use_tma ? len / kBlock * kBlock : 0u) + (threadIdx.x & 31u); e < len; e += 32u)
+    sg.out[first + e] = as_f(lds32((swizzled_row(rows, (int)(e >> 5)) ^ ((e & 28u) << 2)) | ((e & 3u) << 2)));
+  __syncwarp();
 }
 
 // the last CTA to leave re-arms the ticket counter for the next launch (true in thread 0 of that CTA)

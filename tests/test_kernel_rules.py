@@ -74,6 +74,14 @@ def test_a_warp_that_gives_up_waits_for_its_copies(name, index, issued):
     assert re.search(r"for \(;[^;]*< %s; [^)]*\)\s*mbar_wait_bounded\(" % issued, after_the_loop)
 
 
+def test_decode_of_collective_steps_keeps_the_same_rules():
+    """It is launched overlapped too, through hc_decode.cu."""
+    code = _code("hc_decode_step.cuh")
+    assert not re.search(r'"(\\n|\\t|\s)*(bar|barrier)\.', code) and "__restrict__" not in code
+    after_the_loop = code.rsplit("HC_PH_COUNT();", 1)[1]
+    assert re.search(r"for \(; v < jobs; [^)]*\)\s*mbar_wait_bounded\(", after_the_loop)
+
+
 @pytest.mark.skipif(_build.nvcc_path() is None, reason="needs nvcc")
 @pytest.mark.parametrize("name", ["hc_encode.cu", "hc_decode.cu"])
 def test_no_spills(name, tmp_path):
