@@ -29,9 +29,11 @@ namespace dev {
 // As with one stream (below) every warp has a contiguous run of sub-tiles, and its offset in every stream.  What it stages at a time is a
 // BATCH, the payloads of one sub-tile in up to four streams, and everything that goes with one is done for the four at once: lanes
 // 8 s .. 8 s + 7 belong to stream s, each with the rate bytes of four blocks.  Staged one by one, every stream of a sub-tile cost a scan,
-// room in the ring, bounds and a barrier of its own, 300 of its 470 instructions (four streams of 256 MB 198 us, 146 this way; seven
-// of 40 MB 67.6 and 52.1; four of 4 MB 11.0 and 8.7; two of 4 KB 5.2 and 4.9).  A batch whose payloads do not all fit in the ring is
-// staged in parts.  What bounds it: instructions, at 16 warps an SM; short runs the same trips to L2 as one stream's.
+// room in the ring, bounds and a barrier of its own, 300 of its 470 instructions (four streams of 256 MB 198 us, 143 this way; seven
+// of 40 MB 67.6 and 48.1; four of 4 MB 11.0 and 8.7; two of 4 KB 5.2 and 4.9).  So are the totals of a run and the offsets of its pool,
+// which stream by stream were 5 to 8 % of seven streams of 40 MB.  A batch whose payloads do not all fit in the ring is staged in parts.
+// What bounds it: instructions, at 16 warps an SM (four streams of 256 MB: 84 us of memory traffic); short runs the same trips to L2 as
+// one stream's.
 constexpr int kSumWarps = 16;
 constexpr uint32_t kSumRing = 10240, kSumUsable = kSumRing - 160;  // (see kDecRingUsable)
 constexpr int kSumWarpBytes = kSubBytes + (int)kSumRing;
@@ -43,6 +45,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   __shared__ uint64_t s_full[kSumWarps][2];
   __shared__ uint32_t s_tot[kSumWarps][kMaxDst];  // payload bytes of a run
   __shared__ uint64_t s_pre[kMaxDst];
+  __shared__ uint64_t s_end[kSumWarps][kMaxDst];         // offset behind the payloads of a run
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* const obuf = smem + warp * kSubBytes;
@@ -69,42 +72,45 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   const uint32_t pool = p.pool;  // sub-tiles at the end of every run that are handed out one by one
   uint32_t it = run_of(gw);
   const uint32_t run_end = run_of(gw + 1u), own_end = run_end - pool;
-  // Payload bytes of the run in every stream.  Runs of up to four sub-tiles: eight lanes a stream, four streams at a time (a
-  // load per stream, its code eight times over, took 0.5 us more where all is start-up)
+  auto sum8 = [&](uint32_t v) -> uint32_t {  // over the lanes of a stream
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  // Payload bytes of the run in every stream: eight lanes a stream, 16 rate bytes a lane
+  const uint32_t mine = lane >> 3, part = lane & 7u;  // stream of the four
+  uint32_t sum = 0, sum_2 = 0;                        // of streams `mine` and 4 + `mine`
   if (p.run_all + (p.run_more ? 1u : 0u) <= 4u) {
-    const uint32_t l = lane & 7u, q0 = lane >> 3, q1 = q0 + 4u;
-    uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
-    if (q0 < Q) v0 = rates16(p.seg[q0].in, p.seg[q0].in_size, it, run_end, l);
-    if (q1 < Q) v1 = rates16(p.seg[q1].in, p.seg[q1].in_size, it, run_end, l);
-    uint32_t s0 = payload_len16(v0), s1 = payload_len16(v1);  // below 2^16 each: 4 * 32 * 132 at most
-    s0 |= s1 << 16;
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    if (l == 0) {
-      s_tot[warp][q0] = s0 & 0xffffu;
-      s_tot[warp][q1] = s0 >> 16;
-    }
+    uint4 v = make_uint4(0, 0, 0, 0), v_2 = v;
+    if (mine < Q) v = rates16(p.seg[mine].in, p.seg[mine].in_size, it, run_end, part);
+    if (mine + 4u < Q) v_2 = rates16(p.seg[mine + 4u].in, p.seg[mine + 4u].in_size, it, run_end, part);
+    sum = sum8(payload_len16(v) | payload_len16(v_2) << 16);  // below 2^16 each: 4 * 32 * 132 at most
+    sum_2 = sum >> 16;
+    sum &= 0xffffu;
   } else {
-    // Longer runs: 16 sub-tiles of four streams are asked for before the first is added (one stream after the other: eight of
-    // 40 MB 96.0 us, 92.6 this way; four of 256 MB 240.9 and 237.1; two of 128 MB 70.4 and 70.0)
+    // Longer runs: 16 sub-tiles of all streams are asked for before the first is added (one stream after the other: eight of
+    // 40 MB 96.0 us, 92.6 with four at a time)
 #pragma unroll 1
-    for (uint32_t q4 = 0; q4 < Q; q4 += 4u) {
-      uint32_t sum[4] = {0, 0, 0, 0};
-#pragma unroll 1
-      for (uint32_t l = lane; it * kSubBlocks + 16u * l < run_end * kSubBlocks; l += 32u) {
-        uint4 v[4];
+    for (uint32_t at = it; at < run_end; at += 16u) {
+      uint4 v[8];
 #pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u)
-          v[u] = q4 + u < Q ? rates16(p.seg[q4 + u].in, p.seg[q4 + u].in_size, it, run_end, l) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (uint32_t u = 0; u < 4u; ++u) sum[u] += payload_len16(v[u]);
+      for (uint32_t j = 0; j < 8u; ++j) {
+        const uint32_t q = mine + 4u * (j & 1u), first = at + 4u * (j >> 1);
+        v[j] = q < Q && first < run_end ? rates16(p.seg[q].in, p.seg[q].in_size, first, run_end, part) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
-      for (uint32_t u = 0; u < 4u; ++u) {
-        sum[u] = __reduce_add_sync(0xffffffffu, sum[u]);
-        if (lane == 0) s_tot[warp][q4 + u] = sum[u];  // (room for kMaxDst streams, a multiple of four)
+      for (uint32_t j = 0; j < 4u; ++j) {
+        if (at + 4u * j >= run_end) break;
+        sum += payload_len16(v[2u * j]);
+        if (Q > 4u) sum_2 += payload_len16(v[2u * j + 1u]);
       }
     }
+    sum = sum8(sum);
+    if (Q > 4u) sum_2 = sum8(sum_2);
+  }
+  if (part == 0u) {
+    s_tot[warp][mine] = sum;
+    s_tot[warp][mine + 4u] = sum_2;
   }
 
   // ---- units: a sub-tile in streams 4 half .. 4 half + 3 ------------------------------------------------------------------
@@ -134,7 +140,6 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     return run_of(w + 1u) - pool + k;
   };
   auto pool_flag = [&](uint32_t t, uint32_t q) -> uint64_t* { return p.flags + (size_t)q * pool * nw + (t & ~kPool); };
-  const uint32_t mine = lane >> 3, part = lane & 7u;  // stream of the four, blocks 4 part .. 4 part + 3
   struct Unit {
     uint32_t item, half;
     uint32_t sub;
@@ -146,8 +151,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     u.rates = 0;
     u.flag = 0;
     if (u.item == kNoTile || q >= Q) return;
-    const DecSegment& sg = p.seg[q];
-    u.rates = load_rates4(sg.in, sg.in_size, (uint64_t)u.sub * kSubBlocks + 4u * part);
+    u.rates = load_rates4(p.seg[q].in, p.seg[q].in_size, (uint64_t)u.sub * kSubBlocks + 4u * part);
     if (u.item & kPool) u.flag = ld_relaxed_gpu_u64(pool_flag(u.item, q));
   };
   // (an earlier launch that timed out, and nobody has cleared its status: no output)
@@ -164,14 +168,17 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     if (lane == 0) s_pre[q] = pre;
   }
   __syncthreads();
-  uint64_t own_off = 0, own_off_2 = 0;  // of the next own sub-tile's payload in the lane's stream of this half, of the other one
-  if (mine < Q) own_off = rate_bytes(p.seg[0].n) + s_pre[mine];
-  if (mine + 4u < Q) own_off_2 = rate_bytes(p.seg[0].n) + s_pre[mine + 4u];
-#pragma unroll 1
-  for (uint32_t w = 0; w < warp; ++w) {
-    own_off += s_tot[w][mine];
-    own_off_2 += s_tot[w][mine + 4u];
+  // offset of the next own sub-tile's payload in the lane's stream of this half, of the other one
+  auto before_me = [&](uint32_t q) -> uint64_t {
+    const uint32_t v = (part < warp ? s_tot[part][q] : 0u) + (part + 8u < warp ? s_tot[part + 8u][q] : 0u);
+    return rate_bytes(p.seg[0].n) + (q < Q ? s_pre[q] : 0u) + sum8(v);
+  };
+  uint64_t own_off = before_me(mine), own_off_2 = Q > 4u ? before_me(mine + 4u) : 0u;
+  if (pool && part == 0u) {
+    s_end[warp][mine] = own_off + sum;
+    s_end[warp][mine + 4u] = own_off_2 + sum_2;
   }
+  __syncwarp();
 
   // ---- staging -------------------------------------------------------------------------------------------------------
   struct Batch {
@@ -311,15 +318,13 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
       // copies have been issued, so that it delays nothing
       announced = true;
 #pragma unroll 1
-      for (uint32_t q = 0; q < Q; ++q) {
-        const DecSegment& sg = p.seg[q];
-        uint64_t off = rate_bytes(sg.n) + s_pre[q];
-        for (uint32_t w = 0; w <= warp; ++w) off += s_tot[w][q];
-#pragma unroll 1
+      for (uint32_t q = mine; q - mine < Q; q += 4u) {
+        uint64_t off = s_end[warp][q];
+#pragma unroll 2
         for (uint32_t k = pool; k-- > 0u;) {
-          const uint64_t b = (uint64_t)(own_end + k) * kSubBlocks + lane;
-          off -= __reduce_add_sync(0xffffffffu, payload_len(b < sg.in_size ? ld_cg_u8(sg.in + b) : 0u));
-          if (lane == 0) st_relaxed_gpu_u64(pool_flag(k * nw + gw, q), flag_pack(p.ring_epoch, off));
+          const uint32_t r4 = q < Q ? load_rates4(p.seg[q].in, p.seg[q].in_size, (uint64_t)(own_end + k) * kSubBlocks + 4u * part) : 0u;
+          off -= sum8(payload_len4(r4));
+          if (part == 0u && q < Q) st_relaxed_gpu_u64(pool_flag(k * nw + gw, q), flag_pack(p.ring_epoch, off));
         }
       }
     }
