@@ -353,21 +353,46 @@ __device__ __forceinline__ void sum_clear(PlaneSum& s) {
   for (int j = 0; j < kNarrow; ++j) s.A[j] = 0;
   s.apart = s.bound = 0;
 }
-// planes 8 B .. 8 B + 7 of a block (zero at and above F); word: the one that plane 8 B begins in
+// Which of the first 16 planes a block of F planes has: all ones or zero for each, a row of 16 words for every F.  Comparing and
+// selecting takes two operations a plane of the pipe that bounds the sums; with a mask from shared memory, the selection and the
+// exclusive or with the sign are one.  Unit c of row F (four masks) stands at unit c ^ (F / 2 % 4), so that eight neighbouring F
+// have no banks in common.
+constexpr int kMaskWords = 17 * 16;
+__device__ __forceinline__ void fill_masks(uint32_t* masks) {
+  for (uint32_t i = threadIdx.x; i < (uint32_t)kMaskWords; i += blockDim.x) {
+    const uint32_t F = i >> 4, j = ((i >> 2 & 3u) ^ (F >> 1 & 3u)) << 2 | (i & 3u);
+    masks[i] = j < F ? 0xffffffffu : 0u;
+  }
+}
+// (t & m) ^ s
+__device__ __forceinline__ uint32_t and_xor(uint32_t t, uint32_t m, uint32_t s) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(d) : "r"(t), "r"(m), "r"(s));
+  return d;
+}
+// planes 8 B .. 8 B + 7 of a block (zero at and above F), exclusive or sign; word: the one that plane 8 B begins in; row: masks of F
 template <int B>
-__device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F, uint32_t& word, uint32_t (&T)[32]) {
-  uint32_t w[8];
+__device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F, uint32_t row, uint32_t sign, uint32_t& word, uint32_t (&X)[32]) {
+  uint32_t w[8], m[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) w[j] = lds32(wp + 4 * (8 * B + 2 + j));
+  if (B < 2) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(m[4 * c]), "=r"(m[4 * c + 1]), "=r"(m[4 * c + 2]), "=r"(m[4 * c + 3])
+                   : "r"(row ^ (uint32_t)((2 * B + c) << 4))
+                   : "memory");
+  }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const uint32_t x = __funnelshift_r(j ? w[j - 1] : word, w[j], sh);
-    T[8 * B + j] = (uint32_t)(8 * B + j) < F ? x : 0u;
+    X[8 * B + j] = B < 2 ? and_xor(x, m[j], sign) : ((uint32_t)(8 * B + j) < F ? x : 0u) ^ sign;
   }
   word = w[7];
 }
-// Adds a staged payload (see read_planes).
-__device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, uint32_t pos, uint32_t rate) {
+// Adds a staged payload (see read_planes); masks: see fill_masks.
+__device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, const uint32_t* masks, uint32_t pos, uint32_t rate) {
   const uint32_t F = rate & 31u, W = __reduce_max_sync(0xffffffffu, F);
   uint32_t p2 = pos, a0 = 0;
   if (__any_sync(0xffffffffu, rate & 0x80u)) {
@@ -379,14 +404,15 @@ __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, uint32_
     }
   }
   const uint32_t sh = 8u * (p2 & 3u), wp = smem_u32(buf) + (p2 & ~3u);
-  uint32_t T[32], word0 = lds32(wp), word = lds32(wp + 4u);
+  const uint32_t Fm = F < 16u ? F : 16u, row = (smem_u32(masks) + 64u * Fm) | (8u * Fm & 0x30u);
+  uint32_t X[32], word0 = lds32(wp), word = lds32(wp + 4u);
   const uint32_t sign = __funnelshift_r(word0, word, sh);
-  read_eight<0>(wp, sh, F, word, T);
+  read_eight<0>(wp, sh, F, row, sign, word, X);
   if (W > 8u) {
-    read_eight<1>(wp, sh, F, word, T);
+    read_eight<1>(wp, sh, F, row, sign, word, X);
   } else {
 #pragma unroll
-    for (int j = 8; j < 16; ++j) T[j] = 0;
+    for (int j = 8; j < 16; ++j) X[j] = sign;
   }
   s.apart += sign & kFirst ? 0u - a0 : a0;
   const bool was_wide = sum_wide(s);
@@ -397,15 +423,15 @@ __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, uint32_
       for (int j = kNarrow; j < 32; ++j) s.A[j] = s.A[kNarrow - 1];
     }
     if (W > 16u) {
-      read_eight<2>(wp, sh, F, word, T);
-      read_eight<3>(wp, sh, F, word, T);
+      read_eight<2>(wp, sh, F, row, sign, word, X);
+      read_eight<3>(wp, sh, F, row, sign, word, X);
     } else {
 #pragma unroll
-      for (int j = 16; j < 32; ++j) T[j] = 0;
+      for (int j = 16; j < 32; ++j) X[j] = sign;
     }
-    add_planes<32, 32>(s.A, T, sign);
+    add_planes<32, 32>(s.A, X, sign);
   } else {
-    add_planes<16, kNarrow>(s.A, T, sign);
+    add_planes<16, kNarrow>(s.A, X, sign);
   }
 }
 // Sum -> values (float bits).  In planes the sum of k streams costs k additions and one transposition.  The rows come out with B

@@ -45,7 +45,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   __shared__ uint64_t s_full[kSumWarps][2];
   __shared__ uint32_t s_tot[kSumWarps][kMaxDst];  // payload bytes of a run
   __shared__ uint64_t s_pre[kMaxDst];
-  __shared__ uint64_t s_end[kSumWarps][kMaxDst];         // offset behind the payloads of a run
+  __shared__ __align__(64) uint32_t masks[kMaskWords];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* const obuf = smem + warp * kSubBytes;
@@ -55,6 +55,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   if (lane < 2u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
+  fill_masks(masks);
   grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   __syncwarp();
   const uint32_t Q = p.n_seg;
@@ -174,11 +175,6 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     return rate_bytes(p.seg[0].n) + (q < Q ? s_pre[q] : 0u) + sum8(v);
   };
   uint64_t own_off = before_me(mine), own_off_2 = Q > 4u ? before_me(mine + 4u) : 0u;
-  if (pool && part == 0u) {
-    s_end[warp][mine] = own_off + sum;
-    s_end[warp][mine + 4u] = own_off_2 + sum_2;
-  }
-  __syncwarp();
 
   // ---- staging -------------------------------------------------------------------------------------------------------
   struct Batch {
@@ -319,7 +315,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
       announced = true;
 #pragma unroll 1
       for (uint32_t q = mine; q - mine < Q; q += 4u) {
-        uint64_t off = s_end[warp][q];
+        uint64_t off = before_me(q) + s_tot[warp][q];
 #pragma unroll 2
         for (uint32_t k = pool; k-- > 0u;) {
           const uint32_t r4 = q < Q ? load_rates4(p.seg[q].in, p.seg[q].in_size, (uint64_t)(own_end + k) * kSubBlocks + 4u * part) : 0u;
@@ -341,7 +337,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
       const uint32_t rate = rates >> (8u * (lane & 3u)) & 0xffu, at = pos + payload_len4(rates & ahead);
       rates = __shfl_sync(0xffffffffu, cur.rates, (int)(8u * s + 8u + (lane >> 2)));  // (past the last one: unused)
       pos = __shfl_sync(0xffffffffu, cur.pos, (int)(8u * s + 8u + (lane >> 2)));
-      sum_add(acc, ring, at, rate);
+      sum_add(acc, ring, masks, at, rate);
     }
     __syncwarp();
     if (tid == 0) HC_PH(3);

@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, SUM ? 4 : 5)
 hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t s_full[kDecWarps][4];
+  __shared__ __align__(64) uint32_t masks[SUM ? kMaskWords : 4];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* const obuf = smem + warp * kSubBytes;
@@ -36,6 +37,10 @@ hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   if (lane < 4u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
+  if (SUM) {
+    fill_masks(masks);
+    __syncthreads();
+  }
   __syncwarp();
 
   const uint32_t Q = SUM ? p.n_seg : 1u;  // streams per sub-tile
@@ -239,7 +244,7 @@ hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     uint32_t w[32];
     if (SUM) {
       if (cur.seg == 0) sum_clear(acc);
-      sum_add(acc, ring, cur.pos, cur.rate);
+      sum_add(acc, ring, masks, cur.pos, cur.rate);
       __syncwarp();
       if (threadIdx.x == 0) HC_PH(3);
       last = cur.seg + 1 == Q;

@@ -227,14 +227,14 @@ HC_HD uint32_t majority(uint32_t a, uint32_t b, uint32_t c) {
   return (a & b) | (c & (a | b));
 #endif
 }
-// A += the integers with magnitude planes T[0 .. W-1] and sign map `sign`, modulo 2^N
+// A += the integers with magnitude planes X[0 .. W-1] ^ sign and sign map `sign`, modulo 2^N
 template <int W, int N>
-HC_HD void add_planes(uint32_t (&A)[32], const uint32_t (&T)[32], uint32_t sign) {
+HC_HD void add_planes(uint32_t (&A)[32], const uint32_t (&X)[32], uint32_t sign) {
   static_assert(W <= N && N <= 32, "planes");
   uint32_t c = sign;  // -m = ~m + 1
 #pragma unroll
   for (int j = 0; j < N; ++j) {
-    const uint32_t x = j < W ? T[j] ^ sign : sign, a = A[j];
+    const uint32_t x = j < W ? X[j] : sign, a = A[j];
     A[j] = xor3(a, x, c);
     if (j + 1 < N) c = majority(a, x, c);
   }
