@@ -119,14 +119,43 @@ __device__ __forceinline__ uint32_t payload_len4(uint32_t r4) {
   return 4u * __dp4a(F, 0x01010101u, 0u) + 4u * __popc(live) + __popc(outl) + __dp4a(extra, 0x01010101u, 0u);
 }
 
+// Which of the first 16 planes a block of F planes has: all ones or zero for each, a row of 16 words for every F.  Comparing and
+// selecting takes two operations a plane of the half-rate pipe; with a mask from shared memory it is one, in sums together with the
+// exclusive or with the sign (decode of 64 MB 22.5 us, 21.2 this way, of 256 MB 61.8 and 60.9; four streams of 256 MB added 143.5 and
+// 138.8; the decode of an allreduce step of 64 MB at 8 ranks 33.1 and 32.0).  Not in the add of one stream and fp32: of 64 MB 38.6 us,
+// 38.4 with masks, but of 4 MB 7.7 and 7.8, for the time that the rows take at the start.  Unit c of row F (four masks) stands at unit c ^ (F / 2 % 4), so that eight neighbouring F
+// have no banks in common.
+constexpr int kMaskWords = 17 * 16;
+__device__ __forceinline__ void fill_masks(uint32_t* masks) {
+  for (uint32_t i = threadIdx.x; i < (uint32_t)kMaskWords; i += blockDim.x) {
+    const uint32_t F = i >> 4, j = ((i >> 2 & 3u) ^ (F >> 1 & 3u)) << 2 | (i & 3u);
+    masks[i] = j < F ? 0xffffffffu : 0u;
+  }
+}
+// (t & m) ^ s
+__device__ __forceinline__ uint32_t and_xor(uint32_t t, uint32_t m, uint32_t s) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(d) : "r"(t), "r"(m), "r"(s));
+  return d;
+}
+// four masks of the row at `row`, from plane 4 C on
+template <int C>
+__device__ __forceinline__ void four_masks(uint32_t row, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(row ^ (uint32_t)(C << 4)) : "memory");
+}
+__device__ __forceinline__ uint32_t mask_row(const uint32_t* masks, uint32_t F) {
+  const uint32_t f = F < 16u ? F : 16u;
+  return (smem_u32(masks) + 64u * f) | (8u * f & 0x30u);
+}
+
 // ---- stream -> block --------------------------------------------------------------------------------
 // Reads the payload of the block with rate byte `rate` at byte `pos` of a staged stream: planes into T[0..W-1]
 // (zero at and above F), the sign map in the planes' bit order, |d0| of an outlier block (else 0).  Every
 // word is rebuilt from two neighbours by a funnel shift, whatever the block's alignment: with outlier blocks
 // about, the lanes of a warp have all four alignments, and a second path for aligned blocks ran on top.
 // Blocks without payload give zeros; up to 4 W + 8 bytes behind the payload are read (and ignored).
-template <int W>
-__device__ __forceinline__ void read_planes(const uint8_t* buf, uint32_t pos, uint32_t rate, bool any_outlier,
+template <int W, bool MASKS>
+__device__ __forceinline__ void read_planes(const uint8_t* buf, const uint32_t* masks, uint32_t pos, uint32_t rate, bool any_outlier,
                                             uint32_t& sign, uint32_t& a0, uint32_t (&T)[32]) {
   const uint32_t F = rate & 31u;
   uint32_t p2 = pos;
@@ -145,10 +174,18 @@ __device__ __forceinline__ void read_planes(const uint8_t* buf, uint32_t pos, ui
 #pragma unroll
   for (int j = 0; j < W + 2; ++j) word[j] = lds32(wp + 4 * j);
   sign = __funnelshift_r(word[0], word[1], sh);
+  uint32_t m[16];
+  if (MASKS && W <= 16) {
+    const uint32_t row = mask_row(masks, F);
+    if (W > 0) four_masks<0>(row, m[0], m[1], m[2], m[3]);
+    if (W > 4) four_masks<1>(row, m[4], m[5], m[6], m[7]);
+    if (W > 8) four_masks<2>(row, m[8], m[9], m[10], m[11]);
+    if (W > 12) four_masks<3>(row, m[12], m[13], m[14], m[15]);
+  }
 #pragma unroll
   for (int j = 1; j <= W; ++j) {
     const uint32_t x = __funnelshift_r(word[j], word[j + 1], sh);
-    T[j - 1] = (uint32_t)j <= F ? x : 0u;
+    T[j - 1] = MASKS && W <= 16 ? x & m[(j - 1) & 15] : (uint32_t)j <= F ? x : 0u;
   }
 }
 
@@ -172,15 +209,17 @@ __device__ __forceinline__ void rows_of_block(uint32_t (&T)[32], uint32_t rate, 
 // staged payload -> rows, sign map with element i at bit 31 - i; W (plane_width of the largest F of the warp) is warp-uniform.  The widths that data at the usual error
 // bounds has come first and in line, so that the loop's instructions lie together (as a switch, with the longest
 // variants in between: add of 64 MB 41.7 us, 40.3 this way; decode of 64 MB 22.4, 21.6)
-__device__ __forceinline__ void decode_rows(const uint8_t* buf, uint32_t pos, uint32_t rate, int W, uint32_t& sign,
+// MASKS: see fill_masks
+template <bool MASKS>
+__device__ __forceinline__ void decode_rows(const uint8_t* buf, const uint32_t* masks, uint32_t pos, uint32_t rate, int W, uint32_t& sign,
                                             uint32_t& a0, uint32_t (&T)[32]) {
   const bool outl = __any_sync(0xffffffffu, rate & 0x80u);
-  if (__builtin_expect(W == 12, 1)) { read_planes<12>(buf, pos, rate, outl, sign, a0, T); rows_of_block<12>(T, rate, a0); }
-  else if (__builtin_expect(W == 8, 1)) { read_planes<8>(buf, pos, rate, outl, sign, a0, T); rows_of_block<8>(T, rate, a0); }
-  else if (__builtin_expect(W == 16, 1)) { read_planes<16>(buf, pos, rate, outl, sign, a0, T); rows_of_block<16>(T, rate, a0); }
-  else if (W == 4) { read_planes<4>(buf, pos, rate, outl, sign, a0, T); rows_of_block<4>(T, rate, a0); }
-  else if (__builtin_expect(W == 0, 0)) { read_planes<0>(buf, pos, rate, outl, sign, a0, T); rows_of_block<0>(T, rate, a0); }
-  else { read_planes<32>(buf, pos, rate, outl, sign, a0, T); rows_of_block<32>(T, rate, a0); }
+  if (__builtin_expect(W == 12, 1)) { read_planes<12, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<12>(T, rate, a0); }
+  else if (__builtin_expect(W == 8, 1)) { read_planes<8, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<8>(T, rate, a0); }
+  else if (__builtin_expect(W == 16, 1)) { read_planes<16, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<16>(T, rate, a0); }
+  else if (W == 4) { read_planes<4, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<4>(T, rate, a0); }
+  else if (__builtin_expect(W == 0, 0)) { read_planes<0, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<0>(T, rate, a0); }
+  else { read_planes<32, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<32>(T, rate, a0); }
   sign = swap_order(sign);
 }
 
@@ -353,23 +392,6 @@ __device__ __forceinline__ void sum_clear(PlaneSum& s) {
   for (int j = 0; j < kNarrow; ++j) s.A[j] = 0;
   s.apart = s.bound = 0;
 }
-// Which of the first 16 planes a block of F planes has: all ones or zero for each, a row of 16 words for every F.  Comparing and
-// selecting takes two operations a plane of the pipe that bounds the sums; with a mask from shared memory, the selection and the
-// exclusive or with the sign are one.  Unit c of row F (four masks) stands at unit c ^ (F / 2 % 4), so that eight neighbouring F
-// have no banks in common.
-constexpr int kMaskWords = 17 * 16;
-__device__ __forceinline__ void fill_masks(uint32_t* masks) {
-  for (uint32_t i = threadIdx.x; i < (uint32_t)kMaskWords; i += blockDim.x) {
-    const uint32_t F = i >> 4, j = ((i >> 2 & 3u) ^ (F >> 1 & 3u)) << 2 | (i & 3u);
-    masks[i] = j < F ? 0xffffffffu : 0u;
-  }
-}
-// (t & m) ^ s
-__device__ __forceinline__ uint32_t and_xor(uint32_t t, uint32_t m, uint32_t s) {
-  uint32_t d;
-  asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(d) : "r"(t), "r"(m), "r"(s));
-  return d;
-}
 // planes 8 B .. 8 B + 7 of a block (zero at and above F), exclusive or sign; word: the one that plane 8 B begins in; row: masks of F
 template <int B>
 __device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F, uint32_t row, uint32_t sign, uint32_t& word, uint32_t (&X)[32]) {
@@ -377,12 +399,8 @@ __device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F,
 #pragma unroll
   for (int j = 0; j < 8; ++j) w[j] = lds32(wp + 4 * (8 * B + 2 + j));
   if (B < 2) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                   : "=r"(m[4 * c]), "=r"(m[4 * c + 1]), "=r"(m[4 * c + 2]), "=r"(m[4 * c + 3])
-                   : "r"(row ^ (uint32_t)((2 * B + c) << 4))
-                   : "memory");
+    four_masks<2 * B>(row, m[0], m[1], m[2], m[3]);
+    four_masks<2 * B + 1>(row, m[4], m[5], m[6], m[7]);
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -404,7 +422,7 @@ __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, const u
     }
   }
   const uint32_t sh = 8u * (p2 & 3u), wp = smem_u32(buf) + (p2 & ~3u);
-  const uint32_t Fm = F < 16u ? F : 16u, row = (smem_u32(masks) + 64u * Fm) | (8u * Fm & 0x30u);
+  const uint32_t row = mask_row(masks, F);
   uint32_t X[32], word0 = lds32(wp), word = lds32(wp + 4u);
   const uint32_t sign = __funnelshift_r(word0, word, sh);
   read_eight<0>(wp, sh, F, row, sign, word, X);

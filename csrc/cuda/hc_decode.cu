@@ -10,8 +10,8 @@
 // look-back, no second kernel.  The SMs do not run at the same pace (with equal static shares the first warp of a 256 MB launch
 // finished at 42 us, the last at 70), so the last eighth of every run goes to whoever is free first; the payload
 // offsets of those sub-tiles are written to the workspace after the first one has been decoded.
-// What bounds the decode of one stream: 256 MB the memory (62.1 us; 61.9 with the arithmetic left out, 50.4 without the stores), 64 MB
-// the memory and the start (22.8; 20.8, 19.0), smaller ones the way to the first payload: rate bytes, exchange, payload, one trip to
+// What bounds the decode of one stream: 256 MB the memory (60.9 us), 64 MB the memory and the start (21.2; before the masks 22.8, with
+// 20.8 without the arithmetic and 19.0 without the stores), smaller ones the way to the first payload: rate bytes, exchange, payload, one trip to
 // L2 after the other (8 MB: of 6.1 us on the device 3.3; 5.1 of 7.5 when 64-bit divisions, the status and the offsets of the pool
 // stood in between).
 //
@@ -389,6 +389,7 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t s_full[kRunWarps][4];
   __shared__ uint32_t s_tot[kRunWarps];
+  __shared__ __align__(64) uint32_t masks[kMaskWords];
   __shared__ uint64_t s_pre;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -399,6 +400,7 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
   if (lane < 4u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
+  fill_masks(masks);
   grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   __syncwarp();
   const DecSegment& sg = p.seg[0];
@@ -549,7 +551,7 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
     uint32_t pos = at % kRing + inc - len;
     if (pos >= kRing) pos -= kRing;
     uint32_t T[32], sign, a0;
-    decode_rows(ring, pos, rate, plane_width(__reduce_max_sync(0xffffffffu, rate & 31u)), sign, a0, T);
+    decode_rows<true>(ring, masks, pos, rate, plane_width(__reduce_max_sync(0xffffffffu, rate & 31u)), sign, a0, T);
     const bool little = (rate & 31u) <= 16u && a0 < (1u << 23);
     const uint32_t cur = sub;
     __syncwarp();

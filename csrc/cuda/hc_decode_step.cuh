@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, SUM ? 4 : 5)
 hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t s_full[kDecWarps][4];
-  __shared__ __align__(64) uint32_t masks[SUM ? kMaskWords : 4];
+  __shared__ __align__(64) uint32_t masks[kMaskWords];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* const obuf = smem + warp * kSubBytes;
@@ -37,11 +37,8 @@ hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   if (lane < 4u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
-  if (SUM) {
-    fill_masks(masks);
-    __syncthreads();
-  }
-  __syncwarp();
+  fill_masks(masks);
+  __syncthreads();
 
   const uint32_t Q = SUM ? p.n_seg : 1u;  // streams per sub-tile
   const uint32_t gw = blockIdx.x * n_warps + warp, nw = gridDim.x * n_warps;
@@ -252,7 +249,7 @@ hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     } else {
       const int W = plane_width(__reduce_max_sync(0xffffffffu, cur.rate & 31u));
       uint32_t T[32], sign, a0;
-      decode_rows(ring, cur.pos, cur.rate, W, sign, a0, T);
+      decode_rows<true>(ring, masks, cur.pos, cur.rate, W, sign, a0, T);
       __syncwarp();
       if (threadIdx.x == 0) HC_PH(3);
       // ---- signs, prefix sum, scaling ------------------------------------------------------------------------------
