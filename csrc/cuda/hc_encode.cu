@@ -33,12 +33,15 @@ constexpr int kEncWarps = 23;
 __host__ __device__ constexpr int enc_warps(int op) { return op == kOpCompress ? kEncWarps : 15; }
 // packed payloads: a payload of 4096 bytes, 4 bytes pack_block adds, 16 copy_ring looks ahead
 __host__ __device__ constexpr int enc_out_ring(int op) { return op == kOpCompress ? 5376 : 5120; }
-// incoming payloads: see hc_decode.cu
-__host__ __device__ constexpr int enc_in_ring(int op) { return op == kOpCompress ? 0 : 4864; }
-__host__ __device__ constexpr int enc_warp_bytes(int op) { return kSubBytes + enc_out_ring(op) + enc_in_ring(op); }
-constexpr int kInUsable = 4864 - 160;
+// rows of the local operand, which stream + stream has not: it takes their room for payloads, so that two of up to 4.4 KB are on
+// their way (a random walk, 3.3 KB each: 64 MB 53.9 us, 52.4 this way, 16 MB 20.2 and 19.9; payloads of 1 KB no change)
+__host__ __device__ constexpr int enc_stage(int op) { return op == kOpAddStream ? 0 : kSubBytes; }
+// incoming payloads, and in front of the ring's end what read_planes may look at behind one
+__host__ __device__ constexpr int enc_in_ring(int op) { return op == kOpCompress ? 0 : op == kOpAddStream ? 4864 + kSubBytes : 4864; }
+__host__ __device__ constexpr int enc_in_usable(int op) { return enc_in_ring(op) - 160; }
+__host__ __device__ constexpr int enc_warp_bytes(int op) { return enc_stage(op) + enc_out_ring(op) + enc_in_ring(op); }
 static_assert(kEncWarps * 4096 < (1 << 24), "EncShared::sum");
-static_assert(32 * 132 + 32 <= kInUsable, "one payload must fit");
+static_assert(32 * 132 + 32 <= enc_in_usable(kOpAddF32), "one payload must fit");
 
 struct EncShared {
   uint64_t stage_full[kEncWarps];
@@ -280,9 +283,9 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   }
 
   // ============================================ compute warps ==========================================================
-  uint8_t* const stage = smem + warp * kSubBytes;
-  uint8_t* const inring = smem + nc * kSubBytes + warp * enc_in_ring(OP);
-  const uint32_t oring = smem_u32(smem + nc * (kSubBytes + enc_in_ring(OP)) + warp * enc_out_ring(OP));
+  uint8_t* const stage = smem + warp * enc_stage(OP);
+  uint8_t* const inring = smem + nc * enc_stage(OP) + warp * enc_in_ring(OP);
+  const uint32_t oring = smem_u32(smem + nc * (enc_stage(OP) + enc_in_ring(OP)) + warp * enc_out_ring(OP));
   constexpr uint32_t kOutBytes = (uint32_t)enc_out_ring(OP);
   struct Where {
     uint32_t seg, sub;  // segment, sub-tile inside it
@@ -328,9 +331,9 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     const uint32_t inc = warp_inclusive_scan(len, (int)lane);
     uint32_t tot = __shfl_sync(0xffffffffu, inc, 31), rate = praw;
     uint32_t at = staged ? live_end : 0u;
-    if (tot && at + tot + 31u > (uint32_t)kInUsable) {
+    if (tot && at + tot + 31u > (uint32_t)enc_in_usable(OP)) {
       at = 0;
-      if (tot + 31u > (staged ? live_at : (uint32_t)kInUsable)) return;
+      if (tot + 31u > (staged ? live_at : (uint32_t)enc_in_usable(OP))) return;
     }
     const uint64_t off = sh.in_at[pk % kInSlots][pq][warp];
     if (tot && off + tot > p.in_size[pq]) {  // stream shorter than its rate bytes imply
