@@ -119,17 +119,26 @@ __device__ __forceinline__ uint32_t payload_len4(uint32_t r4) {
   return 4u * __dp4a(F, 0x01010101u, 0u) + 4u * __popc(live) + __popc(outl) + __dp4a(extra, 0x01010101u, 0u);
 }
 
+// element 0 of a block in the order of the stream's words
+constexpr uint32_t kFirst = 0x80u;
+
 // Which of the first 16 planes a block of F planes has: all ones or zero for each, a row of 16 words for every F.  Comparing and
 // selecting takes two operations a plane of the half-rate pipe; with a mask from shared memory it is one, in sums together with the
 // exclusive or with the sign (decode of 64 MB 22.5 us, 21.2 this way, of 256 MB 61.8 and 60.9; four streams of 256 MB added 143.5 and
 // 138.8; the decode of an allreduce step of 64 MB at 8 ranks 33.1 and 32.0).  Not in the add of one stream and fp32: of 64 MB 38.6 us,
-// 38.4 with masks, but of 4 MB 7.7 and 7.8, for the time that the rows take at the start.  Unit c of row F (four masks) stands at unit c ^ (F / 2 % 4), so that eight neighbouring F
-// have no banks in common.
-constexpr int kMaskWords = 17 * 16;
+// 38.4 with masks, but of 4 MB 7.7 and 7.8, for the time that the rows take at the start.  Rows lie 20 words apart, so that eight
+// neighbouring ones have no banks in common and a row's four loads are one address.
+// Sums have a second set of rows, kOutlierRows further on, for outlier blocks: whatever such a block's planes hold for element 0 does
+// not count (four streams of 256 MB 138.4 us without them, 140.3 with; from 17 to 21 rows apart they take the same).
+constexpr int kMaskRows = 17, kOutlierRows = 17, kSumMaskRows = kOutlierRows + kMaskRows, kMaskPitch = 20;
+template <int ROWS>
 __device__ __forceinline__ void fill_masks(uint32_t* masks) {
-  for (uint32_t i = threadIdx.x; i < (uint32_t)kMaskWords; i += blockDim.x) {
-    const uint32_t F = i >> 4, j = ((i >> 2 & 3u) ^ (F >> 1 & 3u)) << 2 | (i & 3u);
-    masks[i] = j < F ? 0xffffffffu : 0u;
+  for (uint32_t i = threadIdx.x; i < 4u * ROWS; i += blockDim.x) {
+    const int row = (int)(i >> 2), j = 4 * (int)(i & 3u);
+    const int F = row < kOutlierRows ? row : row - kOutlierRows;
+    const uint32_t all = row < kOutlierRows ? 0xffffffffu : ~kFirst;
+    *reinterpret_cast<uint4*>(masks + kMaskPitch * row + j) =
+        make_uint4(F > j ? all : 0u, F > j + 1 ? all : 0u, F > j + 2 ? all : 0u, F > j + 3 ? all : 0u);
   }
 }
 // (t & m) ^ s
@@ -141,12 +150,9 @@ __device__ __forceinline__ uint32_t and_xor(uint32_t t, uint32_t m, uint32_t s) 
 // four masks of the row at `row`, from plane 4 C on
 template <int C>
 __device__ __forceinline__ void four_masks(uint32_t row, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(row ^ (uint32_t)(C << 4)) : "memory");
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4 + %5];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(row), "n"(16 * C) : "memory");
 }
-__device__ __forceinline__ uint32_t mask_row(const uint32_t* masks, uint32_t F) {
-  const uint32_t f = F < 16u ? F : 16u;
-  return (smem_u32(masks) + 64u * f) | (8u * f & 0x30u);
-}
+__device__ __forceinline__ uint32_t mask_row(const uint32_t* masks, uint32_t row) { return smem_u32(masks) + 4u * kMaskPitch * row; }
 
 // ---- stream -> block --------------------------------------------------------------------------------
 // Reads the payload of the block with rate byte `rate` at byte `pos` of a staged stream: planes into T[0..W-1]
@@ -176,7 +182,7 @@ __device__ __forceinline__ void read_planes(const uint8_t* buf, const uint32_t* 
   sign = __funnelshift_r(word[0], word[1], sh);
   uint32_t m[16];
   if (MASKS && W <= 16) {
-    const uint32_t row = mask_row(masks, F);
+    const uint32_t row = mask_row(masks, F < 16u ? F : 16u);
     if (W > 0) four_masks<0>(row, m[0], m[1], m[2], m[3]);
     if (W > 4) four_masks<1>(row, m[4], m[5], m[6], m[7]);
     if (W > 8) four_masks<2>(row, m[8], m[9], m[10], m[11]);
@@ -191,8 +197,6 @@ __device__ __forceinline__ void read_planes(const uint8_t* buf, const uint32_t* 
 
 // sign map in the order of the stream's words <-> element i at bit 31 - i
 __device__ __forceinline__ uint32_t swap_order(uint32_t sign) { return __byte_perm(sign, 0, 0x0123); }
-// element 0 of a block in the order of the stream's words
-constexpr uint32_t kFirst = 0x80u;
 
 // planes -> rows: on return T[i ^ 7] = |d_i|
 template <int W>
@@ -392,7 +396,7 @@ __device__ __forceinline__ void sum_clear(PlaneSum& s) {
   for (int j = 0; j < kNarrow; ++j) s.A[j] = 0;
   s.apart = s.bound = 0;
 }
-// planes 8 B .. 8 B + 7 of a block (zero at and above F), exclusive or sign; word: the one that plane 8 B begins in; row: masks of F
+// planes 8 B .. 8 B + 7 of a block (zero at and above F), exclusive or sign; word: the one that plane 8 B begins in; row: its masks
 template <int B>
 __device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F, uint32_t row, uint32_t sign, uint32_t& word, uint32_t (&X)[32]) {
   uint32_t w[8], m[8];
@@ -409,7 +413,8 @@ __device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F,
   }
   word = w[7];
 }
-// Adds a staged payload (see read_planes); masks: see fill_masks.
+// Adds a staged payload (see read_planes); masks: see fill_masks.  As everywhere, d_0 of an outlier block is the 31 bits of its bytes,
+// and nothing of what its planes may hold for element 0 (an encoder that does not mask |INT_MIN|, a damaged stream).
 __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, const uint32_t* masks, uint32_t pos, uint32_t rate) {
   const uint32_t F = rate & 31u, W = __reduce_max_sync(0xffffffffu, F);
   uint32_t p2 = pos, a0 = 0;
@@ -417,12 +422,12 @@ __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, const u
     if (rate & 0x80u) {
       const uint32_t nout = ((rate >> 5) & 3u) + 1u;
       const uint32_t wa = smem_u32(buf) + (pos & ~3u);
-      a0 = __funnelshift_r(lds32(wa), lds32(wa + 4u), 8u * (pos & 3u)) & (0xffffffffu >> (32u - 8u * nout));
+      a0 = __funnelshift_r(lds32(wa), lds32(wa + 4u), 8u * (pos & 3u)) & (0xffffffffu >> (32u - 8u * nout)) & 0x7fffffffu;
       p2 += nout;
     }
   }
   const uint32_t sh = 8u * (p2 & 3u), wp = smem_u32(buf) + (p2 & ~3u);
-  const uint32_t row = mask_row(masks, F);
+  const uint32_t row = mask_row(masks, (F < 16u ? F : 16u) + (rate & 0x80u ? (uint32_t)kOutlierRows : 0u));
   uint32_t X[32], word0 = lds32(wp), word = lds32(wp + 4u);
   const uint32_t sign = __funnelshift_r(word0, word, sh);
   read_eight<0>(wp, sh, F, row, sign, word, X);
@@ -443,6 +448,10 @@ __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, const u
     if (W > 16u) {
       read_eight<2>(wp, sh, F, row, sign, word, X);
       read_eight<3>(wp, sh, F, row, sign, word, X);
+      if (rate & 0x80u) {  // (what the masks do for the planes below; as a mask of read_eight it cost the blocks without such planes 2 us of 140)
+#pragma unroll
+        for (int j = 16; j < 32; ++j) X[j] = bit_select(X[j], sign, ~kFirst);
+      }
     } else {
 #pragma unroll
       for (int j = 16; j < 32; ++j) X[j] = sign;

@@ -35,7 +35,7 @@ namespace dev {
 // What bounds it: instructions, at 16 warps an SM (four streams of 256 MB: 84 us of memory traffic); short runs the same trips to L2 as
 // one stream's.
 constexpr int kSumWarps = 16;
-constexpr uint32_t kSumRing = 10240, kSumUsable = kSumRing - 160;  // (see kDecRingUsable)
+constexpr uint32_t kSumRing = 10112, kSumUsable = kSumRing - 160;  // (see kDecRingUsable)
 constexpr int kSumWarpBytes = kSubBytes + (int)kSumRing;
 static_assert(32 * 132 + 32 <= kSumUsable, "one payload must fit");
 
@@ -45,7 +45,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   __shared__ uint64_t s_full[kSumWarps][2];
   __shared__ uint32_t s_tot[kSumWarps][kMaxDst];  // payload bytes of a run
   __shared__ uint64_t s_pre[kMaxDst];
-  __shared__ __align__(64) uint32_t masks[kMaskWords];
+  __shared__ __align__(64) uint32_t masks[kMaskPitch * kSumMaskRows];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* const obuf = smem + warp * kSubBytes;
@@ -55,7 +55,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   if (lane < 2u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
-  fill_masks(masks);
+  fill_masks<kSumMaskRows>(masks);
   grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   __syncwarp();
   const uint32_t Q = p.n_seg;
@@ -389,7 +389,7 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t s_full[kRunWarps][4];
   __shared__ uint32_t s_tot[kRunWarps];
-  __shared__ __align__(64) uint32_t masks[kMaskWords];
+  __shared__ __align__(64) uint32_t masks[kMaskPitch * kMaskRows];
   __shared__ uint64_t s_pre;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -400,7 +400,7 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
   if (lane < 4u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
-  fill_masks(masks);
+  fill_masks<kMaskRows>(masks);
   grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   __syncwarp();
   const DecSegment& sg = p.seg[0];

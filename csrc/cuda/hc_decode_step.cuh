@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, SUM ? 4 : 5)
 hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t s_full[kDecWarps][4];
-  __shared__ __align__(64) uint32_t masks[kMaskWords];
+  __shared__ __align__(64) uint32_t masks[kMaskPitch * (SUM ? kSumMaskRows : kMaskRows)];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n_warps = blockDim.x >> 5;
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* const obuf = smem + warp * kSubBytes;
@@ -37,7 +37,7 @@ hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   if (lane < 4u) mbar_init(&full[lane], 1);
   fence_mbar_init();
   if (tid == 0) launch_dependents();
-  fill_masks(masks);
+  fill_masks<SUM ? kSumMaskRows : kMaskRows>(masks);
   __syncthreads();
 
   const uint32_t Q = SUM ? p.n_seg : 1u;  // streams per sub-tile

@@ -244,7 +244,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
   constexpr bool kPlanes = kHasIn && kFloat && !ONE;  // contributions are added as planes (see PlaneSum)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ EncShared sh;
-  __shared__ __align__(64) uint32_t masks[kPlanes ? kMaskWords : 4];
+  __shared__ __align__(64) uint32_t masks[kPlanes ? kMaskPitch * kSumMaskRows : 4];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t nc = (blockDim.x >> 5) - 1u;  // compute warps
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -266,7 +266,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     if (kHasIn && lane < (uint32_t)kMaxIn) sh.in_run[lane] = 0;
   }
   fence_mbar_init();
-  if (kPlanes) fill_masks(masks);
+  if (kPlanes) fill_masks<kSumMaskRows>(masks);
   if (tid == 0) launch_dependents();
   grid_dependency_wait();  // nothing in global memory is touched before (see launch_overlapped)
   if (tid == 0) {

@@ -64,3 +64,40 @@ def test_decode_of_sums_at_the_edges(k, bits, sign):
     y = codec.decompress_sum([gpu] * k, n, eb, stream_bytes=[stream.size] * k)
     np.testing.assert_array_equal(y.cpu().numpy(), ops.cpu_decompress(want, n, eb))
     assert codec.status() == 0
+
+
+def _any_stream(n, planes, first_bytes, seed):
+    """A stream of random rate bytes and random payloads: outlier blocks with a |d_0| of 32 bits, and with planes that hold something
+    for element 0 too, as this library does not write them."""
+    rng = np.random.default_rng(seed)
+    blocks = -(-n // 32)
+    planes = rng.integers(0, planes + 1, blocks)
+    rates = np.where(rng.random(blocks) < 0.5, planes, 128 | rng.integers(0, first_bytes, blocks) << 5 | planes)
+    rates = np.append(rates, np.zeros(-blocks % 1024, rates.dtype))
+    lens = np.where(rates & 128, 5 + 4 * (rates & 31) + (rates >> 5 & 3), np.where(rates & 31, 4 + 4 * (rates & 31), 0))
+    return np.append(rates, rng.integers(0, 256, lens.sum())).astype(np.uint8)
+
+
+@pytest.mark.parametrize("planes,first_bytes", [(0, 4), (4, 1), (8, 2), (10, 2), (12, 4), (14, 2), (16, 4), (18, 1), (31, 4)])
+def test_sums_of_streams_that_another_encoder_wrote(planes, first_bytes):
+    """d_0 of an outlier block is its bytes, 31 bits of them, and nothing but them."""
+    n, eb, k = 37 * 1024 + 77, 0.5, 8
+    codec = ops.Codec((k + 1) * 65536)
+    x = _walk(n, 8, planes)
+    streams = [_any_stream(n, planes, first_bytes, 10 * planes + i) for i in range(k)]
+    gpu = [_gpu(s) for s in streams]
+    sizes = [s.size for s in streams]
+    for mode in ("outlier", "plain", "vec"):
+        out, size = codec.hom_add(gpu[0], torch.from_numpy(x).cuda(), eb, mode, stream_bytes=sizes[0])
+        np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), ops.cpu_hom_add(streams[0], x, eb, mode))
+        out, size = codec.hom_add_streams(gpu[0], gpu[1], n, mode, a_bytes=sizes[0], b_bytes=sizes[1])
+        np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), ops.cpu_hom_add_streams(streams[0], streams[1], n, mode))
+    want = streams[0]
+    for i in range(1, k):
+        want = ops.cpu_hom_add_streams(want, streams[i], n)
+        if i in (1, 2, 4, 7):
+            y = codec.decompress_sum(gpu[:i + 1], n, eb, stream_bytes=sizes[:i + 1])
+            np.testing.assert_array_equal(y.cpu().numpy(), ops.cpu_decompress(want, n, eb))
+            out, size = codec.hom_add_multi(gpu[:i + 1], torch.from_numpy(x).cuda(), eb, stream_bytes=sizes[:i + 1])
+            np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), ops.cpu_hom_add(want, x, eb))
+    assert codec.status() == 0
