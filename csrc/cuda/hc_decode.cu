@@ -38,6 +38,7 @@ constexpr int kSumWarps = 16;
 constexpr uint32_t kSumRing = 10112, kSumUsable = kSumRing - 160;  // (see kDecRingUsable)
 constexpr int kSumWarpBytes = kSubBytes + (int)kSumRing;
 static_assert(32 * 132 + 32 <= kSumUsable, "one payload must fit");
+static_assert(kSumWarps <= 16, "runs_before");
 
 __global__ void __launch_bounds__(kSumWarps * 32, 1)
 hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant__ DecParams p) {
@@ -73,7 +74,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   const uint32_t pool = p.pool;  // sub-tiles at the end of every run that are handed out one by one
   uint32_t it = run_of(gw);
   const uint32_t run_end = run_of(gw + 1u), own_end = run_end - pool;
-  auto sum8 = [&](uint32_t v) -> uint32_t {  // over the lanes of a stream
+  auto sum8 = [&](auto v) {  // over the lanes of a stream
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
@@ -171,8 +172,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
   __syncthreads();
   // offset of the next own sub-tile's payload in the lane's stream of this half, of the other one
   auto before_me = [&](uint32_t q) -> uint64_t {
-    const uint32_t v = (part < warp ? s_tot[part][q] : 0u) + (part + 8u < warp ? s_tot[part + 8u][q] : 0u);
-    return rate_bytes(p.seg[0].n) + (q < Q ? s_pre[q] : 0u) + sum8(v);
+    return rate_bytes(p.seg[0].n) + (q < Q ? s_pre[q] : 0u) + sum8(runs_before(s_tot, q, warp, part));
   };
   uint64_t own_off = before_me(mine), own_off_2 = Q > 4u ? before_me(mine + 4u) : 0u;
 

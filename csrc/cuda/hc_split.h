@@ -69,6 +69,11 @@ inline RunSplit split_runs(uint64_t subs, uint32_t sms, uint32_t max_warps) {
   s.pool = run < 4 ? 0u : run < 8 ? 1u : (uint32_t)(run / 8);
   return s;
 }
+// Payload bytes, in stream q, of the runs of a CTA's warps before `warp`, of up to 16: the share of lane `part` of eight.  The total of
+// one run fits 32 bits; that of a CTA need not, where a large array meets few SMs.
+HC_HD uint64_t runs_before(const uint32_t (*totals)[kMaxDst], uint32_t q, uint32_t warp, uint32_t part) {
+  return (uint64_t)(part < warp ? totals[part][q] : 0u) + (part + 8u < warp ? totals[part + 8u][q] : 0u);
+}
 // a word per pooled sub-tile and stream for its payload offset
 inline uint64_t run_words(const RunSplit& s, uint32_t streams) { return (uint64_t)s.pool * s.grid * s.warps * streams; }
 

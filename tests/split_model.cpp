@@ -1,5 +1,5 @@
 // Every call that the entry points accept (their conditions in brackets) fits the words of its workspace, and the split
-// covers all sub-tiles with CTAs that fit the exchange.  Prints what does not; "ok <calls>" at the end.
+// covers all sub-tiles with CTAs that fit the exchange; offsets inside a CTA beyond 32 bits.  Prints what does not; "ok <calls>" at the end.
 #include <stdio.h>
 
 #include <random>
@@ -35,7 +35,24 @@ static void decode(const char* what, size_t max_elems, size_t n, unsigned k, uns
   }
 }
 
+// the lanes' shares of the runs before a warp, with runs as long as they can be: 60 GB in a CTA
+static void offsets() {
+  uint32_t totals[16][hc::kMaxDst];
+  for (unsigned w = 0; w < 16; ++w)
+    for (unsigned q = 0; q < (unsigned)hc::kMaxDst; ++q) totals[w][q] = 0xffffffffu - 1000u * w - q;
+  for (unsigned q = 0; q < (unsigned)hc::kMaxDst; ++q) {
+    uint64_t want = 0;
+    for (unsigned warp = 0; warp < 16; ++warp) {
+      uint64_t sum = 0;
+      for (unsigned part = 0; part < 8; ++part) sum += hc::runs_before(totals, q, warp, part);
+      expect(sum == want, "runs before a warp", warp, q, 0, 0);
+      want += totals[warp][q];
+    }
+  }
+}
+
 int main() {
+  offsets();
   std::mt19937_64 rng(1);
   auto size = [&](size_t most) {  // spread over the logarithm, edges of sub-tiles, tiles and chunks among them
     const double e = std::uniform_real_distribution<double>(0, 1)(rng);
