@@ -64,6 +64,32 @@ def test_no_non_coherent_loads(name):
         assert "__restrict__" not in code.split(kernel + "(", 1)[1].split("{", 1)[0]
 
 
+def _launched_overlapped(code, headers=""):
+    """{kernel: its arguments} of all kernels that a source may launch overlapped.  A launch that gets its kernel by a variable may mean
+    any kernel of the source and of the headers."""
+    kernels = {re.search(r"(hc_\w+)\(", k)[1]: k.split("{", 1)[0].split("hc_", 1)[1] for k in (code + headers).split("__global__")[1:]}
+    names = re.findall(r"launch_overlapped\((?:dev::)?(\w+)", code)
+    return kernels if any(n not in kernels for n in names) else {n: kernels[n] for n in names}
+
+
+@pytest.mark.parametrize("name,headers,count", [("hc_encode.cu", [], 1), ("hc_decode.cu", ["hc_decode_step.cuh"], 3), ("hc_kernels.cu", [], 1)])
+def test_every_kernel_launched_overlapped_is_looked_at(name, headers, count):
+    code, headers = _code(name), "".join(_code(h) for h in headers)
+    kernels = _launched_overlapped(code, headers)
+    assert len(kernels) == count
+    for arguments in kernels.values():
+        assert "__restrict__" not in arguments
+    # an argument that breaks the rule is seen, however the launch names its kernel
+    for kernel in kernels:
+        broken = (code + headers).replace(kernel + "(const __grid_constant__", kernel + "(const int* __restrict__ x, const __grid_constant__", 1)
+        assert broken != code + headers and "__restrict__" in _launched_overlapped(broken)[kernel]
+
+
+def test_no_other_source_launches_overlapped():
+    names = [p.name for p in sorted(CUDA.glob("hc_*.cu*")) if p.name != "hc_host.cuh" and "launch_overlapped(" in _code(p.name)]
+    assert names == ["hc_decode.cu", "hc_encode.cu", "hc_kernels.cu"]
+
+
 @pytest.mark.parametrize("name,index,issued", [("hc_encode.cu", 0, "jobs"), ("hc_decode.cu", 0, "jobs"), ("hc_decode.cu", 1, "issued")])
 def test_a_warp_that_gives_up_waits_for_its_copies(name, index, issued):
     """Bulk copies land in shared memory; the CTA does not leave it while one may be on its way."""
