@@ -125,6 +125,32 @@ def test_sums_of_payloads_that_fill_the_ring(k, bits):
     assert c.status() == 2
 
 
+@pytest.mark.parametrize("k,bits", [(2, 22), (3, 1), (4, 20), (5, 16), (8, 19)])
+def test_sums_of_payloads_of_no_bytes(k, bits):
+    """Sub-tiles without payload in some of the streams of a batch, and in all of them: such a copy has no bytes, such a batch no copy."""
+    n = 148 * 16 * 1024 * 5 + 1025
+    subs = (n + 1023) // 1024
+    g = torch.Generator("cuda").manual_seed(100 + k)
+    c = ops.Codec(k * ((n + 32767) // 32768 * 32768))
+    in_all = torch.rand(subs, device="cuda", generator=g) < 0.2
+    want, streams, sizes, empty = torch.zeros(n, device="cuda"), [], [], []
+    for i in range(k):
+        none = in_all | (torch.rand(subs, device="cuda", generator=g) < 0.4)
+        x = torch.randint(-2 ** bits, 2 ** bits, (n,), device="cuda", generator=g)
+        x = x.masked_fill(none.repeat_interleave(1024)[:n], 0).float()
+        s, size = c.compress(x, EB)
+        want += x
+        streams.append(s)
+        sizes.append(int(size))
+        empty.append((s[:subs * 32].reshape(subs, 32) == 0).all(1))  # rate bytes
+    empty = torch.stack(empty)
+    for half in (empty[:4], empty[4:]):  # the streams of a batch
+        assert len(half) == 0 or half.all(0).sum() > subs / 10
+        assert len(half) < 2 or (half.any(0) & ~half.all(0)).sum() > subs / 10
+    assert torch.equal(c.decompress_sum(streams, n, EB, stream_bytes=sizes), want)
+    assert c.status() == 0
+
+
 def test_launches_of_all_grids_behind_one_another():
     """A launch leaves words of the exchange as they are; the next one, with more CTAs or fewer, starts from there."""
     rng = np.random.default_rng(3)
