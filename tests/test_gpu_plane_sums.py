@@ -46,6 +46,44 @@ def test_sums_of_streams(bits, mode):
     assert codec.status() == 0
 
 
+def _with_gaps(n, bits, seed):
+    """Differences of up to `bits` bits, and blocks that are all zero: next to one another in the sub-tiles, in some of which all are."""
+    rng = np.random.default_rng(seed)
+    blocks = -(-n // 32)
+    d = rng.integers(-(2 ** bits) + 1, 2 ** bits, (blocks, 32))
+    d[:, 0] >>= rng.integers(0, bits + 1, blocks)
+    d[rng.random(blocks) < 0.5] = 0
+    d[(np.arange(blocks) // 32 + seed) % 5 == 0] = 0
+    return np.clip(d.cumsum(1).reshape(-1)[:n], -(2 ** 29), 2 ** 29).astype(np.float32)
+
+
+@pytest.mark.parametrize("mode", ["outlier", "plain", "vec"])
+@pytest.mark.parametrize("bits", [1, 4, 8, 12, 16, 17, 18, 20, 24])
+def test_sums_with_blocks_of_no_planes(bits, mode):
+    """What stands where the sign map of a block without payload would be belongs to another block, and has no effect."""
+    n, eb, k = 10 * 1024 + 77, 0.5, 8
+    codec = ops.Codec((k + 1) * 32768)
+    xs = [_with_gaps(n, bits, 10 * bits + i) for i in range(k + 1)]
+    streams = [ops.cpu_compress(x, eb, mode) for x in xs]
+    for s in streams:
+        planes = (s[:10 * 32] & 31).reshape(10, 32)  # of whole sub-tiles
+        assert ((planes == 0).any(1) & (planes.max(1) >= bits)).sum() >= 7 and (planes.max(1) == 0).sum() >= 2
+    gpu = [_gpu(s) for s in streams]
+    want = streams[0]
+    for i in range(1, k):
+        last, want = want, ops.cpu_hom_add_streams(want, streams[i], n, mode)
+        out, size = codec.hom_add_streams(_gpu(last), gpu[i], n, mode, a_bytes=last.size, b_bytes=streams[i].size)
+        np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), want)
+        if i in (1, 2, 6, 7):
+            sizes = [s.size for s in streams[:i + 1]]
+            out, size = codec.hom_add_multi(gpu[:i + 1], torch.from_numpy(xs[k]).cuda(), eb, mode, stream_bytes=sizes)
+            np.testing.assert_array_equal(out[:int(size)].cpu().numpy(), ops.cpu_hom_add(want, xs[k], eb, mode))
+            if mode != "vec":  # (streams with the stride-1 predictor only)
+                y = codec.decompress_sum(gpu[:i + 1], n, eb, stream_bytes=sizes)
+                np.testing.assert_array_equal(y.cpu().numpy(), ops.cpu_decompress(want, n, eb, mode))
+    assert codec.status() == 0
+
+
 @pytest.mark.parametrize("sign", [1, -1])
 @pytest.mark.parametrize("k,bits", [(2, 6), (2, 10), (8, 8), (3, 10), (2, 11), (2, 14), (8, 12), (3, 14), (5, 14), (8, 15), (8, 16), (2, 20)])
 def test_decode_of_sums_at_the_edges(k, bits, sign):
