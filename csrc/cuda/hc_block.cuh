@@ -413,8 +413,10 @@ __device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F,
   }
   word = w[7];
 }
-// Adds a staged payload (see read_planes); masks: see fill_masks.  As everywhere, d_0 of an outlier block is the 31 bits of its bytes,
+// Adds the staged payload at byte `pos` of buf; masks: see fill_masks.  However short it is, the 10 words from its sign map on are read,
+// 18 if a block of the warp has more than 8 planes, 34 with more than 16: kSumReads bytes from `pos` on at most.  As everywhere, d_0 of an outlier block is the 31 bits of its bytes,
 // and nothing of what its planes may hold for element 0 (an encoder that does not mask |INT_MIN|, a damaged stream).
+constexpr int kSumReads = 4 + 4 * 34;  // bytes of d_0, words from the sign map on
 __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, const uint32_t* masks, uint32_t pos, uint32_t rate) {
   const uint32_t F = rate & 31u, W = __reduce_max_sync(0xffffffffu, F);
   uint32_t p2 = pos, a0 = 0;

@@ -38,6 +38,7 @@ constexpr int kSumWarps = 16;
 constexpr uint32_t kSumRing = 10112, kSumUsable = kSumRing - 160;  // (see kDecRingUsable)
 constexpr int kSumWarpBytes = kSubBytes + (int)kSumRing;
 static_assert(32 * 132 + 32 <= kSumUsable, "one payload must fit");
+static_assert((uint32_t)kSumReads <= kSumRing - kSumUsable, "sum_add reads on behind a payload");
 static_assert(kSumWarps <= 16, "runs_before");
 
 __global__ void __launch_bounds__(kSumWarps * 32, 1)

@@ -14,11 +14,12 @@ namespace dev {
 // thread) or, in sums, 16 (128) on an SM
 constexpr int kDecWarps = 4;
 // payload ring of a warp: the largest payload of corrupt rate bytes (32 x 132) with its 16-byte phase, and in
-// front of the ring's end what read_planes may look at behind a payload
+// front of the ring's end what read_planes and sum_add may look at behind a payload
 constexpr int kDecRing = 6144;
 constexpr int kDecRingUsable = kDecRing - 160;
 constexpr int kDecWarpBytes = kSubBytes + kDecRing;
 static_assert(32 * 132 + 32 <= kDecRingUsable, "one payload must fit");
+static_assert(kSumReads <= kDecRing - kDecRingUsable, "sum_add reads on behind a payload");
 
 // Steps of a collective.  SUM: the n_seg streams hold contributions to ONE array; a warp stages the same sub-tile of every stream in
 // turn, adds the deltas in registers, as bit planes, and writes seg[0].out once.

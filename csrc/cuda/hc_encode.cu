@@ -33,15 +33,17 @@ constexpr int kEncWarps = 23;
 __host__ __device__ constexpr int enc_warps(int op) { return op == kOpCompress ? kEncWarps : 15; }
 // packed payloads: a payload of 4096 bytes, 4 bytes pack_block adds, 16 copy_ring looks ahead
 __host__ __device__ constexpr int enc_out_ring(int op) { return op == kOpCompress ? 5376 : 5120; }
-// rows of the local operand, which stream + stream has not: it takes their room for payloads, so that two of up to 4.4 KB are on
+// rows of the local operand, which stream + stream has not: it takes their room for payloads, so that two of any length are on
 // their way (a random walk, 3.3 KB each: 64 MB 53.9 us, 52.4 this way, 16 MB 20.2 and 19.9; payloads of 1 KB no change)
 __host__ __device__ constexpr int enc_stage(int op) { return op == kOpAddStream ? 0 : kSubBytes; }
-// incoming payloads, and in front of the ring's end what read_planes may look at behind one
+// incoming payloads, and in front of the ring's end what read_planes and sum_add may look at behind one
 __host__ __device__ constexpr int enc_in_ring(int op) { return op == kOpCompress ? 0 : op == kOpAddStream ? 4864 + kSubBytes : 4864; }
 __host__ __device__ constexpr int enc_in_usable(int op) { return enc_in_ring(op) - 160; }
 __host__ __device__ constexpr int enc_warp_bytes(int op) { return enc_stage(op) + enc_out_ring(op) + enc_in_ring(op); }
 static_assert(kEncWarps * 4096 < (1 << 24), "EncShared::sum");
 static_assert(32 * 132 + 32 <= enc_in_usable(kOpAddF32), "one payload must fit");
+static_assert(2 * (32 * 132 + 32) <= enc_in_usable(kOpAddStream), "two payloads are to fit");
+static_assert(kSumReads <= enc_in_ring(kOpAddF32) - enc_in_usable(kOpAddF32), "sum_add reads on behind a payload");
 
 struct EncShared {
   uint64_t stage_full[kEncWarps];

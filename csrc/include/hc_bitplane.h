@@ -103,7 +103,8 @@ HC_HD void planes_from_rows(uint32_t (&A)[32]) {
     if ((k & 1) == 0) swap_stage<1>(A[k], A[k + 1]);
 }
 
-// The same for a width known at run time, at most 16 (a multiple of four): planes 0 .. W-1 in one piece of code for all of them.
+// The same for rows of W bits, W known at run time and from 0 to 16, in one piece of code for all of them: planes 0 .. 7, from W = 9 on
+// 0 .. 11, from W = 13 on 0 .. 15.  What the entries behind them hold is not said.
 HC_HD void planes_up_to_16(uint32_t (&A)[32], uint32_t W) {
 #pragma unroll
   for (int k = 0; k < 16; ++k) A[k] = perm(A[k], A[k + 16], 0x5410);
