@@ -468,7 +468,7 @@ __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, const u
 // whole number of B, comes off by an addition on the same pipe, where signs would take a shift and a logic operation a value.
 // Widths: 12 planes for sums of up to 11 bits, 16 for up to 15; the rest, with 32, goes by way of int32 (four streams of a random
 // walk of 16 MB 25.1 us by way of a row for every stream, 20.4 this way).
-template <int S, int W>
+template <int W>
 __device__ __forceinline__ void biased_values(PlaneSum& s, float scale, uint32_t (&w)[32]) {
   constexpr int B = 1 << (W - 1);
   s.A[W - 1] = ~s.A[W - 1];
@@ -477,17 +477,17 @@ __device__ __forceinline__ void biased_values(PlaneSum& s, float scale, uint32_t
   const float apart = __fmul_rn((float)(int32_t)s.apart, 0x1p-23f);
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    q[i] = __fmaf_rn(as_f(s.A[i ^ 7]), 0x1p126f, i >= S ? q[i - S] : i == 0 ? apart : 0.0f);
-    w[i] = as_u(__fmul_rn(__fadd_rn(q[i], -0x1p-23f * (float)((i / S + 1) * B)), scale));
+    q[i] = __fmaf_rn(as_f(s.A[i ^ 7]), 0x1p126f, i ? q[i - 1] : apart);
+    w[i] = as_u(__fmul_rn(__fadd_rn(q[i], -0x1p-23f * (float)((i + 1) * B)), scale));
   }
 }
-template <int S>
+// (stride-1 predictor only: no sum of streams of mode vec is decoded)
 __device__ __forceinline__ void sum_values(PlaneSum& s, float scale, float eb, uint32_t (&w)[32]) {
   // no sum of a row leaves 24 bits: 32 magnitudes of 15 bits and B for each, and |d_0|'s part that is apart
   const bool exact = scale != 0.0f && s.bound <= 1u << 15 && s.apart + (1u << 22) < (1u << 23);
   if (__builtin_expect(__all_sync(0xffffffffu, exact), 1)) {
-    if (__builtin_expect(__all_sync(0xffffffffu, s.bound <= 1u << 11), 1)) biased_values<S, 12>(s, scale, w);
-    else biased_values<S, 16>(s, scale, w);
+    if (__builtin_expect(__all_sync(0xffffffffu, s.bound <= 1u << 11), 1)) biased_values<12>(s, scale, w);
+    else biased_values<16>(s, scale, w);
     return;
   }
   if (!sum_wide(s)) {
@@ -498,7 +498,7 @@ __device__ __forceinline__ void sum_values(PlaneSum& s, float scale, float eb, u
   uint32_t q[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    q[i] = s.A[i ^ 7] + (i >= S ? q[i - S] : i == 0 ? s.apart : 0u);
+    q[i] = s.A[i ^ 7] + (i ? q[i - 1] : s.apart);
     w[i] = as_u(__fmul_rn(__fmul_rn((float)(int32_t)q[i], eb), 2.0f));
   }
 }

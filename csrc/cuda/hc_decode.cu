@@ -344,7 +344,7 @@ hc_decode_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_constant
     if (tid == 0) HC_PH(3);
     if (cur.last) {
       uint32_t w[32];
-      sum_values<1>(acc, p.scale, p.eb, w);
+      sum_values(acc, p.scale, p.eb, w);
       if (tid == 0) HC_PH(4);
       const uint64_t first = (uint64_t)cur.sub * kSubValues;
       if (lane == 0) tma_wait_group_read<0>();  // the rows of a turn ago have left the buffer
@@ -534,7 +534,7 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
 
   while (item != kNoTile) {
     const uint32_t len = payload_len(rate);
-    const uint32_t inc = warp_inclusive_scan(len, (int)lane);
+    const uint32_t inc = warp_inclusive_scan(len);
     const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
     if (tot && at + tot > limit) {  // stream shorter than its rate bytes imply
       if (lane == 0) note_error(ws.ctrl, kErrTruncated);

@@ -160,7 +160,7 @@ hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       }
       if (!un.raw_ok) un.raw = load_raw(tk, q);
       const uint32_t sum = payload_len4(un.raw);
-      inc = warp_inclusive_scan(sum, (int)lane);
+      inc = warp_inclusive_scan(sum);
       excl = inc - sum;
       scanned = true;
       // the next unit's flag and rate bytes are on their way while this one is worked on
@@ -237,17 +237,17 @@ hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
     if (!warp_wait(&full[v & 3u], (v >> 2) & 1u, ws, kSiteDecodeInFull)) break;
     ++v;
     if (threadIdx.x == 0) HC_PH(2);
-    constexpr int S = MODE == kModeVec ? 4 : 1;
     bool last = true;
     uint32_t w[32];
-    if (SUM) {
+    if constexpr (SUM) {
       if (cur.seg == 0) sum_clear(acc);
       sum_add(acc, ring, masks, cur.pos, cur.rate);
       __syncwarp();
       if (threadIdx.x == 0) HC_PH(3);
       last = cur.seg + 1 == Q;
-      if (last) sum_values<S>(acc, p.scale, p.eb, w);
+      if (last) sum_values(acc, p.scale, p.eb, w);
     } else {
+      constexpr int S = MODE == kModeVec ? 4 : 1;
       const int W = plane_width(__reduce_max_sync(0xffffffffu, cur.rate & 31u));
       uint32_t T[32], sign, a0;
       decode_rows<true>(ring, masks, cur.pos, cur.rate, W, sign, a0, T);

@@ -188,7 +188,7 @@ __device__ __forceinline__ uint64_t st_value(uint64_t w) { return w & ((1ull << 
 
 // ---- warp / block scans ---------------------------------------------------------------------------
 // (the shuffle itself says whether there is a lane to add)
-__device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, int) {
+__device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v) {
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1)
     asm volatile(

@@ -128,7 +128,7 @@ __device__ __forceinline__ void input_offsets(const SoloParams& p, EncShared& sh
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t a = t * nc, b = a + nc < subs ? a + nc : subs;
   const uint32_t sum = payload_len16(rates16(p.in[q], p.in_size[q], a, b, lane));  // half a sub-tile per lane
-  const uint32_t inc = warp_inclusive_scan(sum, (int)lane);
+  const uint32_t inc = warp_inclusive_scan(sum);
   const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
   uint64_t base = sh.in_run[q];
   if (p.one_round) base = take_total(p.ws.sums + (1u + q) * kSumWords, p.ws);
@@ -176,7 +176,7 @@ __device__ __forceinline__ void clerk(const SoloParams& p, EncShared& sh, uint32
     const uint32_t r = k % kSlots;
     if (!totals_wait(sh, k, ws)) return;
     const uint32_t tot = lane < nc ? sh.tot[r][lane] : 0u;
-    const uint32_t inc = warp_inclusive_scan(tot, (int)lane);
+    const uint32_t inc = warp_inclusive_scan(tot);
     const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
     const Chunk c = segs ? chunk_of<true>(p, t) : Chunk{0u, t};
     if (c.seg != seg) {  // every segment is a stream of its own
@@ -330,7 +330,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       return;
     }
     const uint32_t len = payload_len(praw);
-    const uint32_t inc = warp_inclusive_scan(len, (int)lane);
+    const uint32_t inc = warp_inclusive_scan(len);
     uint32_t tot = __shfl_sync(0xffffffffu, inc, 31), rate = praw;
     uint32_t at = staged ? live_end : 0u;
     if (tot && at + tot + 31u > (uint32_t)enc_in_usable(OP)) {
@@ -534,7 +534,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       if constexpr (kPlanes) return sum_code<MODE>(sum);
       else return code_of<MODE>(d, or_tail);
     }();
-    const uint32_t inc = warp_inclusive_scan(code.len, (int)lane);
+    const uint32_t inc = warp_inclusive_scan(code.len);
     const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
     uint32_t before = 0;
     if (lane == 0) {

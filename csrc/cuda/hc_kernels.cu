@@ -89,7 +89,7 @@ __device__ __forceinline__ void loader_stage_stream(const uint8_t* in, uint64_t 
     len[k] = payload_len(rate[k]);
     sum += len[k];
   }
-  const uint32_t inc = warp_inclusive_scan(sum, lane);
+  const uint32_t inc = warp_inclusive_scan(sum);
   const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
   // collective steps: the producer's arrival flag carries the tile's byte offset, no look-back
   bool ok = true;

@@ -375,7 +375,7 @@ __device__ __forceinline__ bool compute_barrier_or(bool leaves) {
 constexpr uint32_t kLeaveTotal = 1u << 24;  // far above any total
 __device__ __forceinline__ uint32_t compute_exclusive_scan(uint32_t v, uint32_t* s_wsum, uint32_t* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t inc = warp_inclusive_scan(v, lane);
+  uint32_t inc = warp_inclusive_scan(v);
   if (lane == 31) s_wsum[warp] = inc;
   compute_barrier();
   uint32_t pre = 0, tot = 0;
