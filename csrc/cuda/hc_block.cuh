@@ -126,8 +126,10 @@ constexpr uint32_t kFirst = 0x80u;
 // selecting takes two operations a plane of the half-rate pipe; with a mask from shared memory it is one, in sums together with the
 // exclusive or with the sign (decode of 64 MB 22.5 us, 21.2 this way, of 256 MB 61.8 and 60.9; four streams of 256 MB added 143.5 and
 // 138.8; the decode of an allreduce step of 64 MB at 8 ranks 33.1 and 32.0).  Not in the add of one stream and fp32: of 64 MB 38.6 us,
-// 38.4 with masks, but of 4 MB 7.7 and 7.8, for the time that the rows take at the start.  Rows lie 20 words apart, so that eight
-// neighbouring ones have no banks in common and a row's four loads are one address.
+// 38.4 with masks, but of 4 MB 7.7 and 7.8, for the time that the rows take at the start.  Nor for blocks of 13 to 16 planes in the decode
+// of one stand-alone stream (a random walk of 256 MB 90.6 us, 94.0 with them, of 64 MB 26.4 and 27.2, of 16 MB 10.2 and 10.5, normal-
+// distributed values of 16 MB 9.8 and 10.0); in the steps of a collective they gain nothing and cost nothing there.
+// Rows lie 20 words apart, so that eight neighbouring ones have no banks in common and a row's four loads are one address.
 // Sums have a second set of rows, kOutlierRows further on, for outlier blocks: whatever such a block's planes hold for element 0 does
 // not count (four streams of 256 MB 138.4 us without them, 140.3 with; from 17 to 21 rows apart they take the same).
 constexpr int kMaskRows = 17, kOutlierRows = 17, kSumMaskRows = kOutlierRows + kMaskRows, kMaskPitch = 20;
@@ -160,7 +162,7 @@ __device__ __forceinline__ uint32_t mask_row(const uint32_t* masks, uint32_t row
 // word is rebuilt from two neighbours by a funnel shift, whatever the block's alignment: with outlier blocks
 // about, the lanes of a warp have all four alignments, and a second path for aligned blocks ran on top.
 // Blocks without payload give zeros; up to 4 W + 8 bytes behind the payload are read (and ignored).
-template <int W, bool MASKS>
+template <int W, int MASKED>
 __device__ __forceinline__ void read_planes(const uint8_t* buf, const uint32_t* masks, uint32_t pos, uint32_t rate, bool any_outlier,
                                             uint32_t& sign, uint32_t& a0, uint32_t (&T)[32]) {
   const uint32_t F = rate & 31u;
@@ -180,9 +182,10 @@ __device__ __forceinline__ void read_planes(const uint8_t* buf, const uint32_t* 
 #pragma unroll
   for (int j = 0; j < W + 2; ++j) word[j] = lds32(wp + 4 * j);
   sign = __funnelshift_r(word[0], word[1], sh);
+  constexpr bool kMasks = W <= MASKED;
   uint32_t m[16];
-  if (MASKS && W <= 16) {
-    const uint32_t row = mask_row(masks, F < 16u ? F : 16u);
+  if (kMasks) {
+    const uint32_t row = mask_row(masks, F);  // (F <= W)
     if (W > 0) four_masks<0>(row, m[0], m[1], m[2], m[3]);
     if (W > 4) four_masks<1>(row, m[4], m[5], m[6], m[7]);
     if (W > 8) four_masks<2>(row, m[8], m[9], m[10], m[11]);
@@ -191,7 +194,7 @@ __device__ __forceinline__ void read_planes(const uint8_t* buf, const uint32_t* 
 #pragma unroll
   for (int j = 1; j <= W; ++j) {
     const uint32_t x = __funnelshift_r(word[j], word[j + 1], sh);
-    T[j - 1] = MASKS && W <= 16 ? x & m[(j - 1) & 15] : (uint32_t)j <= F ? x : 0u;
+    T[j - 1] = kMasks ? x & m[(j - 1) & 15] : (uint32_t)j <= F ? x : 0u;
   }
 }
 
@@ -213,17 +216,17 @@ __device__ __forceinline__ void rows_of_block(uint32_t (&T)[32], uint32_t rate, 
 // staged payload -> rows, sign map with element i at bit 31 - i; W (plane_width of the largest F of the warp) is warp-uniform.  The widths that data at the usual error
 // bounds has come first and in line, so that the loop's instructions lie together (as a switch, with the longest
 // variants in between: add of 64 MB 41.7 us, 40.3 this way; decode of 64 MB 22.4, 21.6)
-// MASKS: see fill_masks
-template <bool MASKS>
+// MASKED: widest blocks that are read with masks (see fill_masks)
+template <int MASKED>
 __device__ __forceinline__ void decode_rows(const uint8_t* buf, const uint32_t* masks, uint32_t pos, uint32_t rate, int W, uint32_t& sign,
                                             uint32_t& a0, uint32_t (&T)[32]) {
   const bool outl = __any_sync(0xffffffffu, rate & 0x80u);
-  if (__builtin_expect(W == 12, 1)) { read_planes<12, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<12>(T, rate, a0); }
-  else if (__builtin_expect(W == 8, 1)) { read_planes<8, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<8>(T, rate, a0); }
-  else if (__builtin_expect(W == 16, 1)) { read_planes<16, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<16>(T, rate, a0); }
-  else if (W == 4) { read_planes<4, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<4>(T, rate, a0); }
-  else if (__builtin_expect(W == 0, 0)) { read_planes<0, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<0>(T, rate, a0); }
-  else { read_planes<32, MASKS>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<32>(T, rate, a0); }
+  if (__builtin_expect(W == 12, 1)) { read_planes<12, MASKED>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<12>(T, rate, a0); }
+  else if (__builtin_expect(W == 8, 1)) { read_planes<8, MASKED>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<8>(T, rate, a0); }
+  else if (__builtin_expect(W == 16, 1)) { read_planes<16, MASKED>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<16>(T, rate, a0); }
+  else if (W == 4) { read_planes<4, MASKED>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<4>(T, rate, a0); }
+  else if (__builtin_expect(W == 0, 0)) { read_planes<0, MASKED>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<0>(T, rate, a0); }
+  else { read_planes<32, MASKED>(buf, masks, pos, rate, outl, sign, a0, T); rows_of_block<32>(T, rate, a0); }
   sign = swap_order(sign);
 }
 

@@ -552,7 +552,7 @@ hc_decode_run_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_cons
     uint32_t pos = at % kRing + inc - len;
     if (pos >= kRing) pos -= kRing;
     uint32_t T[32], sign, a0;
-    decode_rows<true>(ring, masks, pos, rate, plane_width(__reduce_max_sync(0xffffffffu, rate & 31u)), sign, a0, T);
+    decode_rows<12>(ring, masks, pos, rate, plane_width(__reduce_max_sync(0xffffffffu, rate & 31u)), sign, a0, T);
     const bool little = (rate & 31u) <= 16u && a0 < (1u << 23);
     const uint32_t cur = sub;
     __syncwarp();

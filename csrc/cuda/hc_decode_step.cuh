@@ -250,7 +250,7 @@ hc_decode_step_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
       constexpr int S = MODE == kModeVec ? 4 : 1;
       const int W = plane_width(__reduce_max_sync(0xffffffffu, cur.rate & 31u));
       uint32_t T[32], sign, a0;
-      decode_rows<true>(ring, masks, cur.pos, cur.rate, W, sign, a0, T);
+      decode_rows<16>(ring, masks, cur.pos, cur.rate, W, sign, a0, T);
       __syncwarp();
       if (threadIdx.x == 0) HC_PH(3);
       // ---- signs, prefix sum, scaling ------------------------------------------------------------------------------

@@ -485,7 +485,7 @@ hc_encode_solo_kernel(const __grid_constant__ TensorMaps tmaps, const __grid_con
           __syncwarp();
         } else {
           uint32_t T[32], sign, a0;
-          decode_rows<false>(inring, nullptr, cur_pos, cur_rate, plane_width(__reduce_max_sync(0xffffffffu, cur_rate & 31u)), sign, a0, T);
+          decode_rows<-1>(inring, nullptr, cur_pos, cur_rate, plane_width(__reduce_max_sync(0xffffffffu, cur_rate & 31u)), sign, a0, T);
           __syncwarp();
           // |d_1| .. |d_31| small enough for sums in subnormals: so with up to 16 planes, else to be looked at (a
           // plain block may have many planes for the sake of d_0 alone, which is summed in int32)
