@@ -131,7 +131,8 @@ constexpr uint32_t kFirst = 0x80u;
 // distributed values of 16 MB 9.8 and 10.0); in the steps of a collective they gain nothing and cost nothing there.
 // Rows lie 20 words apart, so that eight neighbouring ones have no banks in common and a row's four loads are one address.
 // Sums have a second set of rows, kOutlierRows further on, for outlier blocks: whatever such a block's planes hold for element 0 does
-// not count (four streams of 256 MB 138.4 us without them, 140.3 with; from 17 to 21 rows apart they take the same).
+// not count (four streams of 256 MB 139.1 us without them, 139.8 with, 140.9 where every block chooses its set, not the outlier ones
+// alone; from 17 to 21 rows apart they take the same).
 constexpr int kMaskRows = 17, kOutlierRows = 17, kSumMaskRows = kOutlierRows + kMaskRows, kMaskPitch = 20;
 template <int ROWS>
 __device__ __forceinline__ void fill_masks(uint32_t* masks) {
@@ -386,6 +387,9 @@ __device__ __forceinline__ void pack_blocks(uint32_t base, uint32_t rel, const B
 // streams and fp32 3550 and 4380: 16 MB of a random walk 23.8 -> 20.3 us, 64 MB of gradients 49.2 -> 44.5, seven streams of 8 MB and
 // their decode 25.1 -> 23.0.  With ONE stream and fp32 as many instructions are left (the rows of the local operand are there
 // already) and their chain is longer: 64 MB 38.4 us by way of rows, 40.5 this way.
+// A stream of 17 or 18 planes, which twenty would hold, is read in the wide code, for the masks of a block end at 16 (64 MB of blocks of
+// 16, 17, 18 and 19 planes added 49.2, 53.8, 54.9 and 57.3 us; by way of rows 63.7, 72.9, 75.9 and 78.9); blocks of up to 4 planes are
+// read like those of 8 (a smooth field of 64 MB 38.6 us; by way of rows, with code of their own width, 40.8).
 // Two pieces of code, narrow and wide, not one for each width (44.0 us where this takes 44.5, but 21.6 against 20.3 for the random walk
 // and 44.2 against 37.7 for three of them), and not groups of four planes as far as they are needed (46.4).
 constexpr int kNarrow = 20;
@@ -422,17 +426,17 @@ __device__ __forceinline__ void read_eight(uint32_t wp, uint32_t sh, uint32_t F,
 constexpr int kSumReads = 4 + 4 * 34;  // bytes of d_0, words from the sign map on
 __device__ __forceinline__ void sum_add(PlaneSum& s, const uint8_t* buf, const uint32_t* masks, uint32_t pos, uint32_t rate) {
   const uint32_t F = rate & 31u, W = __reduce_max_sync(0xffffffffu, F);
-  uint32_t p2 = pos, a0 = 0;
+  uint32_t p2 = pos, a0 = 0, row = mask_row(masks, F < 16u ? F : 16u);
   if (__any_sync(0xffffffffu, rate & 0x80u)) {
     if (rate & 0x80u) {
       const uint32_t nout = ((rate >> 5) & 3u) + 1u;
       const uint32_t wa = smem_u32(buf) + (pos & ~3u);
       a0 = __funnelshift_r(lds32(wa), lds32(wa + 4u), 8u * (pos & 3u)) & (0xffffffffu >> (32u - 8u * nout)) & 0x7fffffffu;
       p2 += nout;
+      row += 4u * kMaskPitch * kOutlierRows;
     }
   }
   const uint32_t sh = 8u * (p2 & 3u), wp = smem_u32(buf) + (p2 & ~3u);
-  const uint32_t row = mask_row(masks, (F < 16u ? F : 16u) + (rate & 0x80u ? (uint32_t)kOutlierRows : 0u));
   uint32_t X[32], word0 = lds32(wp), word = lds32(wp + 4u);
   const uint32_t sign = __funnelshift_r(word0, word, sh);
   read_eight<0>(wp, sh, F, row, sign, word, X);

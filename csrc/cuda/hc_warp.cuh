@@ -30,7 +30,9 @@ __device__ __forceinline__ void note_timeout(const Workspace& ws, uint32_t site)
 }
 // Bounded mbarrier wait of a whole warp; false: gave up (recorded).  The lanes try together and vote, so that the loop is the same
 // for all of them: as a loop per lane every wait carried the code for lanes that leave it apart (a sub-tile of an add 1237 warp
-// instructions, 1206 this way; compress of 4 KB 3.45 us and 3.38, decode of 64 MB 22.8 and 22.4).
+// instructions, 1206 this way; compress of 4 KB 3.84 us and 3.75, of 256 MB 63.6 and 62.4, decode of 64 MB 22.8 and 22.4).  Compress of
+// 16 MB takes 7.35 us, 7.2 with a loop per lane in the wait for the rows alone, but then 4 KB 3.84 and 256 MB 63.2; from 8 to 32 MB no
+// other size was found to lose.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const Workspace& ws, uint32_t site) {
   if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
   long long t0 = 0;
